@@ -186,13 +186,6 @@ __device__ __forceinline__ void tab2_build_warp(uint2 *T, uint32_t c0, uint32_t 
     for (int j = 0; j < 4; ++j) T[32 * j + lane] = make_uint2(v0[j], v1[j]);
 }
 
-// Same product with the table at byte offset base + off of the shared
-// array `sm`, base a multiple of 256 (its low byte is zero) and off a
-// constant after unrolling.  Byte j of a (b) holds 4 * nibble 2j (2j+1) of
-// w, the byte offset of that window's entry; one byte-permute splices it
-// under `base`, and off + the window's 64-byte slot fold into the load's
-// immediate.  Per product: 2 multiplies and 2 ANDs to spread the nibbles, 8
-// permutes, 8 loads, 4 XORs.
 // p + t * stride_bytes as one wide multiply-add on the multiply-add pipe
 // (the strided FFT passes address 2^K pencil values this way, keeping the
 // integer-logic pipe for the field products)
@@ -206,12 +199,24 @@ __device__ __forceinline__ T *strided(T *p, uint32_t t, uint32_t stride_bytes) {
 __device__ __forceinline__ uint32_t shared_addr(const void *p) {
     return (uint32_t)__cvta_generic_to_shared(p);
 }
-// The two nibble spreads' shifts run as multiplies on the multiply-add pipe
-// (w * 4, and the high word of w * 2^30 = w >> 2): a table product is
-// otherwise all integer-logic work (the byte permutes and XORs), and that
-// pipe is what bounds the table kernels.  The multipliers come from
-// constant memory so the compiler keeps them multiplies.
+// Product with the table at byte offset base + off of the shared array
+// `sm`, off a constant after unrolling.  Byte j of a (b) holds 4 * nibble 2j
+// (2j+1) of w, the byte offset of that window's entry; a four-byte dot
+// product with 1 at byte j adds it to `base`, and off + the window's 64-byte
+// slot fold into the load's immediate.  Per product: 2 multiplies and 2 ANDs
+// to spread the nibbles, 8 dot products, 8 loads, 4 XORs.
+// What bounds it: 8 shared-memory wavefronts, one a clock and SM.  The
+// shifts of the nibble spreads (w * 4, and the high word of w * 2^30 = w >>
+// 2) and the dot products run on the multiply-add pipe, so the logic pipe
+// (64 lanes a clock and SM) has 7 instructions left instead of 15 with a
+// byte-permute per window: in a loop of nothing but products both forms come
+// to 8.0-8.2 clocks per 32 products, but the logic pipe then had 9% left for
+// everything else around the products (a 4-stage strided FFT pass at 2^18 x
+// 256 columns took 177 us with permutes, 168 us with dot products).  The
+// multipliers come from constant memory so the compiler keeps them
+// multiplies.
 static __constant__ uint32_t kSpreadMul[2] = {4u, 1u << 30};
+static __constant__ uint32_t kByteSel[4] = {1u, 1u << 8, 1u << 16, 1u << 24};
 __device__ __forceinline__ uint32_t tab_mul_sa(const uint8_t *__restrict__ sm, uint32_t base, uint32_t off,
                                                uint32_t w) {
     uint32_t a, b;
@@ -219,16 +224,15 @@ __device__ __forceinline__ uint32_t tab_mul_sa(const uint8_t *__restrict__ sm, u
     asm("mul.hi.u32 %0, %1, %2;" : "=r"(b) : "r"(w), "r"(kSpreadMul[1]));
     a &= 0x3C3C3C3Cu;
     b &= 0x3C3C3C3Cu;
-#define LGD_LD(x, sel, o) (*reinterpret_cast<const uint32_t *>(sm + __byte_perm((x), base, (sel)) + off + (o)))
-    const uint32_t r0 = LGD_LD(a, 0x7650, 0), r1 = LGD_LD(b, 0x7650, 64);
-    const uint32_t r2 = LGD_LD(a, 0x7651, 128), r3 = LGD_LD(b, 0x7651, 192);
-    const uint32_t r4 = LGD_LD(a, 0x7652, 256), r5 = LGD_LD(b, 0x7652, 320);
-    const uint32_t r6 = LGD_LD(a, 0x7653, 384), r7 = LGD_LD(b, 0x7653, 448);
+#define LGD_LD(x, j, o) (*reinterpret_cast<const uint32_t *>(sm + __dp4a((x), kByteSel[j], base) + off + (o)))
+    const uint32_t r0 = LGD_LD(a, 0, 0), r1 = LGD_LD(b, 0, 64);
+    const uint32_t r2 = LGD_LD(a, 1, 128), r3 = LGD_LD(b, 1, 192);
+    const uint32_t r4 = LGD_LD(a, 2, 256), r5 = LGD_LD(b, 2, 320);
+    const uint32_t r6 = LGD_LD(a, 3, 384), r7 = LGD_LD(b, 3, 448);
 #undef LGD_LD
     return (r0 ^ r1 ^ r2) ^ (r3 ^ r4 ^ r5) ^ (r6 ^ r7);
 }
-// w times both constants of the pair table at byte offset base of `sm`
-// (base a multiple of 256): byte j of a (b) holds 8 * nibble 2j (2j+1) of
+// w times both constants of the pair table at byte offset base of `sm`: byte j of a (b) holds 8 * nibble 2j (2j+1) of
 // w, the byte offset of that window's 8-byte entry.
 static __constant__ uint32_t kSpreadMul2[2] = {8u, 1u << 31};
 __device__ __forceinline__ uint2 tab2_mul_sa(const uint8_t *__restrict__ sm, uint32_t base, uint32_t w) {
@@ -237,11 +241,11 @@ __device__ __forceinline__ uint2 tab2_mul_sa(const uint8_t *__restrict__ sm, uin
     asm("mul.hi.u32 %0, %1, %2;" : "=r"(b) : "r"(w), "r"(kSpreadMul2[1]));
     a &= 0x78787878u;
     b &= 0x78787878u;
-#define LGD_LD2(x, sel, o) (*reinterpret_cast<const uint2 *>(sm + __byte_perm((x), base, (sel)) + (o)))
-    const uint2 r0 = LGD_LD2(a, 0x7650, 0), r1 = LGD_LD2(b, 0x7650, 128);
-    const uint2 r2 = LGD_LD2(a, 0x7651, 256), r3 = LGD_LD2(b, 0x7651, 384);
-    const uint2 r4 = LGD_LD2(a, 0x7652, 512), r5 = LGD_LD2(b, 0x7652, 640);
-    const uint2 r6 = LGD_LD2(a, 0x7653, 768), r7 = LGD_LD2(b, 0x7653, 896);
+#define LGD_LD2(x, j, o) (*reinterpret_cast<const uint2 *>(sm + __dp4a((x), kByteSel[j], base) + (o)))
+    const uint2 r0 = LGD_LD2(a, 0, 0), r1 = LGD_LD2(b, 0, 128);
+    const uint2 r2 = LGD_LD2(a, 1, 256), r3 = LGD_LD2(b, 1, 384);
+    const uint2 r4 = LGD_LD2(a, 2, 512), r5 = LGD_LD2(b, 2, 640);
+    const uint2 r6 = LGD_LD2(a, 3, 768), r7 = LGD_LD2(b, 3, 896);
 #undef LGD_LD2
     return make_uint2((r0.x ^ r1.x ^ r2.x) ^ (r3.x ^ r4.x ^ r5.x) ^ (r6.x ^ r7.x),
                       (r0.y ^ r1.y ^ r2.y) ^ (r3.y ^ r4.y ^ r5.y) ^ (r6.y ^ r7.y));
