@@ -129,7 +129,13 @@ uint8_t *pinned(lg_ctx *c, size_t bytes) {
     return c->pinned;
 }
 
-void sync(lg_ctx *c) { CK(c, cudaStreamSynchronize(c->stream)); }
+void sync(lg_ctx *c) {
+    CK(c, cudaStreamSynchronize(c->stream));
+    if (*static_cast<volatile uint32_t *>(c->L.fault)) {  // a kernel gave up waiting for a copy
+        *c->L.fault = 0;
+        CK(c, cudaErrorLaunchTimeout);
+    }
+}
 
 // lg_dump_intermediates: hand the caller a host copy of `bytes` device
 // bytes once the stream has produced them; nothing happens otherwise.
@@ -312,19 +318,17 @@ struct Witness {  // RecursiveLigeroWitness, src/data_structures.rs:32-40
 };
 
 // encode_non_systematic (src/reed_solomon.rs:104-113) of n columns into E
-// (column-major, 4m rows): the columns scaled by pis are written once to
-// `scaled` (n columns of m words) and the first FFT pass of all four
-// quarters reads them from there, instead of spreading four copies through
-// HBM; codes short enough for a single FFT pass spread them.
+// (column-major, 4m rows): the first FFT pass reads each input column once,
+// scales it by pis and starts all four quarters from it; codes short enough
+// for a single FFT pass spread four scaled copies first.
 void rs_encode(lg_ctx *c, const Code &code, const uint32_t *d_poly, uint32_t log_m, uint32_t n, uint32_t *E,
-               uint64_t col_stride, uint32_t *scaled, lgk::FftPasses passes = lgk::FFT_ALL) {
+               uint64_t col_stride, lgk::FftPasses passes = lgk::FFT_ALL) {
     const uint64_t m = 1ull << log_m;
     if (log_m > 6) {
-        CK(c, lgk::rs_scale(c->L, d_poly, code.pis, scaled, log_m, n));
         lgk::FftSrc src;
-        src.p = scaled;
+        src.p = d_poly;
         src.col_stride = m;
-        src.q_stride = 0;
+        src.pis = code.pis;
         CK(c, lgk::fft_vectors(c->L, E, code.tw, log_m, n, col_stride, 4, m, 4, false, passes, &src));
     } else {
         CK(c, lgk::rs_scale_spread(c->L, d_poly, code.pis, E, log_m, n));
@@ -336,10 +340,7 @@ void rs_encode(lg_ctx *c, const Code &code, const uint32_t *d_poly, uint32_t log
 void commit_into(lg_ctx *c, const uint32_t *d_poly, uint32_t log_m, uint32_t n, uint32_t *E, uint32_t *tree) {
     const Code code = get_code(c, log_m);
     const uint64_t m = 1ull << log_m, rows = 4 * m;
-    {
-        DBuf scaled(c, log_m > 6 ? 4ull * n * m : 0);
-        rs_encode(c, code, d_poly, log_m, n, E, rows, scaled.u32());
-    }
+    rs_encode(c, code, d_poly, log_m, n, E, rows);
     CK(c, lgk::leaf_hashes(c->L, E, rows, n, tree));
     CK(c, lgk::merkle_upper(c->L, tree, rows));
 }
@@ -411,7 +412,6 @@ Witness commit_from_host(lg_ctx *c, Scratch &sc, const uint32_t *h_poly, uint32_
     cudaGetLastError();
     const std::vector<uint32_t> groups = host_copy_groups(n);
     const uint32_t U = host_hash_unit(n);
-    DBuf scaled(c, log_m > 6 ? 4ull * n * m : 0);
     // staging for pageable input: two pinned chunks, reused after their copy
     constexpr size_t kChunk = 4u << 20;
     uint8_t *slot[2] = {nullptr, nullptr};
@@ -445,8 +445,7 @@ Witness commit_from_host(lg_ctx *c, Scratch &sc, const uint32_t *h_poly, uint32_
         CK(c, cudaEventRecord(c->copy_ev[g % 4], c->copy_stream));
         CK(c, cudaStreamWaitEvent(c->stream, c->copy_ev[g % 4], 0));
         uint32_t *Eg = w.E.u32() + (uint64_t)j0 * rows;
-        rs_encode(c, code, d_poly + (uint64_t)j0 * m, log_m, cols, Eg, rows, scaled.u32() + (uint64_t)j0 * m,
-                  lgk::FFT_HEAD);
+        rs_encode(c, code, d_poly + (uint64_t)j0 * m, log_m, cols, Eg, rows, lgk::FFT_HEAD);
         j0 += cols;
         if (j0 % U == 0 || j0 == n) {  // a hash unit is complete
             const uint32_t u = (j0 - 1) / U, ju = u * U, ucols = j0 - ju;
@@ -845,10 +844,7 @@ BatchWitness commit_batch(lg_ctx *c, const uint32_t *d_polys, uint32_t log_m, ui
     w.B = B;
     w.E = DBuf(c, 4ull * B * w.e_stride());
     w.tree = DBuf(c, 4ull * B * w.t_stride());
-    {
-        DBuf scaled(c, log_m > 6 ? 4ull * B * n << log_m : 0);
-        rs_encode(c, code, d_polys, log_m, B * n, w.E.u32(), w.rows, scaled.u32());
-    }
+    rs_encode(c, code, d_polys, log_m, B * n, w.E.u32(), w.rows);
     CK(c, lgk::leaf_hashes(c->L, w.E.u32(), w.rows, n, w.tree.u32(), B, w.e_stride(), w.t_stride()));
     CK(c, lgk::merkle_upper(c->L, w.tree.u32(), w.rows, B, w.t_stride()));
     return w;
@@ -1649,7 +1645,8 @@ lg_status lg_ctx_create(int device, uint64_t budget, lg_ctx **out) {
         return LG_ERR_CUDA;
     }
     if (cudaMalloc((void **)&c->L.dtab, lgk::kDtabSlots * lgk::kDtabWords * 4) != cudaSuccess ||
-        cudaMalloc((void **)&c->L.tickets, 256) != cudaSuccess || cudaMemset(c->L.tickets, 0, 256) != cudaSuccess) {
+        cudaMalloc((void **)&c->L.tickets, 256) != cudaSuccess || cudaMemset(c->L.tickets, 0, 256) != cudaSuccess ||
+        cudaMallocHost((void **)&c->L.fault, 64) != cudaSuccess) {
         cudaGetLastError();
         if (c->L.dtab) cudaFree(c->L.dtab);
         if (c->L.tickets) cudaFree(c->L.tickets);
@@ -1658,6 +1655,7 @@ lg_status lg_ctx_create(int device, uint64_t budget, lg_ctx **out) {
         delete c;
         return LG_ERR_OUT_OF_MEMORY;
     }
+    *c->L.fault = 0;
     for (auto &e : c->copy_ev) cudaEventCreateWithFlags(&e, cudaEventDisableTiming);
     cudaMemPool_t pool;
     if (cudaDeviceGetDefaultMemPool(&pool, device) == cudaSuccess) {
@@ -1696,6 +1694,7 @@ void lg_ctx_destroy(lg_ctx *c) {
     if (c->dev_arena) cudaFree(c->dev_arena);
     if (c->L.dtab) cudaFree(c->L.dtab);
     if (c->L.tickets) cudaFree(c->L.tickets);
+    if (c->L.fault) cudaFreeHost(c->L.fault);
     c->L.release();
     for (auto e : c->copy_ev) if (e) cudaEventDestroy(e);
     if (c->copy_stream) cudaStreamDestroy(c->copy_stream);
@@ -1958,8 +1957,7 @@ lg_status lg_rs_encode_cols(lg_ctx *c, const uint32_t *d_poly, uint32_t log_m, u
     return guarded(c, [&] {
         CK(c, cudaSetDevice(c->device));
         const Code code = get_code(c, log_m);
-        DBuf scaled(c, log_m > 6 ? 4ull * n << log_m : 0);
-        rs_encode(c, code, d_poly, log_m, n, d_enc, 4ull << log_m, scaled.u32());
+        rs_encode(c, code, d_poly, log_m, n, d_enc, 4ull << log_m);
         sync(c);
     });
 }

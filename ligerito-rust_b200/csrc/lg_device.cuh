@@ -27,6 +27,54 @@ __device__ __forceinline__ void pdl_begin() {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
+// ------------------------------------------------------------ bulk copies
+// Untiled bulk copies (16-byte aligned addresses and sizes) between global
+// and shared memory.  They pass the load/store unit by, whose wavefronts
+// bound the table kernels.
+__device__ __forceinline__ void mbar_init(uint64_t *bar, uint32_t arrivals) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"((uint32_t)__cvta_generic_to_shared(bar)), "r"(arrivals)
+                 : "memory");
+}
+// generic-proxy writes to shared memory (a barrier's init, a tile to be
+// copied out) before async-proxy accesses of it
+__device__ __forceinline__ void fence_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
+__device__ __forceinline__ void mbar_expect(uint64_t *bar, uint32_t bytes) {
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"((uint32_t)__cvta_generic_to_shared(bar)),
+                 "r"(bytes)
+                 : "memory");
+}
+__device__ __forceinline__ void bulk_load(void *dst, const void *src, uint32_t bytes, uint64_t *bar) {
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                     (uint32_t)__cvta_generic_to_shared(dst)),
+                 "l"(src), "r"(bytes), "r"((uint32_t)__cvta_generic_to_shared(bar))
+                 : "memory");
+}
+__device__ __forceinline__ void bulk_store(void *dst, const void *src, uint32_t bytes) {
+    asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(dst),
+                 "r"((uint32_t)__cvta_generic_to_shared(src)), "r"(bytes)
+                 : "memory");
+}
+// this thread's bulk stores have left shared memory and are written
+__device__ __forceinline__ void bulk_store_wait() {
+    asm volatile("cp.async.bulk.commit_group;\n\tcp.async.bulk.wait_group 0;" ::: "memory");
+}
+// Waits for the barrier's phase of that parity; a wait that does not end
+// within the limit (a copy that never completes) is reported in *fault, a
+// word of host memory that the host looks at after it synchronises.
+__device__ __forceinline__ void mbar_wait(uint64_t *bar, uint32_t parity, uint32_t *fault) {
+    const uint32_t a = (uint32_t)__cvta_generic_to_shared(bar);
+    for (uint32_t tries = 0; tries < (1u << 18); ++tries) {
+        uint32_t done;
+        asm volatile(
+            "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+            : "=r"(done)
+            : "r"(a), "r"(parity)
+            : "memory");
+        if (done) return;
+    }
+    *reinterpret_cast<volatile uint32_t *>(fault) = 1;
+}
+
 constexpr uint32_t kTail = 0x8299u;  // x^32 mod p
 
 __device__ __forceinline__ uint32_t red_small(uint32_t t) {
@@ -43,10 +91,17 @@ __device__ __forceinline__ uint32_t gf_mulxk(uint32_t a) {
     return (a << K) ^ red_small(a >> (32 - K));
 }
 
+// hi x^32 + lo mod p.  The tail x^15 + x^9 + x^7 + x^4 + x^3 + 1 is
+// (1 + x^3)(1 + x^4) + x^9 + x^15; one wide multiply gives both words of a
+// shifted hi.
 __device__ __forceinline__ uint32_t gf_reduce(uint32_t hi, uint32_t lo) {
-    uint32_t lo2 = hi ^ (hi << 3) ^ (hi << 4) ^ (hi << 7) ^ (hi << 9) ^ (hi << 15);
-    uint32_t ov = (hi >> 29) ^ (hi >> 28) ^ (hi >> 25) ^ (hi >> 23) ^ (hi >> 17);
-    return lo ^ lo2 ^ red_small(ov);
+    const uint64_t s3 = (uint64_t)hi * 8u, s9 = (uint64_t)hi * 512u, s15 = (uint64_t)hi * 32768u;
+    const uint32_t a0 = hi ^ (uint32_t)s3, a1 = (uint32_t)(s3 >> 32);  // hi (1 + x^3)
+    const uint64_t s4 = (uint64_t)a0 * 16u;
+    const uint32_t l = a0 ^ (uint32_t)s4 ^ (uint32_t)s9 ^ (uint32_t)s15;
+    const uint32_t t = a1 ^ (a1 << 4) ^ (uint32_t)(s4 >> 32) ^ (uint32_t)(s9 >> 32) ^ (uint32_t)(s15 >> 32);
+    const uint32_t b = t ^ (t << 3);  // deg t <= 14: t times the tail does not overflow
+    return lo ^ l ^ b ^ (b << 4) ^ (t << 9) ^ (t << 15);
 }
 
 // Carry-less 32 x 32 -> 64-bit product: 16 integer multiplies of operands
@@ -60,8 +115,15 @@ __device__ __forceinline__ uint64_t clmul32(uint32_t a, uint32_t b) {
     uint64_t z1 = ((uint64_t)a0 * b1) ^ ((uint64_t)a1 * b0) ^ ((uint64_t)a2 * b3) ^ ((uint64_t)a3 * b2);
     uint64_t z2 = ((uint64_t)a0 * b2) ^ ((uint64_t)a1 * b1) ^ ((uint64_t)a2 * b0) ^ ((uint64_t)a3 * b3);
     uint64_t z3 = ((uint64_t)a0 * b3) ^ ((uint64_t)a1 * b2) ^ ((uint64_t)a2 * b1) ^ ((uint64_t)a3 * b0);
-    return (z0 & 0x1111111111111111ull) | (z1 & 0x2222222222222222ull) | (z2 & 0x4444444444444444ull) |
-           (z3 & 0x8888888888888888ull);
+    // one bit select per word joins two classes (bits 0, 1 and 2, 3 of each
+    // nibble), one more the two pairs
+    auto join = [](uint32_t x0, uint32_t x1, uint32_t x2, uint32_t x3) {
+        const uint32_t p = (x0 & 0x55555555u) | (x1 & 0xAAAAAAAAu), q = (x2 & 0x55555555u) | (x3 & 0xAAAAAAAAu);
+        return (p & 0x33333333u) | (q & 0xCCCCCCCCu);
+    };
+    const uint32_t lo = join((uint32_t)z0, (uint32_t)z1, (uint32_t)z2, (uint32_t)z3);
+    const uint32_t hi = join((uint32_t)(z0 >> 32), (uint32_t)(z1 >> 32), (uint32_t)(z2 >> 32), (uint32_t)(z3 >> 32));
+    return ((uint64_t)hi << 32) | lo;
 }
 
 __device__ __forceinline__ uint32_t gf_mul(uint32_t a, uint32_t b) {

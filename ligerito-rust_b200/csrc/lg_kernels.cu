@@ -93,125 +93,6 @@ __global__ void k_rs_scale_spread(const uint32_t *__restrict__ poly, const uint3
     }
 }
 
-__global__ void k_rs_scale(const uint32_t *__restrict__ poly, const uint32_t *__restrict__ pis,
-                           uint32_t *__restrict__ out, uint32_t log_m, uint64_t total) {
-    pdl_begin();
-    const uint64_t m = 1ull << log_m;
-    for (uint64_t idx = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; idx < total;
-         idx += (uint64_t)gridDim.x * blockDim.x)
-        out[idx] = gf_mul(poly[idx], pis[idx & (m - 1)]);
-}
-
-// The same scaling for many columns: every column multiplies row i by the
-// same pis[i], so a block takes tiles of 32 rows x up to 64 columns, builds
-// the 32 rows' multiplication tables and multiplies with table lookups that
-// every lane of a warp shares.  A tile goes through shared memory with an
-// odd column stride: rows along lanes for the coalesced global accesses,
-// columns along lanes for the lookups, both free of bank conflicts.  Blocks
-// loop over tiles and load the next tile into registers before multiplying
-// the current one, so its HBM latency hides behind the table builds and
-// lookups.
-constexpr uint32_t kScaleRows = 32, kScaleCols = 64, kScaleThreads = 256;
-static_assert(kScaleCols == 64 && kScaleRows % (kScaleThreads / 32) == 0, "two column halves per lane");
-constexpr uint32_t kScalePer = kScaleRows * kScaleCols / kScaleThreads;  // words per thread
-__global__ void __launch_bounds__(kScaleThreads, 4) k_rs_scale_tab(const uint32_t *__restrict__ poly,
-                                                                const uint32_t *__restrict__ pis,
-                                                                uint32_t *__restrict__ out, uint32_t log_m, uint32_t n) {
-    pdl_begin();
-    __shared__ __align__(512) uint32_t tabs[kScaleRows][kTabWords];
-    __shared__ uint32_t tile[kScaleCols * (kScaleRows + 1)];
-    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const uint64_t m = 1ull << log_m;
-    const uint32_t ntiles = (uint32_t)(m / kScaleRows);
-    const uint32_t j0 = blockIdx.y * kScaleCols, ncol = min(kScaleCols, n - j0);
-    // thread's slots c = threadIdx.x + 256 i: column c / 32, row c % 32
-    uint32_t pre[kScalePer];
-    auto load = [&](uint32_t t) {
-        const uint64_t i0 = (uint64_t)t * kScaleRows;
-#pragma unroll
-        for (uint32_t i = 0; i < kScalePer; ++i) {
-            const uint32_t c = threadIdx.x + kScaleThreads * i, j = c / kScaleRows, r = c % kScaleRows;
-            pre[i] = j < ncol ? __ldg(poly + (uint64_t)(j0 + j) * m + i0 + r) : 0u;
-        }
-    };
-    // each warp builds the tables of rows warp + 8 rr (rr < 4); their pis
-    // words are loaded a tile ahead with the data
-    constexpr uint32_t kRowsPerWarp = kScaleRows / (kScaleThreads / 32);
-    uint32_t pc[kRowsPerWarp], pn[kRowsPerWarp];
-    auto load_pis = [&](uint32_t t, uint32_t (&dst)[kRowsPerWarp]) {
-#pragma unroll
-        for (uint32_t rr = 0; rr < kRowsPerWarp; ++rr)
-            dst[rr] = __ldg(pis + (uint64_t)t * kScaleRows + warp + (kScaleThreads / 32) * rr);
-    };
-    uint32_t t = blockIdx.x;
-    if (t < ntiles) {
-        load(t);
-        load_pis(t, pc);
-    }
-    for (; t < ntiles; t += gridDim.x) {
-        const uint64_t i0 = (uint64_t)t * kScaleRows;
-#pragma unroll
-        for (uint32_t rr = 0; rr < kRowsPerWarp; ++rr)
-            tab_build_warp_logic(tabs[warp + (kScaleThreads / 32) * rr], pc[rr], lane);
-#pragma unroll
-        for (uint32_t i = 0; i < kScalePer; ++i) {
-            const uint32_t c = threadIdx.x + kScaleThreads * i;
-            tile[(c / kScaleRows) * (kScaleRows + 1) + c % kScaleRows] = pre[i];
-        }
-        __syncthreads();
-        if (t + gridDim.x < ntiles) {  // in flight during the lookups
-            load(t + gridDim.x);
-            load_pis(t + gridDim.x, pn);
-        }
-        // 8 independent products per lane: rows warp + 8 rr, columns lane + 32 jj
-        uint32_t x[kRowsPerWarp][2];
-#pragma unroll
-        for (uint32_t rr = 0; rr < kRowsPerWarp; ++rr)
-#pragma unroll
-            for (uint32_t jj = 0; jj < 2; ++jj) {
-                const uint32_t j = lane + 32 * jj, r = warp + (kScaleThreads / 32) * rr;
-                x[rr][jj] = j < ncol ? tab_mul_sa(reinterpret_cast<const uint8_t *>(tabs), 512u * r, 0,
-                                                  tile[j * (kScaleRows + 1) + r])
-                                     : 0u;
-            }
-#pragma unroll
-        for (uint32_t rr = 0; rr < kRowsPerWarp; ++rr)
-#pragma unroll
-            for (uint32_t jj = 0; jj < 2; ++jj) {
-                const uint32_t j = lane + 32 * jj, r = warp + (kScaleThreads / 32) * rr;
-                if (j < ncol) tile[j * (kScaleRows + 1) + r] = x[rr][jj];
-            }
-        __syncthreads();
-#pragma unroll
-        for (uint32_t i = 0; i < kScalePer; ++i) {
-            const uint32_t c = threadIdx.x + kScaleThreads * i, j = c / kScaleRows, r = c % kScaleRows;
-            if (j < ncol) out[(uint64_t)(j0 + j) * m + i0 + r] = tile[j * (kScaleRows + 1) + r];
-        }
-#pragma unroll
-        for (uint32_t rr = 0; rr < kRowsPerWarp; ++rr) pc[rr] = pn[rr];
-        __syncthreads();  // the tile and tables are rewritten next
-    }
-}
-
-cudaError_t rs_scale(Launcher &L, const uint32_t *poly, const uint32_t *pis, uint32_t *out, uint32_t log_m,
-                     uint32_t n) {
-    if (n >= kScaleCols / 2 && log_m >= 5) {
-        // a table costs about as much as 30 general products: worth it from
-        // 32 columns on
-        // a few tiles per block: about four blocks per SM in one wave
-        const uint64_t ntiles = (1ull << log_m) / kScaleRows;
-        const dim3 grid((unsigned)std::min<uint64_t>(ntiles, 148ull * 4), (n + kScaleCols - 1) / kScaleCols);
-        L.note(8.0 * n * (1ull << log_m), (double)n * (1ull << log_m));
-        LGK_LAUNCH(L, "rs_scale", launch_k(k_rs_scale_tab, grid, 256, 0, L.stream, poly, pis, out, log_m, n));
-        return cudaGetLastError();
-    }
-    const uint64_t total = (uint64_t)n << log_m;
-    const unsigned blocks = (unsigned)std::min<uint64_t>((total + 255) / 256, 148ull * 16);
-    L.note(8.0 * total, (double)total);
-    LGK_LAUNCH(L, "rs_scale", launch_k(k_rs_scale, blocks, 256, 0, L.stream, poly, pis, out, log_m, total));
-    return cudaGetLastError();
-}
-
 cudaError_t rs_scale_spread(Launcher &L, const uint32_t *poly, const uint32_t *pis, uint32_t *E,
                             uint32_t log_m, uint32_t n) {
     uint64_t total = (uint64_t)n << log_m;
@@ -231,11 +112,14 @@ struct PassArgs {
     const uint32_t *tw;
     const uint4 *dtab;  // this pass's D tables (see build_pass_tables)
     uint64_t col_stride, q_stride;
-    uint32_t L, d0, log_S, log_nvec_p2, nvec, log_bpg, log_B, root_base;
+    uint32_t L, d0, log_S, nvec, bpg, root_base;  // bpg: strided passes, units per (q, P)
+    uint32_t bulk;                                // strided passes: rows come in by bulk copies
+    uint32_t *fault;                              // set when a copy's wait gives up
     uint32_t vchunk, nchunks;  // last pass: vectors per block, blocks per (q, P)
     uint64_t units;            // strided passes: (group, chunk) work units
     const uint32_t *src;       // strided passes: input, when not data (FftSrc)
     uint64_t src_col_stride, src_q_stride;
+    const uint32_t *pis;       // k_rs_first: the row scaling
 };
 
 // The 2^K - 1 node tables of one (q, P), in 512-byte slots at the start of
@@ -293,7 +177,9 @@ __global__ void k_fft_dtab(const uint32_t *__restrict__ tw, DtabArgs d, uint32_t
 // stages root-first.  Inverse: ifft_twiddles / ifft_mul (:161-178,
 // 194-206), leaves-first.  One flat loop so every register index is a
 // compile-time constant after unrolling.
-template <int KP, int S0, bool INV>
+// ZERO0: the twiddle of each stage's node 0 is zero (its products are left
+// out).
+template <int KP, int S0, bool INV, bool ZERO0 = false>
 __device__ __forceinline__ void pencil_stages(uint32_t (&v)[1 << KP], const uint8_t *sm, uint32_t tb,
                                               uint32_t gshift_slot) {
 #pragma unroll
@@ -309,7 +195,7 @@ __device__ __forceinline__ void pencil_stages(uint32_t (&v)[1 << KP], const uint
         const uint32_t base = tb + 512u * (gshift_slot << sl);
         const uint32_t off = 512u * ((1u << s) - 1u + (uint32_t)tp);
         if (!INV) {
-            v[x] ^= tab_mul_sa(sm, base, off, v[y]);
+            if (!ZERO0 || tp != 0) v[x] ^= tab_mul_sa(sm, base, off, v[y]);
             v[y] ^= v[x];
         } else {
             v[y] ^= v[x];
@@ -321,172 +207,318 @@ __device__ __forceinline__ void pencil_stages(uint32_t (&v)[1 << KP], const uint
 // Strided passes: a thread owns one "pencil", the 2^K rows
 // P*2^(L-d0) + t*S + o (t < 2^K) of one vector, S = 2^(L-d0-K) > 1, in
 // registers.  Threads of a block share (q, P) and hence every twiddle of
-// the pass; lanes run over o, so each row access is coalesced.  With
-// K <= 4 a thread also holds the next unit's pencil, loaded before this
-// one's stages run so that its HBM latency hides behind them (64
-// registers, 4 blocks per SM: measured faster than 6 blocks without it);
-// larger pencils would spill.
+// the pass; lanes run over o, so each row access is coalesced.
+// Work units are (group (q, P), chunk of blockDim.x pencils) in group-major
+// order; block b takes the contiguous range [b U / B, (b+1) U / B), so one
+// wave of blocks gets equal shares, and builds the node tables again only
+// where its range enters the next group.
+// Bulk copies of a unit's 2^K rows into buf[2^K][B], issued by the whole block
+// (a.bulk: rows of S >= 32 words, 16-byte aligned): `cnt` pencils from the
+// one at `src` on, columns `cs` words apart.
+template <int K>
+__device__ __forceinline__ void issue_unit(const uint32_t *src, uint64_t cs, uint32_t log_S, uint32_t cnt, uint32_t *buf,
+                                           uint64_t *bar) {
+    constexpr uint32_t R = 1u << K;
+    const uint32_t B = blockDim.x, tid = threadIdx.x, S4 = 4u << log_S;
+    if (tid == 0) mbar_expect(bar, 4 * R * cnt);
+    if ((1ull << log_S) >= B) {  // one column's run of B words per row
+        for (uint32_t t = tid; t < R; t += B) bulk_load(buf + t * B, strided(src, t, S4), 4 * B, bar);
+    } else {  // B / S whole columns
+        const uint32_t n = R * (cnt >> log_S);
+        for (uint32_t c = tid; c < n; c += B) {
+            const uint32_t t = c & (R - 1), col = c >> K;
+            bulk_load(buf + t * B + (col << log_S), strided(src + col * cs, t, S4), S4, bar);
+        }
+    }
+}
+
+// K <= 4: a thread also holds the next unit's pencil, loaded before this
+// one's stages run so that its HBM latency hides behind them (64 registers,
+// 4 blocks per SM; at 2^18 x 256 columns 168 us against 176 us with the rows
+// staged by bulk copies, whose hand-over is a block barrier per unit).
+// Larger pencils leave no registers for that: with a.bulk, bulk copies bring
+// a unit's rows into shared memory, the next unit's issued as soon as this
+// one's values are in registers (K = 6 at 2^12 x 1472 columns x 4: 143 us
+// without, 100 us with them).
 template <int K, bool INV>
-__global__ void __launch_bounds__(256, K <= 4 ? 4 : (K == 5 ? 4 : 2)) k_fft_pass(PassArgs a) {
+__global__ void __launch_bounds__(256, K <= 4 ? 4 : (K == 5 ? 3 : 2)) k_fft_pass(PassArgs a) {
     pdl_begin();
     extern __shared__ __align__(16) uint8_t smraw[];
-    // Work units (group (q, P), chunk of 2^log_B pencils) in group-major
-    // order; block b takes the contiguous range [b U / B, (b+1) U / B), so
-    // one wave of blocks gets equal shares, and builds the node tables again
-    // only where its range enters the next group.
+    constexpr uint32_t R = 1u << K;
+    constexpr bool PF = K <= 4;
+    const uint32_t B = blockDim.x, tid = threadIdx.x;
+    uint32_t *buf = reinterpret_cast<uint32_t *>(smraw + (R - 1) * 512);  // a.bulk: [R][B]
+    uint64_t *bar = reinterpret_cast<uint64_t *>(buf + R * B);
     const uint32_t U = (uint32_t)a.units, nb = gridDim.x;
     const uint32_t u0 = (uint32_t)((uint64_t)blockIdx.x * U / nb), u1 = (uint32_t)((uint64_t)(blockIdx.x + 1) * U / nb);
-    const uint64_t S = 1ull << a.log_S;
-    const uint32_t S4 = 4u << a.log_S;  // bytes between pencil values (a vector is < 4 GiB)
-    uint32_t cur = 0xFFFFFFFFu;
-    const bool own_src = a.src != nullptr;
-    const uint64_t scs = own_src ? a.src_col_stride : a.col_stride;
-    // Pencil of unit u for this thread: load pointer, store pointer and
-    // whether the thread has a vector there (nvec need not be a power of 2).
-    auto locate = [&](uint32_t u, const uint32_t *&lb, uint32_t *&sb) -> bool {
-        const uint32_t grp = u >> a.log_bpg, chunk = u & ((1u << a.log_bpg) - 1);
-        const unsigned P = grp & ((1u << a.d0) - 1), q = grp >> a.d0;
-        const uint64_t row0 = (uint64_t)P << (a.L - a.d0);
-        const uint32_t g = (chunk << a.log_B) + threadIdx.x;
-        const uint32_t o = g & ((1u << a.log_S) - 1), j = g >> a.log_S;
-        sb = a.data + q * a.q_stride + row0 + j * a.col_stride + o;
-        lb = own_src ? a.src + q * a.src_q_stride + row0 + j * scs + o : sb;
-        return j < a.nvec;
+    const uint64_t G = (uint64_t)a.nvec << a.log_S;  // pencils of a group
+    const uint32_t S4 = 4u << a.log_S;               // bytes between pencil values (a vector is < 4 GiB)
+    // the group's first word, and where pencil g of it starts
+    auto group = [&](uint32_t grp) {
+        return a.data + (grp >> a.d0) * a.q_stride + ((uint64_t)(grp & ((1u << a.d0) - 1)) << (a.L - a.d0));
     };
-    constexpr bool PF = K <= 4;
-    constexpr int NP = PF ? (1 << K) : 1;
-    uint32_t v[1 << K], nv[NP];
-    const uint32_t *lb;
-    uint32_t *sb;
-    bool have = PF && u0 < u1 && locate(u0, lb, sb);
-    if (PF && have) {
+    auto pencil = [&](uint32_t *gp, uint64_t g) { return gp + (g >> a.log_S) * a.col_stride + (g & ((1ull << a.log_S) - 1)); };
+    uint32_t grp = u0 / a.bpg, ch = u0 - grp * a.bpg, parity = 0;
+    uint32_t *gp = group(grp);
+    uint32_t nv[PF ? R : 1], *p = gp;
+    bool mine = false;
+    auto prefetch = [&]() {  // the pencil of chunk ch of the group at gp
+        const uint64_t g = (uint64_t)ch * B + tid;
+        mine = g < G;
+        p = pencil(gp, g);
+        if (PF && mine) {
 #pragma unroll
-        for (int t = 0; t < NP; ++t) nv[t] = *strided(lb, (uint32_t)t, S4);
-    }
-    for (uint32_t u = u0; u < u1; ++u) {
-        const uint32_t grp = u >> a.log_bpg;
-        if (grp != cur) {
-            if (cur != 0xFFFFFFFFu) __syncthreads();  // every thread is done with the old tables
-            const unsigned P = grp & ((1u << a.d0) - 1), q = grp >> a.d0;
-            build_pass_tables<K>(smraw, a, q, P);  // ends with the block synchronised
-            cur = grp;
+            for (uint32_t t = 0; PF && t < R; ++t) nv[t] = *strided(p, t, S4);
         }
-        bool mine;
-        uint32_t *base;
+    };
+    auto issue = [&]() {
+        const uint64_t g0 = (uint64_t)ch * B;
+        issue_unit<K>(pencil(gp, g0), a.col_stride, a.log_S, (uint32_t)min((uint64_t)B, G - g0), buf, bar);
+    };
+    if (!PF && a.bulk) {
+        if (tid == 0) {
+            mbar_init(bar, 1);
+            fence_async();
+        }
+        __syncthreads();
+        issue();
+    }
+    prefetch();
+    bool fresh = true;  // the group's tables are to be built
+    for (uint32_t u = u0; u < u1; ++u) {
+        if (fresh) {
+            if (u != u0) __syncthreads();  // every thread is done with the old tables
+            build_pass_tables<K>(smraw, a, grp >> a.d0, grp & ((1u << a.d0) - 1));  // ends with the block synchronised
+        }
+        uint32_t *const base = p;
+        const bool here = mine;
+        uint32_t v[R];
+        fresh = ++ch == a.bpg;
+        if (fresh) {
+            ch = 0;
+            gp = group(++grp);
+        }
         if constexpr (PF) {
-            mine = have;
-            base = sb;
 #pragma unroll
-            for (int t = 0; t < NP; ++t) v[t] = nv[t];
-            have = u + 1 < u1 && locate(u + 1, lb, sb);
-            if (have) {
-#pragma unroll
-                for (int t = 0; t < NP; ++t) nv[t] = *strided(lb, (uint32_t)t, S4);
-            }
+            for (uint32_t t = 0; t < R; ++t) v[t] = nv[t];
+            if (u + 1 < u1) prefetch();
         } else {
-            mine = locate(u, lb, sb);
-            base = sb;
+            if (a.bulk) {
+                mbar_wait(bar, parity, a.fault);
+                parity ^= 1;
+                if (here) {
+#pragma unroll
+                    for (uint32_t t = 0; t < R; ++t) v[t] = buf[t * B + tid];
+                }
+                __syncthreads();  // the values are in registers: the next unit's copies may land
+                if (u + 1 < u1) issue();
+            } else if (here) {
+#pragma unroll
+                for (uint32_t t = 0; t < R; ++t) v[t] = *strided(base, t, S4);
+            }
+            prefetch();
+        }
+        if (!here) continue;
+        pencil_stages<K, 0, INV>(v, smraw, 0, 0);
+#pragma unroll
+        for (uint32_t t = 0; t < R; ++t) *strided(base, t, S4) = v[t];
+    }
+}
+
+// The first pass of a Reed-Solomon encoding (rate 1/4): quarters q < 4 of
+// each output column are the transforms under heap nodes 4 + q of the same
+// input column scaled row by row with pis.  A thread loads its pencil of the
+// input once, scales it and runs the K stages of all four quarters:
+//   * the scaling is a general product per value (a row's constant serves
+//     one value of each column, too few for a table); it uses the multiply
+//     and logic pipes, the stages the shared-memory one;
+//   * the roots' twiddles are GF(2)-linear in q and zero for q = 0, so the
+//     first stage takes the products with roots 1 and 2 only (2 instead of
+//     4 per pair), and q = 3 adds both;
+//   * quarter 0's first node of every stage has twiddle zero too.
+// For K = 4 that is 105 table products and 16 scalings a pencil instead of
+// 128, 64 row loads less, and no scaled copy of the input in memory.
+template <int K>
+__global__ void __launch_bounds__(256, K <= 4 ? 3 : 2) k_rs_first(PassArgs a) {
+    pdl_begin();
+    extern __shared__ __align__(16) uint8_t smraw[];
+    constexpr uint32_t R = 1u << K, H = R / 2, QT = (R - 1) * 512;  // QT: bytes of a quarter's tables
+    const uint32_t B = blockDim.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nw = B >> 5;
+    uint32_t *buf = reinterpret_cast<uint32_t *>(smraw + 4 * QT);  // a.bulk: [R][B]
+    uint64_t *bar = reinterpret_cast<uint64_t *>(buf + R * B);
+    // units blockIdx.x, + gridDim.x, ...: every SM's blocks get the same number
+    // of units to one (contiguous shares of 9 or 10 units a block left SMs
+    // with 27 to 30)
+    const uint32_t U = (uint32_t)a.units, u0 = blockIdx.x, nb = gridDim.x;
+    const uint64_t G = (uint64_t)a.nvec << a.log_S;  // pencils
+    const uint32_t S4 = 4u << a.log_S;               // bytes between pencil values
+    auto issue = [&](uint32_t u) {
+        const uint64_t g0 = (uint64_t)u * B;
+        issue_unit<K>(a.src + (g0 >> a.log_S) * a.src_col_stride + (g0 & ((1ull << a.log_S) - 1)), a.src_col_stride,
+                      a.log_S, (uint32_t)min((uint64_t)B, G - g0), buf, bar);
+    };
+    if (a.bulk) {
+        if (tid == 0) {
+            mbar_init(bar, 1);
+            fence_async();
+        }
+        __syncthreads();
+        issue(u0);
+    }
+    // the node tables of all four quarters (see build_pass_tables)
+    for (uint32_t i = warp; i < 4 * K; i += nw) {
+        const uint32_t q = i / K, s = i % K;
+        tab_build_warp(reinterpret_cast<uint32_t *>(smraw + q * QT + ((1u << s) - 1) * 512),
+                       __ldg(a.tw + ((4u + q) << s) - 1), lane);
+    }
+    __syncthreads();
+    for (uint32_t i = tid; i < 4 * (R - 1) * 32; i += B) {
+        const uint32_t q = i / ((R - 1) * 32), e = i - q * (R - 1) * 32, slot = e >> 5, first = (1u << (31 - __clz(slot + 1))) - 1;
+        if (slot == first) continue;
+        uint4 *T = reinterpret_cast<uint4 *>(smraw + q * QT);
+        uint4 c = T[first * 32 + (e & 31)];
+        const uint4 d = __ldg(a.dtab + e);
+        c.x ^= d.x; c.y ^= d.y; c.z ^= d.z; c.w ^= d.w;
+        T[e] = c;
+    }
+    __syncthreads();
+    uint32_t parity = 0;
+    for (uint32_t u = u0; u < U; u += nb) {
+        const uint64_t g = (uint64_t)u * B + tid;
+        const bool mine = g < G;
+        const uint64_t col = g >> a.log_S, o = g & ((1ull << a.log_S) - 1);
+        uint32_t v[R];
+        const uint32_t *pp = a.pis + o;
+        if (a.bulk) {
+            mbar_wait(bar, parity, a.fault);
+            parity ^= 1;
             if (mine) {
 #pragma unroll
-                for (int t = 0; t < (1 << K); ++t) v[t] = *strided(lb, (uint32_t)t, S4);
+                for (uint32_t t = 0; t < R; ++t) v[t] = buf[t * B + tid];
             }
+            __syncthreads();  // the values are in registers: the next unit's copies may land
+            if (u + nb < U) issue(u + nb);
+        } else if (mine) {
+            const uint32_t *lb = a.src + col * a.src_col_stride + o;
+#pragma unroll
+            for (uint32_t t = 0; t < R; ++t) v[t] = *strided(lb, t, S4);
         }
         if (!mine) continue;
-        pencil_stages<K, 0, INV>(v, smraw, 0, 0);
-        if constexpr (!PF) {
-            // recompute the store addresses instead of keeping 2^K pointers live
-            uint64_t S2;
-            asm volatile("mov.b64 %0, %1;" : "=l"(S2) : "l"(S));
-            asm volatile("mov.b64 %0, %1;" : "=l"(base) : "l"(base));
 #pragma unroll
-            for (int t = 0; t < (1 << K); ++t) base[t * S2] = v[t];
-        } else {
+        for (uint32_t t = 0; t < R; ++t) v[t] = gf_mul(v[t], __ldg(strided(pp, t, S4)));
+        uint32_t p1[H], p2[H];  // the first stage's products with roots 1 and 2
 #pragma unroll
-            for (int t = 0; t < (1 << K); ++t) *strided(base, (uint32_t)t, S4) = v[t];
+        for (uint32_t i = 0; i < H; ++i) {
+            p1[i] = tab_mul_sa(smraw, 0, QT, v[H + i]);
+            p2[i] = tab_mul_sa(smraw, 0, 2 * QT, v[H + i]);
+        }
+        uint32_t *out = a.data + col * a.col_stride + o;
+        {
+            uint32_t x[H], y[H];
+#pragma unroll
+            for (uint32_t i = 0; i < H; ++i) {
+                x[i] = v[i];
+                y[i] = v[H + i] ^ v[i];
+            }
+            if constexpr (K > 1) {
+                pencil_stages<K - 1, 1, false, true>(x, smraw, 0, 0);
+                pencil_stages<K - 1, 1, false>(y, smraw, 0, 1);
+            }
+#pragma unroll
+            for (uint32_t i = 0; i < H; ++i) {
+                *strided(out, i, S4) = x[i];
+                *strided(out, H + i, S4) = y[i];
+            }
+        }
+#pragma unroll 1
+        for (uint32_t q = 1; q < 4; ++q) {
+            out += a.q_stride;
+            const uint32_t m1 = 0u - (q & 1), m2 = 0u - (q >> 1);
+            uint32_t x[H], y[H];
+#pragma unroll
+            for (uint32_t i = 0; i < H; ++i) {
+                x[i] = v[i] ^ (p1[i] & m1) ^ (p2[i] & m2);
+                y[i] = v[H + i] ^ x[i];
+            }
+            if constexpr (K > 1) {
+                pencil_stages<K - 1, 1, false>(x, smraw, q * QT, 0);
+                pencil_stages<K - 1, 1, false>(y, smraw, q * QT, 1);
+            }
+#pragma unroll
+            for (uint32_t i = 0; i < H; ++i) {
+                *strided(out, i, S4) = x[i];
+                *strided(out, H + i, S4) = y[i];
+            }
         }
     }
 }
 
 // Last pass (contiguous blocks of 2^K rows): one block per (q, P) tile of
-// 2^K rows x nvec vectors.  The tile is loaded with coalesced 16-byte reads
-// into shared memory with an odd column stride (2^K + 1 words), so both a
-// lane-per-vector walk down a column and a lane-per-row walk across the
-// columns are bank-conflict free.  All warps build the 2^K - 1 tables, then
-// the stages run in two register phases of about K/2 stages each.  Lanes
-// run over vectors, so a warp shares every table it reads; the block has
-// as many threads as a phase has pencils (up to 256), so a tile of few
-// vectors still keeps every thread busy.
+// 2^K rows x nvec vectors.  All warps build the 2^K - 1 tables, then the
+// stages run in two register phases of about K/2 stages each.  A warp shares
+// every table it reads; the block has as many threads as a phase has pencils
+// (up to 256), so a tile of few vectors still keeps every thread busy.
+// The load/store unit's wavefronts bound this kernel (93% of their peak with
+// the tile staged through registers), so a column's 2^K words enter and
+// leave the tile as one bulk copy each, which takes none.  The tile's column
+// stride is 2^K + 4 words (an odd number of 16-byte pieces): phase A reads
+// and writes words with lanes over 8 columns x 4 rows, phase B 16-byte
+// pieces with lanes over columns, both free of bank conflicts.
 template <int K, bool INV>
 __global__ void __launch_bounds__(256, 4) k_fft_tail(PassArgs a) {
     pdl_begin();
-    constexpr int KA = K / 2, KB = K - KA, RB = 1 << KB, R = 1 << K, STRIDE = R + 1, CPC = R / 4;
+    constexpr int KA = K / 2, KB = K - KA, RB = 1 << KB, R = 1 << K, STRIDE = R + 4;
     extern __shared__ __align__(16) uint8_t smraw[];
     const unsigned chunk = blockIdx.x % a.nchunks, rest = blockIdx.x / a.nchunks;
     const unsigned P = rest & ((1u << a.d0) - 1);
     const unsigned q = rest >> a.d0;
     const uint32_t nvec = min(a.vchunk, a.nvec - chunk * a.vchunk);
-    const uint32_t tb = 0;
-    uint32_t *tile = reinterpret_cast<uint32_t *>(smraw + tb + ((1 << K) - 1) * 512);
+    uint32_t *tile = reinterpret_cast<uint32_t *>(smraw + (R - 1) * 512);
+    uint64_t *bar = reinterpret_cast<uint64_t *>(tile + a.vchunk * STRIDE);
     uint32_t *gbase = a.data + (uint64_t)chunk * a.vchunk * a.col_stride + q * a.q_stride + ((uint64_t)P << K);
-    // the tile's 16-byte pieces are loaded into registers first, so that
-    // their HBM latency passes while the block builds its tables (up to
-    // kTilePieces per thread: 64 vectors of 64 rows over 256 threads)
-    constexpr int kTilePieces = 4;
-    uint4 pre[kTilePieces];
-#pragma unroll
-    for (int i = 0; i < kTilePieces; ++i) {
-        const uint32_t c = threadIdx.x + i * blockDim.x;
-        if (c < nvec * CPC) {
-            const uint32_t j = c / CPC, piece = c % CPC;
-            pre[i] = *reinterpret_cast<const uint4 *>(gbase + j * a.col_stride + 4 * piece);
-        }
-    }
-    build_pass_tables<K>(smraw, a, q, P);
-#pragma unroll
-    for (int i = 0; i < kTilePieces; ++i) {
-        const uint32_t c = threadIdx.x + i * blockDim.x;
-        if (c < nvec * CPC) {
-            const uint32_t j = c / CPC, piece = c % CPC;
-            uint32_t *d = tile + j * STRIDE + 4 * piece;
-            d[0] = pre[i].x; d[1] = pre[i].y; d[2] = pre[i].z; d[3] = pre[i].w;
-        }
-    }
-    // pieces past the registers' share (smaller blocks on wider tiles)
-    for (uint32_t c = threadIdx.x + kTilePieces * blockDim.x; c < nvec * CPC; c += blockDim.x) {
-        const uint32_t j = c / CPC, piece = c % CPC;
-        const uint4 x = *reinterpret_cast<const uint4 *>(gbase + j * a.col_stride + 4 * piece);
-        uint32_t *d = tile + j * STRIDE + 4 * piece;
-        d[0] = x.x; d[1] = x.y; d[2] = x.z; d[3] = x.w;
+    if (threadIdx.x == 0) {
+        mbar_init(bar, 1);
+        fence_async();
+        mbar_expect(bar, 4 * R * nvec);
     }
     __syncthreads();
+    for (uint32_t j = threadIdx.x; j < nvec; j += blockDim.x)
+        bulk_load(tile + j * STRIDE, gbase + j * a.col_stride, 4 * R, bar);
+    build_pass_tables<K>(smraw, a, q, P);
+    mbar_wait(bar, 0, a.fault);
 
     // Two register phases: KA stages on pencils of 2^KA values at stride
     // 2^KB, then KB stages on contiguous pencils of 2^KB values.  Work items
-    // run over (vector, pencil) with the vector index in the low bits (a
-    // power-of-two span, so the split is a mask and a shift).
-    const uint32_t lnv = 32 - __clz(nvec - 1), vmask = (1u << lnv) - 1;
+    // run over (vector, pencil) with a power-of-two span of vectors, so the
+    // split is masks and shifts.
+    const uint32_t lnv = 32 - __clz(nvec - 1), cl = min(3u, lnv);
     auto phase_a = [&]() {
+        // item bits: 8 vectors, pencil, the other vectors
         for (uint32_t item = threadIdx.x; item < ((uint32_t)RB << lnv); item += blockDim.x) {
-            const uint32_t j = item & vmask, u = item >> lnv;
+            const uint32_t u = (item >> cl) & (RB - 1), j = (item >> (cl + KB) << cl) | (item & ((1u << cl) - 1));
             if (j >= nvec) continue;
             uint32_t v[1 << KA];
 #pragma unroll
             for (int i = 0; i < (1 << KA); ++i) v[i] = tile[j * STRIDE + u + RB * i];
-            pencil_stages<KA, 0, INV>(v, smraw, tb, 0);
+            pencil_stages<KA, 0, INV>(v, smraw, 0, 0);
 #pragma unroll
             for (int i = 0; i < (1 << KA); ++i) tile[j * STRIDE + u + RB * i] = v[i];
         }
     };
     auto phase_b = [&]() {
         for (uint32_t item = threadIdx.x; item < ((1u << KA) << lnv); item += blockDim.x) {
-            const uint32_t j = item & vmask, gq = item >> lnv;
+            const uint32_t j = item & ((1u << lnv) - 1), gq = item >> lnv;
             if (j >= nvec) continue;
+            uint4 *p = reinterpret_cast<uint4 *>(tile + j * STRIDE + RB * gq);
             uint32_t v[RB];
 #pragma unroll
-            for (int i = 0; i < RB; ++i) v[i] = tile[j * STRIDE + RB * gq + i];
-            pencil_stages<KB, KA, INV>(v, smraw, tb, gq);
+            for (int i = 0; i < RB / 4; ++i) {
+                const uint4 x = p[i];
+                v[4 * i] = x.x; v[4 * i + 1] = x.y; v[4 * i + 2] = x.z; v[4 * i + 3] = x.w;
+            }
+            pencil_stages<KB, KA, INV>(v, smraw, 0, gq);
 #pragma unroll
-            for (int i = 0; i < RB; ++i) tile[j * STRIDE + RB * gq + i] = v[i];
+            for (int i = 0; i < RB / 4; ++i) p[i] = make_uint4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
         }
     };
     if (!INV) {
@@ -498,24 +530,25 @@ __global__ void __launch_bounds__(256, 4) k_fft_tail(PassArgs a) {
         __syncthreads();
         phase_a();
     }
+    fence_async();  // this thread's tile words, before the copies out
     __syncthreads();
-
-    for (uint32_t c = threadIdx.x; c < nvec * CPC; c += blockDim.x) {
-        const uint32_t j = c / CPC, piece = c % CPC;
-        const uint32_t *d = tile + j * STRIDE + 4 * piece;
-        *reinterpret_cast<uint4 *>(gbase + j * a.col_stride + 4 * piece) = make_uint4(d[0], d[1], d[2], d[3]);
-    }
+    for (uint32_t j = threadIdx.x; j < nvec; j += blockDim.x)
+        bulk_store(gbase + j * a.col_stride, tile + j * STRIDE, 4 * R);
+    bulk_store_wait();  // the tile is read, and the words are written when the grid ends
 }
 
 constexpr uint32_t kTailChunk = 64;  // vectors per tile of the last pass
 static size_t pass_smem(int K) { return (size_t)((1 << K) - 1) * 512; }
-static size_t tail_smem(int K, uint32_t vchunk) { return pass_smem(K) + (size_t)vchunk * ((1u << K) + 1) * 4; }
+static size_t tail_smem(int K, uint32_t vchunk) { return pass_smem(K) + (size_t)vchunk * ((1u << K) + 4) * 4 + 16; }
+// strided pass: tables, then (bulk copies) the unit's rows and the barrier
+static size_t strided_smem(int K, unsigned threads, bool bulk, bool rs_first = false) {
+    return pass_smem(K) * (rs_first ? 4 : 1) + (bulk ? ((size_t)threads << K) * 4 + 16 : 0);
+}
 
-// One wave of strided-pass blocks: as many as fit on the device at once
-// (occupancy of this instantiation, cached), at most one per unit.
-template <int K, bool INV>
-static unsigned pass_grid(uint64_t units, unsigned threads, size_t smem) {
-    static std::atomic<int> sms_c{0}, occ_c[257];  // idempotent fills; contexts may run on several threads
+// One wave of blocks of a kernel: as many as fit on the device at once
+// (occupancy at this size, cached by the caller's array), at most one per unit.
+static unsigned wave_grid(const void *kernel, std::atomic<int> *occ_c, uint64_t units, unsigned threads, size_t smem) {
+    static std::atomic<int> sms_c{0};  // idempotent fills; contexts may run on several threads
     int sms = sms_c.load(std::memory_order_relaxed);
     if (!sms) {
         int dev = 0;
@@ -523,11 +556,10 @@ static unsigned pass_grid(uint64_t units, unsigned threads, size_t smem) {
             sms = 148;
         sms_c.store(sms, std::memory_order_relaxed);
     }
-    int o = occ_c[threads].load(std::memory_order_relaxed);
+    int o = occ_c->load(std::memory_order_relaxed);
     if (!o) {
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o, k_fft_pass<K, INV>, (int)threads, smem) != cudaSuccess || o < 1)
-            o = 1;
-        occ_c[threads].store(o, std::memory_order_relaxed);
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o, kernel, (int)threads, smem) != cudaSuccess || o < 1) o = 1;
+        occ_c->store(o, std::memory_order_relaxed);
     }
     return (unsigned)std::min<uint64_t>(units, (uint64_t)sms * o);
 }
@@ -536,17 +568,45 @@ template <bool INV>
 static cudaError_t launch_pass(Launcher &L, int K, PassArgs a, unsigned threads) {
     char nmbuf[48];
     std::snprintf(nmbuf, sizeof nmbuf, "%s_L%u_K%d_n%u", INV ? "ifft_pass" : "fft_pass", a.L, K, a.nvec);
-    const size_t smem = pass_smem(K);
+    if (K <= 4) a.bulk = 0;  // those hold the next unit's values in registers
+    const size_t smem = strided_smem(K, threads, a.bulk);
+    // the kernel's limit is always set to its largest unit: contexts on other
+    // threads launch the same kernel with other sizes, and a smaller limit
+    // set between another thread's set and launch would fail it
+    const int smem_max = (int)strided_smem(K, 256, K > 4);
     switch (K) {
 #define LGK_CASE(k)                                                                                  \
     case k: {                                                                                        \
-        if (smem > 48 * 1024)                                                                        \
-            cudaFuncSetAttribute(k_fft_pass<k, INV>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
-        const unsigned blocks = pass_grid<k, INV>(a.units, threads, smem);                           \
+        static std::atomic<int> occ[2][257];                                                         \
+        const void *fn = reinterpret_cast<const void *>(k_fft_pass<k, INV>);                         \
+        if (smem_max > 48 * 1024) cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_max); \
+        const unsigned blocks = wave_grid(fn, &occ[a.bulk][threads], a.units, threads, smem);        \
         LGK_LAUNCH(L, nmbuf, launch_k(k_fft_pass<k, INV>, blocks, threads, smem, L.stream, a));      \
         break;                                                                                       \
     }
         LGK_CASE(1) LGK_CASE(2) LGK_CASE(3) LGK_CASE(4) LGK_CASE(5) LGK_CASE(6)
+#undef LGK_CASE
+        default: return cudaErrorInvalidValue;
+    }
+    return cudaGetLastError();
+}
+
+static cudaError_t launch_rs_first(Launcher &L, int K, const PassArgs &a, unsigned threads) {
+    char nmbuf[48];
+    std::snprintf(nmbuf, sizeof nmbuf, "fft_pass_L%u_K%d_n%u_rs", a.L, K, a.nvec);
+    const size_t smem = strided_smem(K, threads, a.bulk, true);
+    const int smem_max = (int)strided_smem(K, 256, true, true);  // as in launch_pass
+    switch (K) {
+#define LGK_CASE(k)                                                                                  \
+    case k: {                                                                                        \
+        static std::atomic<int> occ[2][257];                                                         \
+        const void *fn = reinterpret_cast<const void *>(k_rs_first<k>);                              \
+        if (smem_max > 48 * 1024) cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_max); \
+        const unsigned blocks = wave_grid(fn, &occ[a.bulk][threads], a.units, threads, smem);        \
+        LGK_LAUNCH(L, nmbuf, launch_k(k_rs_first<k>, blocks, threads, smem, L.stream, a));           \
+        break;                                                                                       \
+    }
+        LGK_CASE(1) LGK_CASE(2) LGK_CASE(3) LGK_CASE(4) LGK_CASE(5)
 #undef LGK_CASE
         default: return cudaErrorInvalidValue;
     }
@@ -558,9 +618,6 @@ static cudaError_t launch_tail(Launcher &L, int K, PassArgs a, unsigned blocks) 
     char nmbuf[48];
     std::snprintf(nmbuf, sizeof nmbuf, "%s_L%u_K%d_n%u", INV ? "ifft_tail" : "fft_tail", a.L, K, a.nvec);
     const size_t smem = tail_smem(K, a.vchunk);
-    // the kernel's limit is always set to its largest tile: contexts on other
-    // threads launch the same kernel with other tile sizes, and a smaller
-    // limit set between another thread's set and launch would fail it
     const int smem_max = (int)tail_smem(K, kTailChunk);
     uint32_t vp2 = 1;
     while (vp2 < a.vchunk) vp2 <<= 1;
@@ -611,13 +668,18 @@ cudaError_t fft_vectors(Launcher &L, uint32_t *data, const uint32_t *tw, uint32_
                         uint32_t root_base, bool inverse, FftPasses passes, const FftSrc *src) {
     if (log_len == 0 || nvec == 0) return cudaSuccess;
     if (inverse && passes != FFT_ALL) return cudaErrorInvalidValue;
-    if (src && (inverse || log_len <= 6 || passes == FFT_LAST)) return cudaErrorInvalidValue;
+    // a source is a Reed-Solomon encoding's: one input for the four quarters
+    if (src && (inverse || log_len <= 6 || passes == FFT_LAST || Q != 4 || root_base != 4 || !src->pis))
+        return cudaErrorInvalidValue;
     // the roots root_base + q (q < Q) must share one heap layer
     const uint32_t lr = 31 - __builtin_clz(root_base);
     if (!L.dtab || root_base == 0 || ((root_base + Q - 1) >> lr) != 1) return cudaErrorInvalidValue;
     // head / last calls on column groups must agree on the split, so only
     // whole transforms take tuned plans
     FftPlan plan = default_fft_plan(log_len);
+    if (src && plan.ks[0] > kMaxRsFirst) {  // (log_len = 12)
+        plan = FftPlan{3, {plan.ks[0] / 2, plan.ks[0] - plan.ks[0] / 2, plan.ks[1]}};
+    }
     if (passes == FFT_ALL && !L.forced_plan) {
         const TuneKey tk{L.device, log_len, nvec, Q, src != nullptr, inverse, 0};
         if (!tuned_fft_plan(tk, &plan) && L.autotune) {
@@ -626,7 +688,7 @@ cudaError_t fft_vectors(Launcher &L, uint32_t *data, const uint32_t *tw, uint32_
         }
     }
     if (L.forced_plan) plan = *L.forced_plan;
-    if (!plan_valid(plan, log_len)) return cudaErrorInvalidValue;
+    if (!plan_valid(plan, log_len) || (src && plan.ks[0] > kMaxRsFirst)) return cudaErrorInvalidValue;
     const uint32_t np = plan.np;
     std::vector<uint32_t> ks(plan.ks, plan.ks + np);
     std::vector<uint32_t> d0s(np);
@@ -663,16 +725,17 @@ cudaError_t fft_vectors(Launcher &L, uint32_t *data, const uint32_t *tw, uint32_
         a.dtab = reinterpret_cast<const uint4 *>(dtab + (size_t)p * 63 * kTabWords);
         a.src = (src && p == 0) ? src->p : nullptr;
         a.src_col_stride = src ? src->col_stride : 0;
-        a.src_q_stride = src ? src->q_stride : 0;
+        a.src_q_stride = 0;
+        a.pis = a.src ? src->pis : nullptr;
         a.L = log_len; a.d0 = d0; a.log_S = log_len - d0 - K;
-        a.log_nvec_p2 = ilog2u(nvec_p2); a.nvec = nvec; a.root_base = root_base;
+        a.nvec = nvec; a.root_base = root_base; a.fault = L.fault;
         const bool tail = a.log_S == 0 && K >= 4 && aligned;
         {
             // every vector read (the source once when all Q subtrees share
             // it) and written once; one product per butterfly and stage
             const double words = (double)Q * nvec * (1ull << log_len);
-            const double rd = (a.src && src->q_stride == 0) ? words / Q : words;
-            L.note(4.0 * (rd + words), words / 2 * K);
+            if (a.src) L.note(4.0 * (words / Q + words), words / Q + words / 2 * K);
+            else L.note(8.0 * words, words / 2 * K);
         }
         if (tail) {
             a.vchunk = std::min<uint32_t>(nvec, kTailChunk);
@@ -684,13 +747,17 @@ cudaError_t fft_vectors(Launcher &L, uint32_t *data, const uint32_t *tw, uint32_
             if (e != cudaSuccess) return e;
             continue;
         }
-        const uint64_t G = (uint64_t)nvec_p2 << a.log_S;  // threads per (q, P)
-        const uint32_t B = (uint32_t)std::max<uint64_t>(32, std::min<uint64_t>(G, 256));
-        a.log_B = ilog2u(B);
-        a.log_bpg = ilog2u(G / B);
-        a.units = ((uint64_t)Q << d0) << a.log_bpg;
+        const uint64_t G = (uint64_t)nvec << a.log_S;  // pencils per (q, P)
+        const uint32_t B = (uint32_t)std::max<uint64_t>(32, std::min<uint64_t>((uint64_t)nvec_p2 << a.log_S, 256));
+        a.bpg = (uint32_t)((G + B - 1) / B);
+        a.units = a.src ? a.bpg : ((uint64_t)Q << d0) * a.bpg;  // k_rs_first: all quarters in a unit
         a.nchunks = 0;
-        cudaError_t e = inverse ? launch_pass<true>(L, (int)K, a, B) : launch_pass<false>(L, (int)K, a, B);
+        const bool src_aligned = !a.src || ((uintptr_t)a.src % 16 == 0 && a.src_col_stride % 4 == 0);
+        // rows of at least 32 words: below that a bulk copy moves too little
+        a.bulk = aligned && src_aligned && a.log_S >= 5;
+        cudaError_t e = a.src     ? launch_rs_first(L, (int)K, a, B)
+                        : inverse ? launch_pass<true>(L, (int)K, a, B)
+                                  : launch_pass<false>(L, (int)K, a, B);
         if (e != cudaSuccess) return e;
     }
     return cudaSuccess;
@@ -2049,7 +2116,7 @@ cudaError_t tune_fft(Launcher &L, const TuneKey &k, uint32_t *data, const uint32
     (void)data;
     const uint64_t n = 1ull << k.log_len;
     const uint64_t extent = (uint64_t)(k.nvec - 1) * col_stride + (uint64_t)(k.Q - 1) * q_stride + n;
-    const uint64_t src_extent = src ? (uint64_t)(k.nvec - 1) * src->col_stride + (uint64_t)(k.Q - 1) * src->q_stride + n : 0;
+    const uint64_t src_extent = src ? (uint64_t)(k.nvec - 1) * src->col_stride + n : 0;
     uint32_t *sd = nullptr, *ss = nullptr;
     if (cudaMallocAsync(&sd, 4 * extent, L.stream) != cudaSuccess ||
         (src && cudaMallocAsync(&ss, 4 * src_extent, L.stream) != cudaSuccess)) {
@@ -2074,6 +2141,7 @@ cudaError_t tune_fft(Launcher &L, const TuneKey &k, uint32_t *data, const uint32
     float best_ms = 1e30f;
     cudaError_t err = cudaSuccess;
     for (const FftPlan &c : fft_candidates(k.log_len)) {
+        if (src && c.ks[0] > kMaxRsFirst) continue;
         L.forced_plan = &c;
         float ms = 1e30f;
         for (int rep = 0; rep < 3 && err == cudaSuccess; ++rep) {

@@ -48,6 +48,10 @@ struct Launcher {
     // device words, owned by the context and zero between launches: block
     // tickets of kernels whose last block to finish does the final step
     uint32_t *tickets = nullptr;
+    // a word of pinned host memory, owned by the context: a kernel whose wait
+    // for one of its copies gave up sets it, and the context reports it at
+    // its next synchronisation
+    uint32_t *fault = nullptr;
     struct DtabKey {
         const uint32_t *tw = nullptr;
         uint32_t log_len = 0, root_base = 0, plan = 0;
@@ -133,11 +137,6 @@ std::string tuned_choices();
 // copies, so quarter q then needs the m-point FFT under heap node 4+q.
 cudaError_t rs_scale_spread(Launcher &L, const uint32_t *poly, const uint32_t *pis, uint32_t *E,
                             uint32_t log_m, uint32_t n);
-// The same scaling without the spread: out[j*m + i] = poly[j*m + i] * pis[i]
-// (n columns of m), for an FFT whose first pass reads all four quarters'
-// input from it (FftSrc).
-cudaError_t rs_scale(Launcher &L, const uint32_t *poly, const uint32_t *pis, uint32_t *out, uint32_t log_m,
-                     uint32_t n);
 
 // In-place additive FFT / IFFT (src/binary_fft.rs:109-206) of `nvec * Q`
 // vectors of 2^log_len: vector (j, q) starts at data + j*col_stride +
@@ -149,13 +148,16 @@ cudaError_t rs_scale(Launcher &L, const uint32_t *poly, const uint32_t *pis, uin
 // last; forward only) -- vectors are independent, so a caller may run the
 // head passes on column groups as they arrive and the last pass on larger
 // batches.
-// src: where the first pass reads its input instead of data (vector (j, q)
-// at src + j*col_stride + q*q_stride; q_stride 0 lets all Q subtrees start
-// from one copy); the first pass must then be a strided pass (log_len > 6).
+// src: a Reed-Solomon encoding (Q = 4 under root_base 4): the first pass
+// reads column j's words at src.p + j*col_stride, scales row i by pis[i] and
+// runs its stages for all four quarters; it must be a strided pass (log_len >
+// 6) of at most kMaxRsFirst stages.
 enum FftPasses { FFT_ALL = 0, FFT_HEAD = 1, FFT_LAST = 2 };
+constexpr uint32_t kMaxRsFirst = 5;
 struct FftSrc {
     const uint32_t *p = nullptr;
-    uint64_t col_stride = 0, q_stride = 0;
+    uint64_t col_stride = 0;
+    const uint32_t *pis = nullptr;
 };
 cudaError_t fft_vectors(Launcher &L, uint32_t *data, const uint32_t *tw, uint32_t log_len,
                         uint32_t nvec, uint64_t col_stride, uint32_t Q, uint64_t q_stride,
