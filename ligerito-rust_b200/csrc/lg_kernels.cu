@@ -764,82 +764,70 @@ cudaError_t fft_vectors(Launcher &L, uint32_t *data, const uint32_t *tw, uint32_
 }
 
 // =============================================================== Merkle
+// a tree node (or chaining value): 8 words, two 16-byte accesses
+__device__ __forceinline__ void load_node(const uint32_t *p, uint32_t (&h)[8]) {
+    const uint4 x = reinterpret_cast<const uint4 *>(p)[0], y = reinterpret_cast<const uint4 *>(p)[1];
+    h[0] = x.x; h[1] = x.y; h[2] = x.z; h[3] = x.w; h[4] = y.x; h[5] = y.y; h[6] = y.z; h[7] = y.w;
+}
+__device__ __forceinline__ void store_node(uint32_t *p, const uint32_t (&h)[8]) {
+    reinterpret_cast<uint4 *>(p)[0] = make_uint4(h[0], h[1], h[2], h[3]);
+    reinterpret_cast<uint4 *>(p)[1] = make_uint4(h[4], h[5], h[6], h[7]);
+}
+
 // Leaf = the row's n words as LE bytes, one BLAKE3 chunk (n <= 256):
 // blocks of 16 words, CHUNK_START on the first, CHUNK_END|ROOT on the last.
-__global__ void k_leaf_hash(const uint32_t *__restrict__ E, uint64_t rows, uint32_t ncols,
-                            uint32_t *__restrict__ out, uint32_t one, uint64_t e_stride, uint64_t out_stride) {
+// A thread hashes blocks b0 .. b0 + nb_run - 1 of one row's leaf, from the IV
+// or from the chaining value an earlier call left in out.  Bound by the
+// compression (lg_device.cuh); a whole block's 16 loads take one
+// multiply-add each for their address and no predicate.
+__global__ void __launch_bounds__(128) k_leaf_hash(const uint32_t *__restrict__ E, uint64_t rows, uint32_t ncols,
+                                                   uint32_t b0, uint32_t nb_run, uint32_t *__restrict__ out,
+                                                   uint64_t e_stride, uint64_t out_stride) {
     pdl_begin();
     E += blockIdx.y * e_stride;  // lockstep batch: proof blockIdx.y
     out += blockIdx.y * out_stride;
     const uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
     if (i >= rows) return;
-    const uint32_t nb = (ncols + 15) / 16;
+    const uint32_t nb = (ncols + 15) / 16, rows4 = (uint32_t)(4 * rows);  // a column is < 4 GiB
     uint32_t cv[8];
-    b3_iv(cv);
-    for (uint32_t b = 0; b < nb; ++b) {
+    if (b0 == 0) b3_iv(cv);
+    else load_node(out + 8 * i, cv);
+    const uint32_t *p = E + 16ull * b0 * rows + i;
+    for (uint32_t b = b0; b < b0 + nb_run; ++b, p += 16 * rows) {
         uint32_t m[16];
+        if (16 * (b + 1) <= ncols) {
 #pragma unroll
-        for (int w = 0; w < 16; ++w) {
-            const uint32_t j = b * 16 + w;
-            m[w] = j < ncols ? __ldg(E + (uint64_t)j * rows + i) : 0u;
+            for (uint32_t w = 0; w < 16; ++w) m[w] = __ldg(strided(p, w, rows4));
+        } else {
+#pragma unroll
+            for (uint32_t w = 0; w < 16; ++w) m[w] = b * 16 + w < ncols ? __ldg(strided(p, w, rows4)) : 0u;
         }
         const bool last = b + 1 == nb;
         const uint32_t blen = last ? 4 * ncols - 64 * (nb - 1) : 64;
         const uint32_t flags = (b == 0 ? B3_CHUNK_START : 0u) | (last ? (B3_CHUNK_END | B3_ROOT) : 0u);
-        b3_compress(cv, m, blen, flags, one);
+        b3_compress(cv, m, blen, flags);
     }
-    uint4 *o = reinterpret_cast<uint4 *>(out + 8 * i);
-    o[0] = make_uint4(cv[0], cv[1], cv[2], cv[3]);
-    o[1] = make_uint4(cv[4], cv[5], cv[6], cv[7]);
-}
-
-__global__ void k_leaf_block(const uint32_t *__restrict__ E, uint64_t rows, uint32_t ncols, uint32_t b0,
-                             uint32_t nb_run, uint32_t *__restrict__ out, uint32_t one) {
-    pdl_begin();
-    const uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
-    if (i >= rows) return;
-    const uint32_t nb = (ncols + 15) / 16;
-    uint4 *o = reinterpret_cast<uint4 *>(out + 8 * i);
-    uint32_t cv[8];
-    if (b0 == 0) {
-        b3_iv(cv);
-    } else {
-        const uint4 x = o[0], y = o[1];
-        cv[0] = x.x; cv[1] = x.y; cv[2] = x.z; cv[3] = x.w;
-        cv[4] = y.x; cv[5] = y.y; cv[6] = y.z; cv[7] = y.w;
-    }
-    for (uint32_t b = b0; b < b0 + nb_run; ++b) {
-        uint32_t m[16];
-#pragma unroll
-        for (int w = 0; w < 16; ++w) {
-            const uint32_t j = b * 16 + w;
-            m[w] = j < ncols ? __ldg(E + (uint64_t)j * rows + i) : 0u;
-        }
-        const bool last = b + 1 == nb;
-        const uint32_t blen = last ? 4 * ncols - 64 * (nb - 1) : 64;
-        const uint32_t flags = (b == 0 ? B3_CHUNK_START : 0u) | (last ? (B3_CHUNK_END | B3_ROOT) : 0u);
-        b3_compress(cv, m, blen, flags, one);
-    }
-    o[0] = make_uint4(cv[0], cv[1], cv[2], cv[3]);
-    o[1] = make_uint4(cv[4], cv[5], cv[6], cv[7]);
+    store_node(out + 8 * i, cv);
 }
 
 cudaError_t leaf_hash_block(Launcher &L, const uint32_t *E, uint64_t rows, uint32_t ncols, uint32_t b0,
                             uint32_t nb, uint32_t *out) {
-    if (ncols == 0 || ncols > 256 || nb == 0 || b0 + nb > (ncols + 15) / 16) return cudaErrorInvalidValue;
+    if (ncols == 0 || ncols > 256 || nb == 0 || b0 + nb > (ncols + 15) / 16 || rows >= (1ull << 30))
+        return cudaErrorInvalidValue;
     const unsigned blocks = (unsigned)((rows + 127) / 128);
     const uint32_t cols = std::min<uint32_t>(16 * nb, ncols - 16 * b0);
     L.note((double)rows * (4.0 * cols + (b0 ? 64.0 : 32.0)), 0, (double)rows * nb);
-    LGK_LAUNCH(L, "leaf_hash_block", launch_k(k_leaf_block, blocks, 128, 0, L.stream, E, rows, ncols, b0, nb, out, 1u));
+    LGK_LAUNCH(L, "leaf_hash_block", launch_k(k_leaf_hash, blocks, 128, 0, L.stream, E, rows, ncols, b0, nb, out, 0, 0));
     return cudaGetLastError();
 }
 
 cudaError_t leaf_hashes(Launcher &L, const uint32_t *E, uint64_t rows, uint32_t ncols, uint32_t *out, uint32_t B,
                         uint64_t e_stride, uint64_t out_stride) {
-    if (B == 0 || B > 65535) return cudaErrorInvalidValue;
+    if (B == 0 || B > 65535 || ncols == 0 || rows >= (1ull << 30)) return cudaErrorInvalidValue;
+    const uint32_t nb = (ncols + 15) / 16;
     const dim3 blocks((unsigned)((rows + 127) / 128), B);
-    L.note((double)B * rows * (4.0 * ncols + 32.0), 0, (double)B * rows * ((ncols + 15) / 16));
-    LGK_LAUNCH(L, "leaf_hash", launch_k(k_leaf_hash, blocks, 128, 0, L.stream, E, rows, ncols, out, 1u, e_stride,
+    L.note((double)B * rows * (4.0 * ncols + 32.0), 0, (double)B * rows * nb);
+    LGK_LAUNCH(L, "leaf_hash", launch_k(k_leaf_hash, blocks, 128, 0, L.stream, E, rows, ncols, 0, nb, out, e_stride,
                                         out_stride));
     return cudaGetLastError();
 }
@@ -847,13 +835,14 @@ cudaError_t leaf_hashes(Launcher &L, const uint32_t *E, uint64_t rows, uint32_t 
 // Node = blake3(left || right): one 64-byte block, CHUNK_START|CHUNK_END|ROOT
 // (src/merkle_tree.rs:42-51).  A block reduces 2^c consecutive nodes of one
 // layer through c layers in shared memory and writes every layer it makes.
-__device__ __forceinline__ void hash_node(const uint32_t *l, const uint32_t *r, uint32_t *o, uint32_t one) {
+template <bool MA = true>
+__device__ __forceinline__ void hash_node(const uint32_t *l, const uint32_t *r, uint32_t *o) {
     uint32_t m[16];
 #pragma unroll
     for (int w = 0; w < 8; ++w) { m[w] = l[w]; m[8 + w] = r[w]; }
     uint32_t cv[8];
     b3_iv(cv);
-    b3_compress(cv, m, 64, B3_CHUNK_START | B3_CHUNK_END | B3_ROOT, one);
+    b3_compress<MA>(cv, m, 64, B3_CHUNK_START | B3_CHUNK_END | B3_ROOT);
 #pragma unroll
     for (int w = 0; w < 8; ++w) o[w] = cv[w];
 }
@@ -863,21 +852,12 @@ __device__ __forceinline__ void hash_node(const uint32_t *l, const uint32_t *r, 
 // and hashes the 7 nodes of the three layers above them, keeping at most
 // three pending hashes; every lane does full work, so these launches run
 // at hashing throughput.
-__device__ __forceinline__ void load_node(const uint32_t *p, uint32_t (&h)[8]) {
-    const uint4 x = reinterpret_cast<const uint4 *>(p)[0], y = reinterpret_cast<const uint4 *>(p)[1];
-    h[0] = x.x; h[1] = x.y; h[2] = x.z; h[3] = x.w; h[4] = y.x; h[5] = y.y; h[6] = y.z; h[7] = y.w;
-}
-__device__ __forceinline__ void store_node(uint32_t *p, const uint32_t (&h)[8]) {
-    reinterpret_cast<uint4 *>(p)[0] = make_uint4(h[0], h[1], h[2], h[3]);
-    reinterpret_cast<uint4 *>(p)[1] = make_uint4(h[4], h[5], h[6], h[7]);
-}
-__device__ __forceinline__ void hash_pair(const uint32_t (&l)[8], const uint32_t (&r)[8], uint32_t (&o)[8],
-                                          uint32_t one) {
-    hash_node(l, r, o, one);
+__device__ __forceinline__ void hash_pair(const uint32_t (&l)[8], const uint32_t (&r)[8], uint32_t (&o)[8]) {
+    hash_node(l, r, o);
 }
 
 __global__ void __launch_bounds__(128) k_merkle_thread3(uint32_t *__restrict__ tree, uint64_t in_off, uint64_t n_in,
-                                                        uint32_t one, uint64_t tree_stride) {
+                                                        uint64_t tree_stride) {
     pdl_begin();
     tree += blockIdx.y * tree_stride;  // lockstep batch: proof blockIdx.y
     const uint64_t t = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
@@ -894,7 +874,7 @@ __global__ void __launch_bounds__(128) k_merkle_thread3(uint32_t *__restrict__ t
     load_node(src + 8, r);
 #pragma unroll 1
     for (uint32_t i = 0; i < 7; ++i) {
-        hash_pair(l, r, h, one);
+        hash_pair(l, r, h);
         const uint64_t at = (i == 6)                ? off3 + t
                             : (i == 2 || i == 5)    ? off2 + 2 * t + (i == 5)
                                                     : off1 + 4 * t + (i < 2 ? i : i - 1);
@@ -937,7 +917,7 @@ constexpr uint32_t kNarrowNodes = 512, kNarrowMax = kNarrowNodes * kNarrowNodes;
 // src_tree: the first layer is read from the tree with loads that bypass
 // L1 (nodes other blocks wrote).  Ends with the block synchronised.
 __device__ __forceinline__ void narrow_climb(uint32_t *__restrict__ tree, uint64_t off, uint64_t n, uint64_t first,
-                                             uint32_t m, uint32_t *buf_a, uint32_t *buf_b, uint32_t one) {
+                                             uint32_t m, uint32_t *buf_a, uint32_t *buf_b) {
     const uint32_t t = threadIdx.x;
     if (t < m / 2) {
         uint32_t l[8], r[8], h[8];
@@ -945,7 +925,7 @@ __device__ __forceinline__ void narrow_climb(uint32_t *__restrict__ tree, uint64
         const uint4 a0 = __ldcg(pl), a1 = __ldcg(pl + 1), b0 = __ldcg(pl + 2), b1 = __ldcg(pl + 3);
         l[0] = a0.x; l[1] = a0.y; l[2] = a0.z; l[3] = a0.w; l[4] = a1.x; l[5] = a1.y; l[6] = a1.z; l[7] = a1.w;
         r[0] = b0.x; r[1] = b0.y; r[2] = b0.z; r[3] = b0.w; r[4] = b1.x; r[5] = b1.y; r[6] = b1.z; r[7] = b1.w;
-        hash_pair(l, r, h, one);
+        hash_pair(l, r, h);
         store_node(tree + 8 * (off + n + first / 2 + t), h);
 #pragma unroll
         for (int j = 0; j < 8; ++j) buf_a[j * (kNarrowNodes / 2) + t] = h[j];
@@ -966,7 +946,7 @@ __device__ __forceinline__ void narrow_climb(uint32_t *__restrict__ tree, uint64
                 l[j] = x.x;
                 r[j] = x.y;
             }
-            hash_pair(l, r, h, one);
+            hash_pair(l, r, h);
             store_node(tree + 8 * (off + n + first / 2 + t), h);
 #pragma unroll
             for (int j = 0; j < 8; ++j) dst[j * ds + t] = h[j];
@@ -986,7 +966,7 @@ __device__ __forceinline__ void narrow_climb(uint32_t *__restrict__ tree, uint64
 }
 
 __global__ void __launch_bounds__(256) k_merkle_narrow(uint32_t *__restrict__ tree, uint64_t in_off, uint64_t n_in,
-                                                       uint32_t *ticket, uint32_t one, uint64_t tree_stride) {
+                                                       uint32_t *ticket, uint64_t tree_stride) {
     pdl_begin();
     tree += blockIdx.y * tree_stride;  // lockstep batch: proof blockIdx.y, its own ticket
     ticket += blockIdx.y;
@@ -996,7 +976,7 @@ __global__ void __launch_bounds__(256) k_merkle_narrow(uint32_t *__restrict__ tr
     __shared__ __align__(16) uint32_t buf_b[8 * (kNarrowNodes / 4)];
     __shared__ uint32_t last;
     const uint32_t per = (uint32_t)(n_in < kNarrowNodes ? n_in : kNarrowNodes), nb = gridDim.x;
-    narrow_climb(tree, in_off, n_in, (uint64_t)blockIdx.x * per, per, buf_a, buf_b, one);
+    narrow_climb(tree, in_off, n_in, (uint64_t)blockIdx.x * per, per, buf_a, buf_b);
     if (nb == 1) return;
     // the layer of the blocks' roots
     uint64_t off = in_off, n = n_in;
@@ -1007,7 +987,7 @@ __global__ void __launch_bounds__(256) k_merkle_narrow(uint32_t *__restrict__ tr
     if (!last) return;
     __threadfence();
     if (threadIdx.x == 0) *ticket = 0;  // ready for the next launch on the stream
-    narrow_climb(tree, off, n, 0, nb, buf_a, buf_b, one);
+    narrow_climb(tree, off, n, 0, nb, buf_a, buf_b);
 }
 
 cudaError_t merkle_upper(Launcher &L, uint32_t *tree, uint64_t num_leaves, uint32_t B, uint64_t tree_stride) {
@@ -1023,14 +1003,14 @@ cudaError_t merkle_upper(Launcher &L, uint32_t *tree, uint64_t num_leaves, uint3
             const uint64_t threads = n / 8;
             L.note(32.0 * B * (n + n / 2 + n / 4 + n / 8), (double)0, (double)B * (n / 2 + n / 4 + n / 8));
             LGK_LAUNCH(L, "merkle_thread3", launch_k(k_merkle_thread3, dim3((unsigned)((threads + 127) / 128), B), 128,
-                                                     0, L.stream, tree, off, n, 1u, tree_stride));
+                                                     0, L.stream, tree, off, n, tree_stride));
             e = cudaGetLastError();
             for (int l = 0; l < 3; ++l) { off += n; n /= 2; }
         } else {
             const uint64_t per = std::min<uint64_t>(n, kNarrowNodes);
             L.note(32.0 * B * (2 * n - 1), 0, (double)B * (n - 1));
             LGK_LAUNCH(L, "merkle_narrow", launch_k(k_merkle_narrow, dim3((unsigned)(n / per), B), 256, 0, L.stream,
-                                                    tree, off, n, L.tickets, 1u, tree_stride));
+                                                    tree, off, n, L.tickets, tree_stride));
             e = cudaGetLastError();
             n = 1;
         }
@@ -1876,7 +1856,7 @@ cudaError_t induce_fused(Launcher &L, const InducePlan &p, const uint32_t *d_row
 __global__ void __launch_bounds__(256) k_opening_check(const uint32_t *__restrict__ rows, uint32_t ncols,
                                                        const uint64_t *__restrict__ q, uint32_t nq,
                                                        const uint32_t *__restrict__ proof, uint32_t depth,
-                                                       uint32_t *__restrict__ out, uint32_t one) {
+                                                       uint32_t *__restrict__ out) {
     pdl_begin();
     __shared__ uint32_t h[256][8];
     __shared__ uint64_t qs[256];
@@ -1896,7 +1876,7 @@ __global__ void __launch_bounds__(256) k_opening_check(const uint32_t *__restric
             const bool last = b + 1 == nb;
             const uint32_t blen = last ? 4 * ncols - 64 * (nb - 1) : 64;
             const uint32_t flags = (b == 0 ? B3_CHUNK_START : 0u) | (last ? (B3_CHUNK_END | B3_ROOT) : 0u);
-            b3_compress(cv, m, blen, flags, one);
+            b3_compress<false>(cv, m, blen, flags);
         }
 #pragma unroll
         for (int w = 0; w < 8; ++w) h[t][w] = cv[w];
@@ -1929,13 +1909,13 @@ __global__ void __launch_bounds__(256) k_opening_check(const uint32_t *__restric
             if (paired) {
 #pragma unroll
                 for (int w = 0; w < 8; ++w) other[w] = h[t + 1][w];
-                hash_node(mine, other, parent, one);
+                hash_node<false>(mine, other, parent);
             } else {
                 const uint32_t *nd = proof + 8ull * (pc_base + pidx);
 #pragma unroll
                 for (int w = 0; w < 8; ++w) other[w] = nd[w];
-                if (qi & 1) hash_node(other, mine, parent, one);
-                else hash_node(mine, other, parent, one);
+                if (qi & 1) hash_node<false>(other, mine, parent);
+                else hash_node<false>(mine, other, parent);
             }
         }
         __syncthreads();
@@ -1955,7 +1935,7 @@ cudaError_t opening_check(Launcher &L, const uint32_t *rows, uint32_t ncols, con
                           const uint32_t *proof, uint32_t depth, uint32_t *out) {
     if (nq == 0 || nq > 256 || ncols == 0 || ncols > 256 || depth > 63) return cudaErrorInvalidValue;
     LGK_LAUNCH(L, "opening_check", launch_k(k_opening_check, 1, 256, 0, L.stream, rows, ncols, q, nq, proof, depth,
-                                            out, 1u));
+                                            out));
     return cudaGetLastError();
 }
 
