@@ -717,16 +717,9 @@ void prove_impl(lg_ctx *c, Scratch &sc, const lg_config &cfg, const uint32_t *d_
     dump_dev(c, "enforced_sum", 0, t + 3, 4);
     w0.E.reset();
     w0.tree.reset();
-    uint32_t *r = next_chal(1);
-    // SumcheckProverInstance::new, then :93 (src/ligerito.rs:35) and the
-    // first challenge of :97
-    const lgk::FsTail t0 = tail(true, 1, r);
-    CK(c, lgk::eval013(c->L, f.u32(), B.u32(), fv, t, &t0));
-    dump_triple(t);
-
     DBuf f2(c, 4ull << (fv - 1)), B2(c, 4ull << (fv - 1));
+    DBuf bi;  // the basis a step starts by gluing into B (none at the first)
     for (uint32_t i = 0; i < steps; ++i) {
-        const uint32_t *rs = r;  // this step's ks[i] round challenges are consecutive
         // The last commitment is final here: a side stream brings its matrix
         // and tree to the host during this step's rounds, so the final
         // opening needs no second round trip (when they are small and the
@@ -745,9 +738,48 @@ void prove_impl(lg_ctx *c, Scratch &sc, const lg_config &cfg, const uint32_t *d_
             CK(c, cudaMemcpyAsync(h + eb, wprev.tree.p, tb, cudaMemcpyDeviceToHost, c->copy_stream));
             CK(c, cudaEventRecord(c->copy_ev[6], c->copy_stream));
         }
-        for (uint32_t k = 0; k < cfg.ks[i]; ++k) {  // :97-102
+        // The step's opening triple: SumcheckProverInstance::new, then :93
+        // (src/ligerito.rs:35) and the first challenge of :97; or
+        // introduce_new, :187-193 (src/ligerito.rs:52), the glue challenge,
+        // then the first round challenge, and the glue.  A step small enough
+        // runs in one launch with its rounds; a larger one's last rounds do.
+        const uint32_t nsq = i ? 2 : 1, rounds = cfg.ks[i];
+        uint32_t *ec = next_chal(nsq);
+        uint32_t *r = ec + nsq - 1;
+        const uint32_t *rs = r;  // this step's ks[i] round challenges are consecutive
+        const bool whole = !c->dump_cb && lgk::sum_step_fits(fv, rounds, 1, i > 0);
+        if (!whole) {
+            const lgk::FsTail te = tail(true, nsq, ec);
+            CK(c, lgk::eval013(c->L, f.u32(), i ? bi.u32() : B.u32(), fv, t, &te));
+            dump_triple(t);
+            if (i) {
+                CK(c, lgk::axpy(c->L, B.u32(), bi.u32(), fv, 0, ec));
+                dump_dev(c, "beta", i, ec, 4);
+                dump_dev(c, "basis_sum", i, B.p, 4ull << fv);
+            }
+        }
+        for (uint32_t k = 0; k < rounds;) {  // :97-102
+            const bool rest = whole || (!c->dump_cb && lgk::sum_step_fits(fv, rounds - k, 1, false));
+            if (rest) {
+                lgk::SumStep s;
+                s.f = f.u32(); s.B = B.u32(); s.bi = whole && i ? bi.u32() : nullptr;
+                s.log_len = fv; s.rounds = rounds - k;
+                s.eval = whole; s.nsq = nsq;
+                s.tri = whole ? t : next_tri();
+                for (uint32_t j = whole ? 0 : 1; j < s.rounds; ++j) next_tri();
+                s.chal = whole ? ec : r;
+                next_chal(s.rounds - 1);
+                s.fo = f2.u32(); s.Bo = B2.u32(); s.fs = fs;
+                CK(c, lgk::sum_step(c->L, s));
+                std::swap(f, f2);
+                std::swap(B, B2);
+                fv -= s.rounds;
+                round_no += s.rounds;
+                k = rounds;
+                continue;
+            }
             t = next_tri();
-            const bool more = k + 1 < cfg.ks[i];
+            const bool more = ++k < rounds;
             uint32_t *rn = more ? next_chal(1) : nullptr;
             const lgk::FsTail tk = tail(false, more ? 1 : 0, rn);
             CK(c, lgk::fold_round(c->L, f.u32(), B.u32(), fv, 0, f2.u32(), B2.u32(), t, r, &tk));
@@ -797,22 +829,12 @@ void prove_impl(lg_ctx *c, Scratch &sc, const lg_config &cfg, const uint32_t *d_
         root_m = root_later(&P.recursive_roots[i + 1]);
         uint32_t *al = next_chal(1);
         auto op = open_rows_dev(c, sc, wprev, fs, wn.root(), 1, al, &P.recursive[i], root_m);  // :156-172
-        DBuf bi(c, 4ull << fv);
+        bi = DBuf(c, 4ull << fv);
         t = next_tri();
         induce_dev(c, sc, fv, op.first, LG_NUM_QUERIES, nullptr, cfg.ks[i], op.second, 0, bi.u32(), t + 3, rs, al);
         dump_opening(i + 1, op, wprev.cols, al);
         dump_dev(c, "basis", i + 1, bi.p, 4ull << fv);
         dump_dev(c, "enforced_sum", i + 1, t + 3, 4);
-        // introduce_new, :187-193 (src/ligerito.rs:52): the glue challenge,
-        // then the next step's first round challenge
-        uint32_t *beta = next_chal(2);
-        const lgk::FsTail ti = tail(true, 2, beta);
-        CK(c, lgk::eval013(c->L, f.u32(), bi.u32(), fv, t, &ti));
-        dump_triple(t);
-        r = beta + 1;
-        CK(c, lgk::axpy(c->L, B.u32(), bi.u32(), fv, 0, beta));  // glue
-        dump_dev(c, "beta", i + 1, beta, 4);
-        dump_dev(c, "basis_sum", i + 1, B.p, 4ull << fv);
         wprev = std::move(wn);
     }
     throw ProverAssert{};  // :198
@@ -1068,16 +1090,42 @@ void prove_batch_impl(lg_ctx *c, Scratch &sc, const lg_config &cfg, const uint32
                  B);  // :78-85
     w0.E.reset();
     w0.tree.reset();
-    uint32_t *r = next_chal(1);
-    const lgk::FsTail t0 = tail(true, 1, r);
-    CK(c, lgk::eval013(c->L, f.u32(), Bv.u32(), fv, t, &t0, B, rstr(fv)));
 
     DBuf f2(c, (4ull << (fv - 1)) * B), B2(c, (4ull << (fv - 1)) * B);
+    DBuf bi;
     for (uint32_t i = 0; i < steps; ++i) {
+        const uint32_t nsq = i ? 2 : 1, rounds = cfg.ks[i];
+        uint32_t *ec = next_chal(nsq);
+        uint32_t *r = ec + nsq - 1;
         const uint32_t *rs = r;
-        for (uint32_t k = 0; k < cfg.ks[i]; ++k) {  // :97-102
+        const bool whole = lgk::sum_step_fits(fv, rounds, B, i > 0);
+        if (!whole) {
+            const lgk::FsTail te = tail(true, nsq, ec);
+            CK(c, lgk::eval013(c->L, f.u32(), i ? bi.u32() : Bv.u32(), fv, t, &te, B, rstr(fv)));
+            if (i) CK(c, lgk::axpy(c->L, Bv.u32(), bi.u32(), fv, 0, ec, B, rstr(fv)));  // glue
+        }
+        for (uint32_t k = 0; k < rounds;) {  // :97-102
+            if (whole || lgk::sum_step_fits(fv, rounds - k, B, false)) {
+                lgk::SumStep s;
+                s.f = f.u32(); s.B = Bv.u32(); s.bi = whole && i ? bi.u32() : nullptr;
+                s.log_len = fv; s.rounds = rounds - k;
+                s.eval = whole; s.nsq = nsq;
+                s.tri = whole ? t : next_tri();
+                for (uint32_t j = whole ? 0 : 1; j < s.rounds; ++j) next_tri();
+                s.chal = whole ? ec : r;
+                next_chal(s.rounds - 1);
+                s.fo = f2.u32(); s.Bo = B2.u32(); s.fs = fs;
+                lgk::RoundStrides st = rstr(fv);
+                st.fo = st.go = 1ull << (fv - s.rounds);
+                CK(c, lgk::sum_step(c->L, s, B, st));
+                std::swap(f, f2);
+                std::swap(Bv, B2);
+                fv -= s.rounds;
+                k = rounds;
+                continue;
+            }
             t = next_tri();
-            const bool more = k + 1 < cfg.ks[i];
+            const bool more = ++k < rounds;
             uint32_t *rn = more ? next_chal(1) : nullptr;
             const lgk::FsTail tk = tail(false, more ? 1 : 0, rn);
             CK(c, lgk::fold_round(c->L, f.u32(), Bv.u32(), fv, 0, f2.u32(), B2.u32(), t, r, &tk, B, rstr(fv)));
@@ -1126,15 +1174,9 @@ void prove_batch_impl(lg_ctx *c, Scratch &sc, const lg_config &cfg, const uint32
         uint32_t *al = next_chal(1);
         BatchOpened o = open_rows_batch(c, sc, wprev, fs, wn.root(), wn.t_stride(), 1, al, CH,
                                         each([ii](lg::Proof *p) { return &p->recursive[ii]; }), root_m);  // :156-172
-        DBuf bi(c, (4ull << fv) * B);
+        bi = DBuf(c, (4ull << fv) * B);
         t = next_tri();
         induce_batch(c, sc, fv, o.rows, o.stride, nq, cfg.ks[i], o.q, bi.u32(), t + 3, TR, rs, al, CH, B);
-        uint32_t *beta = next_chal(2);
-        const lgk::FsTail ti = tail(true, 2, beta);
-        CK(c, lgk::eval013(c->L, f.u32(), bi.u32(), fv, t, &ti, B, rstr(fv)));
-        r = beta + 1;
-        lgk::RoundStrides ax = rstr(fv);
-        CK(c, lgk::axpy(c->L, Bv.u32(), bi.u32(), fv, 0, beta, B, ax));  // glue
         wprev = std::move(wn);
     }
     throw ProverAssert{};  // :198

@@ -1359,6 +1359,214 @@ cudaError_t axpy(Launcher &L, uint32_t *B, const uint32_t *bi, uint32_t log_len,
     return cudaGetLastError();
 }
 
+// A whole sumcheck step, or its last rounds, in one launch: a cluster of C
+// blocks keeps f and the basis in its shared memory, evaluates the step's
+// opening triple and folds round after round, and warp 0 of its first block
+// runs the transcript between them.
+//   * Block c holds the words whose index modulo M = 2^(log_len - rounds - 1)
+//     lies in [c M / C, (c+1) M / C): every fold and every triple pairs words
+//     that differ in a higher bit, so no round moves data between blocks.
+//   * A round is one product table, the folds and products, an XOR reduction,
+//     two cluster barriers (the blocks' partial triples to the first block,
+//     its challenge back) and the transcript's one or two SHA-256
+//     compressions.
+// Bound by that chain's latency: a step of 2^10 words (opening triple and four
+// rounds) takes 29 us in one launch, 54 us as five (event-timed), one of 2^14
+// with its glue 33 against 70 us as six.
+struct SumStepArgs {
+    const uint32_t *f, *B, *bi;  // bi: the basis to glue into B (after the opening triple), or null
+    uint32_t log_len, rounds;
+    uint32_t eval, nsq;          // eval: opening triple over (f, bi or B), checked against tri[3], then nsq challenges
+    uint32_t *tri;               // 4 words a triple: the opening one's, then one a round
+    uint32_t *chal;              // the opening's challenges and the rounds' after them; !eval: the first round's is there
+    uint32_t *fo, *Bo;           // 2^(log_len - rounds) words
+    FsState *fs;
+};
+// in shared memory, without its words
+struct SumStepShared {
+    FsState S;
+    fsd::Batch batch;
+    uint32_t part[8][4];  // the blocks' partial triples (first block)
+    uint32_t red[8][4];   // the warps'
+    uint32_t r[4];        // the challenges the first block hands out
+};
+constexpr uint32_t kSumThreads = 256;
+__device__ __forceinline__ uint32_t cluster_rank() {
+    uint32_t r;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return r;
+}
+__device__ __forceinline__ void cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+}
+__device__ __forceinline__ void cluster_store(const uint32_t *p, uint32_t rank, uint32_t v) {
+    asm volatile("{\n\t.reg .b32 a;\n\tmapa.shared::cluster.u32 a, %0, %1;\n\tst.shared::cluster.u32 [a], %2;\n\t}" ::"r"(
+                     (uint32_t)__cvta_generic_to_shared(p)),
+                 "r"(rank), "r"(v)
+                 : "memory");
+}
+__global__ void __launch_bounds__(kSumThreads) k_sum_step(SumStepArgs a, RoundStrides st, uint32_t C) {
+    pdl_begin();
+    extern __shared__ __align__(512) uint8_t ssraw[];
+    {
+        const uint32_t b = blockIdx.y;  // lockstep batch: proof b
+        a.f += b * st.f;
+        a.B += b * st.g;
+        if (a.bi) a.bi += b * st.f;
+        a.tri += b * st.acc;
+        a.chal += b * st.out;
+        a.fo += b * st.fo;
+        a.Bo += b * st.go;
+        a.fs += b * st.fs;
+    }
+    uint32_t *T = reinterpret_cast<uint32_t *>(ssraw);  // the table of the challenge
+    SumStepShared &sh = *reinterpret_cast<SumStepShared *>(ssraw + 4 * kTabWords);
+    const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, c = cluster_rank();
+    const uint32_t lw = a.log_len - a.rounds - 1 - (31 - __clz(C)), w = 1u << lw;  // 2^lw words a run of this block
+    uint32_t len = w << (a.rounds + 1);                                            // its words
+    uint32_t *F = reinterpret_cast<uint32_t *>(ssraw + 4 * kTabWords + ((sizeof(SumStepShared) + 15) & ~15u)), *G = F + len;
+    uint32_t *I = G + len;  // bi's words
+    // global index of local word x: run x >> lw, offset x & (w - 1)
+    auto at = [&](uint32_t x) { return (x >> lw << (lw + 31 - __clz(C))) + c * w + (x & (w - 1)); };
+    for (uint32_t x = tid; x < len; x += kSumThreads) {
+        F[x] = a.f[at(x)];
+        G[x] = a.B[at(x)];
+        if (a.bi) I[x] = a.bi[at(x)];
+    }
+    if (c == 0)
+        for (uint32_t i = tid; i < fsd::kFsStateWords; i += kSumThreads)
+            reinterpret_cast<uint32_t *>(&sh.S)[i] = reinterpret_cast<const uint32_t *>(a.fs)[i];
+    cluster_sync();  // the block's words are there, and every block of the cluster has started
+    const uint8_t *t8 = reinterpret_cast<const uint8_t *>(T);
+    // the triple s0, s1, s2 over the whole cluster, absorbed by the first
+    // block (checked against tri[3] if `check`), then nsq challenges; the
+    // last one, and the one before it in beta's place, in sh.r everywhere
+    uint32_t *tri = a.tri, *chal = a.eval ? a.chal : a.chal + 1;
+    auto transcript = [&](uint32_t s0, uint32_t s1, uint32_t s2, bool check, uint32_t nsq) {
+        s0 = __reduce_xor_sync(0xffffffffu, s0);
+        s1 = __reduce_xor_sync(0xffffffffu, s1);
+        s2 = __reduce_xor_sync(0xffffffffu, s2);
+        if (lane == 0) { sh.red[warp][0] = s0; sh.red[warp][1] = s1; sh.red[warp][2] = s2; }
+        __syncthreads();
+        if (tid < 3) {
+            uint32_t x = 0;
+#pragma unroll
+            for (uint32_t i = 0; i < kSumThreads / 32; ++i) x ^= sh.red[i][tid];
+            cluster_store(&sh.part[c][tid], 0, x);
+        }
+        cluster_sync();
+        if (c == 0 && warp == 0) {
+            if (lane < 3) {
+                uint32_t x = 0;
+                for (uint32_t i = 0; i < C; ++i) x ^= sh.part[i][lane];
+                sh.part[0][lane] = x;
+                tri[lane] = x;
+            }
+            __syncwarp();
+            if (lane == 0) {
+                if (check && (sh.part[0][0] ^ sh.part[0][1]) != tri[3]) sh.S.err |= FS_ERR_SUMCHECK;
+                fsd::fs_absorb(sh.S, sh.part[0], 3);
+                fsd::fs_chain(sh.S, sh.batch, nsq);
+            }
+            __syncwarp();
+            uint32_t v = 0;
+            if (lane < nsq) {
+                v = (uint32_t)fsd::fs_squeeze_at(sh.S, sh.batch, lane);
+                chal[lane] = v;
+            }
+            __syncwarp();
+            if (lane == 0) fsd::fs_commit(sh.S, sh.batch, nsq);
+            for (uint32_t i = 0; i < nsq; ++i) {
+                const uint32_t x = __shfl_sync(0xffffffffu, v, i);
+                if (lane < C) cluster_store(&sh.r[i], lane, x);
+            }
+        }
+        tri += 4;
+        chal += nsq;
+        if (nsq) cluster_sync();
+    };
+    auto table = [&](uint32_t x) {  // T = the table of x; the block's words are settled too
+        if (warp == 0) tab_build_warp(T, x, lane);
+        __syncthreads();
+    };
+    uint32_t nsq = 1;
+    if (a.eval) {
+        const uint32_t *g = a.bi ? I : G;
+        uint32_t s0 = 0, s1 = 0, s2 = 0;
+        for (uint32_t x = tid; x < len / 2; x += kSumThreads) {
+            const uint32_t f0 = F[x], f1 = F[len / 2 + x], g0 = g[x], g1 = g[len / 2 + x];
+            s0 ^= gf_mul(f0, g0);
+            s1 ^= gf_mul(f1, g1);
+            s2 ^= gf_mul(at3(f0, f1), at3(g0, g1));
+        }
+        nsq = a.nsq;
+        transcript(s0, s1, s2, true, nsq);
+        if (a.bi) {  // glue: B += beta bi
+            table(sh.r[0]);
+            for (uint32_t x = tid; x < len; x += kSumThreads) G[x] ^= tab_mul_sa(t8, 0, 0, I[x]);
+            __syncthreads();
+        }
+    } else {
+        if (tid == 0) sh.r[0] = *a.chal;
+        __syncthreads();
+    }
+    for (uint32_t k = 0; k < a.rounds; ++k) {
+        table(sh.r[k == 0 ? nsq - 1 : 0]);
+        const uint32_t q = len / 4;
+        uint32_t s0 = 0, s1 = 0, s2 = 0;
+        for (uint32_t i = tid; i < q; i += kSumThreads) {
+            const uint32_t a0 = F[i], a1 = F[q + i], a2 = F[2 * q + i], a3 = F[3 * q + i];
+            const uint32_t c0 = G[i], c1 = G[q + i], c2 = G[2 * q + i], c3 = G[3 * q + i];
+            const uint32_t flo = a0 ^ tab_mul_sa(t8, 0, 0, a0 ^ a2), fhi = a1 ^ tab_mul_sa(t8, 0, 0, a1 ^ a3);
+            const uint32_t blo = c0 ^ tab_mul_sa(t8, 0, 0, c0 ^ c2), bhi = c1 ^ tab_mul_sa(t8, 0, 0, c1 ^ c3);
+            F[i] = flo; F[q + i] = fhi;
+            G[i] = blo; G[q + i] = bhi;
+            s0 ^= gf_mul(flo, blo);
+            s1 ^= gf_mul(fhi, bhi);
+            s2 ^= gf_mul(at3(flo, fhi), at3(blo, bhi));
+        }
+        len /= 2;
+        transcript(s0, s1, s2, false, k + 1 < a.rounds ? 1 : 0);
+    }
+    __syncthreads();
+    for (uint32_t x = tid; x < len; x += kSumThreads) {
+        a.fo[at(x)] = F[x];
+        a.Bo[at(x)] = G[x];
+    }
+    if (c == 0)
+        for (uint32_t i = tid; i < fsd::kFsStateWords; i += kSumThreads)
+            reinterpret_cast<uint32_t *>(a.fs)[i] = reinterpret_cast<const uint32_t *>(&sh.S)[i];
+}
+static size_t sum_step_smem(uint32_t log_len, uint32_t C, bool bi) {
+    return 4 * kTabWords + ((sizeof(SumStepShared) + 15) & ~size_t(15)) + ((bi ? 12ull : 8ull) << log_len) / C;
+}
+// Blocks of a step's cluster: enough that a round gives a thread one or two
+// items, at most 8 (the portable size) and no more than the device's SMs for
+// the whole batch; 0 when the step does not fit.
+static uint32_t sum_step_cluster(uint32_t log_len, uint32_t rounds, uint32_t NB, bool bi) {
+    if (rounds == 0 || log_len < rounds + 1 || log_len > kSumStepMaxLog) return 0;
+    uint32_t C = 1;
+    while (C < 8 && (1ull << (log_len - 2)) / C > kSumThreads && 2 * C * NB <= 148 && (2 * C >> (log_len - rounds - 1)) == 0)
+        C *= 2;
+    return sum_step_smem(log_len, C, bi) <= 200 * 1024 ? C : 0;
+}
+bool sum_step_fits(uint32_t log_len, uint32_t rounds, uint32_t NB, bool glue) {
+    return sum_step_cluster(log_len, rounds, NB, glue) != 0;
+}
+cudaError_t sum_step(Launcher &L, const SumStep &s, uint32_t NB, const RoundStrides &st) {
+    const uint32_t C = sum_step_cluster(s.log_len, s.rounds, NB, s.bi != nullptr);
+    if (C == 0 || NB == 0 || NB > 65535 || s.nsq > 2 || (s.eval && s.nsq == 0)) return cudaErrorInvalidValue;
+    SumStepArgs a;
+    a.f = s.f; a.B = s.B; a.bi = s.bi; a.log_len = s.log_len; a.rounds = s.rounds; a.eval = s.eval; a.nsq = s.nsq;
+    a.tri = s.tri; a.chal = s.chal; a.fo = s.fo; a.Bo = s.Bo; a.fs = s.fs;
+    const size_t smem = sum_step_smem(s.log_len, C, s.bi != nullptr);
+    if (smem > 48 * 1024) cudaFuncSetAttribute(k_sum_step, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+    const double n = (double)NB * (1ull << s.log_len);
+    L.note(12.0 * n, 7.0 * n / 2);
+    LGK_LAUNCH(L, "fold_round", launch_kc(k_sum_step, dim3(C, NB), kSumThreads, C, smem, L.stream, a, st, C));
+    return cudaGetLastError();
+}
+
 // ================================================================ induce
 // basis[t] = sum_k apow[k] prod_{bit i of t} S_k[i]   (t < 2^n)
 //          = sum_k Hi_k[t >> b] * Lo_k[t & (2^b-1)]

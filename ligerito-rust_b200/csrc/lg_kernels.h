@@ -87,20 +87,33 @@ struct Launcher {
 // the previous grid's completion before touching memory.  LG_PDL=0 in the
 // environment turns it off.
 bool pdl_enabled();
+// launch_kc: in clusters of `cluster` blocks along x.
 template <typename... KArgs, typename... Args>
-cudaError_t launch_k(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
-                     Args... args) {
+cudaError_t launch_kc(void (*kernel)(KArgs...), dim3 grid, dim3 block, unsigned cluster, size_t smem,
+                      cudaStream_t stream, Args... args) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = block;
     cfg.dynamicSmemBytes = smem;
     cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchAttribute attr[2];
     cfg.attrs = attr;
-    cfg.numAttrs = pdl_enabled() ? 1 : 0;
+    if (pdl_enabled()) {
+        attr[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[cfg.numAttrs++].val.programmaticStreamSerializationAllowed = 1;
+    }
+    if (cluster) {
+        attr[cfg.numAttrs].id = cudaLaunchAttributeClusterDimension;
+        attr[cfg.numAttrs].val.clusterDim.x = cluster;
+        attr[cfg.numAttrs].val.clusterDim.y = attr[cfg.numAttrs].val.clusterDim.z = 1;
+        ++cfg.numAttrs;
+    }
     return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
+}
+template <typename... KArgs, typename... Args>
+cudaError_t launch_k(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
+                     Args... args) {
+    return launch_kc(kernel, grid, block, 0, smem, stream, args...);
 }
 
 // A kernel launch on L's stream, counted and (when timing) bracketed.
@@ -312,6 +325,25 @@ struct FsTail {
     uint32_t nsq = 0;
     uint32_t *out = nullptr;
 };
+
+// A sumcheck step of at most 2^kSumStepMaxLog words, or its last rounds, in
+// one launch.  eval: first the triple of (f, bi or B) at tri (checked against
+// the enforced sum tri[3]) and nsq challenges at chal; then, with bi, B +=
+// chal[0] * bi.  Then `rounds` folds of f and B by the last of those
+// challenges (!eval: by *chal) and the ones squeezed after each round but the
+// last, each with its triple at the next 4 words of tri.  fo, Bo: 2^(log_len
+// - rounds) words.
+constexpr uint32_t kSumStepMaxLog = 16;
+struct SumStep {
+    const uint32_t *f = nullptr, *B = nullptr, *bi = nullptr;
+    uint32_t log_len = 0, rounds = 0;
+    bool eval = false;
+    uint32_t nsq = 0;
+    uint32_t *tri = nullptr, *chal = nullptr, *fo = nullptr, *Bo = nullptr;
+    FsState *fs = nullptr;
+};
+bool sum_step_fits(uint32_t log_len, uint32_t rounds, uint32_t NB, bool glue);
+cudaError_t sum_step(Launcher &L, const SumStep &s, uint32_t NB = 1, const RoundStrides &st = RoundStrides{});
 
 // Lockstep batches: B transcripts d[0..B), one block each; per-proof
 // strides of the step / query arguments' buffers (in their elements).
