@@ -50,7 +50,7 @@ struct lg_ctx {
     int device = 0;
     cudaStream_t stream = nullptr;
     cudaStream_t copy_stream = nullptr;  // host->device input copies overlapped with compute
-    cudaEvent_t copy_ev[8] = {};
+    cudaEvent_t copy_ev[8] = {}, side_ev = nullptr;
     lgk::Launcher L;
     uint64_t budget = 0, in_use = 0;
     std::string err;
@@ -209,17 +209,16 @@ const uint32_t *get_fft_tw(lg_ctx *c, uint32_t log_n) {
 // call that outgrows it gets extra pinned blocks, valid until the call
 // ends, and the next call starts with an arena that size), and
 // host-side results of downloads (openings) are materialised by finalizers
-// after the call's last synchronisation.  Deferred downloads (of arena
-// buffers, which live until the call ends) are only queued by flush(), so
-// that the kernels between them run back to back and the copies go out
-// while the host has other work.
+// after the call's last synchronisation.  Side downloads (of arena buffers,
+// which live until the call ends) go out on the copy stream as soon as the
+// kernels queued so far are done, so they travel beside the later kernels
+// and break no chain of dependent launches.
 struct Scratch {
     lg_ctx *c;
     std::vector<DBuf> dev_overflow;
     std::vector<uint8_t *> pin_overflow;
     std::vector<std::function<void()>> finalizers;
-    struct Deferred { uint8_t *h; const void *d; size_t bytes; };
-    std::vector<Deferred> deferred;
+    bool side = false;  // copies on the copy stream that finish() waits for
     static constexpr size_t kPin = 8u << 20, kDevArena = 32u << 20;
     explicit Scratch(lg_ctx *ctx) : c(ctx) {
         constexpr size_t kDev = kDevArena;
@@ -239,14 +238,10 @@ struct Scratch {
         c->pin_used = 0;
         c->dev_used = 0;
     }
-    void flush() {
-        for (auto &x : deferred) CK(c, cudaMemcpyAsync(x.h, x.d, x.bytes, cudaMemcpyDeviceToHost, c->stream));
-        deferred.clear();
-    }
     // all pending transfers done, then hand the host copies over
     void finish() {
-        flush();
         sync(c);
+        if (side) CK(c, cudaStreamSynchronize(c->copy_stream));
         for (auto &f : finalizers) f();
         finalizers.clear();
     }
@@ -300,10 +295,13 @@ struct Scratch {
         return reinterpret_cast<const T *>(h);
     }
     template <class T>
-    const T *download_deferred(const T *d, size_t count) {  // valid after finish()
+    const T *download_side(const T *d, size_t count) {  // valid after finish()
         const size_t bytes = count * sizeof(T);
         uint8_t *h = pin(bytes);
-        deferred.push_back({h, d, bytes});
+        CK(c, cudaEventRecord(c->side_ev, c->stream));
+        CK(c, cudaStreamWaitEvent(c->copy_stream, c->side_ev, 0));
+        CK(c, cudaMemcpyAsync(h, d, bytes, cudaMemcpyDeviceToHost, c->copy_stream));
+        side = true;
         return reinterpret_cast<const T *>(h);
     }
 };
@@ -538,7 +536,7 @@ std::pair<const uint32_t *, const uint64_t *> open_rows_dev(lg_ctx *c, Scratch &
     a.mirror = absorb_mirror;
     CK(c, lgk::fs_queries(c->L, fs, a));
     CK(c, lgk::gather_opening(c->L, w.E.u32(), w.rows, w.cols, d_q, nq, w.tree.u32(), d_nodes, cap, d_cnt, d_out));
-    const uint32_t *h = sc.download_deferred(d_out, nq * w.cols + (size_t)cap * 8 + 1);
+    const uint32_t *h = sc.download_side(d_out, nq * w.cols + (size_t)cap * 8 + 1);
     const uint32_t cols = w.cols;
     sc.finalizers.push_back([h, nq, cap, cols, op]() {
         op->rows.assign_fixed(h, nq, cols);
@@ -628,28 +626,20 @@ void prove_impl(lg_ctx *c, Scratch &sc, const lg_config &cfg, const uint32_t *d_
     uint32_t nrounds = 0;
     for (uint32_t i = 0; i < steps; ++i) nrounds += cfg.ks[i];
     const uint32_t ntri = 1 + nrounds + (steps - 1);  // sumcheck triples, in transcript order
-    auto *fs = static_cast<lgk::FsState *>(sc.dev(sizeof(lgk::FsState)));
     uint32_t *chal = static_cast<uint32_t *>(sc.dev(4ull * (cfg.initial_k + nrounds + 3 * steps + 4)));
-    // s0, s1, s2, enforced sum per triple, then the fused steps' block ticket
-    uint32_t *tri = static_cast<uint32_t *>(sc.dev(16ull * ntri + 16));
-    uint32_t *ticket = tri + 4 * ntri;
+    // What the host reads at the end, in one run of words (one download): the
+    // transcript state; s0, s1, s2, enforced sum per triple, then the fused
+    // steps' block ticket; the roots (the transcript kernel absorbing one
+    // copies it here; the tree itself may be freed before the download); yr.
+    const uint32_t fve = cfg.initial_log_m - nrounds;  // log2 |yr|
+    constexpr uint32_t kFsW = sizeof(lgk::FsState) / 4;
+    const size_t end_words = kFsW + 4ull * ntri + 4 + 8ull * (steps + 1) + (1ull << fve);
+    uint32_t *end_d = static_cast<uint32_t *>(sc.dev(4 * end_words));
+    auto *fs = reinterpret_cast<lgk::FsState *>(end_d);
+    uint32_t *tri = end_d + kFsW, *ticket = tri + 4 * ntri, *roots = ticket + 4, *yr_d = roots + 8 * (steps + 1);
     uint32_t nchal = 0, ntri_used = 0;
     auto next_chal = [&](uint32_t n) { uint32_t *p = chal + nchal; nchal += n; return p; };
     auto next_tri = [&]() { return tri + 4 * ntri_used++; };
-    CK(c, cudaMemsetAsync(tri, 0, 16ull * ntri + 16, c->stream));
-    CK(c, lgk::fs_init(c->L, fs, LG_FS_SEED));
-    // A root reaches the host from the arena copy that the transcript
-    // kernel absorbing it writes (the tree itself may be freed before the
-    // deferred copies are queued).
-    auto root_later = [&](std::vector<uint8_t> *dst) {
-        uint32_t *mirror = static_cast<uint32_t *>(sc.dev(32));
-        const uint32_t *h = sc.download_deferred(mirror, 8);
-        sc.finalizers.push_back([h, dst]() {
-            const uint8_t *b = reinterpret_cast<const uint8_t *>(h);
-            dst->assign(b, b + 32);
-        });
-        return mirror;
-    };
     auto tail = [&](bool check, uint32_t nsq, uint32_t *out) {
         lgk::FsTail a;
         a.fs = fs;
@@ -658,17 +648,6 @@ void prove_impl(lg_ctx *c, Scratch &sc, const lg_config &cfg, const uint32_t *d_
         a.nsq = nsq;
         a.out = out;
         return a;
-    };
-    auto step = [&](const uint32_t *src, uint32_t nwords, bool check, uint32_t nsq, uint32_t *out,
-                    uint32_t *mirror) {
-        lgk::FsStep a;
-        a.mirror = mirror;
-        a.src = src;
-        a.nwords = nwords;
-        a.check = check;
-        a.nsq = nsq;
-        a.out = out;
-        CK(c, lgk::fs_step(c->L, fs, a));
     };
     // lg_dump_intermediates only (no-ops otherwise)
     auto dump_commit = [&](uint32_t level, uint32_t log_m, const Witness &w) {
@@ -692,11 +671,22 @@ void prove_impl(lg_ctx *c, Scratch &sc, const lg_config &cfg, const uint32_t *d_
                                            1u << cfg.initial_log_n)
                         : commit(c, d_poly, cfg.initial_log_m, 1u << cfg.initial_log_n);  // :32-37
     dump_commit(0, cfg.initial_log_m, w0);
-    uint32_t *root_m = root_later(&P.initial_root);
     P.recursive_roots.resize(steps);
     P.recursive.resize(steps - 1);  // openings are filled in by pointer later
-    const uint32_t *pe0 = next_chal(cfg.initial_k);
-    step(w0.root(), 8, false, cfg.initial_k, const_cast<uint32_t *>(pe0), root_m);  // :48-50
+    uint32_t *pe0 = next_chal(cfg.initial_k);
+    {
+        lgk::FsStep a;
+        a.src = w0.root();
+        a.nwords = 8;
+        a.nsq = cfg.initial_k;
+        a.out = pe0;
+        a.mirror = roots;
+        a.init = 1;
+        a.seed = LG_FS_SEED;
+        a.zero = tri;
+        a.nzero = 4 * ntri + 4;
+        CK(c, lgk::fs_step(c->L, fs, a));  // :48-50
+    }
     uint32_t fv = cfg.initial_log_m;  // log2 |f|
     DBuf f(c, 4ull << fv);
     partial_eval_dev(c, d_poly, cfg.initial_log_m + cfg.initial_log_n, nullptr, cfg.initial_k, f.u32(), pe0);  // :52-53
@@ -705,9 +695,8 @@ void prove_impl(lg_ctx *c, Scratch &sc, const lg_config &cfg, const uint32_t *d_
 
     Witness wprev = commit(c, f.u32(), cfg.log_m[0], 1u << cfg.log_n[0]);  // :55-60
     dump_commit(1, cfg.log_m[0], wprev);
-    root_m = root_later(&P.recursive_roots[0]);
     uint32_t *alpha = next_chal(1);
-    auto opened = open_rows_dev(c, sc, w0, fs, wprev.root(), 1, alpha, &P.initial, root_m);  // :64-76
+    auto opened = open_rows_dev(c, sc, w0, fs, wprev.root(), 1, alpha, &P.initial, roots + 8);  // :64-76
     DBuf B(c, 4ull << fv);
     uint32_t *t = next_tri();
     induce_dev(c, sc, fv, opened.first, LG_NUM_QUERIES, nullptr, cfg.initial_k, opened.second, 0, B.u32(), t + 3, pe0,
@@ -719,6 +708,7 @@ void prove_impl(lg_ctx *c, Scratch &sc, const lg_config &cfg, const uint32_t *d_
     w0.tree.reset();
     DBuf f2(c, 4ull << (fv - 1)), B2(c, 4ull << (fv - 1));
     DBuf bi;  // the basis a step starts by gluing into B (none at the first)
+    bool yr_there = false;
     for (uint32_t i = 0; i < steps; ++i) {
         // The last commitment is final here: a side stream brings its matrix
         // and tree to the host during this step's rounds, so the final
@@ -769,9 +759,11 @@ void prove_impl(lg_ctx *c, Scratch &sc, const lg_config &cfg, const uint32_t *d_
                 for (uint32_t j = whole ? 0 : 1; j < s.rounds; ++j) next_tri();
                 s.chal = whole ? ec : r;
                 next_chal(s.rounds - 1);
-                s.fo = f2.u32(); s.Bo = B2.u32(); s.fs = fs;
+                s.fo = i == steps - 1 ? yr_d : f2.u32();
+                s.Bo = B2.u32(); s.fs = fs;
                 CK(c, lgk::sum_step(c->L, s));
-                std::swap(f, f2);
+                if (s.fo != yr_d) std::swap(f, f2);
+                else yr_there = true;
                 std::swap(B, B2);
                 fv -= s.rounds;
                 round_no += s.rounds;
@@ -796,16 +788,17 @@ void prove_impl(lg_ctx *c, Scratch &sc, const lg_config &cfg, const uint32_t *d_
             r = rn;
         }
         if (i == steps - 1) {  // :104-143
-            P.yr.resize(1ull << fv);
-            const uint32_t *hy = sc.download_later(f.u32(), 1ull << fv);
-            const lgk::FsState *hs = sc.download_later(fs, 1);
-            const uint32_t *ht = sc.download_later(tri, 4ull * ntri);
+            if (!yr_there) CK(c, cudaMemcpyAsync(yr_d, f.p, 4ull << fv, cudaMemcpyDeviceToDevice, c->stream));
+            const uint32_t *h = sc.download_later(end_d, end_words);
             if (h_E) CK(c, cudaStreamWaitEvent(c->stream, c->copy_ev[6], 0));
-            // wait for these three only; the deferred downloads (roots,
-            // openings) go out now, while the host finishes the transcript
             sync(c);
-            sc.flush();
-            std::memcpy(P.yr.data(), hy, 4ull << fv);
+            const auto *hs = reinterpret_cast<const lgk::FsState *>(h);
+            const uint32_t *ht = h + kFsW, *hr = h + (roots - end_d), *hy = h + (yr_d - end_d);
+            for (uint32_t j = 0; j <= steps; ++j) {
+                const uint8_t *rb = reinterpret_cast<const uint8_t *>(hr + 8 * j);
+                (j ? P.recursive_roots[j - 1] : P.initial_root).assign(rb, rb + 32);
+            }
+            P.yr.assign(hy, hy + (1ull << fv));
             for (uint32_t j = 0; j < ntri; ++j) P.transcript.push_back({ht[4 * j], ht[4 * j + 1], ht[4 * j + 2]});
             if (hs->err) throw ProverAssert{};
             lg::Transcript fsh(LG_FS_SEED);
@@ -826,9 +819,8 @@ void prove_impl(lg_ctx *c, Scratch &sc, const lg_config &cfg, const uint32_t *d_
         }
         Witness wn = commit(c, f.u32(), cfg.log_m[i + 1], 1u << cfg.log_n[i + 1]);  // :145-155
         dump_commit(i + 2, cfg.log_m[i + 1], wn);
-        root_m = root_later(&P.recursive_roots[i + 1]);
         uint32_t *al = next_chal(1);
-        auto op = open_rows_dev(c, sc, wprev, fs, wn.root(), 1, al, &P.recursive[i], root_m);  // :156-172
+        auto op = open_rows_dev(c, sc, wprev, fs, wn.root(), 1, al, &P.recursive[i], roots + 8 * (i + 2));  // :156-172
         bi = DBuf(c, 4ull << fv);
         t = next_tri();
         induce_dev(c, sc, fv, op.first, LG_NUM_QUERIES, nullptr, cfg.ks[i], op.second, 0, bi.u32(), t + 3, rs, al);
@@ -923,7 +915,7 @@ BatchOpened open_rows_batch(lg_ctx *c, Scratch &sc, const BatchWitness &w, lgk::
     gst.out = os;
     CK(c, lgk::gather_opening(c->L, w.E.u32(), w.rows, w.cols, d_q, nq, w.tree.u32(), d_nodes, cap, d_cnt, d_out, B,
                               gst));
-    const uint32_t *h = sc.download_deferred(d_out, os * B);
+    const uint32_t *h = sc.download_side(d_out, os * B);
     const uint32_t cols = w.cols;
     sc.finalizers.push_back([h, nq, cap, cols, os, ops]() {
         for (size_t b = 0; b < ops.size(); ++b) {
@@ -1014,19 +1006,8 @@ void prove_batch_impl(lg_ctx *c, Scratch &sc, const lg_config &cfg, const uint32
     uint32_t nchal = 0, ntri_used = 0;
     auto next_chal = [&](uint32_t n) { uint32_t *p = chal + nchal; nchal += n; return p; };
     auto next_tri = [&]() { return tri + 4 * ntri_used++; };
-    CK(c, cudaMemsetAsync(tri, 0, 4ull * TR * B, c->stream));
-    CK(c, lgk::fs_init(c->L, fs, LG_FS_SEED, B));
-    auto root_later = [&](std::vector<std::vector<uint8_t> *> dst) {
-        uint32_t *mirror = static_cast<uint32_t *>(sc.dev(32ull * B));
-        const uint32_t *h = sc.download_deferred(mirror, 8ull * B);
-        sc.finalizers.push_back([h, dst]() {
-            for (size_t b = 0; b < dst.size(); ++b) {
-                const uint8_t *p = reinterpret_cast<const uint8_t *>(h + 8 * b);
-                dst[b]->assign(p, p + 32);
-            }
-        });
-        return mirror;
-    };
+    // each root's copies (8 words a proof), downloaded together at the end
+    uint32_t *roots = static_cast<uint32_t *>(sc.dev(32ull * B * (steps + 1)));
     auto each = [&](auto get) {
         std::vector<decltype(get(P[0]))> v;
         for (auto *p : P) v.push_back(get(p));
@@ -1059,19 +1040,23 @@ void prove_batch_impl(lg_ctx *c, Scratch &sc, const lg_config &cfg, const uint32
         p->recursive.resize(steps - 1);
     }
     BatchWitness w0 = commit_batch(c, d_polys, cfg.initial_log_m, 1u << cfg.initial_log_n, B);  // :32-37
-    uint32_t *root_m = root_later(each([](lg::Proof *p) { return &p->initial_root; }));
-    const uint32_t *pe0 = next_chal(cfg.initial_k);
+    uint32_t *pe0 = next_chal(cfg.initial_k);
     {
         lgk::FsStep a;
         a.src = w0.root();
         a.nwords = 8;
         a.nsq = cfg.initial_k;
-        a.out = const_cast<uint32_t *>(pe0);
-        a.mirror = root_m;
+        a.out = pe0;
+        a.mirror = roots;
+        a.init = 1;
+        a.seed = LG_FS_SEED;
+        a.zero = tri;
+        a.nzero = (uint32_t)TR;
         lgk::FsStrides st;
         st.src = w0.t_stride();
         st.out = CH;
         st.mirror = 8;
+        st.zero = TR;
         CK(c, lgk::fs_step(c->L, fs, a, B, st));  // :48-50
     }
     uint32_t fv = cfg.initial_log_m;
@@ -1080,10 +1065,9 @@ void prove_batch_impl(lg_ctx *c, Scratch &sc, const lg_config &cfg, const uint32
                        B);  // :52-53
 
     BatchWitness wprev = commit_batch(c, f.u32(), cfg.log_m[0], 1u << cfg.log_n[0], B);  // :55-60
-    root_m = root_later(each([](lg::Proof *p) { return &p->recursive_roots[0]; }));
     uint32_t *alpha = next_chal(1);
     BatchOpened op = open_rows_batch(c, sc, w0, fs, wprev.root(), wprev.t_stride(), 1, alpha, CH,
-                                     each([](lg::Proof *p) { return &p->initial; }), root_m);  // :64-76
+                                     each([](lg::Proof *p) { return &p->initial; }), roots + 8 * B);  // :64-76
     DBuf Bv(c, (4ull << fv) * B);
     uint32_t *t = next_tri();
     induce_batch(c, sc, fv, op.rows, op.stride, nq, cfg.initial_k, op.q, Bv.u32(), t + 3, TR, pe0, alpha, CH,
@@ -1152,12 +1136,17 @@ void prove_batch_impl(lg_ctx *c, Scratch &sc, const lg_config &cfg, const uint32
                             each([](lg::Proof *p) { return &p->final_; }), nullptr);
             // (f is freed when this returns: its copy is queued now)
             const uint32_t *hy = sc.download_later(f.u32(), ny * B);
-            const lgk::FsState *hs = sc.download_deferred(fs, B);
-            const uint32_t *ht = sc.download_deferred(tri, TR * B);
+            const lgk::FsState *hs = sc.download_later(fs, B);
+            const uint32_t *ht = sc.download_later(tri, TR * B);
+            const uint32_t *hr = sc.download_later(roots, 8ull * B * (steps + 1));
             std::vector<char> *flags = &bad;
-            sc.finalizers.push_back([hy, hs, ht, ny, ntri, TR, P, flags]() {
+            sc.finalizers.push_back([hy, hs, ht, hr, steps, ny, ntri, TR, P, flags]() {
                 for (size_t b = 0; b < P.size(); ++b) {
                     lg::Proof &pb = *P[b];
+                    for (uint32_t j = 0; j <= steps; ++j) {
+                        const uint8_t *rb = reinterpret_cast<const uint8_t *>(hr + 8 * (j * P.size() + b));
+                        (j ? pb.recursive_roots[j - 1] : pb.initial_root).assign(rb, rb + 32);
+                    }
                     pb.yr.assign(hy + b * ny, hy + (b + 1) * ny);
                     for (uint32_t j = 0; j < ntri; ++j) {
                         const uint32_t *x = ht + b * TR + 4 * j;
@@ -1169,11 +1158,11 @@ void prove_batch_impl(lg_ctx *c, Scratch &sc, const lg_config &cfg, const uint32
             return;
         }
         BatchWitness wn = commit_batch(c, f.u32(), cfg.log_m[i + 1], 1u << cfg.log_n[i + 1], B);  // :145-155
-        const uint32_t ip1 = i + 1, ii = i;
-        root_m = root_later(each([ip1](lg::Proof *p) { return &p->recursive_roots[ip1]; }));
+        const uint32_t ii = i;
         uint32_t *al = next_chal(1);
         BatchOpened o = open_rows_batch(c, sc, wprev, fs, wn.root(), wn.t_stride(), 1, al, CH,
-                                        each([ii](lg::Proof *p) { return &p->recursive[ii]; }), root_m);  // :156-172
+                                        each([ii](lg::Proof *p) { return &p->recursive[ii]; }),
+                                        roots + 8 * B * (i + 2));  // :156-172
         bi = DBuf(c, (4ull << fv) * B);
         t = next_tri();
         induce_batch(c, sc, fv, o.rows, o.stride, nq, cfg.ks[i], o.q, bi.u32(), t + 3, TR, rs, al, CH, B);
@@ -1699,6 +1688,7 @@ lg_status lg_ctx_create(int device, uint64_t budget, lg_ctx **out) {
     }
     *c->L.fault = 0;
     for (auto &e : c->copy_ev) cudaEventCreateWithFlags(&e, cudaEventDisableTiming);
+    cudaEventCreateWithFlags(&c->side_ev, cudaEventDisableTiming);
     cudaMemPool_t pool;
     if (cudaDeviceGetDefaultMemPool(&pool, device) == cudaSuccess) {
         uint64_t thr = UINT64_MAX;
@@ -1739,6 +1729,7 @@ void lg_ctx_destroy(lg_ctx *c) {
     if (c->L.fault) cudaFreeHost(c->L.fault);
     c->L.release();
     for (auto e : c->copy_ev) if (e) cudaEventDestroy(e);
+    if (c->side_ev) cudaEventDestroy(c->side_ev);
     if (c->copy_stream) cudaStreamDestroy(c->copy_stream);
     cudaStreamDestroy(c->stream);
     delete c;

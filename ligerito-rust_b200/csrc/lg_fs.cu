@@ -26,24 +26,6 @@ namespace {
 using namespace fsd;
 using lgd::pdl_begin;
 
-__global__ void k_fs_init(FsState *g, uint32_t seed) {
-    pdl_begin();
-    g += blockIdx.x;  // lockstep batch: one block per proof
-    __shared__ FsState S;
-    if (threadIdx.x == 0) {
-        const uint32_t iv[8] = {0x6a09e667, 0xbb67ae85, 0x3c6ef372, 0xa54ff53a,
-                                0x510e527f, 0x9b05688c, 0x1f83d9ab, 0x5be0cd19};
-        for (int k = 0; k < 8; ++k) S.h[k] = iv[k];
-        S.nw = 0;
-        S.total = 0;
-        S.counter = 0;
-        S.err = 0;
-        S.pad = 0;
-        fs_absorb(S, &seed, 1);  // FS::new(seed): the seed's LE bytes
-    }
-    store_state(S, g);
-}
-
 __global__ void k_fs_step(FsState *g, FsStep a, FsStrides st) {
     pdl_begin();
     {
@@ -52,12 +34,26 @@ __global__ void k_fs_step(FsState *g, FsStep a, FsStrides st) {
         a.src += b * st.src;
         if (a.out) a.out += b * st.out;
         if (a.mirror) a.mirror += b * st.mirror;
+        if (a.zero) a.zero += b * st.zero;
     }
     __shared__ FsState S;
     __shared__ Batch B;
     __shared__ uint32_t stage[32];
     __shared__ uint32_t kw[kKwBlocks][64];
-    load_state(S, g);
+    for (uint32_t i = threadIdx.x; i < a.nzero; i += blockDim.x) a.zero[i] = 0;
+    if (a.init) {  // FS::new(seed): the seed's LE bytes absorbed
+        for (uint32_t i = threadIdx.x; i < sizeof(FsState) / 4; i += blockDim.x) reinterpret_cast<uint32_t *>(&S)[i] = 0;
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            const uint32_t iv[8] = {0x6a09e667, 0xbb67ae85, 0x3c6ef372, 0xa54ff53a,
+                                    0x510e527f, 0x9b05688c, 0x1f83d9ab, 0x5be0cd19};
+            for (int k = 0; k < 8; ++k) S.h[k] = iv[k];
+            fs_absorb(S, &a.seed, 1);
+        }
+        __syncthreads();
+    } else {
+        load_state(S, g);
+    }
     const bool bad = threadIdx.x == 0 && a.check && (a.src[0] ^ a.src[1]) != a.src[3];
     // long runs (yr) with the message schedules in parallel
     if (a.nwords >= 64) fs_absorb_sched(S, a.src, a.nwords, kw, a.mirror);
@@ -339,15 +335,9 @@ __global__ void __launch_bounds__(kQBlock) k_fs_queries(FsState *g, FsQueries a,
 
 }  // namespace
 
-cudaError_t fs_init(Launcher &L, FsState *d, uint32_t seed, uint32_t B) {
-    if (B == 0 || B > 65535) return cudaErrorInvalidValue;
-    LGK_LAUNCH(L, "fs_init", launch_k(k_fs_init, B, 32, 0, L.stream, d, seed));
-    return cudaGetLastError();
-}
-
 cudaError_t fs_step(Launcher &L, FsState *d, const FsStep &a, uint32_t B, const FsStrides &st) {
     if (a.nwords > 1024 || (a.nwords && !a.src) || a.nsq > 256 || (a.nsq && !a.out) ||
-        (a.check && (!a.src || a.nwords < 3)) || B == 0 || B > 65535)
+        (a.check && (!a.src || a.nwords < 3)) || (a.nzero && !a.zero) || B == 0 || B > 65535)
         return cudaErrorInvalidValue;
     LGK_LAUNCH(L, "fs_step", launch_k(k_fs_step, B, 32, 0, L.stream, d, a, st));
     return cudaGetLastError();

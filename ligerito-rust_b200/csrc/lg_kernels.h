@@ -347,11 +347,10 @@ cudaError_t sum_step(Launcher &L, const SumStep &s, uint32_t NB = 1, const Round
 
 // Lockstep batches: B transcripts d[0..B), one block each; per-proof
 // strides of the step / query arguments' buffers (in their elements).
-struct FsStrides { uint64_t src = 0, out = 0, mirror = 0, q = 0, nodes = 0, nnodes = 0; };
+struct FsStrides { uint64_t src = 0, out = 0, mirror = 0, q = 0, nodes = 0, nnodes = 0, zero = 0; };
 
-// FS::new(seed)
-cudaError_t fs_init(Launcher &L, FsState *d, uint32_t seed, uint32_t B = 1);
-// If check: flag FS_ERR_SUMCHECK unless src[0] ^ src[1] == src[3] (a
+// If init: start from FS::new(seed), and zero nzero words at `zero` (the
+// proof's triples and tickets, before the kernels that add to them).  If check: flag FS_ERR_SUMCHECK unless src[0] ^ src[1] == src[3] (a
 // sumcheck triple and its enforced sum).  Then absorb nwords u32s of src
 // (their LE bytes) and squeeze nsq field elements into out.
 struct FsStep {
@@ -360,6 +359,9 @@ struct FsStep {
     uint32_t nsq = 0;
     uint32_t *out = nullptr;
     uint32_t *mirror = nullptr;  // when set, also receives the absorbed words
+    uint32_t init = 0, seed = 0;
+    uint32_t *zero = nullptr;
+    uint32_t nzero = 0;
 };
 cudaError_t fs_step(Launcher &L, FsState *d, const FsStep &a, uint32_t B = 1, const FsStrides &st = FsStrides{});
 // Absorb nwords u32s of src; get_distinct_queries(n, s) sorted into q
