@@ -514,6 +514,12 @@ def decode_proof(b: bytes) -> ProofFields:
     return ProofFields(root0, rr, init, rec, yr, fin, tr)
 
 
+_new_bytes = ctypes.pythonapi.PyBytes_FromStringAndSize
+_new_bytes.restype, _new_bytes.argtypes = ctypes.py_object, [ctypes.c_char_p, ctypes.c_ssize_t]
+_bytes_ptr = ctypes.pythonapi.PyBytes_AsString
+_bytes_ptr.restype, _bytes_ptr.argtypes = ctypes.c_void_p, [ctypes.py_object]
+
+
 class FinalizedLigeritoProof:
     """Opaque proof handle (lg_proof) with the canonical byte encoding."""
 
@@ -530,9 +536,11 @@ class FinalizedLigeritoProof:
     def to_bytes(self) -> bytes:
         n = ctypes.c_uint64()
         _check(lib.lg_proof_serialize(self.handle, None, ctypes.byref(n)))
-        out = bytearray(n.value)
-        _check(lib.lg_proof_serialize(self.handle, (ctypes.c_char * len(out)).from_buffer(out), ctypes.byref(n)))
-        return bytes(out)
+        # written straight into a new bytes object of that size, which nobody
+        # else holds yet
+        out = _new_bytes(None, n.value)
+        _check(lib.lg_proof_serialize(self.handle, _bytes_ptr(out), ctypes.byref(n)))
+        return out
 
     @classmethod
     def from_bytes(cls, b: bytes) -> "FinalizedLigeritoProof":

@@ -1936,9 +1936,8 @@ lg_status lg_proof_serialize(const lg_proof *p, uint8_t *buf, uint64_t *len) {
         *len = need;
         return ask ? LG_OK : LG_ERR_INVALID_ARGUMENT;
     }
-    std::vector<uint8_t> b = lg::serialize(p->p);
-    std::memcpy(buf, b.data(), b.size());
-    *len = b.size();
+    lg::serialize(p->p, buf);
+    *len = need;
     return LG_OK;
 }
 

@@ -381,28 +381,38 @@ lg_status config_check(const lg_config &c, uint64_t poly_len) {
 // FinalizedLigeritoProof in order; byte strings and vectors carry a u32
 // count (layout documented in the public header's design notes).
 namespace {
-struct Writer {
-    std::vector<uint8_t> b;
-    void raw(const void *p, size_t n) {
-        const size_t at = b.size();
-        b.resize(at + n);
-        if (n) std::memcpy(b.data() + at, p, n);
+// little-endian words, whole runs at a time
+inline void put_words(uint8_t *d, const uint32_t *v, size_t n) {
+#if __BYTE_ORDER__ == __ORDER_LITTLE_ENDIAN__
+    if (n) std::memcpy(d, v, 4 * n);
+#else
+    for (size_t i = 0; i < n; ++i, d += 4) {
+        const uint32_t x = v[i];
+        d[0] = (uint8_t)x; d[1] = (uint8_t)(x >> 8); d[2] = (uint8_t)(x >> 16); d[3] = (uint8_t)(x >> 24);
     }
-    void u32(uint32_t v) {
-        const uint8_t x[4] = {(uint8_t)v, (uint8_t)(v >> 8), (uint8_t)(v >> 16), (uint8_t)(v >> 24)};
-        raw(x, 4);
+#endif
+}
+inline void get_words(uint32_t *v, const uint8_t *d, size_t n) {
+#if __BYTE_ORDER__ == __ORDER_LITTLE_ENDIAN__
+    if (n) std::memcpy(v, d, 4 * n);
+#else
+    for (size_t i = 0; i < n; ++i, d += 4)
+        v[i] = (uint32_t)d[0] | (uint32_t)d[1] << 8 | (uint32_t)d[2] << 16 | (uint32_t)d[3] << 24;
+#endif
+}
+struct Writer {  // into the caller's buffer of serialized_size bytes
+    uint8_t *p;
+    void u32(uint32_t v) { put_words(p, &v, 1); p += 4; }
+    void bytes(const uint8_t *v, size_t n) {
+        u32((uint32_t)n);
+        if (n) std::memcpy(p, v, n);
+        p += n;
     }
-    void bytes(const uint8_t *p, size_t n) { u32((uint32_t)n); raw(p, n); }
     void bytes(const std::vector<uint8_t> &v) { bytes(v.data(), v.size()); }
     void words(const uint32_t *v, size_t n) {
         u32((uint32_t)n);
-        const size_t at = b.size();
-        b.resize(at + 4 * n);
-        uint8_t *d = b.data() + at;
-        for (size_t i = 0; i < n; ++i, d += 4) {
-            const uint32_t x = v[i];
-            d[0] = (uint8_t)x; d[1] = (uint8_t)(x >> 8); d[2] = (uint8_t)(x >> 16); d[3] = (uint8_t)(x >> 24);
-        }
+        put_words(p, v, n);
+        p += 4 * n;
     }
     void words(const std::vector<uint32_t> &v) { words(v.data(), v.size()); }
     void opening(const Opening &o) {
@@ -431,18 +441,26 @@ struct Reader {
         uint32_t c = u32();
         if (!count(c, 4)) return;
         v.resize(c);
-        for (auto &x : v) x = u32();
+        get_words(v.data(), p + at, c);
+        at += 4ull * c;
     }
     void opening(Opening &o) {
         uint32_t r = u32();
         if (!count(r, 4)) return;
         o.rows.clear();
         o.rows.off.reserve(r + 1);
-        std::vector<uint32_t> row;
         for (uint32_t i = 0; i < r && !bad; ++i) {
-            words(row);
-            if (!bad) o.rows.push(row.data(), row.size());
+            const uint32_t c = u32();
+            if (!count(c, 4)) return;
+            // rows are of one length nearly always: room for all by the first
+            if (i == 0 && (uint64_t)r * c * 4 <= n - at) o.rows.data.reserve((size_t)r * c);
+            const size_t w = o.rows.data.size();
+            o.rows.data.resize(w + c);
+            get_words(o.rows.data.data() + w, p + at, c);
+            o.rows.off.push_back(w + c);
+            at += 4ull * c;
         }
+        if (bad) return;
         uint32_t s = u32();
         if (!count(s, 4)) return;
         o.merkle.clear();
@@ -471,10 +489,9 @@ size_t serialized_size(const Proof &p) {
     return s;
 }
 
-std::vector<uint8_t> serialize(const Proof &p) {
-    Writer w;
-    w.b.reserve(serialized_size(p));
-    w.b.insert(w.b.end(), {'L', 'G', 'R', 'P'});
+void serialize(const Proof &p, uint8_t *out) {
+    std::memcpy(out, "LGRP", 4);
+    Writer w{out + 4};
     w.u32(1);
     w.u32(4);
     w.bytes(p.initial_root);
@@ -487,7 +504,6 @@ std::vector<uint8_t> serialize(const Proof &p) {
     w.opening(p.final_);
     w.u32((uint32_t)p.transcript.size());
     for (auto &t : p.transcript) { w.u32(t[0]); w.u32(t[1]); w.u32(t[2]); }
-    return std::move(w.b);
 }
 
 bool deserialize(const uint8_t *buf, size_t len, Proof &p) {
