@@ -10,10 +10,9 @@
 // repeats and sorts.  Everything absorbed is whole u32s, so the pending
 // message is kept as big-endian words.
 //
-// Absorbing is serial (one thread).  Squeezes are batched: squeeze i of a
-// batch finalises the state after i+1 more counters, so one thread
-// compresses the full blocks those counters complete (the only serial
-// part), then every thread finalises its own clone in parallel.
+// Squeeze i of a batch finalises the state after i+1 more counters, so one
+// thread compresses the full blocks that the absorbed words and the counters
+// complete (the only serial part), then every thread finalises its own clone.
 #include <cstdint>
 
 #include "lg_device.cuh"
@@ -38,8 +37,9 @@ __global__ void k_fs_step(FsState *g, FsStep a, FsStrides st) {
     }
     __shared__ FsState S;
     __shared__ Batch B;
-    __shared__ uint32_t stage[32];
-    __shared__ uint32_t kw[kKwBlocks][64];
+    __shared__ uint32_t stage[64];
+    __shared__ FsWork W;
+    static_assert(kKwBlocks <= 32, "the long runs' schedules share the step's rows");
     for (uint32_t i = threadIdx.x; i < a.nzero; i += blockDim.x) a.zero[i] = 0;
     if (a.init) {  // FS::new(seed): the seed's LE bytes absorbed
         for (uint32_t i = threadIdx.x; i < sizeof(FsState) / 4; i += blockDim.x) reinterpret_cast<uint32_t *>(&S)[i] = 0;
@@ -55,9 +55,22 @@ __global__ void k_fs_step(FsState *g, FsStep a, FsStrides st) {
         load_state(S, g);
     }
     const bool bad = threadIdx.x == 0 && a.check && (a.src[0] ^ a.src[1]) != a.src[3];
+    if (a.nwords <= kStepMax && a.nsq <= kStepMax) {
+        if (threadIdx.x < a.nwords) {
+            stage[threadIdx.x] = a.src[threadIdx.x];
+            if (a.mirror) a.mirror[threadIdx.x] = stage[threadIdx.x];
+        }
+        __syncthreads();
+        fs_step_warps(S, W, stage, a.nwords, a.nsq);
+        __syncthreads();
+        if (threadIdx.x == 0 && bad) S.err |= FS_ERR_SUMCHECK;
+        if (threadIdx.x < a.nsq) a.out[threadIdx.x] = W.sq[threadIdx.x];
+        store_state(S, g);
+        return;
+    }
     // long runs (yr) with the message schedules in parallel
-    if (a.nwords >= 64) fs_absorb_sched(S, a.src, a.nwords, kw, a.mirror);
-    else fs_absorb_block(S, a.src, a.nwords, stage, 32, a.mirror);
+    if (a.nwords >= 64) fs_absorb_sched(S, a.src, a.nwords, W.kw, a.mirror);
+    else fs_absorb_block(S, a.src, a.nwords, stage, 64, a.mirror);
     if (bad) S.err |= FS_ERR_SUMCHECK;
     __syncthreads();
     fs_fields(S, B, a.nsq, a.out);
@@ -99,31 +112,21 @@ __device__ uint32_t hash_insert(unsigned long long *key, uint32_t *rank, uint64_
     return kHash - 1;  // unreachable: the table is never more than half full
 }
 
-// The chain of a batch (see fs_chain) from schedules prepared by the block:
-// thread t < full writes K + W of chain block t to kw[t], then thread 0
-// runs only the rounds.  The whole block calls it.
-__device__ void fs_chain_block(const FsState &S, Batch &B, uint32_t cnt, uint32_t (*kw)[64]) {
-    const uint32_t full = (S.nw + cnt) / 16;
-    if (threadIdx.x < full) {
-        uint32_t blk[16];
-#pragma unroll
-        for (int k = 0; k < 16; ++k) blk[k] = stream_word(S, 16 * threadIdx.x + k);
-        sha_schedule_kw(blk, kw[threadIdx.x]);
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        uint32_t st[8];
-#pragma unroll
-        for (int k = 0; k < 8; ++k) B.chain[0][k] = st[k] = S.h[k];
-        for (uint32_t f = 0; f < full; ++f) {
-            sha_rounds_kw(st, kw[f]);
-#pragma unroll
-            for (int k = 0; k < 8; ++k) B.chain[f + 1][k] = st[k];
-        }
-    }
-    __syncthreads();
-}
+// Squeezes of a batch, and the blocks hashed in it: the full blocks of the
+// chain, one final block a squeeze and a second one for the squeezes whose
+// last data leaves no room for the padding (two words of each 16).
+constexpr uint32_t kBatch = 176;
+constexpr uint32_t kChainRows = (15 + kStepMax + kBatch) / 16 + 1;
+constexpr uint32_t kFinalRows = kBatch + 2 * (kBatch / 16 + 2);
+constexpr size_t kQuerySmem = (size_t)(kChainRows + kFinalRows) * kKwStride * 4;
+// p' < p with p' % 16 >= 14
+__device__ __forceinline__ uint32_t two_below(uint32_t p) { return 2 * (p >> 4) + ((p & 15) > 14 ? 1u : 0u); }
 
+// Warp 0 runs the chain of full blocks the batch's counters complete (about
+// ten), warp 1 ahead of it their schedules and the other warps meanwhile the
+// schedules of every squeeze's final blocks, which depend on the counters
+// only; then all squeezes finish side by side.  Bound by the chain: rounds of
+// one warp, about 1 us a block.
 __global__ void __launch_bounds__(kQBlock) k_fs_queries(FsState *g, FsQueries a, FsStrides st) {
     pdl_begin();
     {
@@ -136,23 +139,30 @@ __global__ void __launch_bounds__(kQBlock) k_fs_queries(FsState *g, FsQueries a,
         a.nodes += b * st.nodes;
         a.nnodes += b * st.nnodes;
     }
+    extern __shared__ __align__(16) uint32_t kw_rows[];
+    auto chain_kw = [&](uint32_t f) { return kw_rows + f * kKwStride; };
+    auto final_kw = [&](uint32_t f) { return kw_rows + (kChainRows + f) * kKwStride; };
     __shared__ FsState S;
     __shared__ Batch B;
-    __shared__ uint64_t acc[kQBlock];
+    __shared__ uint32_t root[kStepMax];
+    __shared__ __align__(16) uint32_t acc[kQBlock];  // the queries taken
+    __shared__ uint32_t sorted[kQBlock];
     __shared__ unsigned long long hkey[kHash];
     __shared__ uint32_t hrank[kHash];
-    __shared__ uint32_t lo32[kQBlock];
+    __shared__ uint32_t lo32[kQBlock];  // a batch's squeezes, by index
     __shared__ uint32_t scratch[kQBlock / 32];
-    __shared__ uint32_t wcnt[64][kQBlock / 32], wmask[64][kQBlock / 32];
-    __shared__ uint64_t sq[kQBlock];     // a batch's squeezes, by index
-    __shared__ uint32_t order[kQBlock];  // squeeze index of each thread
+    __shared__ uint32_t wcnt[32][kQBlock / 32], wmask[32][kQBlock / 32];
     __shared__ uint32_t take_sh, batch_sh;
-    __shared__ uint32_t kw[kMaxChain][64];
-    const uint32_t tid = threadIdx.x;
+    const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     load_state(S, g);
-    fs_absorb_block(S, a.src, a.nwords, lo32, kQBlock, a.mirror);
+    uint32_t na = a.nwords;  // words absorbed with the first batch
+    if (tid < na) {
+        root[tid] = a.src[tid];
+        if (a.mirror) a.mirror[tid] = root[tid];
+    }
+    __syncthreads();
     const bool ok = a.n >= a.s && a.s >= 1 && a.s <= kQBlock;
-    const uint64_t mask = a.n - 1;  // n is a power of two: % n is a mask
+    const uint32_t mask = (uint32_t)(a.n - 1);  // n is a power of two: % n is a mask
     uint32_t count = 0, batch = 0, take = 0;
     // get_distinct_queries in batches of squeezes; the round bound only
     // guards a state that cannot progress (n >= s always can)
@@ -160,43 +170,87 @@ __global__ void __launch_bounds__(kQBlock) k_fs_queries(FsState *g, FsQueries a,
         // the queries still needed, about twice the repeats expected among
         // them (need (need/2 + count) / n) plus 2 more, and the challenges
         // squeezed after them: the chain of full blocks a batch completes is
-        // its serial part (~1.2 us a block), so the batch is kept tight; a
-        // short batch just takes another round
+        // its serial part, so the batch is kept tight; a short batch just
+        // takes another round
         const uint32_t need = a.s - count;
         const uint64_t margin = ((uint64_t)need * (need + 2ull * count)) / a.n + 2;
         const uint64_t want = need + margin + a.nsq;
-        batch = want < kQBlock ? (uint32_t)want : kQBlock;
-        fs_chain_block(S, B, batch, kw);
-        // A squeeze whose final data fills 14 or 15 words of its last block
-        // needs a second compression for the padding; those squeezes go to
-        // the first threads, so that only their warps run two compressions
-        // (each warp of consecutive squeezes would otherwise hold some).
+        batch = want < kBatch ? (uint32_t)want : kBatch;
+        const FsStream str(S, root, na);
+        const uint32_t s0 = str.nw + na + 1;  // squeeze i ends after s0 + i words
+        const uint32_t full = (s0 - 1 + batch) / 16, t0 = two_below(s0);
+        for (uint32_t i = tid; i < kHash; i += blockDim.x) {
+            hkey[i] = ~0ull;  // never a value: values are < n <= 2^31
+            hrank[i] = ~0u;
+        }
+        if (warp == 0) {
+            uint32_t h[8];
+#pragma unroll
+            for (int k = 0; k < 8; ++k) h[k] = S.h[k];
+            if (lane == 0)
+#pragma unroll
+                for (int k = 0; k < 8; ++k) B.chain[0][k] = h[k];
+            for (uint32_t f = 0; f < full; ++f) {
+                sha_rounds_kw(h, chain_kw(f), [&](int c) {
+                    if (f == 0) asm volatile("bar.sync %0, 64;" ::"r"(1 + c) : "memory");
+                });
+                if (lane == 0)
+#pragma unroll
+                    for (int k = 0; k < 8; ++k) B.chain[f + 1][k] = h[k];
+            }
+        } else if (warp == 1) {
+            uint32_t blk[16];
+            const uint32_t f = min(lane, kChainRows - 1);
+#pragma unroll
+            for (int k = 0; k < 16; ++k) blk[k] = str.word(16 * f + k);
+            if (full)
+                sha_schedule_kw(blk, chain_kw(f), [](int c) {
+                    __syncwarp();
+                    asm volatile("bar.arrive %0, 64;" ::"r"(1 + c) : "memory");
+                });
+        } else {
+            // row i: squeeze i's first final block; row batch + r: the r-th
+            // two-block squeeze's second
+            const uint32_t n2 = two_below(s0 + batch) - t0;
+            for (uint32_t t = tid - 64; t < batch + n2; t += kQBlock - 64) {
+                uint32_t i = t;
+                if (t >= batch) {
+                    const uint32_t r = t - batch + t0;
+                    i = 16 * (r >> 1) + 14 + (r & 1) - s0;
+                }
+                uint32_t blk[16];
+                str.final_block(i, t >= batch, blk);
+                sha_schedule_kw(blk, final_kw(t));
+            }
+        }
+        __syncthreads();
         {
-            const bool two = tid < batch && ((S.nw + tid + 1) & 15) >= 14;
-            uint32_t total2;
-            const uint32_t r2 = block_rank(two, scratch, &total2);
-            if (tid < batch) order[two ? r2 : total2 + (tid - r2)] = tid;
+            // the two-block squeezes on the first threads, so that only their
+            // warps run two compressions
+            const uint32_t n2 = two_below(s0 + batch) - t0;
+            if (tid < batch) {
+                uint32_t p;
+                if (tid < n2) {
+                    const uint32_t r = tid + t0;
+                    p = 16 * (r >> 1) + 14 + (r & 1);
+                } else {
+                    const uint32_t r = tid - n2 + (s0 - t0);
+                    p = 16 * (r / 14) + r % 14;
+                }
+                const uint32_t i = p - s0, fb = p / 16;
+                uint32_t h[8];
+#pragma unroll
+                for (int k = 0; k < 8; ++k) h[k] = B.chain[fb][k];
+                sha_rounds_kw(h, final_kw(i));
+                if (tid < n2) sha_rounds_kw(h, final_kw(batch + tid));
+                lo32[i] = bswap32(h[0]);
+            }
         }
         __syncthreads();
-        if (tid < batch) {
-            const uint32_t i = order[tid];
-            sq[i] = fs_squeeze_at(S, B, i);
-        }
-        __syncthreads();
-        uint64_t qv = 0;
-        if (tid < batch) {
-            const uint64_t lo = sq[tid];
-            lo32[tid] = (uint32_t)lo;
-            qv = lo & mask;
-        }
+        const uint32_t qv = tid < batch ? lo32[tid] & mask : 0;
         // Repeats: the queries taken so far (rank 0) and this batch's
         // squeezes (rank i + 1) go into a shared hash set that keeps each
         // value's smallest rank; a squeeze is new iff it holds its value's.
-        for (uint32_t i = tid; i < kHash; i += blockDim.x) {
-            hkey[i] = ~0ull;  // never a value: values are < n <= 2^63
-            hrank[i] = ~0u;
-        }
-        __syncthreads();
         if (tid < count) hash_insert(hkey, hrank, acc[tid], 0);
         const uint32_t slot = tid < batch ? hash_insert(hkey, hrank, qv, tid + 1) : 0;
         __syncthreads();
@@ -216,10 +270,20 @@ __global__ void __launch_bounds__(kQBlock) k_fs_queries(FsState *g, FsQueries a,
         // batch when it has them; commit past those too
         const uint32_t extra = count == a.s && take + a.nsq <= batch ? a.nsq : 0;
         if (tid < extra) a.out[tid] = lo32[take + tid];
-        if (tid == 0) {
-            fs_commit(S, B, take + extra);
-            batch_sh = extra;
+        if (warp == 0) {  // the state past them
+            const uint32_t len = str.nw + na + take + extra, rem = len & 15;
+            const uint32_t w = lane < rem ? str.word((len & ~15u) + lane) : 0u;
+            __syncwarp();
+            if (lane < 16) S.w[lane] = w;
+            if (lane < 8) S.h[lane] = B.chain[len / 16][lane];
+            if (lane == 0) {
+                S.nw = rem;
+                S.total += 4ull * (na + take + extra);
+                S.counter += take + extra;
+                batch_sh = extra;
+            }
         }
+        na = 0;
         __syncthreads();
     }
     const uint32_t done_extra = ok && count == a.s ? batch_sh : 0;
@@ -230,97 +294,76 @@ __global__ void __launch_bounds__(kQBlock) k_fs_queries(FsState *g, FsQueries a,
         }
         for (uint32_t i = tid; i < a.s && i < kQBlock; i += blockDim.x) a.q[i] = 0;
     } else {
-        if (tid >= count) acc[tid] = ~0ull;
+        // sorted by rank: the queries are distinct, so a query's place is the
+        // number of smaller ones (four compared a load)
+        if (tid >= count) acc[tid] = ~0u;
         __syncthreads();
-        // bitonic sort of the kQBlock keys, one pair per thread per step
-        for (uint32_t size = 2; size <= kQBlock; size <<= 1)
-            for (uint32_t stride = size >> 1; stride > 0; stride >>= 1) {
-                const uint32_t i = tid, j = i ^ stride;
-                if (j > i) {
-                    const bool up = (i & size) == 0;
-                    const uint64_t x = acc[i], y = acc[j];
-                    if ((x > y) == up) { acc[i] = y; acc[j] = x; }
-                }
-                __syncthreads();
+        const bool have = tid < count;
+        {
+            const uint32_t v = acc[tid];
+            uint32_t below = 0;
+            for (uint32_t j = 0; j < (count + 3) / 4; ++j) {
+                const uint4 x = reinterpret_cast<const uint4 *>(acc)[j];
+                below += (x.x < v) + (x.y < v) + (x.z < v) + (x.w < v);
             }
-        if (tid < count) a.q[tid] = acc[tid];
+            if (have) sorted[below] = v;
+        }
+        __syncthreads();
+        if (have) a.q[tid] = sorted[tid];
         // Multi-proof siblings (merkle_tree::prove, src/merkle_tree.rs:62-111):
         // at layer d the present nodes are x = q >> d; the sibling x ^ 1 is
         // emitted, in order of x, unless it is present too.  Queries are
         // sorted, so the nodes equal to x form a run and x's sibling can only
         // be the run's neighbour: an odd x is settled at its run's first
         // query by the previous query, an even x at its run's last query by
-        // the next one.  Thread i owns query i across all layers.
-        const bool have = tid < count;
-        const uint64_t qi = have ? acc[tid] : 0;
-        const uint64_t qp = have && tid > 0 ? acc[tid - 1] : ~0ull;
-        const uint64_t qn = have && tid + 1 < count ? acc[tid + 1] : ~0ull;
-        const uint32_t lane = tid & 31, warp = tid >> 5;
+        // the next one.  Either emits iff the neighbour is not under x's
+        // parent, i.e. iff it differs from q in a bit above d: so query i
+        // emits in layer d if bit d is set and the previous query's highest
+        // differing bit is above d, or bit d is clear and the next one's is.
+        const uint32_t qi = have ? sorted[tid] : 0;
+        const uint32_t dp = have && tid > 0 ? qi ^ sorted[tid - 1] : ~0u;
+        const uint32_t dn = have && tid + 1 < count ? qi ^ sorted[tid + 1] : ~0u;
         uint32_t nl = 0;
         while ((1ull << nl) < a.n) ++nl;
-        auto emits = [&](uint32_t d, uint64_t &x) {
-            x = qi >> d;
-            if (!have) return false;
-            const bool has_p = qp != ~0ull, has_n = qn != ~0ull;
-            const uint64_t xp = qp >> d, xn = qn >> d;
-            if (x & 1) return (!has_p || xp != x) && !(has_p && xp == (x ^ 1));
-            return (!has_n || xn != x) && !(has_n && xn == (x ^ 1));
-        };
+        // bits below the highest set bit of d (all of them when there is no neighbour)
+        auto under = [](uint32_t d) { return d == ~0u ? ~0u : (1u << (31 - __clz(d))) - 1; };
+        const uint32_t emask =
+            have ? ((qi & under(dp)) | (~qi & under(dn))) & (nl >= 32 ? ~0u : (1u << nl) - 1) : 0u;
         // Per-warp counts of every layer, then one scan gives each warp its
-        // start in each layer (layers in order, threads in query order):
-        // two barriers instead of two per layer.
-        // (each layer's emit bit and warp mask are kept for the write pass)
-        uint64_t x, emask = 0;
+        // start in each layer (layers in order, threads in query order).
         for (uint32_t d = 0; d < nl; ++d) {
-            const bool e = emits(d, x);
-            emask |= (uint64_t)e << d;
-            const uint32_t m = __ballot_sync(0xffffffffu, e);
+            const uint32_t m = __ballot_sync(0xffffffffu, (emask >> d) & 1);
             if (lane == 0) {
                 wcnt[d][warp] = __popc(m);
                 wmask[d][warp] = m;
             }
         }
         __syncthreads();
-        if (warp == 0) {
-            // lane l scans layers l and l + 32: in-layer warp offsets, then
-            // a shuffle scan of the layer totals
-            uint32_t tot[2] = {0, 0};
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                const uint32_t d = lane + 32 * h;
-                if (d < nl)
-                    for (uint32_t w = 0; w < kQBlock / 32; ++w) {
-                        const uint32_t c = wcnt[d][w];
-                        wcnt[d][w] = tot[h];
-                        tot[h] += c;
-                    }
-            }
-            uint32_t inc[2] = {tot[0], tot[1]};
-#pragma unroll
-            for (int h = 0; h < 2; ++h)
-                for (uint32_t o = 1; o < 32; o <<= 1) {
-                    const uint32_t y = __shfl_up_sync(0xffffffffu, inc[h], o);
-                    if (lane >= o) inc[h] += y;
+        if (warp == 0) {  // lane l scans layer l
+            uint32_t tot = 0;
+            if (lane < nl)
+                for (uint32_t w = 0; w < kQBlock / 32; ++w) {
+                    const uint32_t c = wcnt[lane][w];
+                    wcnt[lane][w] = tot;
+                    tot += c;
                 }
-            const uint32_t all0 = __shfl_sync(0xffffffffu, inc[0], 31);
-            const uint32_t start[2] = {inc[0] - tot[0], all0 + inc[1] - tot[1]};
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                const uint32_t d = lane + 32 * h;
-                if (d < nl)
-                    for (uint32_t w = 0; w < kQBlock / 32; ++w) wcnt[d][w] += start[h];
+            uint32_t inc = tot;
+            for (uint32_t o = 1; o < 32; o <<= 1) {
+                const uint32_t y = __shfl_up_sync(0xffffffffu, inc, o);
+                if (lane >= o) inc += y;
             }
-            if (lane == 31) take_sh = all0 + inc[1];
+            if (lane < nl)
+                for (uint32_t w = 0; w < kQBlock / 32; ++w) wcnt[lane][w] += inc - tot;
+            if (lane == 31) take_sh = inc;
         }
         __syncthreads();
-        uint64_t layer_off = 0, width = a.n;
-        for (uint32_t d = 0; d < nl; ++d) {
-            const bool e = (emask >> d) & 1;
-            const uint32_t m = wmask[d][warp];
-            const uint32_t pos = wcnt[d][warp] + __popc(m & ((1u << lane) - 1));
-            if (e && pos < a.nodes_cap) a.nodes[pos] = layer_off + ((qi >> d) ^ 1);
-            layer_off += width;
-            width >>= 1;
+        uint32_t left = emask;
+        while (left) {
+            const uint32_t d = __ffs(left) - 1;
+            left &= left - 1;
+            const uint32_t pos = wcnt[d][warp] + __popc(wmask[d][warp] & ((1u << lane) - 1));
+            // layer d starts after n + n/2 + ... = 2n - 2n/2^d nodes
+            if (pos < a.nodes_cap) a.nodes[pos] = 2 * a.n - (2 * a.n >> d) + ((qi >> d) ^ 1);
         }
         const uint32_t nout = take_sh;
         if (tid == 0) {
@@ -339,15 +382,17 @@ cudaError_t fs_step(Launcher &L, FsState *d, const FsStep &a, uint32_t B, const 
     if (a.nwords > 1024 || (a.nwords && !a.src) || a.nsq > 256 || (a.nsq && !a.out) ||
         (a.check && (!a.src || a.nwords < 3)) || (a.nzero && !a.zero) || B == 0 || B > 65535)
         return cudaErrorInvalidValue;
-    LGK_LAUNCH(L, "fs_step", launch_k(k_fs_step, B, 32, 0, L.stream, d, a, st));
+    LGK_LAUNCH(L, "fs_step", launch_k(k_fs_step, B, 64, 0, L.stream, d, a, st));
     return cudaGetLastError();
 }
 
 cudaError_t fs_queries(Launcher &L, FsState *d, const FsQueries &a, uint32_t B, const FsStrides &st) {
-    if (a.s == 0 || a.s > kQBlock || a.n == 0 || (a.n & (a.n - 1)) || a.nwords > 1024 || (a.nwords && !a.src) ||
+    if (a.s == 0 || a.s > kQBlock || a.n == 0 || (a.n & (a.n - 1)) || a.n > (1ull << 31) || a.nwords > kStepMax ||
+        (a.nwords && !a.src) ||
         a.nsq > kQBlock || (a.nsq && !a.out) || !a.q || !a.nodes || !a.nnodes || B == 0 || B > 65535)
         return cudaErrorInvalidValue;
-    LGK_LAUNCH(L, "fs_queries", launch_k(k_fs_queries, B, kQBlock, 0, L.stream, d, a, st));
+    cudaFuncSetAttribute(k_fs_queries, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kQuerySmem);
+    LGK_LAUNCH(L, "fs_queries", launch_k(k_fs_queries, B, kQBlock, kQuerySmem, L.stream, d, a, st));
     return cudaGetLastError();
 }
 

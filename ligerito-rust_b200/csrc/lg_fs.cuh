@@ -75,40 +75,79 @@ __device__ __forceinline__ void sha_compress(uint32_t st[8], const uint32_t (&bl
     st[4] = addm(st[4], e); st[5] = addm(st[5], f); st[6] = addm(st[6], g); st[7] = addm(st[7], h);
 }
 
-// The 64 rounds of a compression whose K[t] + W[t] are already in kw (the
-// message schedule computed elsewhere): the serial part alone.
-__device__ __forceinline__ void sha_rounds_kw(uint32_t st[8], const uint32_t *kw) {
-    uint32_t a = st[0], b = st[1], c = st[2], d = st[3], e = st[4], f = st[5], g = st[6], h = st[7];
-#pragma unroll 1
-    for (int t0 = 0; t0 < 64; t0 += 16) {
+// One warp issues an instruction every two cycles whatever pipe it goes to, so
+// a compression on one thread costs its instruction count: 14 a round with
+// three-input additions, 10 more a round for the message schedule (measured:
+// 3400-3600 cycles with the schedule, 56 a round; the rounds alone 35).  The
+// serial chains below therefore leave the schedule, which depends on the
+// message only, to other warps.
+
+// 16 rounds on K[t] + W[t] at kw (16-byte aligned shared memory).
+__device__ __forceinline__ void sha_rounds16(uint32_t (&v)[8], const uint32_t *kw) {
 #pragma unroll
-        for (int i = 0; i < 16; ++i) {
-            const uint32_t hk = addm(h, kw[t0 + i]);
-            const uint32_t t1 = addm(addm(hk, rr(e, 6) ^ rr(e, 11) ^ rr(e, 25)), (e & f) ^ (~e & g));
-            const uint32_t t2 = addm(rr(a, 2) ^ rr(a, 13) ^ rr(a, 22), (a & b) ^ (a & c) ^ (b & c));
-            h = g; g = f; f = e; e = addm(d, t1); d = c; c = b; b = a; a = addm(t1, t2);
+    for (int j = 0; j < 4; ++j) {
+        const uint4 k4 = reinterpret_cast<const uint4 *>(kw)[j];
+        const uint32_t k[4] = {k4.x, k4.y, k4.z, k4.w};
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            // a .. h of this round: v rotated by one place a round
+            const int r = 4 * j + i;
+            uint32_t &a = v[(0 - r) & 7], &b = v[(1 - r) & 7], &c = v[(2 - r) & 7], &d = v[(3 - r) & 7];
+            uint32_t &e = v[(4 - r) & 7], &f = v[(5 - r) & 7], &g = v[(6 - r) & 7], &h = v[(7 - r) & 7];
+            const uint32_t t1 = h + k[i] + (rr(e, 6) ^ rr(e, 11) ^ rr(e, 25)) + ((e & f) ^ (~e & g));
+            d += t1;
+            h = t1 + (rr(a, 2) ^ rr(a, 13) ^ rr(a, 22)) + ((a & b) ^ (a & c) ^ (b & c));
         }
     }
-    st[0] = addm(st[0], a); st[1] = addm(st[1], b); st[2] = addm(st[2], c); st[3] = addm(st[3], d);
-    st[4] = addm(st[4], e); st[5] = addm(st[5], f); st[6] = addm(st[6], g); st[7] = addm(st[7], h);
 }
+// The 64 rounds of a compression whose K[t] + W[t] are in kw; before(c) runs
+// ahead of rounds 16 c.
+template <class F>
+__device__ __forceinline__ void sha_rounds_kw(uint32_t (&st)[8], const uint32_t *kw, F before) {
+    uint32_t v[8];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) v[k] = st[k];
+#pragma unroll 1
+    for (int c = 0; c < 4; ++c) {
+        before(c);
+        sha_rounds16(v, kw + 16 * c);
+    }
+#pragma unroll
+    for (int k = 0; k < 8; ++k) st[k] += v[k];
+}
+__device__ __forceinline__ void sha_rounds_kw(uint32_t (&st)[8], const uint32_t *kw) {
+    sha_rounds_kw(st, kw, [](int) {});
+}
+// Words between the schedules of different lanes: 16-byte accesses of a
+// quarter-warp fall on different banks.
+constexpr uint32_t kKwStride = 68;
 
-// K[t] + W[t] (t < 64) of a block of 16 big-endian words.
-__device__ __forceinline__ void sha_schedule_kw(const uint32_t (&blk)[16], uint32_t *kw) {
+// K[t] + W[t] (t < 64) of a block of 16 big-endian words; after(c) runs when
+// words 16 c .. 16 c + 15 are written.
+template <class F>
+__device__ __forceinline__ void sha_schedule_kw(const uint32_t (&blk)[16], uint32_t *kw, F after) {
     uint32_t w[16];
 #pragma unroll
     for (int i = 0; i < 16; ++i) w[i] = blk[i];
 #pragma unroll 1
-    for (int t0 = 0; t0 < 64; t0 += 16) {
+    for (int c = 0; c < 4; ++c) {
+        if (c > 0) {
 #pragma unroll
-        for (int i = 0; i < 16; ++i) {
-            if (t0 > 0) {
+            for (int i = 0; i < 16; ++i) {
                 const uint32_t x = w[(i + 1) & 15], y = w[(i + 14) & 15];
                 w[i] += (rr(x, 7) ^ rr(x, 18) ^ (x >> 3)) + w[(i + 9) & 15] + (rr(y, 17) ^ rr(y, 19) ^ (y >> 10));
             }
-            kw[t0 + i] = kK256[t0 + i] + w[i];
         }
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+            reinterpret_cast<uint4 *>(kw + 16 * c)[i] =
+                make_uint4(kK256[16 * c + 4 * i] + w[4 * i], kK256[16 * c + 4 * i + 1] + w[4 * i + 1],
+                           kK256[16 * c + 4 * i + 2] + w[4 * i + 2], kK256[16 * c + 4 * i + 3] + w[4 * i + 3]);
+        after(c);
     }
+}
+__device__ __forceinline__ void sha_schedule_kw(const uint32_t (&blk)[16], uint32_t *kw) {
+    sha_schedule_kw(blk, kw, [](int) {});
 }
 
 // Serial absorb of nwords u32s (their LE bytes) by one thread.
@@ -151,7 +190,7 @@ __device__ void fs_absorb_block(FsState &S, const uint32_t *src, uint32_t nwords
 // kKwBlocks at a time, into kw) so that thread 0 runs only the 64 rounds
 // of each.  A non-null mirror receives a copy of the words.
 constexpr uint32_t kKwBlocks = 32;
-__device__ void fs_absorb_sched(FsState &S, const uint32_t *src, uint32_t nwords, uint32_t (*kw)[64],
+__device__ void fs_absorb_sched(FsState &S, const uint32_t *src, uint32_t nwords, uint32_t (*kw)[kKwStride],
                                 uint32_t *mirror) {
     const uint32_t head = min(nwords, (16u - S.nw) & 15u);
     const uint32_t full = (nwords - head) / 16, done = head + 16 * full;
@@ -173,8 +212,14 @@ __device__ void fs_absorb_sched(FsState &S, const uint32_t *src, uint32_t nwords
             sha_schedule_kw(blk, kw[t]);
         }
         __syncthreads();
-        if (threadIdx.x == 0)
-            for (uint32_t i = 0; i < nb; ++i) sha_rounds_kw(S.h, kw[i]);
+        if (threadIdx.x == 0) {
+            uint32_t st[8];
+#pragma unroll
+            for (int k = 0; k < 8; ++k) st[k] = S.h[k];
+            for (uint32_t i = 0; i < nb; ++i) sha_rounds_kw(st, kw[i]);
+#pragma unroll
+            for (int k = 0; k < 8; ++k) S.h[k] = st[k];
+        }
         __syncthreads();
     }
     if (threadIdx.x == 0) {
@@ -271,6 +316,124 @@ __device__ void fs_fields(FsState &S, Batch &B, uint32_t nsq, uint32_t *out) {
     }
 }
 
+// A stream of words past the hashed blocks: the pending words, `na` words of
+// `data` (LE bytes), then the counters.
+struct FsStream {
+    const uint32_t *w, *data;
+    uint32_t nw, na, counter;
+    uint64_t total;
+    __device__ __forceinline__ FsStream(const FsState &S, const uint32_t *d, uint32_t n)
+        : w(S.w), data(d), nw(S.nw), na(n), counter(S.counter), total(S.total) {}
+    __device__ __forceinline__ uint32_t word(uint32_t j) const {
+        return j < nw ? w[j] : bswap32(j - nw < na ? data[j - nw] : counter + (j - nw - na));
+    }
+    // squeeze i: its full blocks, the words after them, the blocks it ends in
+    __device__ __forceinline__ uint32_t len(uint32_t i) const { return nw + na + i + 1; }
+    __device__ __forceinline__ uint32_t blocks(uint32_t i) const { return (len(i) & 15) + 3 <= 16 ? 1 : 2; }
+    // block t of squeeze i's end: data, the 0x80 word, the 64-bit length
+    __device__ __forceinline__ void final_block(uint32_t i, uint32_t t, uint32_t (&blk)[16]) const {
+        const uint32_t fb = len(i) / 16, rem = len(i) & 15, nblk = blocks(i);
+        const uint64_t bits = (total + 4ull * (na + i + 1)) * 8;
+#pragma unroll
+        for (int k = 0; k < 16; ++k) {
+            const uint32_t j = 16 * t + k;
+            uint32_t v = 0;
+            if (j < rem) v = word(16 * fb + j);
+            else if (j == rem) v = 0x80000000u;
+            if (j == 16 * nblk - 2) v = (uint32_t)(bits >> 32);
+            if (j == 16 * nblk - 1) v = (uint32_t)bits;
+            blk[k] = v;
+        }
+    }
+};
+
+// A transcript step on warps 0 and 1 of a block: absorb na <= 8 words of
+// `data` (shared memory), squeeze nsq <= 8 field elements into W.sq.  Warp 1
+// writes the schedules of every block the step hashes (one a lane: the full
+// block the new words may complete, each squeeze's final blocks), 16 words
+// at a time; warp 0 follows it with the rounds, the squeezes side by side.
+// Warp 0's threads see the results (S, W.sq) when it returns; other warps
+// after the block's next barrier.
+constexpr uint32_t kStepMax = 8;
+struct alignas(16) FsWork {  // rows are read 16 bytes at a time
+    uint32_t kw[32][kKwStride];  // row: a lane of warp 1
+    uint32_t sq[kStepMax];
+};
+static_assert(1 + 2 * kStepMax <= 32, "one schedule a lane");
+__device__ void fs_step_warps(FsState &S, FsWork &W, const uint32_t *data, uint32_t na, uint32_t nsq) {
+    const uint32_t lane = threadIdx.x & 31;
+    const FsStream st(S, data, na);
+    const uint32_t all = st.nw + na + nsq;  // < 32: at most one full block
+    const bool chain = all >= 16;
+    if (threadIdx.x >= 32) {
+        if (nsq == 0 && !chain) return;
+        uint32_t blk[16];
+        const uint32_t i = (lane - 1) / 2, t = (lane - 1) & 1;
+        if (lane == 0) {
+#pragma unroll
+            for (int k = 0; k < 16; ++k) blk[k] = chain ? st.word(k) : 0u;
+        } else if (i < nsq && t < st.blocks(i)) {
+            st.final_block(i, t, blk);
+        } else {
+#pragma unroll
+            for (int k = 0; k < 16; ++k) blk[k] = 0;
+        }
+        // (lanes past the step's blocks write a spare row of their own)
+        sha_schedule_kw(blk, W.kw[lane], [](int c) {
+            __syncwarp();
+            asm volatile("bar.arrive %0, 64;" ::"r"(1 + c) : "memory");
+        });
+        return;
+    }
+    // warp 0: the words that stay pending, read before anything is written
+    const uint32_t rem = all & 15, next = lane < rem ? st.word((all & ~15u) + lane) : 0u;
+    if (nsq == 0 && !chain) {
+        __syncwarp();
+        if (lane < 16) S.w[lane] = next;
+        if (lane == 0) { S.nw = rem; S.total += 4ull * na; }
+        __syncwarp();
+        return;
+    }
+    bool waited = false;
+    auto wait = [&](int c) {
+        if (!waited) asm volatile("bar.sync %0, 64;" ::"r"(1 + c) : "memory");
+    };
+    uint32_t h0[8], h1[8];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) h0[k] = h1[k] = S.h[k];
+    if (chain) {
+        sha_rounds_kw(h1, W.kw[0], wait);
+        waited = true;
+    }
+    if (nsq) {
+        const uint32_t i = lane < nsq ? lane : 0;
+        const bool after = st.len(i) >= 16;
+        const uint32_t nblk = st.blocks(i), two = __any_sync(0xffffffffu, nblk == 2);
+        uint32_t f[8];
+#pragma unroll
+        for (int k = 0; k < 8; ++k) f[k] = after ? h1[k] : h0[k];
+        sha_rounds_kw(f, W.kw[1 + 2 * i], wait);
+        waited = true;
+        if (two && nblk == 2) sha_rounds_kw(f, W.kw[2 + 2 * i]);
+        __syncwarp();
+        if (lane < nsq) W.sq[lane] = bswap32(f[0]);
+    }
+    __syncwarp();
+    if (lane < 16) S.w[lane] = next;
+    if (lane < 8 && chain) {
+        uint32_t x = 0;
+#pragma unroll
+        for (int k = 0; k < 8; ++k) x = lane == k ? h1[k] : x;
+        S.h[lane] = x;
+    }
+    if (lane == 0) {
+        S.nw = rem;
+        S.total += 4ull * (na + nsq);
+        S.counter += nsq;
+    }
+    __syncwarp();
+}
+
 __device__ void load_state(FsState &S, const FsState *g) {
     const uint32_t *src = reinterpret_cast<const uint32_t *>(g);
     uint32_t *dst = reinterpret_cast<uint32_t *>(&S);
@@ -299,7 +462,7 @@ __device__ __forceinline__ uint32_t fs_tail_prefetch(const FsTail &t) {
 }
 __device__ void fs_tail_block(const FsTail &t, uint32_t *acc3, uint32_t pre) {
     __shared__ FsState S;
-    __shared__ Batch B;
+    __shared__ FsWork W;
     __shared__ uint32_t tri[4];
     __shared__ bool last;
     __threadfence();
@@ -311,14 +474,17 @@ __device__ void fs_tail_block(const FsTail &t, uint32_t *acc3, uint32_t pre) {
     if (threadIdx.x < 4) tri[threadIdx.x] = atomicOr(acc3 + threadIdx.x, 0u);
     if (threadIdx.x < kFsStateWords) reinterpret_cast<uint32_t *>(&S)[threadIdx.x] = pre;
     __syncthreads();
+    if (threadIdx.x >= 64) return;
+    fs_step_warps(S, W, tri, 3, t.nsq);
+    if (threadIdx.x >= 32) return;
     if (threadIdx.x == 0) {
         if (t.check && (tri[0] ^ tri[1]) != tri[3]) S.err |= FS_ERR_SUMCHECK;
-        fs_absorb(S, tri, 3);
         *t.ticket = 0;
     }
-    __syncthreads();
-    fs_fields(S, B, t.nsq, t.out);
-    store_state(S, t.fs);
+    __syncwarp();
+    if (threadIdx.x < t.nsq) t.out[threadIdx.x] = W.sq[threadIdx.x];
+    for (uint32_t i = threadIdx.x; i < kFsStateWords; i += 32)
+        reinterpret_cast<uint32_t *>(t.fs)[i] = reinterpret_cast<const uint32_t *>(&S)[i];
 }
 
 }  // namespace

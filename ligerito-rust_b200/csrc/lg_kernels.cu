@@ -6,6 +6,7 @@
 
 #include <algorithm>
 #include <atomic>
+#include <cstddef>
 #include <cstdio>
 #include <cstdlib>
 #include <map>
@@ -1385,11 +1386,13 @@ struct SumStepArgs {
 // in shared memory, without its words
 struct SumStepShared {
     FsState S;
-    fsd::Batch batch;
+    fsd::FsWork work;
+    uint32_t tri[2][4];   // the triple, a copy for each transcript warp
     uint32_t part[8][4];  // the blocks' partial triples (first block)
     uint32_t red[8][4];   // the warps'
     uint32_t r[4];        // the challenges the first block hands out
 };
+static_assert(offsetof(SumStepShared, work) % 16 == 0, "the schedules' rows are read 16 bytes at a time");
 constexpr uint32_t kSumThreads = 256;
 __device__ __forceinline__ uint32_t cluster_rank() {
     uint32_t r;
@@ -1455,30 +1458,20 @@ __global__ void __launch_bounds__(kSumThreads) k_sum_step(SumStepArgs a, RoundSt
             cluster_store(&sh.part[c][tid], 0, x);
         }
         cluster_sync();
-        if (c == 0 && warp == 0) {
+        if (c == 0 && warp < 2) {
             if (lane < 3) {
                 uint32_t x = 0;
                 for (uint32_t i = 0; i < C; ++i) x ^= sh.part[i][lane];
-                sh.part[0][lane] = x;
-                tri[lane] = x;
+                sh.tri[warp][lane] = x;
+                if (warp == 0) tri[lane] = x;
             }
             __syncwarp();
-            if (lane == 0) {
-                if (check && (sh.part[0][0] ^ sh.part[0][1]) != tri[3]) sh.S.err |= FS_ERR_SUMCHECK;
-                fsd::fs_absorb(sh.S, sh.part[0], 3);
-                fsd::fs_chain(sh.S, sh.batch, nsq);
-            }
-            __syncwarp();
-            uint32_t v = 0;
-            if (lane < nsq) {
-                v = (uint32_t)fsd::fs_squeeze_at(sh.S, sh.batch, lane);
-                chal[lane] = v;
-            }
-            __syncwarp();
-            if (lane == 0) fsd::fs_commit(sh.S, sh.batch, nsq);
-            for (uint32_t i = 0; i < nsq; ++i) {
-                const uint32_t x = __shfl_sync(0xffffffffu, v, i);
-                if (lane < C) cluster_store(&sh.r[i], lane, x);
+            fsd::fs_step_warps(sh.S, sh.work, sh.tri[warp], 3, nsq);
+            if (warp == 0) {
+                if (lane == 0 && check && (sh.tri[0][0] ^ sh.tri[0][1]) != tri[3]) sh.S.err |= FS_ERR_SUMCHECK;
+                if (lane < nsq) chal[lane] = sh.work.sq[lane];
+                for (uint32_t i = 0; i < nsq; ++i)
+                    if (lane < C) cluster_store(&sh.r[i], lane, sh.work.sq[i]);
             }
         }
         tri += 4;

@@ -364,8 +364,8 @@ struct FsStep {
     uint32_t nzero = 0;
 };
 cudaError_t fs_step(Launcher &L, FsState *d, const FsStep &a, uint32_t B = 1, const FsStrides &st = FsStrides{});
-// Absorb nwords u32s of src; get_distinct_queries(n, s) sorted into q
-// (s <= 256, n a power of two); the multi-proof siblings of those leaves
+// Absorb nwords <= 8 u32s of src; get_distinct_queries(n, s) sorted into q
+// (s <= 256, n <= 2^31 a power of two); the multi-proof siblings of those leaves
 // in a tree of n leaves (merkle_tree::prove order) into nodes as node
 // numbers, leaves first, count in *nnodes; then squeeze nsq field elements
 // into out.  n < s flags FS_ERR_QUERIES (the reference loops forever).

@@ -40,3 +40,13 @@ def test_lockstep_steps_match_single(lg, ref, ctx, log_m, ks, B):
     got = lg.prove_lockstep(pc, lg.to_device(polys.ravel()).view(B, -1), ctx)
     for b in (0, B // 2, B - 1):
         assert got[b].to_bytes() == ref.prove(rc, polys[b], nthreads=8)
+
+
+@pytest.mark.parametrize("k0", [2, 3, 4, 5, 7, 8])
+def test_first_challenges_match_oracle(lg, ref, ctx, k0):
+    # the number of challenges squeezed at once moves every later word of the
+    # transcript inside its SHA-256 blocks
+    pc = lg.ProverConfig(2, (1 << 10, 1 << k0), [(1 << 8, 4), (1 << 6, 4)], k0, [2, 2])
+    rc = ref.config(2, 10, k0, [8, 6], [2, 2])
+    poly = lg.splitmix_coeffs(50 + k0, pc.poly_len)
+    assert lg.prover(pc, lg.to_device(poly), ctx).to_bytes() == ref.prove(rc, poly, nthreads=8)
