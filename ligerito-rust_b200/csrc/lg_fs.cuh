@@ -75,12 +75,13 @@ __device__ __forceinline__ void sha_compress(uint32_t st[8], const uint32_t (&bl
     st[4] = addm(st[4], e); st[5] = addm(st[5], f); st[6] = addm(st[6], g); st[7] = addm(st[7], h);
 }
 
-// One warp issues an instruction every two cycles whatever pipe it goes to, so
-// a compression on one thread costs its instruction count: 14 a round with
-// three-input additions, 10 more a round for the message schedule (measured:
-// 3400-3600 cycles with the schedule, 56 a round; the rounds alone 35).  The
-// serial chains below therefore leave the schedule, which depends on the
-// message only, to other warps.
+// A compression on one thread is a chain of dependent instructions (logic,
+// shifts and multiply-adds 5.2 cycles after each other, two- and three-input
+// additions 3.2) that one warp issues at 2 to 3 cycles each: 56 cycles a round
+// with its message schedule, 10 of 24 instructions.  The serial chains below
+// therefore leave the schedule, which depends on the message only, to other
+// warps, and sum h + K + W and d ahead of the round's own sigma and choice
+// (30 cycles a round; 33 without, 35 with the additions as multiply-adds).
 
 // 16 rounds on K[t] + W[t] at kw (16-byte aligned shared memory).
 __device__ __forceinline__ void sha_rounds16(uint32_t (&v)[8], const uint32_t *kw) {
@@ -94,8 +95,14 @@ __device__ __forceinline__ void sha_rounds16(uint32_t (&v)[8], const uint32_t *k
             const int r = 4 * j + i;
             uint32_t &a = v[(0 - r) & 7], &b = v[(1 - r) & 7], &c = v[(2 - r) & 7], &d = v[(3 - r) & 7];
             uint32_t &e = v[(4 - r) & 7], &f = v[(5 - r) & 7], &g = v[(6 - r) & 7], &h = v[(7 - r) & 7];
-            const uint32_t t1 = h + k[i] + (rr(e, 6) ^ rr(e, 11) ^ rr(e, 25)) + ((e & f) ^ (~e & g));
-            d += t1;
+            const uint32_t s1 = rr(e, 6) ^ rr(e, 11) ^ rr(e, 25), ch = (e & f) ^ (~e & g);
+            uint32_t hk = h + k[i], hd, t1;
+            asm volatile("" : "+r"(hk));  // (kept apart: the compiler would sum along the chain)
+            hd = hk + d;
+            asm volatile("" : "+r"(hd));
+            t1 = hk + s1 + ch;
+            asm volatile("" : "+r"(t1));
+            d = hd + s1 + ch;
             h = t1 + (rr(a, 2) ^ rr(a, 13) ^ rr(a, 22)) + ((a & b) ^ (a & c) ^ (b & c));
         }
     }

@@ -366,21 +366,29 @@ __global__ void __launch_bounds__(256, K <= 4 ? 3 : 2) k_rs_first(PassArgs a) {
         __syncthreads();
         issue(u0);
     }
-    // the node tables of all four quarters (see build_pass_tables)
-    for (uint32_t i = warp; i < 4 * K; i += nw) {
-        const uint32_t q = i / K, s = i % K;
+    // The node tables of all four quarters (see build_pass_tables): the
+    // offset of a quarter's first node in its layer is linear in q too, so
+    // its twiddles are 0, C_1, C_2 and C_1 ^ C_2, and only those of quarters
+    // 1 and 2 are built.
+    for (uint32_t i = warp; i < 2 * K; i += nw) {
+        const uint32_t q = 1 + i / K, s = i % K;
         tab_build_warp(reinterpret_cast<uint32_t *>(smraw + q * QT + ((1u << s) - 1) * 512),
                        __ldg(a.tw + ((4u + q) << s) - 1), lane);
     }
     __syncthreads();
-    for (uint32_t i = tid; i < 4 * (R - 1) * 32; i += B) {
-        const uint32_t q = i / ((R - 1) * 32), e = i - q * (R - 1) * 32, slot = e >> 5, first = (1u << (31 - __clz(slot + 1))) - 1;
-        if (slot == first) continue;
-        uint4 *T = reinterpret_cast<uint4 *>(smraw + q * QT);
-        uint4 c = T[first * 32 + (e & 31)];
-        const uint4 d = __ldg(a.dtab + e);
-        c.x ^= d.x; c.y ^= d.y; c.z ^= d.z; c.w ^= d.w;
-        T[e] = c;
+    const uint4 *T1 = reinterpret_cast<const uint4 *>(smraw + QT), *T2 = reinterpret_cast<const uint4 *>(smraw + 2 * QT);
+    for (uint32_t e = 32 + tid; e < (R - 1) * 32; e += B) {  // (the roots' slot 0 is there)
+        const uint32_t slot = e >> 5, first = (1u << (31 - __clz(slot + 1))) - 1, f = first * 32 + (e & 31);
+        uint4 d = make_uint4(0, 0, 0, 0);
+        if (slot != first) d = __ldg(a.dtab + e);
+        const uint4 c1 = T1[f], c2 = T2[f];
+        uint4 *T = reinterpret_cast<uint4 *>(smraw);
+        if (slot != first) {
+            T[e] = d;
+            T[QT / 16 + e] = make_uint4(c1.x ^ d.x, c1.y ^ d.y, c1.z ^ d.z, c1.w ^ d.w);
+            T[2 * (QT / 16) + e] = make_uint4(c2.x ^ d.x, c2.y ^ d.y, c2.z ^ d.z, c2.w ^ d.w);
+        }
+        T[3 * (QT / 16) + e] = make_uint4(c1.x ^ c2.x ^ d.x, c1.y ^ c2.y ^ d.y, c1.z ^ c2.z ^ d.z, c1.w ^ c2.w ^ d.w);
     }
     __syncthreads();
     uint32_t parity = 0;
@@ -538,6 +546,7 @@ __global__ void __launch_bounds__(256, 4) k_fft_tail(PassArgs a) {
     bulk_store_wait();  // the tile is read, and the words are written when the grid ends
 }
 
+constexpr uint32_t kMinPassThreads = 64;
 constexpr uint32_t kTailChunk = 64;  // vectors per tile of the last pass
 static size_t pass_smem(int K) { return (size_t)((1 << K) - 1) * 512; }
 static size_t tail_smem(int K, uint32_t vchunk) { return pass_smem(K) + (size_t)vchunk * ((1u << K) + 4) * 4 + 16; }
@@ -749,7 +758,9 @@ cudaError_t fft_vectors(Launcher &L, uint32_t *data, const uint32_t *tw, uint32_
             continue;
         }
         const uint64_t G = (uint64_t)nvec << a.log_S;  // pencils per (q, P)
-        const uint32_t B = (uint32_t)std::max<uint64_t>(32, std::min<uint64_t>((uint64_t)nvec_p2 << a.log_S, 256));
+        uint32_t B = (uint32_t)std::max<uint64_t>(32, std::min<uint64_t>((uint64_t)nvec_p2 << a.log_S, 256));
+        // small transforms: smaller blocks until every SM has one
+        while (B > kMinPassThreads && (a.src ? 1 : ((uint64_t)Q << d0)) * ((G + B - 1) / B) < 148) B /= 2;
         a.bpg = (uint32_t)((G + B - 1) / B);
         a.units = a.src ? a.bpg : ((uint64_t)Q << d0) * a.bpg;  // k_rs_first: all quarters in a unit
         a.nchunks = 0;
@@ -775,12 +786,15 @@ __device__ __forceinline__ void store_node(uint32_t *p, const uint32_t (&h)[8]) 
     reinterpret_cast<uint4 *>(p)[1] = make_uint4(h[4], h[5], h[6], h[7]);
 }
 
+constexpr uint64_t kHashBound = 1ull << 13;
+
 // Leaf = the row's n words as LE bytes, one BLAKE3 chunk (n <= 256):
 // blocks of 16 words, CHUNK_START on the first, CHUNK_END|ROOT on the last.
 // A thread hashes blocks b0 .. b0 + nb_run - 1 of one row's leaf, from the IV
 // or from the chaining value an earlier call left in out.  Bound by the
 // compression (lg_device.cuh); a whole block's 16 loads take one
-// multiply-add each for their address and no predicate.
+// multiply-add each for their address and no predicate.  MA: see b3_add.
+template <bool MA>
 __global__ void __launch_bounds__(128) k_leaf_hash(const uint32_t *__restrict__ E, uint64_t rows, uint32_t ncols,
                                                    uint32_t b0, uint32_t nb_run, uint32_t *__restrict__ out,
                                                    uint64_t e_stride, uint64_t out_stride) {
@@ -806,10 +820,17 @@ __global__ void __launch_bounds__(128) k_leaf_hash(const uint32_t *__restrict__ 
         const bool last = b + 1 == nb;
         const uint32_t blen = last ? 4 * ncols - 64 * (nb - 1) : 64;
         const uint32_t flags = (b == 0 ? B3_CHUNK_START : 0u) | (last ? (B3_CHUNK_END | B3_ROOT) : 0u);
-        b3_compress(cv, m, blen, flags);
+        b3_compress<MA>(cv, m, blen, flags);
     }
     store_node(out + 8 * i, cv);
 }
+
+// Few hashes wait for their compressions' latency, which plain additions
+// shorten (a 2^12-leaf tree: 13.2 us against 14.0); more are bound by the
+// logic pipe's rate (2^16 leaves of 64 words: 22.8 us with plain additions,
+// 19.4 with multiply-adds; their tree 21.4 and 17.5).
+static bool hash_bound(uint64_t hashes) { return hashes > kHashBound; }
+static auto hash_kernel(uint64_t rows, uint32_t B) { return hash_bound(rows * B) ? k_leaf_hash<true> : k_leaf_hash<false>; }
 
 cudaError_t leaf_hash_block(Launcher &L, const uint32_t *E, uint64_t rows, uint32_t ncols, uint32_t b0,
                             uint32_t nb, uint32_t *out) {
@@ -818,7 +839,7 @@ cudaError_t leaf_hash_block(Launcher &L, const uint32_t *E, uint64_t rows, uint3
     const unsigned blocks = (unsigned)((rows + 127) / 128);
     const uint32_t cols = std::min<uint32_t>(16 * nb, ncols - 16 * b0);
     L.note((double)rows * (4.0 * cols + (b0 ? 64.0 : 32.0)), 0, (double)rows * nb);
-    LGK_LAUNCH(L, "leaf_hash_block", launch_k(k_leaf_hash, blocks, 128, 0, L.stream, E, rows, ncols, b0, nb, out, 0, 0));
+    LGK_LAUNCH(L, "leaf_hash_block", launch_k(hash_kernel(rows, 1), blocks, 128, 0, L.stream, E, rows, ncols, b0, nb, out, 0, 0));
     return cudaGetLastError();
 }
 
@@ -828,7 +849,7 @@ cudaError_t leaf_hashes(Launcher &L, const uint32_t *E, uint64_t rows, uint32_t 
     const uint32_t nb = (ncols + 15) / 16;
     const dim3 blocks((unsigned)((rows + 127) / 128), B);
     L.note((double)B * rows * (4.0 * ncols + 32.0), 0, (double)B * rows * nb);
-    LGK_LAUNCH(L, "leaf_hash", launch_k(k_leaf_hash, blocks, 128, 0, L.stream, E, rows, ncols, 0, nb, out, e_stride,
+    LGK_LAUNCH(L, "leaf_hash", launch_k(hash_kernel(rows, B), blocks, 128, 0, L.stream, E, rows, ncols, 0, nb, out, e_stride,
                                         out_stride));
     return cudaGetLastError();
 }
@@ -917,6 +938,7 @@ constexpr uint32_t kNarrowNodes = 512, kNarrowMax = kNarrowNodes * kNarrowNodes;
 // (nodes first .. first + m - 1 of a layer of n) to their common ancestor;
 // src_tree: the first layer is read from the tree with loads that bypass
 // L1 (nodes other blocks wrote).  Ends with the block synchronised.
+template <bool MA>
 __device__ __forceinline__ void narrow_climb(uint32_t *__restrict__ tree, uint64_t off, uint64_t n, uint64_t first,
                                              uint32_t m, uint32_t *buf_a, uint32_t *buf_b) {
     const uint32_t t = threadIdx.x;
@@ -926,7 +948,7 @@ __device__ __forceinline__ void narrow_climb(uint32_t *__restrict__ tree, uint64
         const uint4 a0 = __ldcg(pl), a1 = __ldcg(pl + 1), b0 = __ldcg(pl + 2), b1 = __ldcg(pl + 3);
         l[0] = a0.x; l[1] = a0.y; l[2] = a0.z; l[3] = a0.w; l[4] = a1.x; l[5] = a1.y; l[6] = a1.z; l[7] = a1.w;
         r[0] = b0.x; r[1] = b0.y; r[2] = b0.z; r[3] = b0.w; r[4] = b1.x; r[5] = b1.y; r[6] = b1.z; r[7] = b1.w;
-        hash_pair(l, r, h);
+        hash_node<MA>(l, r, h);
         store_node(tree + 8 * (off + n + first / 2 + t), h);
 #pragma unroll
         for (int j = 0; j < 8; ++j) buf_a[j * (kNarrowNodes / 2) + t] = h[j];
@@ -947,7 +969,7 @@ __device__ __forceinline__ void narrow_climb(uint32_t *__restrict__ tree, uint64
                 l[j] = x.x;
                 r[j] = x.y;
             }
-            hash_pair(l, r, h);
+            hash_node<MA>(l, r, h);
             store_node(tree + 8 * (off + n + first / 2 + t), h);
 #pragma unroll
             for (int j = 0; j < 8; ++j) dst[j * ds + t] = h[j];
@@ -966,6 +988,7 @@ __device__ __forceinline__ void narrow_climb(uint32_t *__restrict__ tree, uint64
     }
 }
 
+template <bool MA>
 __global__ void __launch_bounds__(256) k_merkle_narrow(uint32_t *__restrict__ tree, uint64_t in_off, uint64_t n_in,
                                                        uint32_t *ticket, uint64_t tree_stride) {
     pdl_begin();
@@ -977,7 +1000,7 @@ __global__ void __launch_bounds__(256) k_merkle_narrow(uint32_t *__restrict__ tr
     __shared__ __align__(16) uint32_t buf_b[8 * (kNarrowNodes / 4)];
     __shared__ uint32_t last;
     const uint32_t per = (uint32_t)(n_in < kNarrowNodes ? n_in : kNarrowNodes), nb = gridDim.x;
-    narrow_climb(tree, in_off, n_in, (uint64_t)blockIdx.x * per, per, buf_a, buf_b);
+    narrow_climb<MA>(tree, in_off, n_in, (uint64_t)blockIdx.x * per, per, buf_a, buf_b);
     if (nb == 1) return;
     // the layer of the blocks' roots
     uint64_t off = in_off, n = n_in;
@@ -988,7 +1011,7 @@ __global__ void __launch_bounds__(256) k_merkle_narrow(uint32_t *__restrict__ tr
     if (!last) return;
     __threadfence();
     if (threadIdx.x == 0) *ticket = 0;  // ready for the next launch on the stream
-    narrow_climb(tree, off, n, 0, nb, buf_a, buf_b);
+    narrow_climb<MA>(tree, off, n, 0, nb, buf_a, buf_b);
 }
 
 cudaError_t merkle_upper(Launcher &L, uint32_t *tree, uint64_t num_leaves, uint32_t B, uint64_t tree_stride) {
@@ -1010,7 +1033,7 @@ cudaError_t merkle_upper(Launcher &L, uint32_t *tree, uint64_t num_leaves, uint3
         } else {
             const uint64_t per = std::min<uint64_t>(n, kNarrowNodes);
             L.note(32.0 * B * (2 * n - 1), 0, (double)B * (n - 1));
-            LGK_LAUNCH(L, "merkle_narrow", launch_k(k_merkle_narrow, dim3((unsigned)(n / per), B), 256, 0, L.stream,
+            LGK_LAUNCH(L, "merkle_narrow", launch_k(hash_bound(n * B) ? k_merkle_narrow<true> : k_merkle_narrow<false>, dim3((unsigned)(n / per), B), 256, 0, L.stream,
                                                     tree, off, n, L.tickets, tree_stride));
             e = cudaGetLastError();
             n = 1;
@@ -1903,8 +1926,8 @@ static cudaError_t launch_induce_main(Launcher &L, const InducePlan &p, uint32_t
         int dev = 0, sms = 148;
         if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
             sms = 148;
-        // at least 32 (proof, t_hi pair, query) triples a block
-        const unsigned grid = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>((work / 2 + 31) / 32, (uint64_t)sms * o));
+        // at least 8 (proof, t_hi pair, query) triples a block: one a warp
+        const unsigned grid = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>((work / 2 + 7) / 8, (uint64_t)sms * o));
         LGK_LAUNCH(L, "induce_main", launch_k(k_induce_main2, grid, 256, 0, L.stream, d_lo, d_hi, n, nq, B, out, st));
         return cudaGetLastError();
     }
@@ -1919,9 +1942,10 @@ static cudaError_t launch_induce_main(Launcher &L, const InducePlan &p, uint32_t
 }
 
 // induce_setup and induce_prep in one launch: block k (query k) first
-// runs the setup of its query on warp 0 (the row's dot product with the
-// Lagrange basis, alpha^k, the subspace values) into shared memory, then
-// the block doubles out Lo_k and Hi_k from them.  Each block leaves its
+// runs the setup of its query (the row's dot product with the Lagrange
+// basis, alpha^k, the subspace values) into shared memory, then the block
+// doubles out Lo_k and Hi_k from them.  Bound by the latency of those serial
+// products, so independent ones run side by side.  Each block leaves its
 // contribution alpha^k * dot_k in contrib[k]; the last block to finish (a
 // ticket, reset by it) XORs them into the enforced sum.
 __global__ void __launch_bounds__(256) k_induce_sp(const uint32_t *__restrict__ rows, uint32_t glen,
@@ -1950,51 +1974,56 @@ __global__ void __launch_bounds__(256) k_induce_sp(const uint32_t *__restrict__ 
          i += (uint64_t)gridDim.x * blockDim.x)
         out[i] = 0;
     extern __shared__ uint32_t sbuf[];  // Lo then Hi, when in_smem
-    __shared__ uint32_t gr[256], Ss[32], apk;
+    __shared__ uint32_t Ss[32], apk;
     __shared__ bool last;
-    for (uint32_t j = threadIdx.x; j < glen; j += blockDim.x) gr[j] = d_rs ? lagrange_at(d_rs, nch, j) : args.gr[j];
-    if (d_alpha) alpha = *d_alpha;
-    __syncthreads();
-    const uint32_t k = blockIdx.x, lane = threadIdx.x & 31;
-    if (threadIdx.x < 32) {  // the setup of query k (as k_induce_setup)
-        uint32_t dot = 0;
-        for (uint32_t j = lane; j < glen; j += 32) dot ^= gf_mul(rows[(uint64_t)k * glen + j], gr[j]);
-        dot = warp_xor(dot);
-        uint32_t a2 = alpha;
-        for (uint32_t i = 0; i < lane && i < 16; ++i) a2 = gf_mul(a2, a2);
-        uint32_t pw = (lane < 16 && ((k >> lane) & 1)) ? a2 : 1u;
-#pragma unroll
-        for (int o = 8; o > 0; o >>= 1) pw = gf_mul(pw, __shfl_xor_sync(0xffffffffu, pw, o));
-        pw = __shfl_sync(0xffffffffu, pw, 0);
+    // The setup of query k (as k_induce_setup), its three parts on warps of
+    // their own: the subspace values on warp 0, alpha^k on warp 1, the row's
+    // dot product with the Lagrange basis on the rest.
+    const uint32_t k = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    __shared__ uint32_t dots[8];
+    if (warp == 0) {
         if (lane == 0) {
-            apk = pw;
-            contrib[k] = gf_mul(dot, pw);
             uint32_t sx = (uint32_t)q[k];
-            if (n) Ss[0] = sx;
+            Ss[0] = sx;
             for (uint32_t i = 1; i < n; ++i) {
                 sx = gf_mul(sx, sx) ^ gf_mul(args.sks[i - 1], sx);
                 Ss[i] = sx;
             }
         }
+    } else if (warp == 1) {
+        uint32_t a2 = d_alpha ? *d_alpha : alpha;
+        for (uint32_t i = 0; i < lane && i < 16 && (k >> i) != 0; ++i) a2 = gf_mul(a2, a2);
+        uint32_t pw = (lane < 16 && ((k >> lane) & 1)) ? a2 : 1u;
+#pragma unroll
+        for (int o = 8; o > 0; o >>= 1) pw = gf_mul(pw, __shfl_xor_sync(0xffffffffu, pw, o));
+        if (lane == 0) apk = pw;
+    } else {
+        uint32_t dot = 0;
+        for (uint32_t j = threadIdx.x - 64; j < glen; j += blockDim.x - 64)
+            dot ^= gf_mul(rows[(uint64_t)k * glen + j], d_rs ? lagrange_at(d_rs, nch, j) : args.gr[j]);
+        dot = __reduce_xor_sync(0xffffffffu, dot);
+        if (lane == 0) dots[warp] = dot;
     }
     __syncthreads();
-    // the prep of query k (as k_induce_prep)
+    // the prep of query k (as k_induce_prep), a level of Lo and one of Hi at a
+    // time
     const uint32_t nlo = 1u << b, nhi = 1u << (n - b);
     uint32_t *glk = lo + ((uint64_t)k << b), *ghk = hi + ((uint64_t)k << (n - b));
     uint32_t *lk = in_smem ? sbuf : glk, *hk = in_smem ? sbuf + nlo : ghk;
     if (threadIdx.x == 0) {
         lk[0] = 1;
         hk[0] = apk;
+        uint32_t dot = 0;
+        for (uint32_t w = 2; w < blockDim.x >> 5; ++w) dot ^= dots[w];
+        contrib[k] = gf_mul(dot, apk);
     }
     __syncthreads();
-    for (uint32_t h = 0; h < b; ++h) {
-        const uint32_t sv = Ss[h];
-        for (uint32_t u = threadIdx.x; u < (1u << h); u += blockDim.x) lk[(1u << h) + u] = gf_mul(lk[u], sv);
-        __syncthreads();
-    }
-    for (uint32_t h = 0; h < n - b; ++h) {
-        const uint32_t sv = Ss[b + h];
-        for (uint32_t c = threadIdx.x; c < (1u << h); c += blockDim.x) hk[(1u << h) + c] = gf_mul(hk[c], sv);
+    for (uint32_t h = 0; h < max(b, n - b); ++h) {
+        const uint32_t m = 1u << h, cl = h < b ? m : 0, ch = h < n - b ? m : 0;
+        for (uint32_t u = threadIdx.x; u < cl + ch; u += blockDim.x) {
+            if (u < cl) lk[m + u] = gf_mul(lk[u], Ss[h]);
+            else hk[m + u - cl] = gf_mul(hk[u - cl], Ss[b + h]);
+        }
         __syncthreads();
     }
     if (in_smem) {
