@@ -123,6 +123,22 @@ struct PassArgs {
     const uint32_t *pis;       // k_rs_first: the row scaling
 };
 
+// Slots f + 1 .. f + n - 1 of a stage whose first slot f holds C's table: C
+// XOR D, a slot a warp, starting with warp `rot` (stages one after another
+// keep every warp equally busy; a loop over all slots that finds its stage by
+// counting leading zeros took 45 M more instructions in a 2^18 x 256 last
+// pass of 247 M).  D's slot of the stage's slot t is df + (t << dsh).
+__device__ __forceinline__ void fill_stage(uint4 *T, const uint4 *dtab, int f, int n, int df, int dsh, int rot) {
+    const int lane = threadIdx.x & 31, nw = blockDim.x >> 5, warp = ((threadIdx.x >> 5) - rot) & (nw - 1);
+    if (1 + warp >= n) return;
+    const uint4 c = T[f * 32 + lane];
+    for (int t = 1 + warp; t < n; t += nw) {
+        uint4 d = __ldg(dtab + (df + (t << dsh)) * 32 + lane);
+        d.x ^= c.x; d.y ^= c.y; d.z ^= c.z; d.w ^= c.w;
+        T[(f + t) * 32 + lane] = d;
+    }
+}
+
 // The 2^K - 1 node tables of one (q, P), in 512-byte slots at the start of
 // `sm` (slot 2^s - 1 + t for node t of in-pass stage s).
 //
@@ -143,15 +159,9 @@ __device__ __forceinline__ void build_pass_tables(uint8_t *sm, const PassArgs &a
     for (int s = warp; s < K; s += nw)
         tab_build_warp(reinterpret_cast<uint32_t *>(sm + ((1 << s) - 1) * 512), __ldg(a.tw + (hbase << s) - 1), lane);
     __syncthreads();
-    uint4 *T = reinterpret_cast<uint4 *>(sm);
-    for (int i = threadIdx.x; i < ((1 << K) - 1) * 32; i += blockDim.x) {
-        const int slot = i >> 5, s = 31 - __clz(slot + 1), first = (1 << s) - 1;
-        if (slot == first) continue;
-        uint4 c = T[first * 32 + (i & 31)];
-        const uint4 d = __ldg(a.dtab + i);
-        c.x ^= d.x; c.y ^= d.y; c.z ^= d.z; c.w ^= d.w;
-        T[i] = c;
-    }
+#pragma unroll
+    for (int s = 1; s < K; ++s)
+        fill_stage(reinterpret_cast<uint4 *>(sm), a.dtab, (1 << s) - 1, 1 << s, (1 << s) - 1, 0, (1 << s) - s - 1);
     __syncthreads();
 }
 
@@ -172,6 +182,19 @@ __global__ void k_fft_dtab(const uint32_t *__restrict__ tw, DtabArgs d, uint32_t
     tab_build_warp(out + ((size_t)p * 63 + slot) * kTabWords, __ldg(tw + ((1ull << (d.l0[p] + s)) - 1) + t), lane);
 }
 
+// The leaf layer's twiddles are unscaled: node u has the polynomial 2u.  The
+// nodes t = 0..3 of a pencil's last stage so have those of the first one plus
+// 0, x, x^2, x^2 + x: one table serves all four, and this is the rest of the
+// product, (2t) v, by shifts as multiplies (the pipe the lookups leave idle).
+static __constant__ uint32_t kLeafMul[4] = {2u, 4u, 0x8289u, 16u};
+__device__ __forceinline__ uint32_t leaf_rest(int t, uint32_t v) {
+    if (t == 0) return 0;
+    const uint64_t a = t & 1 ? fma_mul_wide(v, kLeafMul[0]) : 0, b = t & 2 ? fma_mul_wide(v, kLeafMul[1]) : 0;
+    const uint32_t hi = (uint32_t)(a >> 32) ^ (uint32_t)(b >> 32);  // at most 2 bits past x^31
+    // times the tail 0x8299: {0, 3, 7, 9, 15} and 4 apart, so nothing overlaps
+    return (uint32_t)a ^ (uint32_t)b ^ fma_mul(hi, kLeafMul[2]) ^ fma_mul(hi, kLeafMul[3]);
+}
+
 // K stages over the NV values of a register pencil, node index of value i at
 // in-pass stage s = (i >> (K - s)) + node_off(s); tables at tb + 512 * slot.
 // Forward: fft_twiddles / fft_mul (src/binary_fft.rs:143-159, 180-192),
@@ -179,8 +202,9 @@ __global__ void k_fft_dtab(const uint32_t *__restrict__ tw, DtabArgs d, uint32_t
 // 194-206), leaves-first.  One flat loop so every register index is a
 // compile-time constant after unrolling.
 // ZERO0: the twiddle of each stage's node 0 is zero (its products are left
-// out).
-template <int KP, int S0, bool INV, bool ZERO0 = false>
+// out).  LEAF: the last stage is the transform's; its table is that of the
+// pencil's first node, slot 2^s - 1 + the prefix (see leaf_rest).
+template <int KP, int S0, bool INV, bool ZERO0 = false, bool LEAF = false>
 __device__ __forceinline__ void pencil_stages(uint32_t (&v)[1 << KP], const uint8_t *sm, uint32_t tb,
                                               uint32_t gshift_slot) {
 #pragma unroll
@@ -193,14 +217,17 @@ __device__ __forceinline__ void pencil_stages(uint32_t (&v)[1 << KP], const uint
         const int x = (tp << (lh + 1)) + u, y = x + (1 << lh);
         // gshift_slot: runtime prefix of the node index inside this stage,
         // folded into the (256-aligned) base; the rest is a constant offset
-        const uint32_t base = tb + 512u * (gshift_slot << sl);
-        const uint32_t off = 512u * ((1u << s) - 1u + (uint32_t)tp);
+        const bool leaf = LEAF && sl == KP - 1;
+        const uint32_t base = tb + 512u * (leaf ? gshift_slot : gshift_slot << sl);
+        const uint32_t off = 512u * ((1u << s) - 1u + (leaf ? 0u : (uint32_t)tp));
         if (!INV) {
             if (!ZERO0 || tp != 0) v[x] ^= tab_mul_sa(sm, base, off, v[y]);
+            if (leaf) v[x] ^= leaf_rest(tp, v[y]);
             v[y] ^= v[x];
         } else {
             v[y] ^= v[x];
             v[x] ^= tab_mul_sa(sm, base, off, v[y]);
+            if (leaf) v[x] ^= leaf_rest(tp, v[y]);
         }
     }
 }
@@ -462,17 +489,28 @@ __global__ void __launch_bounds__(256, K <= 4 ? 3 : 2) k_rs_first(PassArgs a) {
     }
 }
 
-// Last pass (contiguous blocks of 2^K rows): one block per (q, P) tile of
-// 2^K rows x nvec vectors.  All warps build the 2^K - 1 tables, then the
-// stages run in two register phases of about K/2 stages each.  A warp shares
-// every table it reads; the block has as many threads as a phase has pencils
-// (up to 256), so a tile of few vectors still keeps every thread busy.
-// The load/store unit's wavefronts bound this kernel (93% of their peak with
-// the tile staged through registers), so a column's 2^K words enter and
-// leave the tile as one bulk copy each, which takes none.  The tile's column
-// stride is 2^K + 4 words (an odd number of 16-byte pieces): phase A reads
-// and writes words with lanes over 8 columns x 4 rows, phase B 16-byte
-// pieces with lanes over columns, both free of bank conflicts.
+// The node tables of a last pass's tile (see build_pass_tables): slots of
+// stages 0 .. K-2, then one slot per phase-B pencil for the leaf stage, that
+// of the pencil's first node (leaf_rest).
+template <int K>
+struct TailTables {
+    static constexpr int KA = K / 2, KB = K - KA;
+    static constexpr int kInner = (1 << (K - 1)) - 1, kSlots = kInner + (1 << KA);
+    static __device__ __forceinline__ void build(uint8_t *sm, const PassArgs &a, unsigned q, unsigned P) {
+        const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+        const uint64_t hbase = ((uint64_t)(a.root_base + q) << a.d0) + P;
+        for (int s = warp; s < K; s += nw)
+            tab_build_warp(reinterpret_cast<uint32_t *>(sm + ((1 << s) - 1) * 512), __ldg(a.tw + (hbase << s) - 1), lane);
+        __syncthreads();
+        uint4 *T = reinterpret_cast<uint4 *>(sm);
+#pragma unroll
+        for (int s = 1; s < K - 1; ++s)
+            fill_stage(T, a.dtab, (1 << s) - 1, 1 << s, (1 << s) - 1, 0, (1 << s) - s - 1);
+        fill_stage(T, a.dtab, kInner, 1 << KA, kInner, KB - 1, kInner - (K - 1));
+        __syncthreads();
+    }
+};
+
 template <int K, bool INV>
 __global__ void __launch_bounds__(256, 4) k_fft_tail(PassArgs a) {
     pdl_begin();
@@ -482,7 +520,7 @@ __global__ void __launch_bounds__(256, 4) k_fft_tail(PassArgs a) {
     const unsigned P = rest & ((1u << a.d0) - 1);
     const unsigned q = rest >> a.d0;
     const uint32_t nvec = min(a.vchunk, a.nvec - chunk * a.vchunk);
-    uint32_t *tile = reinterpret_cast<uint32_t *>(smraw + (R - 1) * 512);
+    uint32_t *tile = reinterpret_cast<uint32_t *>(smraw + TailTables<K>::kSlots * 512);
     uint64_t *bar = reinterpret_cast<uint64_t *>(tile + a.vchunk * STRIDE);
     uint32_t *gbase = a.data + (uint64_t)chunk * a.vchunk * a.col_stride + q * a.q_stride + ((uint64_t)P << K);
     if (threadIdx.x == 0) {
@@ -493,7 +531,7 @@ __global__ void __launch_bounds__(256, 4) k_fft_tail(PassArgs a) {
     __syncthreads();
     for (uint32_t j = threadIdx.x; j < nvec; j += blockDim.x)
         bulk_load(tile + j * STRIDE, gbase + j * a.col_stride, 4 * R, bar);
-    build_pass_tables<K>(smraw, a, q, P);
+    TailTables<K>::build(smraw, a, q, P);
     mbar_wait(bar, 0, a.fault);
 
     // Two register phases: KA stages on pencils of 2^KA values at stride
@@ -525,7 +563,7 @@ __global__ void __launch_bounds__(256, 4) k_fft_tail(PassArgs a) {
                 const uint4 x = p[i];
                 v[4 * i] = x.x; v[4 * i + 1] = x.y; v[4 * i + 2] = x.z; v[4 * i + 3] = x.w;
             }
-            pencil_stages<KB, KA, INV>(v, smraw, 0, gq);
+            pencil_stages<KB, KA, INV, false, true>(v, smraw, 0, gq);
 #pragma unroll
             for (int i = 0; i < RB / 4; ++i) p[i] = make_uint4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
         }
@@ -549,7 +587,10 @@ __global__ void __launch_bounds__(256, 4) k_fft_tail(PassArgs a) {
 constexpr uint32_t kMinPassThreads = 64;
 constexpr uint32_t kTailChunk = 64;  // vectors per tile of the last pass
 static size_t pass_smem(int K) { return (size_t)((1 << K) - 1) * 512; }
-static size_t tail_smem(int K, uint32_t vchunk) { return pass_smem(K) + (size_t)vchunk * ((1u << K) + 4) * 4 + 16; }
+static size_t tail_smem(int K, uint32_t vchunk) {
+    const int slots = K == 4 ? TailTables<4>::kSlots : K == 5 ? TailTables<5>::kSlots : TailTables<6>::kSlots;
+    return (size_t)slots * 512 + (size_t)vchunk * ((1u << K) + 4) * 4 + 16;
+}
 // strided pass: tables, then (bulk copies) the unit's rows and the barrier
 static size_t strided_smem(int K, unsigned threads, bool bulk, bool rs_first = false) {
     return pass_smem(K) * (rs_first ? 4 : 1) + (bulk ? ((size_t)threads << K) * 4 + 16 : 0);
@@ -631,8 +672,12 @@ static cudaError_t launch_tail(Launcher &L, int K, PassArgs a, unsigned blocks) 
     const int smem_max = (int)tail_smem(K, kTailChunk);
     uint32_t vp2 = 1;
     while (vp2 < a.vchunk) vp2 <<= 1;
-    // pencils per phase: vectors x 2^(K - K/2) (the larger phase)
-    const unsigned threads = std::max<unsigned>(32, std::min<unsigned>(256, vp2 << (K - K / 2)));
+    // A thread per pencil of a phase (vectors x 2^(K - K/2), the larger one)
+    // up to 256 threads; with enough tiles for several blocks a SM, 128: two
+    // pencils a thread and more tiles in flight hide a tile's table fill and
+    // barriers better (2^18 points: 64 columns 279 -> 265 us, 32 columns 195 ->
+    // 168 us; 64 tiles of 64 columns 10.7 us with 256, 12.8 with 128).
+    const unsigned threads = std::max<unsigned>(32, std::min<unsigned>(blocks >= 148 * 4 ? 128 : 256, vp2 << (K - K / 2)));
     switch (K) {
 #define LGK_CASE(k)                                                                                 \
     case k:                                                                                         \
