@@ -568,11 +568,15 @@ void induce_dev(lg_ctx *c, Scratch &sc, uint32_t n, const uint32_t *d_rows, uint
 
 // host rows / queries (verifier, kernel-level API) -> induce_dev
 // The enforced sum arrives in pinned memory, valid after sc.finish().
+// (d_rows, d_q: the same rows and queries when they are on the device already)
 const uint32_t *induce_host_rows_later(lg_ctx *c, Scratch &sc, uint32_t n, const uint32_t *rows, size_t nrows,
                                        const uint32_t *vch, uint32_t nch, const std::vector<uint64_t> &q,
-                                       uint32_t alpha, uint32_t *d_out) {
-    const uint32_t *d_rows = sc.upload(rows, nrows << nch);
-    const uint64_t *d_q = sc.upload(q.data(), q.size());
+                                       uint32_t alpha, uint32_t *d_out, const uint32_t *d_rows = nullptr,
+                                       const uint64_t *d_q = nullptr) {
+    if (!d_rows) {
+        d_rows = sc.upload(rows, nrows << nch);
+        d_q = sc.upload(q.data(), q.size());
+    }
     uint32_t *d_sum = static_cast<uint32_t *>(sc.dev(16));
     induce_dev(c, sc, n, d_rows, (uint32_t)nrows, vch, nch, d_q, alpha, d_out, d_sum);
     return sc.download_later(d_sum, 1);
@@ -1212,10 +1216,21 @@ bool opening_ok_host(const std::vector<uint8_t> &root, const lg::Opening &o, siz
 // synchronisation (sc.finish(), which throws their panic).  Nothing the
 // verifier computes depends on them, so deciding them late gives the same
 // outcome as the reference's early panics.
-void check_opening(lg_ctx *c, Scratch &sc, const std::vector<uint8_t> &root, const lg::Opening &o, size_t depth,
-                   const std::vector<uint64_t> &q) {
+// The openings of a proof are checked in one launch, beside each other
+// (run_openings, before that synchronisation).  An opening checked on the
+// device leaves its rows and queries there for the induced basis.
+struct OpeningQueue {
+    lgk::OpeningChecks list;
+    uint32_t count = 0;
+};
+struct DeviceOpening {
+    const uint32_t *rows = nullptr;  // null: checked on the host
+    const uint64_t *q = nullptr;
+};
+DeviceOpening check_opening(lg_ctx *c, Scratch &sc, OpeningQueue &oq, const std::vector<uint8_t> &root,
+                            const lg::Opening &o, size_t depth, const std::vector<uint64_t> &q) {
     const size_t nq = q.size();
-    bool fast = nq >= 1 && nq <= 256 && o.rows.size() >= nq && depth >= 1 && depth <= 63;
+    bool fast = nq >= 1 && nq <= 256 && o.rows.size() >= nq && depth >= 1 && depth <= 31 && oq.count < lgk::kMaxOpenings;
     const size_t ncols = fast ? o.rows.len(0) : 0;
     for (size_t i = 0; fast && i < nq; ++i)
         fast = o.rows.len(i) == ncols && (i == 0 || q[i] > q[i - 1]) && (q[i] >> depth) == 0;
@@ -1228,30 +1243,43 @@ void check_opening(lg_ctx *c, Scratch &sc, const std::vector<uint8_t> &root, con
     }
     if (!fast) {
         if (!opening_ok_host(root, o, depth, q)) throw VerifyPanic{};
-        return;
+        return {};
     }
-    const uint32_t *d_rows = sc.upload(o.rows.data.data(), nq * ncols);
-    const uint64_t *d_q = sc.upload(q.data(), nq);
-    const uint32_t *d_proof = refs.empty() ? nullptr
-                                           : sc.upload(reinterpret_cast<const uint32_t *>(o.merkle.data.data()),
-                                                       8 * refs.size());
-    uint32_t *d_out = static_cast<uint32_t *>(sc.dev(9 * 4));
-    CK(c, lgk::opening_check(c->L, d_rows, (uint32_t)ncols, d_q, (uint32_t)nq, d_proof, (uint32_t)depth, d_out));
-    const uint32_t *h = sc.download_later(d_out, 9);
-    const std::vector<uint8_t> *rp = &root;
-    sc.finalizers.push_back([h, rp]() {
-        if (!(h[8] == 1 && rp->size() == 32 && std::memcmp(h, rp->data(), 32) == 0)) throw VerifyPanic{};
+    // the rows, the proof nodes and the queries as one upload
+    const size_t rw = nq * ncols, rb = (4 * rw + 15) & ~size_t(15), mb = 32 * refs.size(), qb = 8 * nq;
+    uint8_t *h = sc.pin(rb + mb + qb), *d = static_cast<uint8_t *>(sc.dev(rb + mb + qb));
+    std::memcpy(h, o.rows.data.data(), 4 * rw);
+    if (mb) std::memcpy(h + rb, o.merkle.data.data(), mb);
+    std::memcpy(h + rb + mb, q.data(), qb);
+    CK(c, cudaMemcpyAsync(d, h, rb + mb + qb, cudaMemcpyHostToDevice, c->stream));
+    lgk::OpeningCheck &oc = oq.list.c[oq.count++];
+    oc.rows = reinterpret_cast<const uint32_t *>(d);
+    oc.proof = reinterpret_cast<const uint32_t *>(d + rb);
+    oc.q = reinterpret_cast<const uint64_t *>(d + rb + mb);
+    oc.ncols = (uint32_t)ncols;
+    oc.nq = (uint32_t)nq;
+    oc.depth = (uint32_t)depth;
+    return {oc.rows, oc.q};
+}
+void run_openings(lg_ctx *c, Scratch &sc, OpeningQueue &oq, const std::vector<const std::vector<uint8_t> *> &roots) {
+    if (oq.count == 0) return;
+    uint32_t *d_out = static_cast<uint32_t *>(sc.dev(32ull * oq.count));
+    for (uint32_t i = 0; i < oq.count; ++i) oq.list.c[i].out = d_out + 8 * i;
+    CK(c, lgk::opening_check(c->L, oq.list, oq.count));
+    const uint32_t *h = sc.download_later(d_out, 8ull * oq.count);
+    const uint32_t n = oq.count;
+    sc.finalizers.push_back([h, n, roots]() {
+        for (uint32_t i = 0; i < n; ++i)
+            if (!(roots[i]->size() == 32 && std::memcmp(h + 8 * i, roots[i]->data(), 32) == 0)) throw VerifyPanic{};
     });
 }
 
-std::vector<uint32_t> dense(const lg::Opening &o, size_t want_rows, size_t want_len) {
+// want_rows rows of want_len words, back to back, or the panic
+const uint32_t *dense(const lg::Opening &o, size_t want_rows, size_t want_len) {
     if (o.rows.size() != want_rows) throw VerifyPanic{};  // assert_eq (src/sumcheck_polys.rs:98)
-    std::vector<uint32_t> r(want_rows * want_len);
-    for (size_t k = 0; k < want_rows; ++k) {
+    for (size_t k = 0; k < want_rows; ++k)
         if (o.rows.len(k) != want_len) throw VerifyPanic{};  // :97
-        std::copy(o.rows.ptr(k), o.rows.ptr(k) + want_len, r.begin() + k * want_len);
-    }
-    return r;
+    return o.rows.data.data();
 }
 
 // ligero_verify (src/ligero.rs:97-131); rows zip against gr (truncation)
@@ -1285,8 +1313,9 @@ void ligero_verify_host(const std::vector<uint64_t> &q, const lg::Opening &o, co
 // The same check with the per-row work on the device: every panic that
 // does not depend on the field values is decided on the host first, then
 // one block per opened row compares <row, gr> with <yr, basis>.
+// (dop: the opening's rows and queries where check_opening left them, or null)
 void ligero_verify_dev(lg_ctx *c, Scratch &sc, const std::vector<uint64_t> &q, const lg::Opening &o,
-                       const std::vector<uint32_t> &yr, const std::vector<uint32_t> &ch) {
+                       const std::vector<uint32_t> &yr, const std::vector<uint32_t> &ch, const DeviceOpening &dop) {
     const size_t ylen = yr.size();
     if (ylen == 0 || (ylen & (ylen - 1))) throw VerifyPanic{};
     uint32_t nv = 0;
@@ -1299,13 +1328,25 @@ void ligero_verify_dev(lg_ctx *c, Scratch &sc, const std::vector<uint64_t> &q, c
     if (nrows == 0) return;
     const std::vector<uint32_t> gr = lg::lagrange_basis(ch.data(), ch.size());
     const std::vector<uint32_t> sks = lg::eval_sk_at_vks(ylen);
-    const uint32_t *d_rows = sc.upload(o.rows.data.data(), o.rows.data.size());
-    const uint64_t *d_off = sc.upload(o.rows.off.data(), o.rows.off.size());
-    const uint32_t *d_gr = sc.upload(gr.data(), gr.size());
-    const uint32_t *d_yr = sc.upload(yr.data(), ylen);
-    const uint64_t *d_q = sc.upload(q.data(), nrows);
-    uint32_t *d_bad = static_cast<uint32_t *>(sc.dev(4));
-    CK(c, cudaMemsetAsync(d_bad, 0, 4, c->stream));
+    // one upload: the row offsets, a zero word to flag a failure in, gr and
+    // yr; the rows and queries too unless the opening's check left them there
+    // (all rows are there when it saw no more of them than queries)
+    const bool there = dop.rows && nrows == q.size();
+    const size_t no = nrows + 1, nr = there ? 0 : o.rows.data.size(), nqu = there ? 0 : nrows;
+    const size_t bytes = 8 * (no + nqu) + 4 * (1 + gr.size() + ylen + nr);
+    uint8_t *hb = sc.pin(bytes), *db = static_cast<uint8_t *>(sc.dev(bytes));
+    uint64_t *h64 = reinterpret_cast<uint64_t *>(hb);
+    std::memcpy(h64, o.rows.off.data(), 8 * no);
+    if (nqu) std::memcpy(h64 + no, q.data(), 8 * nqu);
+    uint32_t *h32 = reinterpret_cast<uint32_t *>(h64 + no + nqu);
+    h32[0] = 0;
+    std::memcpy(h32 + 1, gr.data(), 4 * gr.size());
+    std::memcpy(h32 + 1 + gr.size(), yr.data(), 4 * ylen);
+    if (nr) std::memcpy(h32 + 1 + gr.size() + ylen, o.rows.data.data(), 4 * nr);
+    CK(c, cudaMemcpyAsync(db, hb, bytes, cudaMemcpyHostToDevice, c->stream));
+    const uint64_t *d_off = reinterpret_cast<const uint64_t *>(db), *d_q = there ? dop.q : d_off + no;
+    uint32_t *d_bad = reinterpret_cast<uint32_t *>(db + 8 * (no + nqu));
+    const uint32_t *d_gr = d_bad + 1, *d_yr = d_gr + gr.size(), *d_rows = there ? dop.rows : d_yr + ylen;
     CK(c, lgk::ligero_check(c->L, d_rows, d_off, (uint32_t)nrows, d_gr, (uint32_t)gr.size(), d_yr, nv, d_q,
                             sks.data(), d_bad));
     const uint32_t *h = sc.download_later(d_bad, 1);
@@ -1326,16 +1367,23 @@ bool verify_impl(lg_ctx *c, Scratch &sc, const lg_config &cfg, const lg::Proof &
     size_t depth = cfg.initial_log_m + log_inv_rate;
     std::vector<uint64_t> q;
     if (!fs.get_distinct_queries(1ull << depth, s, q)) throw VerifyPanic{};
-    check_opening(c, sc, P.initial_root, P.initial, depth, q);  // :42-49
+    OpeningQueue oq;
+    std::vector<const std::vector<uint8_t> *> oroots;  // of the queued openings
+    auto check = [&](const std::vector<uint8_t> &root, const lg::Opening &o) {
+        const DeviceOpening d = check_opening(c, sc, oq, root, o, depth, q);
+        if (d.rows) oroots.push_back(&root);
+        return d;
+    };
+    DeviceOpening dop = check(P.initial_root, P.initial);  // :42-49
     const uint32_t alpha = fs.get_field();
-    std::vector<uint32_t> rows = dense(P.initial, s, 1ull << cfg.initial_k);
+    const uint32_t *rows = dense(P.initial, s, 1ull << cfg.initial_k);
     std::vector<DBuf> basis;
     std::vector<uint32_t> bvars, sep;
     basis.emplace_back(c, 4ull << cfg.initial_log_m);
     bvars.push_back(cfg.initial_log_m);
     sep.push_back(1);
-    const uint32_t *h1 = induce_host_rows_later(c, sc, cfg.initial_log_m, rows.data(), s, pe0.data(),
-                                                cfg.initial_k, q, alpha, basis.back().u32());  // :53-60
+    const uint32_t *h1 = induce_host_rows_later(c, sc, cfg.initial_log_m, rows, s, pe0.data(), cfg.initial_k, q, alpha,
+                                                basis.back().u32(), dop.rows, dop.q);  // :53-60
     // SumcheckVerifierInstance::new (src/ligerito.rs:172-192)
     size_t rd = 0;
     auto read_tr = [&]() {
@@ -1370,8 +1418,9 @@ bool verify_impl(lg_ctx *c, Scratch &sc, const lg_config &cfg, const lg::Proof &
             fs.absorb_u32s(P.yr.data(), P.yr.size());
             depth = cfg.log_m[i] + log_inv_rate;
             if (!fs.get_distinct_queries(1ull << depth, s, q)) throw VerifyPanic{};
-            check_opening(c, sc, root, P.final_, depth, q);
-            ligero_verify_dev(c, sc, q, P.final_, P.yr, rs);
+            dop = check(root, P.final_);
+            run_openings(c, sc, oq, oroots);
+            ligero_verify_dev(c, sc, q, P.final_, P.yr, rs, dop);
             const uint32_t final_r = fs.get_field();  // :114
             const size_t yl = P.yr.size();
             if (yl < 2) throw VerifyPanic{};
@@ -1411,13 +1460,13 @@ bool verify_impl(lg_ctx *c, Scratch &sc, const lg_config &cfg, const lg::Proof &
         fs.absorb(P.recursive_roots[i + 1].data(), P.recursive_roots[i + 1].size());  // :122
         depth = cfg.log_m[i] + log_inv_rate;
         if (!fs.get_distinct_queries(1ull << depth, s, q)) throw VerifyPanic{};  // :126
-        check_opening(c, sc, root, P.recursive[i], depth, q);
+        dop = check(root, P.recursive[i]);
         const uint32_t al = fs.get_field();  // :345
-        std::vector<uint32_t> rr = dense(P.recursive[i], s, 1ull << cfg.ks[i]);
+        const uint32_t *rr = dense(P.recursive[i], s, 1ull << cfg.ks[i]);
         basis.emplace_back(c, 4ull << cfg.log_m[i]);
         bvars.push_back(cfg.log_m[i]);
-        const uint32_t *h = induce_host_rows_later(c, sc, cfg.log_m[i], rr.data(), s, rs.data(), cfg.ks[i], q, al,
-                                                   basis.back().u32());
+        const uint32_t *h = induce_host_rows_later(c, sc, cfg.log_m[i], rr, s, rs.data(), cfg.ks[i], q, al,
+                                                   basis.back().u32(), dop.rows, dop.q);
         g = read_tr();  // introduce_new (src/ligerito.rs:212-220)
         {
             const uint32_t e = g[0] ^ g[1];

@@ -2120,97 +2120,124 @@ cudaError_t induce_fused(Launcher &L, const InducePlan &p, const uint32_t *d_row
 }
 
 // ====================================================== opening check
-// merkle_tree::verify of one opening (src/merkle_tree.rs:120-188) for
-// well-formed inputs, in one block: nq <= 256 sorted distinct queries, their
-// rows of ncols words (1..256) hashed as the leaves, and at least as many
-// 32-byte proof nodes as the opening consumes.  Each layer up, entry i
-// starts a step unless it is the right partner of i-1 (q[i-1] even and
-// q[i] = q[i-1] + 1); a step pairs with its right partner or takes the next
-// proof node (on the left when q[i] is odd); the steps in order are the next
-// layer.  out = the last layer's first hash (8 words) and its size.
-__global__ void __launch_bounds__(256) k_opening_check(const uint32_t *__restrict__ rows, uint32_t ncols,
-                                                       const uint64_t *__restrict__ q, uint32_t nq,
-                                                       const uint32_t *__restrict__ proof, uint32_t depth,
-                                                       uint32_t *__restrict__ out) {
+// merkle_tree::verify (src/merkle_tree.rs:120-188) of well-formed openings,
+// one block each: nq <= 256 sorted distinct queries below 2^depth, their rows
+// of ncols words (1..256) hashed as the leaves, and at least as many 32-byte
+// proof nodes as the opening consumes.
+// Thread i climbs from query i and keeps the hash of the node it stands on in
+// registers.  It and query i-1 meet where their indices' highest differing
+// bit is: there it leaves its hash to the first query under its left sibling
+// and stops.  Everything else about the climb follows from the queries too
+// (which layers have a partner, the place of each proof node: layers in
+// order, nodes in query order), so it is worked out before it, and a layer is
+// one barrier and one compression.  Bound by that chain's latency: the three
+// openings of a 2^24 proof (2^20, 2^16 and 2^12 leaves) take 42 us in one
+// launch (event-timed); a launch each, with the layers compacted in shared
+// memory, took 57 us apiece.
+__global__ void __launch_bounds__(256) k_opening_check(OpeningChecks list) {
     pdl_begin();
-    __shared__ uint32_t h[256][8];
-    __shared__ uint64_t qs[256];
-    __shared__ uint32_t cnt[2][8];
-    const uint32_t t = threadIdx.x, lane = t & 31, warp = t >> 5, nwarps = blockDim.x >> 5;
-    if (t < nq) {
-        const uint32_t nb = (ncols + 15) / 16;
-        uint32_t cv[8];
-        b3_iv(cv);
+    const OpeningCheck o = list.c[blockIdx.x];
+    __shared__ uint32_t qs[256], pmask[256];
+    __shared__ uint32_t slot[2][8][256];
+    __shared__ uint32_t wmask[32][8], wbase[32][8];
+    const uint32_t t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    const bool have = t < o.nq;
+    qs[t] = have ? (uint32_t)o.q[t] : 0u;
+    pmask[t] = 0;
+    __syncthreads();
+    // hp: the layer in which this thread's node meets its left sibling (thread
+    // 0 climbs to the root); owner: the first query under that sibling
+    uint32_t hp = have ? o.depth : 0, owner = 0;
+    const uint32_t qt = qs[t];
+    if (have && t > 0) {
+        hp = 31 - __clz(qt ^ qs[t - 1]);
+        const uint32_t lo = ((qt >> hp) - 1) << hp;
+        uint32_t l = 0, r = t - 1;
+        while (l < r) {
+            const uint32_t m = (l + r) / 2;
+            if (qs[m] < lo) l = m + 1;
+            else r = m;
+        }
+        owner = l;
+        atomicOr(&pmask[owner], 1u << hp);
+    }
+    __syncthreads();
+    const uint32_t partner = pmask[t], act = have ? (hp >= 32 ? ~0u : (1u << hp) - 1) : 0u, uses = act & ~partner;
+    for (uint32_t d = 0; d < o.depth; ++d) {
+        const uint32_t m = __ballot_sync(0xffffffffu, (uses >> d) & 1);
+        if (lane == 0) wmask[d][warp] = m;
+    }
+    // the leaf
+    uint32_t cv[8];
+    b3_iv(cv);
+    if (have) {
+        const uint32_t nb = (o.ncols + 15) / 16;
+        const uint32_t *row = o.rows + (uint64_t)t * o.ncols;
         for (uint32_t b = 0; b < nb; ++b) {
             uint32_t m[16];
 #pragma unroll
-            for (int w = 0; w < 16; ++w) {
-                const uint32_t j = b * 16 + w;
-                m[w] = j < ncols ? rows[(uint64_t)t * ncols + j] : 0u;
-            }
+            for (uint32_t w = 0; w < 16; ++w) m[w] = 16 * b + w < o.ncols ? row[16 * b + w] : 0u;
             const bool last = b + 1 == nb;
-            const uint32_t blen = last ? 4 * ncols - 64 * (nb - 1) : 64;
+            const uint32_t blen = last ? 4 * o.ncols - 64 * (nb - 1) : 64;
             const uint32_t flags = (b == 0 ? B3_CHUNK_START : 0u) | (last ? (B3_CHUNK_END | B3_ROOT) : 0u);
             b3_compress<false>(cv, m, blen, flags);
         }
-#pragma unroll
-        for (int w = 0; w < 8; ++w) h[t][w] = cv[w];
-        qs[t] = q[t];
-    }
-    uint32_t cur = nq, pc_base = 0;
-    for (uint32_t d = 0; d < depth; ++d) {
-        __syncthreads();
-        const bool active = t < cur;
-        const uint64_t qi = active ? qs[t] : 0;
-        const bool right = active && t > 0 && !(qs[t - 1] & 1) && qi == qs[t - 1] + 1;
-        const bool start = active && !right;
-        const bool paired = start && t + 1 < cur && !(qi & 1) && qs[t + 1] == qi + 1;
-        const bool uses = start && !paired;
-        const uint32_t ms = __ballot_sync(0xffffffffu, start), mu = __ballot_sync(0xffffffffu, uses);
-        if (lane == 0) { cnt[0][warp] = __popc(ms); cnt[1][warp] = __popc(mu); }
-        __syncthreads();
-        uint32_t step = __popc(ms & ((1u << lane) - 1)), pidx = __popc(mu & ((1u << lane) - 1));
-        uint32_t nsteps = 0, nuses = 0;
-        for (uint32_t w = 0; w < nwarps; ++w) {
-            if (w < warp) { step += cnt[0][w]; pidx += cnt[1][w]; }
-            nsteps += cnt[0][w];
-            nuses += cnt[1][w];
-        }
-        uint32_t parent[8];
-        if (start) {
-            uint32_t mine[8], other[8];
-#pragma unroll
-            for (int w = 0; w < 8; ++w) mine[w] = h[t][w];
-            if (paired) {
-#pragma unroll
-                for (int w = 0; w < 8; ++w) other[w] = h[t + 1][w];
-                hash_node<false>(mine, other, parent);
-            } else {
-                const uint32_t *nd = proof + 8ull * (pc_base + pidx);
-#pragma unroll
-                for (int w = 0; w < 8; ++w) other[w] = nd[w];
-                if (qi & 1) hash_node<false>(other, mine, parent);
-                else hash_node<false>(mine, other, parent);
-            }
-        }
-        __syncthreads();
-        if (start) {
-#pragma unroll
-            for (int w = 0; w < 8; ++w) h[step][w] = parent[w];
-            qs[step] = qi >> 1;
-        }
-        cur = nsteps;
-        pc_base += nuses;
     }
     __syncthreads();
-    if (t < 8) out[t] = h[0][t];
-    if (t == 8) out[8] = cur;
+    if (warp == 0) {  // lane l: layer l's proof nodes before each warp's
+        uint32_t tot = 0;
+        if (lane < o.depth)
+            for (uint32_t w = 0; w < 8; ++w) {
+                wbase[lane][w] = tot;
+                tot += __popc(wmask[lane][w]);
+            }
+        uint32_t inc = tot;
+        for (uint32_t s = 1; s < 32; s <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xffffffffu, inc, s);
+            if (lane >= s) inc += y;
+        }
+        if (lane < o.depth)
+            for (uint32_t w = 0; w < 8; ++w) wbase[lane][w] += inc - tot;
+    }
+    __syncthreads();
+    uint32_t nxt[8];
+    auto fetch = [&](uint32_t d) {  // this thread's proof node of layer d
+        if (d >= o.depth || !((uses >> d) & 1)) return;
+        const uint32_t pos = wbase[d][warp] + __popc(wmask[d][warp] & ((1u << lane) - 1));
+        load_node(o.proof + 8ull * pos, nxt);
+    };
+    fetch(0);
+    for (uint32_t d = 0; d < o.depth; ++d) {
+        if (have && t > 0 && hp == d) {
+#pragma unroll
+            for (int w = 0; w < 8; ++w) slot[d & 1][w][owner] = cv[w];
+        }
+        __syncthreads();
+        if ((act >> d) & 1) {
+            // even nodes have the other one on the right
+            uint32_t m[16];
+            const bool right = (qt >> d) & 1;
+#pragma unroll
+            for (int w = 0; w < 8; ++w) {
+                const uint32_t x = (partner >> d) & 1 ? slot[d & 1][w][t] : nxt[w];
+                m[w] = right ? x : cv[w];
+                m[8 + w] = right ? cv[w] : x;
+            }
+            fetch(d + 1);
+            b3_iv(cv);
+            b3_compress<false>(cv, m, 64, B3_CHUNK_START | B3_CHUNK_END | B3_ROOT);
+        }
+    }
+    if (t == 0) store_node(o.out, cv);
 }
-cudaError_t opening_check(Launcher &L, const uint32_t *rows, uint32_t ncols, const uint64_t *q, uint32_t nq,
-                          const uint32_t *proof, uint32_t depth, uint32_t *out) {
-    if (nq == 0 || nq > 256 || ncols == 0 || ncols > 256 || depth > 63) return cudaErrorInvalidValue;
-    LGK_LAUNCH(L, "opening_check", launch_k(k_opening_check, 1, 256, 0, L.stream, rows, ncols, q, nq, proof, depth,
-                                            out));
+cudaError_t opening_check(Launcher &L, const OpeningChecks &list, uint32_t count) {
+    if (count == 0) return cudaSuccess;
+    if (count > kMaxOpenings) return cudaErrorInvalidValue;
+    for (uint32_t i = 0; i < count; ++i) {
+        const OpeningCheck &o = list.c[i];
+        if (o.nq == 0 || o.nq > 256 || o.ncols == 0 || o.ncols > 256 || o.depth > 31) return cudaErrorInvalidValue;
+    }
+    LGK_LAUNCH(L, "opening_check", launch_k(k_opening_check, count, 256, 0, L.stream, list));
     return cudaGetLastError();
 }
 

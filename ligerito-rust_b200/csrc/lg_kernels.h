@@ -275,13 +275,21 @@ cudaError_t induce_fused(Launcher &L, const InducePlan &p, const uint32_t *d_row
 
 cudaError_t splitmix(Launcher &L, uint64_t seed, uint32_t *out, uint64_t n);
 
-// --- merkle_tree::verify of one opening (src/merkle_tree.rs:120-188) ------
-// Well-formed inputs only (the caller checks): nq <= 256 sorted distinct
-// queries, their rows (nq x ncols words, 1 <= ncols <= 256) and the 32-byte
-// proof nodes the opening consumes (8 words each, in order).  out (9 words)
-// = the last layer's first hash and the last layer's size.
-cudaError_t opening_check(Launcher &L, const uint32_t *rows, uint32_t ncols, const uint64_t *q, uint32_t nq,
-                          const uint32_t *proof, uint32_t depth, uint32_t *out);
+// --- merkle_tree::verify of openings (src/merkle_tree.rs:120-188) ---------
+// Well-formed ones only (the caller checks): nq <= 256 sorted distinct
+// queries below 2^depth (depth <= 31), their rows (nq x ncols words, 1 <=
+// ncols <= 256) and the 32-byte proof nodes the opening consumes (8 words
+// each, in order, 16-byte aligned).  out (8 words, 16-byte aligned): the root
+// they lead to.
+struct OpeningCheck {
+    const uint32_t *rows = nullptr, *proof = nullptr;
+    const uint64_t *q = nullptr;
+    uint32_t *out = nullptr;
+    uint32_t ncols = 0, nq = 0, depth = 0;
+};
+constexpr uint32_t kMaxOpenings = 10;
+struct OpeningChecks { OpeningCheck c[kMaxOpenings]; };
+cudaError_t opening_check(Launcher &L, const OpeningChecks &list, uint32_t count);
 
 // --- ligero_verify (src/ligero.rs:97-131) ----------------------------------
 // Rows k < nrows at rows[row_off[k] .. row_off[k+1]), the Lagrange basis gr
