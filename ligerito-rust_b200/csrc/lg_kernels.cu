@@ -244,7 +244,7 @@ __device__ __forceinline__ void pencil_stages(uint32_t (&v)[1 << KP], const uint
 // (a.bulk: rows of S >= 32 words, 16-byte aligned): `cnt` pencils from the
 // one at `src` on, columns `cs` words apart.
 template <int K>
-__device__ __forceinline__ void issue_unit(const uint32_t *src, uint64_t cs, uint32_t log_S, uint32_t cnt, uint32_t *buf,
+__device__ __forceinline__ void issue_unit(const uint32_t *src, uint32_t cs, uint32_t log_S, uint32_t cnt, uint32_t *buf,
                                            uint64_t *bar) {
     constexpr uint32_t R = 1u << K;
     const uint32_t B = blockDim.x, tid = threadIdx.x, S4 = 4u << log_S;
@@ -255,7 +255,7 @@ __device__ __forceinline__ void issue_unit(const uint32_t *src, uint64_t cs, uin
         const uint32_t n = R * (cnt >> log_S);
         for (uint32_t c = tid; c < n; c += B) {
             const uint32_t t = c & (R - 1), col = c >> K;
-            bulk_load(buf + t * B + (col << log_S), strided(src + col * cs, t, S4), S4, bar);
+            bulk_load(buf + t * B + (col << log_S), strided(src + (uint64_t)col * cs, t, S4), S4, bar);
         }
     }
 }
@@ -279,19 +279,20 @@ __global__ void __launch_bounds__(256, K <= 4 ? 4 : (K == 5 ? 3 : 2)) k_fft_pass
     uint64_t *bar = reinterpret_cast<uint64_t *>(buf + R * B);
     const uint32_t U = (uint32_t)a.units, nb = gridDim.x;
     const uint32_t u0 = (uint32_t)((uint64_t)blockIdx.x * U / nb), u1 = (uint32_t)((uint64_t)(blockIdx.x + 1) * U / nb);
-    const uint64_t G = (uint64_t)a.nvec << a.log_S;  // pencils of a group
-    const uint32_t S4 = 4u << a.log_S;               // bytes between pencil values (a vector is < 4 GiB)
+    const uint32_t G = a.nvec << a.log_S, smask = (1u << a.log_S) - 1;  // pencils of a group (< 2^32 - 256)
+    const uint32_t S4 = 4u << a.log_S;  // bytes between pencil values (a vector is < 4 GiB)
+    const uint32_t cs = (uint32_t)a.col_stride;
     // the group's first word, and where pencil g of it starts
     auto group = [&](uint32_t grp) {
         return a.data + (grp >> a.d0) * a.q_stride + ((uint64_t)(grp & ((1u << a.d0) - 1)) << (a.L - a.d0));
     };
-    auto pencil = [&](uint32_t *gp, uint64_t g) { return gp + (g >> a.log_S) * a.col_stride + (g & ((1ull << a.log_S) - 1)); };
+    auto pencil = [&](uint32_t *gp, uint32_t g) { return gp + (uint64_t)(g >> a.log_S) * cs + (g & smask); };
     uint32_t grp = u0 / a.bpg, ch = u0 - grp * a.bpg, parity = 0;
     uint32_t *gp = group(grp);
     uint32_t nv[PF ? R : 1], *p = gp;
     bool mine = false;
     auto prefetch = [&]() {  // the pencil of chunk ch of the group at gp
-        const uint64_t g = (uint64_t)ch * B + tid;
+        const uint32_t g = ch * B + tid;
         mine = g < G;
         p = pencil(gp, g);
         if (PF && mine) {
@@ -300,8 +301,8 @@ __global__ void __launch_bounds__(256, K <= 4 ? 4 : (K == 5 ? 3 : 2)) k_fft_pass
         }
     };
     auto issue = [&]() {
-        const uint64_t g0 = (uint64_t)ch * B;
-        issue_unit<K>(pencil(gp, g0), a.col_stride, a.log_S, (uint32_t)min((uint64_t)B, G - g0), buf, bar);
+        const uint32_t g0 = ch * B;
+        issue_unit<K>(pencil(gp, g0), cs, a.log_S, min(B, G - g0), buf, bar);
     };
     if (!PF && a.bulk) {
         if (tid == 0) {
@@ -378,12 +379,12 @@ __global__ void __launch_bounds__(256, K <= 4 ? 3 : 2) k_rs_first(PassArgs a) {
     // of units to one (contiguous shares of 9 or 10 units a block left SMs
     // with 27 to 30)
     const uint32_t U = (uint32_t)a.units, u0 = blockIdx.x, nb = gridDim.x;
-    const uint64_t G = (uint64_t)a.nvec << a.log_S;  // pencils
-    const uint32_t S4 = 4u << a.log_S;               // bytes between pencil values
+    const uint32_t G = a.nvec << a.log_S, smask = (1u << a.log_S) - 1;  // pencils (< 2^32 - 256)
+    const uint32_t S4 = 4u << a.log_S;  // bytes between pencil values
+    const uint32_t cs = (uint32_t)a.col_stride, scs = (uint32_t)a.src_col_stride;
     auto issue = [&](uint32_t u) {
-        const uint64_t g0 = (uint64_t)u * B;
-        issue_unit<K>(a.src + (g0 >> a.log_S) * a.src_col_stride + (g0 & ((1ull << a.log_S) - 1)), a.src_col_stride,
-                      a.log_S, (uint32_t)min((uint64_t)B, G - g0), buf, bar);
+        const uint32_t g0 = u * B;
+        issue_unit<K>(a.src + (uint64_t)(g0 >> a.log_S) * scs + (g0 & smask), scs, a.log_S, min(B, G - g0), buf, bar);
     };
     if (a.bulk) {
         if (tid == 0) {
@@ -420,9 +421,9 @@ __global__ void __launch_bounds__(256, K <= 4 ? 3 : 2) k_rs_first(PassArgs a) {
     __syncthreads();
     uint32_t parity = 0;
     for (uint32_t u = u0; u < U; u += nb) {
-        const uint64_t g = (uint64_t)u * B + tid;
+        const uint32_t g = u * B + tid;
         const bool mine = g < G;
-        const uint64_t col = g >> a.log_S, o = g & ((1ull << a.log_S) - 1);
+        const uint32_t col = g >> a.log_S, o = g & smask;
         uint32_t v[R];
         const uint32_t *pp = a.pis + o;
         if (a.bulk) {
@@ -435,7 +436,7 @@ __global__ void __launch_bounds__(256, K <= 4 ? 3 : 2) k_rs_first(PassArgs a) {
             __syncthreads();  // the values are in registers: the next unit's copies may land
             if (u + nb < U) issue(u + nb);
         } else if (mine) {
-            const uint32_t *lb = a.src + col * a.src_col_stride + o;
+            const uint32_t *lb = a.src + (uint64_t)col * scs + o;
 #pragma unroll
             for (uint32_t t = 0; t < R; ++t) v[t] = *strided(lb, t, S4);
         }
@@ -448,7 +449,7 @@ __global__ void __launch_bounds__(256, K <= 4 ? 3 : 2) k_rs_first(PassArgs a) {
             p1[i] = tab_mul_sa(smraw, 0, QT, v[H + i]);
             p2[i] = tab_mul_sa(smraw, 0, 2 * QT, v[H + i]);
         }
-        uint32_t *out = a.data + col * a.col_stride + o;
+        uint32_t *out = a.data + (uint64_t)col * cs + o;
         {
             uint32_t x[H], y[H];
 #pragma unroll
@@ -718,6 +719,7 @@ static bool plan_valid(const FftPlan &pl, uint32_t log_len) {
     return sum == log_len;
 }
 
+constexpr uint64_t kMaxFftWords = 1ull << 32;  // of a call's vectors: pencils have at least two words
 cudaError_t fft_vectors(Launcher &L, uint32_t *data, const uint32_t *tw, uint32_t log_len,
                         uint32_t nvec, uint64_t col_stride, uint32_t Q, uint64_t q_stride,
                         uint32_t root_base, bool inverse, FftPasses passes, const FftSrc *src) {
@@ -727,6 +729,21 @@ cudaError_t fft_vectors(Launcher &L, uint32_t *data, const uint32_t *tw, uint32_
     if (src && (inverse || log_len <= 6 || passes == FFT_LAST || Q != 4 || root_base != 4 || !src->pis))
         return cudaErrorInvalidValue;
     // the roots root_base + q (q < Q) must share one heap layer
+    // the passes count pencils and stride columns in 32 bits: larger batches
+    // run in parts
+    if (col_stride >> 32 || (src && src->col_stride >> 32)) return cudaErrorInvalidValue;
+    if (((uint64_t)nvec << log_len) > kMaxFftWords && nvec > 1) {
+        const uint32_t half = nvec / 2;
+        FftSrc s2;
+        if (src) {
+            s2 = *src;
+            s2.p += half * src->col_stride;
+        }
+        cudaError_t e = fft_vectors(L, data, tw, log_len, half, col_stride, Q, q_stride, root_base, inverse, passes, src);
+        if (e != cudaSuccess) return e;
+        return fft_vectors(L, data + half * col_stride, tw, log_len, nvec - half, col_stride, Q, q_stride, root_base,
+                           inverse, passes, src ? &s2 : nullptr);
+    }
     const uint32_t lr = 31 - __builtin_clz(root_base);
     if (!L.dtab || root_base == 0 || ((root_base + Q - 1) >> lr) != 1) return cudaErrorInvalidValue;
     // head / last calls on column groups must agree on the split, so only
