@@ -589,15 +589,21 @@ uint32_t induce_host_rows(lg_ctx *c, Scratch &sc, uint32_t n, const uint32_t *ro
     return *h;
 }
 
-// partial_eval by any number of challenges (host rs, or device d_rs),
-// chunks of <= 6 per launch
+// Variables folded by the next launch: all that are left if they split, else
+// at most 6.
+uint32_t fold_step(uint32_t cur, uint32_t left, uint32_t B) {
+    if (lgk::fold_splits(cur, left, B)) return left;
+    return std::min<uint32_t>(6, left);
+}
+// partial_eval by any number of challenges (host rs, or device d_rs), a few
+// of them per launch
 void partial_eval_dev(lg_ctx *c, const uint32_t *d_in, uint32_t log_len, const uint32_t *rs, uint32_t k,
                       uint32_t *d_out, const uint32_t *d_rs = nullptr) {
     DBuf tmp[2];
     const uint32_t *src = d_in;
     uint32_t cur = log_len, done = 0, which = 0;
     while (done < k) {
-        const uint32_t kk = std::min<uint32_t>(6, k - done);
+        const uint32_t kk = fold_step(cur, k - done, 1);
         uint32_t *dst;
         if (done + kk == k) dst = d_out;
         else {
@@ -970,7 +976,7 @@ void partial_eval_batch(lg_ctx *c, const uint32_t *d_in, uint64_t in_stride, uin
     uint64_t src_stride = in_stride;
     uint32_t cur = log_len, done = 0, which = 0;
     while (done < k) {
-        const uint32_t kk = std::min<uint32_t>(6, k - done);
+        const uint32_t kk = fold_step(cur, k - done, B);
         uint32_t *dst;
         if (done + kk == k) dst = d_out;
         else {

@@ -1154,6 +1154,30 @@ __device__ __forceinline__ uint32_t lagrange_at(const uint32_t *rs, uint32_t k, 
     return p;
 }
 
+// ============================================================== clusters
+__device__ __forceinline__ uint32_t cluster_rank() {
+    uint32_t r;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return r;
+}
+__device__ __forceinline__ void cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+}
+__device__ __forceinline__ uint32_t cluster_load(const uint32_t *p, uint32_t rank) {
+    uint32_t v;
+    asm volatile("{\n\t.reg .b32 a;\n\tmapa.shared::cluster.u32 a, %1, %2;\n\tld.shared::cluster.u32 %0, [a];\n\t}"
+                 : "=r"(v)
+                 : "r"((uint32_t)__cvta_generic_to_shared(p)), "r"(rank)
+                 : "memory");
+    return v;
+}
+__device__ __forceinline__ void cluster_store(const uint32_t *p, uint32_t rank, uint32_t v) {
+    asm volatile("{\n\t.reg .b32 a;\n\tmapa.shared::cluster.u32 a, %0, %1;\n\tst.shared::cluster.u32 [a], %2;\n\t}" ::"r"(
+                     (uint32_t)__cvta_generic_to_shared(p)),
+                 "r"(rank), "r"(v)
+                 : "memory");
+}
+
 // ================================================================= folds
 // partial_eval over the top k variables (src/multilinear_poly.rs:66-87):
 // out[i] = sum_j eq(rs, j) in[j*M + i], j's top bit with rs[0] -- the
@@ -1166,7 +1190,7 @@ __device__ __forceinline__ uint32_t lagrange_at(const uint32_t *rs, uint32_t k, 
 // once and then loops over outputs, four consecutive ones per thread (one
 // 16-byte load per term); every product in an inner sum is independent of
 // the others, so loads and lookups overlap.
-struct Rs6 { uint32_t v[6]; };
+struct Rs6 { uint32_t v[kMaxFold]; };
 
 template <int KH, int KL, int V>
 __global__ void __launch_bounds__(256) k_fold_eq(const uint32_t *__restrict__ in, uint32_t *__restrict__ out,
@@ -1248,16 +1272,101 @@ __global__ void __launch_bounds__(256) k_fold_eq(const uint32_t *__restrict__ in
     }
 }
 
+// The same sum when there are few outputs: a cluster of 8 blocks takes 256
+// of them, block c the terms of its NH / 8 high indexes jh, and the blocks'
+// partial sums meet in shared memory (block c adds up outputs 32 c .. 32 c +
+// 31).  Bound by latency: a term's load, product and sum are 8 times fewer a
+// thread, and up to 9 variables fold at once.
+template <int KH, int KL>
+__global__ void __launch_bounds__(256) k_fold_split(const uint32_t *__restrict__ in, uint32_t *__restrict__ out,
+                                                    uint64_t M, Rs6 rs, const uint32_t *d_rs, FoldStrides st) {
+    pdl_begin();
+    in += blockIdx.y * st.in;  // lockstep batch: proof blockIdx.y
+    out += blockIdx.y * st.out;
+    if (d_rs) d_rs += blockIdx.y * st.rs;
+    constexpr int NH = 1 << KH, NL = 1 << KL, H = NH / 8;
+    __shared__ __align__(512) uint32_t tabs[NL + H][kTabWords];  // EL tables, then this block's EH
+    __shared__ uint32_t r[KH + KL], ec[NL + H], part[256], red[8][32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const uint32_t c = cluster_rank();
+    const uint64_t o0 = (uint64_t)(blockIdx.x / 8) * 256, o = o0 + threadIdx.x;
+    const bool mine = o < M;
+    uint32_t v[H * NL];
+    if (mine) {
+#pragma unroll
+        for (int j = 0; j < H * NL; ++j) v[j] = __ldg(in + o + (uint64_t)(c * H * NL + j) * M);
+    }
+    if (threadIdx.x < KH + KL) r[threadIdx.x] = d_rs ? d_rs[threadIdx.x] : rs.v[threadIdx.x];
+    __syncthreads();
+    if (threadIdx.x < NL + H) {  // the constants as in k_fold_eq
+        const int t = threadIdx.x;
+        const bool lo = t < NL;
+        const int j = lo ? t : (int)c * H + t - NL, nb = lo ? KL : KH, off = lo ? KH : 0;
+        uint32_t e = 1;
+        for (int b = 0; b < nb; ++b) e = gf_mul(e, ((j >> (nb - 1 - b)) & 1) ? r[off + b] : 1u ^ r[off + b]);
+        ec[t] = e;
+    }
+    __syncthreads();
+    for (int t = warp; t < NL + H; t += 8) tab_build_warp(tabs[t], ec[t], lane);
+    __syncthreads();
+    const uint8_t *t8 = reinterpret_cast<const uint8_t *>(&tabs[0][0]);
+    uint32_t acc = 0;
+    if (mine) {
+#pragma unroll
+        for (int h = 0; h < H; ++h) {
+            uint32_t sum = 0;
+#pragma unroll
+            for (int j = 0; j < NL; ++j) sum ^= tab_mul_sa(t8, 512u * j, 0, v[h * NL + j]);
+            acc ^= tab_mul_sa(t8, 512u * (NL + h), 0, sum);
+        }
+    }
+    part[threadIdx.x] = acc;
+    cluster_sync();
+    red[warp][lane] = cluster_load(&part[32 * c + lane], warp);
+    __syncthreads();
+    if (warp == 0) {
+        uint32_t x = 0;
+#pragma unroll
+        for (int w = 0; w < 8; ++w) x ^= red[w][lane];
+        if (o0 + 32 * c + lane < M) out[o0 + 32 * c + lane] = x;
+    }
+    cluster_sync();  // no block leaves while its sums may still be read
+}
+
+// Few outputs: the split form, where one thread an output would leave most of
+// the device idle (2^10 outputs of 64 terms on 4 blocks: 5.8 us, split 3.6).
+// More than 6 variables at once only for very few outputs: 2^22 words by 9
+// take 22 us so, 13 us as 6 and then 3.
+bool fold_splits(uint32_t log_len, uint32_t k, uint32_t B) {
+    if (k < 4 || k > kMaxFold || log_len < k) return false;
+    const uint64_t chunks = (((1ull << (log_len - k)) + 255) / 256) * B;
+    return chunks <= (k <= 6 ? 64 : 8);
+}
+
 static bool tuned_fold(const TuneKey &k, int *bps);
 static void tune_fold(Launcher &L, const TuneKey &k, const uint32_t *rs, const uint32_t *d_rs);
 
 cudaError_t fold_eq(Launcher &L, const uint32_t *in, uint32_t *out, uint32_t log_len, uint32_t k,
                     const uint32_t *rs, const uint32_t *d_rs, uint32_t B, const FoldStrides &st) {
-    if (k < 1 || k > 6 || k > log_len || (!rs && !d_rs) || B == 0 || B > 65535) return cudaErrorInvalidValue;
+    const bool split = fold_splits(log_len, k, B) && !L.forced_fold_bps;
+    if (k < 1 || (k > 6 && !split) || k > log_len || (!rs && !d_rs) || B == 0 || B > 65535) return cudaErrorInvalidValue;
     Rs6 c{};
     if (!d_rs)
         for (uint32_t j = 0; j < k; ++j) c.v[j] = rs[j];
     const uint64_t M = 1ull << (log_len - k);
+    if (split) {
+        const dim3 grid((unsigned)((M + 255) / 256) * 8, B);
+        L.note(B * (4.0 * (M << k) + 4.0 * M), (double)B * M * (1u << k));
+        switch (k) {
+#define LGK_CASE(kk, kh)                                                                                   \
+    case kk:                                                                                               \
+        LGK_LAUNCH(L, "fold_eq", launch_kc(k_fold_split<kh, kk - kh>, grid, 256, 8, 0, L.stream, in, out, M, c, d_rs, st)); \
+        break;
+            LGK_CASE(4, 3) LGK_CASE(5, 3) LGK_CASE(6, 3) LGK_CASE(7, 3) LGK_CASE(8, 4) LGK_CASE(9, 4)
+#undef LGK_CASE
+        }
+        return cudaGetLastError();
+    }
     const uint32_t kh = k / 2;
     // grid choice: blocks per SM in the low byte, bit 8 for four outputs
     // per thread; tuned per shape (one output per thread, 4 blocks per SM
@@ -1479,20 +1588,6 @@ struct SumStepShared {
 };
 static_assert(offsetof(SumStepShared, work) % 16 == 0, "the schedules' rows are read 16 bytes at a time");
 constexpr uint32_t kSumThreads = 256;
-__device__ __forceinline__ uint32_t cluster_rank() {
-    uint32_t r;
-    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-    return r;
-}
-__device__ __forceinline__ void cluster_sync() {
-    asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
-}
-__device__ __forceinline__ void cluster_store(const uint32_t *p, uint32_t rank, uint32_t v) {
-    asm volatile("{\n\t.reg .b32 a;\n\tmapa.shared::cluster.u32 a, %0, %1;\n\tst.shared::cluster.u32 [a], %2;\n\t}" ::"r"(
-                     (uint32_t)__cvta_generic_to_shared(p)),
-                 "r"(rank), "r"(v)
-                 : "memory");
-}
 __global__ void __launch_bounds__(kSumThreads) k_sum_step(SumStepArgs a, RoundStrides st, uint32_t C) {
     pdl_begin();
     extern __shared__ __align__(512) uint8_t ssraw[];
@@ -1899,19 +1994,27 @@ __global__ void __launch_bounds__(256, 2) k_induce_main2(const uint32_t *__restr
         uint32_t acc0[ACC], acc1[ACC];
 #pragma unroll
         for (int c = 0; c < ACC; ++c) acc0[c] = acc1[c] = 0;
-        // the query's Lo words are loaded (from L2) before the warp builds
-        // its table, so their latency passes under the build
-        for (uint32_t k = k0 + warp; k < k1; k += nw) {
-            const uint32_t *lk = lop + (uint64_t)k * nlo + lane;
-            uint32_t v[ACC];
+        // the next query's Hi pair and Lo words are loaded (from L2) while the
+        // current one's are multiplied: each Lo word right after the product
+        // that frees its register
+        uint32_t v[ACC];
+        uint2 h = make_uint2(0, 0);
+        if (k0 + warp < k1) {
+            const uint32_t *lk = lop + (uint64_t)(k0 + warp) * nlo + lane;
 #pragma unroll
             for (int c = 0; c < ACC; ++c) v[c] = __ldg(lk + 32 * c);
-            const uint2 h = __ldg(reinterpret_cast<const uint2 *>(hip + (uint64_t)k * nhi) + tp);
+            h = __ldg(reinterpret_cast<const uint2 *>(hip + (uint64_t)(k0 + warp) * nhi) + tp);
+        }
+        for (uint32_t k = k0 + warp; k < k1; k += nw) {
             tab2_build_warp(tabs[warp], h.x, h.y, lane);
             __syncwarp();
+            const uint32_t kn = k + nw < k1 ? k + nw : k;
+            const uint32_t *lk = lop + (uint64_t)kn * nlo + lane;
+            h = __ldg(reinterpret_cast<const uint2 *>(hip + (uint64_t)kn * nhi) + tp);
 #pragma unroll
             for (int c = 0; c < ACC; ++c) {
                 const uint2 r = tab2_mul_sa(tab8, 1024u * warp, v[c]);
+                v[c] = __ldg(lk + 32 * c);
                 acc0[c] ^= r.x;
                 acc1[c] ^= r.y;
             }
@@ -2128,7 +2231,10 @@ cudaError_t induce_fused(Launcher &L, const InducePlan &p, const uint32_t *d_row
     L.note(4.0 * B * (vec + nq * (glen + 2)), B * (vec + nq * (glen + 2.0 * n + 20)));
     const size_t words = (1ull << p.b) + (1ull << (n - p.b));
     const int in_smem = words <= 10240;  // with the static arrays, under the 48 KB that needs no opt-in
-    LGK_LAUNCH(L, "induce_sp", launch_k(k_induce_sp, dim3(nq, B), 256, in_smem ? 4 * words : 0, L.stream, d_rows, glen,
+    // one block a query: more than the device holds at 256 threads go out with
+    // 128, twice as many at a time (23 x 148 queries of 2^12: 40 -> 30 us)
+    const unsigned threads = (uint64_t)nq * B > 148 * 8 ? 128 : 256;
+    LGK_LAUNCH(L, "induce_sp", launch_k(k_induce_sp, dim3(nq, B), threads, in_smem ? 4 * words : 0, L.stream, d_rows, glen,
                                         d_q, nq, alpha, n, p.b, args, d_rs, ilog2u(glen), d_alpha, d_apow, d_lo, d_hi,
                                         d_sum, in_smem, out, L.tickets, st));
     cudaError_t e = cudaGetLastError();

@@ -210,7 +210,10 @@ cudaError_t gather_opening(Launcher &L, const uint32_t *E, uint64_t rows, uint32
 // --- multilinear folds (src/multilinear_poly.rs:66-87) -------------------
 // partial_eval of the top k variables (1 <= k <= 6): out (M = 2^log_len >> k
 // words) = sum_j eq(rs, j) * in[j*M + i], rs[0] for j's top bit; the k
-// challenges on the host (rs) or the device (d_rs).
+// challenges on the host (rs) or the device (d_rs).  Up to kMaxFold variables
+// where fold_splits says so (few outputs).
+constexpr uint32_t kMaxFold = 9;
+bool fold_splits(uint32_t log_len, uint32_t k, uint32_t B);
 struct FoldStrides { uint64_t in = 0, out = 0, rs = 0; };
 cudaError_t fold_eq(Launcher &L, const uint32_t *in, uint32_t *out, uint32_t log_len, uint32_t k,
                     const uint32_t *rs, const uint32_t *d_rs = nullptr, uint32_t B = 1,
