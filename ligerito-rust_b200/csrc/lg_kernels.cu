@@ -692,17 +692,35 @@ static cudaError_t launch_tail(Launcher &L, int K, PassArgs a, unsigned blocks) 
     return cudaGetLastError();
 }
 
-// Stage split: the last pass (register phases over shared-memory tiles,
-// many warps per SM) takes up to 6 stages; the strided passes before it
-// hold a 2^K-value pencil per thread, and K = 4-5 keeps twice the warps per
-// SM of K = 6 (measured faster per stage) while still doing several stages
-// per trip through HBM.  The autotuner may replace it per shape.
-FftPlan default_fft_plan(uint32_t log_len) {
+// Stage split of `words` words in all (rs: of a Reed-Solomon encoding, whose
+// first pass runs all four quarters of a pencil).
+//   * The last pass (tiles in shared memory) takes 6 stages, fewer when the
+//     transform is small: its blocks are then few and each waits for its
+//     tables, which double with every stage (2^12 x 64 columns: 37 us as 6 + 6,
+//     24 as 4 + 3 + 5; 2^10 x 64: 24 as 4 + 6, 20 as 3 + 3 + 4; from 2^22 words
+//     on the splits lie within 8% of each other and past that 6 wins), or when
+//     a tile holds few vectors to share its tables (one of 2^22: 500 us with
+//     6, 340 with 5).
+//   * The strided passes before it hold a 2^K-value pencil a thread.  5 stages
+//     cost 40 us a stage at 2^20 x 64, 4 stages 41; 6 stages and a first pass
+//     of 5 over all quarters need so many registers and so much code that they
+//     lose (2^16 x 64 x 4: 225 us as 5 + 5 + 6, 207 as 3 + 3 + 4 + 6).  So as
+//     few passes of at most 5 (4) as will do, the shorter ones first; of at
+//     most 4 where the transform is small and more threads hide more latency
+//     (2^14 x 64: 37 us as 4 + 4 + 6, 31.5 as 3 + 3 + 3 + 5).
+// The autotuner may replace it per shape.
+FftPlan default_fft_plan(uint32_t log_len, uint64_t words, uint32_t nvec, bool rs) {
     FftPlan pl;
-    const uint32_t kt = std::min<uint32_t>(6, log_len), rem = log_len - kt;
-    const uint32_t nps = rem == 0 ? 0 : (rem <= 6 ? 1 : (rem + 4) / 5);
+    uint32_t kt = std::min<uint32_t>(6, log_len);
+    if (log_len >= (rs ? 9u : 7u) && log_len <= 24) {  // (at most kMaxFftPasses passes)
+        if (words <= (1ull << 17)) kt = 4;
+        else if ((words <= (1ull << 20) || nvec < 8) && !(rs && log_len <= 10)) kt = 5;
+    }
+    const uint32_t rem = log_len - kt, most = kt < 6 ? 4 : 5, first = rs ? kRsFirstStages : most;
+    uint32_t nps = 0;
+    while (rem > 0 && (nps == 0 || first + most * (nps - 1) < rem)) ++nps;
     pl.np = nps + 1;
-    for (uint32_t i = 0; i < nps && i < kMaxFftPasses; ++i) pl.ks[i] = rem / nps + (i < rem % nps ? 1 : 0);
+    for (uint32_t i = 0; i < nps && i < kMaxFftPasses; ++i) pl.ks[i] = rem / nps + (nps - i <= rem % nps ? 1 : 0);
     if (nps < kMaxFftPasses) pl.ks[nps] = kt;
     return pl;
 }
@@ -748,10 +766,9 @@ cudaError_t fft_vectors(Launcher &L, uint32_t *data, const uint32_t *tw, uint32_
     if (!L.dtab || root_base == 0 || ((root_base + Q - 1) >> lr) != 1) return cudaErrorInvalidValue;
     // head / last calls on column groups must agree on the split, so only
     // whole transforms take tuned plans
-    FftPlan plan = default_fft_plan(log_len);
-    if (src && plan.ks[0] > kMaxRsFirst) {  // (log_len = 12)
-        plan = FftPlan{3, {plan.ks[0] / 2, plan.ks[0] - plan.ks[0] / 2, plan.ks[1]}};
-    }
+    // (nor does the size of one group change the default)
+    const uint64_t words = passes == FFT_ALL ? (uint64_t)Q * nvec << log_len : ~0ull;
+    FftPlan plan = default_fft_plan(log_len, words, passes == FFT_ALL ? nvec : ~0u, src != nullptr || passes != FFT_ALL);
     if (passes == FFT_ALL && !L.forced_plan) {
         const TuneKey tk{L.device, log_len, nvec, Q, src != nullptr, inverse, 0};
         if (!tuned_fft_plan(tk, &plan) && L.autotune) {
@@ -1344,17 +1361,34 @@ bool fold_splits(uint32_t log_len, uint32_t k, uint32_t B) {
 }
 
 static bool tuned_fold(const TuneKey &k, int *bps);
-static void tune_fold(Launcher &L, const TuneKey &k, const uint32_t *rs, const uint32_t *d_rs);
+static void tune_fold(Launcher &L, const TuneKey &k, bool few);
+constexpr int kFoldVec4 = 0x100, kFoldSplit = 0x200;
 
 cudaError_t fold_eq(Launcher &L, const uint32_t *in, uint32_t *out, uint32_t log_len, uint32_t k,
                     const uint32_t *rs, const uint32_t *d_rs, uint32_t B, const FoldStrides &st) {
-    const bool split = fold_splits(log_len, k, B) && !L.forced_fold_bps;
-    if (k < 1 || (k > 6 && !split) || k > log_len || (!rs && !d_rs) || B == 0 || B > 65535) return cudaErrorInvalidValue;
+    const bool few = fold_splits(log_len, k, B);
+    if (k < 1 || (k > 6 && !few) || k > log_len || (!rs && !d_rs) || B == 0 || B > 65535) return cudaErrorInvalidValue;
     Rs6 c{};
     if (!d_rs)
         for (uint32_t j = 0; j < k; ++j) c.v[j] = rs[j];
     const uint64_t M = 1ull << (log_len - k);
-    if (split) {
+    const uint32_t kh = k / 2;
+    // choice: blocks per SM in the low byte, kFoldVec4 for four outputs per
+    // thread, or kFoldSplit; tuned per shape (by default split with few
+    // outputs, else one output per thread and 4 blocks per SM)
+    int choice = few ? kFoldSplit : 4;
+    if (k > 6) {
+        // only split
+    } else if (L.forced_fold) {
+        choice = L.forced_fold;
+    } else {
+        const TuneKey tk{L.device, log_len, k, 1, false, false, 1};
+        if (!tuned_fold(tk, &choice) && L.autotune) {
+            tune_fold(L, tk, few);
+            tuned_fold(tk, &choice);
+        }
+    }
+    if (choice == kFoldSplit && few) {
         const dim3 grid((unsigned)((M + 255) / 256) * 8, B);
         L.note(B * (4.0 * (M << k) + 4.0 * M), (double)B * M * (1u << k));
         switch (k) {
@@ -1367,22 +1401,9 @@ cudaError_t fold_eq(Launcher &L, const uint32_t *in, uint32_t *out, uint32_t log
         }
         return cudaGetLastError();
     }
-    const uint32_t kh = k / 2;
-    // grid choice: blocks per SM in the low byte, bit 8 for four outputs
-    // per thread; tuned per shape (one output per thread, 4 blocks per SM
-    // by default)
-    int choice = 4;
-    if (L.forced_fold_bps) {
-        choice = L.forced_fold_bps;
-    } else {
-        const TuneKey tk{L.device, log_len, k, 1, false, false, 1};
-        if (!tuned_fold(tk, &choice)) {
-            if (L.autotune) tune_fold(L, tk, rs, d_rs);
-            if (!tuned_fold(tk, &choice)) choice = 4;
-        }
-    }
+    if (choice == kFoldSplit) choice = 4;  // tuned for fewer proofs at a time
     const int bps = choice & 0xFF;
-    const bool vec4 = (choice & 0x100) && M % 4 == 0 && (uintptr_t)in % 16 == 0 && (uintptr_t)out % 16 == 0;
+    const bool vec4 = (choice & kFoldVec4) && M % 4 == 0 && (uintptr_t)in % 16 == 0 && (uintptr_t)out % 16 == 0;
     const uint64_t groups = vec4 ? M / 4 : M;
     const dim3 blocks(
         (unsigned)std::max<uint64_t>(1, std::min<uint64_t>((groups + 255) / 256, 148ull * (uint64_t)bps)), B);
@@ -2475,8 +2496,8 @@ std::map<TuneKey, int> g_fold_bps;
 
 // Candidate splits: the last pass 4-6 stages, the strided passes before it
 // 3-6 each (at most kMaxFftPasses passes), the default first.
-std::vector<FftPlan> fft_candidates(uint32_t log_len) {
-    std::vector<FftPlan> out{default_fft_plan(log_len)};
+std::vector<FftPlan> fft_candidates(uint32_t log_len, uint64_t words, uint32_t nvec, bool rs) {
+    std::vector<FftPlan> out{default_fft_plan(log_len, words, nvec, rs)};
     if (log_len <= 6) return out;
     auto add = [&](const FftPlan &p) {
         for (auto &q : out)
@@ -2519,7 +2540,7 @@ bool tuned_fft_plan(const TuneKey &k, FftPlan *out) {
 cudaError_t tune_fft(Launcher &L, const TuneKey &k, uint32_t *data, const uint32_t *tw, uint64_t col_stride,
                      uint64_t q_stride, uint32_t root_base, const FftSrc *src, FftPlan *out) {
     (void)data;
-    const uint64_t n = 1ull << k.log_len;
+    const uint64_t n = 1ull << k.log_len, words = (uint64_t)k.Q * k.nvec * n;
     const uint64_t extent = (uint64_t)(k.nvec - 1) * col_stride + (uint64_t)(k.Q - 1) * q_stride + n;
     const uint64_t src_extent = src ? (uint64_t)(k.nvec - 1) * src->col_stride + n : 0;
     uint32_t *sd = nullptr, *ss = nullptr;
@@ -2527,7 +2548,7 @@ cudaError_t tune_fft(Launcher &L, const TuneKey &k, uint32_t *data, const uint32
         (src && cudaMallocAsync(&ss, 4 * src_extent, L.stream) != cudaSuccess)) {
         cudaGetLastError();
         if (sd) cudaFreeAsync(sd, L.stream);
-        *out = default_fft_plan(k.log_len);
+        *out = default_fft_plan(k.log_len, words, k.nvec, src != nullptr);
         return cudaSuccess;
     }
     FftSrc s2;
@@ -2542,10 +2563,10 @@ cudaError_t tune_fft(Launcher &L, const TuneKey &k, uint32_t *data, const uint32
     cudaEventCreate(&b);
     const bool timing = L.timing;
     L.timing = false;
-    FftPlan best = default_fft_plan(k.log_len);
+    FftPlan best = default_fft_plan(k.log_len, words, k.nvec, src != nullptr);
     float best_ms = 1e30f;
     cudaError_t err = cudaSuccess;
-    for (const FftPlan &c : fft_candidates(k.log_len)) {
+    for (const FftPlan &c : fft_candidates(k.log_len, words, k.nvec, src != nullptr)) {
         if (src && c.ks[0] > kMaxRsFirst) continue;
         L.forced_plan = &c;
         float ms = 1e30f;
@@ -2589,9 +2610,9 @@ static bool tuned_fold(const TuneKey &k, int *bps) {
 }
 
 // Times the fold grid at 1, 2, 3 and 4 blocks per SM, one or four outputs
-// per thread, on scratch buffers and keeps the fastest (nothing is recorded
+// per thread, and split where there are few outputs, on scratch buffers and keeps the fastest (nothing is recorded
 // if they cannot be allocated).
-static void tune_fold(Launcher &L, const TuneKey &k, const uint32_t *rs, const uint32_t *d_rs) {
+static void tune_fold(Launcher &L, const TuneKey &k, bool few) {
     const uint64_t n = 1ull << k.log_len;
     uint32_t *in = nullptr, *out = nullptr, *drs = nullptr;
     if (cudaMallocAsync(&in, 4 * n, L.stream) != cudaSuccess ||
@@ -2612,11 +2633,11 @@ static void tune_fold(Launcher &L, const TuneKey &k, const uint32_t *rs, const u
     cudaEventCreate(&b);
     const bool timing = L.timing;
     L.timing = false;
-    int best = 4;
+    int best = few ? kFoldSplit : 4;
     float best_ms = 1e30f;
-    for (int cand = 0; cand < 8; ++cand) {
-        const int bps = 1 + (cand & 3), choice = bps | ((cand >> 2) << 8);
-        L.forced_fold_bps = choice;
+    for (int cand = 0; cand < (few ? 9 : 8); ++cand) {
+        const int choice = cand == 8 ? kFoldSplit : (1 + (cand & 3)) | (cand >= 4 ? kFoldVec4 : 0);
+        L.forced_fold = choice;
         float ms = 1e30f;
         for (int rep = 0; rep < 3; ++rep) {
             if (flush) cudaMemsetAsync(flush, rep, kFlush, L.stream);
@@ -2630,7 +2651,7 @@ static void tune_fold(Launcher &L, const TuneKey &k, const uint32_t *rs, const u
         }
         if (ms < best_ms) { best_ms = ms; best = choice; }
     }
-    L.forced_fold_bps = 0;
+    L.forced_fold = 0;
     L.timing = timing;
     cudaEventDestroy(a);
     cudaEventDestroy(b);
@@ -2638,8 +2659,6 @@ static void tune_fold(Launcher &L, const TuneKey &k, const uint32_t *rs, const u
     cudaFreeAsync(out, L.stream);
     cudaFreeAsync(drs, L.stream);
     if (flush) cudaFreeAsync(flush, L.stream);
-    (void)rs;
-    (void)d_rs;
     if (cudaGetLastError() != cudaSuccess) return;
     std::lock_guard<std::mutex> lk(g_tune_mu);
     g_fold_bps[k] = best;
@@ -2658,9 +2677,13 @@ std::string tuned_choices() {
         s += "\n";
     }
     for (auto &kv : g_fold_bps) {
-        std::snprintf(buf, sizeof buf, "fold device %d log_len %u k %u : blocks/SM %d outputs/thread %d\n",
-                      kv.first.device, kv.first.log_len, kv.first.nvec, kv.second & 0xFF,
-                      (kv.second & 0x100) ? 4 : 1);
+        if (kv.second == kFoldSplit)
+            std::snprintf(buf, sizeof buf, "fold device %d log_len %u k %u : split over clusters\n", kv.first.device,
+                          kv.first.log_len, kv.first.nvec);
+        else
+            std::snprintf(buf, sizeof buf, "fold device %d log_len %u k %u : blocks/SM %d outputs/thread %d\n",
+                          kv.first.device, kv.first.log_len, kv.first.nvec, kv.second & 0xFF,
+                          (kv.second & kFoldVec4) ? 4 : 1);
         s += buf;
     }
     return s;

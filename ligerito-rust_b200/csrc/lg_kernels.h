@@ -39,7 +39,7 @@ struct Launcher {
     // fastest for the process; forced_plan overrides the split (tuning runs).
     bool autotune = false;
     const FftPlan *forced_plan = nullptr;
-    int forced_fold_bps = 0;
+    int forced_fold = 0;
     // device scratch of kDtabSlots x kDtabWords, owned by the context: sets
     // of the FFT passes' shared twiddle tables (fft_vectors), rebuilt in
     // stream order, each with the twiddle subtree it was built for and its
@@ -137,7 +137,8 @@ struct TuneKey {
     uint32_t kind;  // 0 FFT, 1 fold
     bool operator<(const TuneKey &o) const;
 };
-FftPlan default_fft_plan(uint32_t log_len);
+constexpr uint32_t kRsFirstStages = 4;  // stages of a Reed-Solomon first pass by default
+FftPlan default_fft_plan(uint32_t log_len, uint64_t words, uint32_t nvec, bool rs);
 bool tuned_fft_plan(const TuneKey &k, FftPlan *out);
 cudaError_t tune_fft(Launcher &L, const TuneKey &k, uint32_t *data, const uint32_t *tw, uint64_t col_stride,
                      uint64_t q_stride, uint32_t root_base, const struct FftSrc *src, FftPlan *out);
