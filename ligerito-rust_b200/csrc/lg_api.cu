@@ -567,26 +567,25 @@ void induce_dev(lg_ctx *c, Scratch &sc, uint32_t n, const uint32_t *d_rows, uint
 }
 
 // host rows / queries (verifier, kernel-level API) -> induce_dev
-// The enforced sum arrives in pinned memory, valid after sc.finish().
-// (d_rows, d_q: the same rows and queries when they are on the device already)
+// The kernel writes the enforced sum straight into pinned memory, valid after
+// sc.finish() (or a synchronisation).  d_rows, d_q: the same rows and queries
+// when they are on the device already; else they go up together.
 const uint32_t *induce_host_rows_later(lg_ctx *c, Scratch &sc, uint32_t n, const uint32_t *rows, size_t nrows,
-                                       const uint32_t *vch, uint32_t nch, const std::vector<uint64_t> &q,
-                                       uint32_t alpha, uint32_t *d_out, const uint32_t *d_rows = nullptr,
+                                       const uint32_t *vch, uint32_t nch, const uint64_t *q, uint32_t alpha,
+                                       uint32_t *d_out, const uint32_t *d_rows = nullptr,
                                        const uint64_t *d_q = nullptr) {
     if (!d_rows) {
-        d_rows = sc.upload(rows, nrows << nch);
-        d_q = sc.upload(q.data(), q.size());
+        const size_t qb = 8 * nrows, rb = 4 * (nrows << nch);
+        uint8_t *h = sc.pin(qb + rb), *d = static_cast<uint8_t *>(sc.dev(qb + rb));
+        std::memcpy(h, q, qb);
+        std::memcpy(h + qb, rows, rb);
+        CK(c, cudaMemcpyAsync(d, h, qb + rb, cudaMemcpyHostToDevice, c->stream));
+        d_q = reinterpret_cast<const uint64_t *>(d);
+        d_rows = reinterpret_cast<const uint32_t *>(d + qb);
     }
-    uint32_t *d_sum = static_cast<uint32_t *>(sc.dev(16));
-    induce_dev(c, sc, n, d_rows, (uint32_t)nrows, vch, nch, d_q, alpha, d_out, d_sum);
-    return sc.download_later(d_sum, 1);
-}
-uint32_t induce_host_rows(lg_ctx *c, Scratch &sc, uint32_t n, const uint32_t *rows, size_t nrows,
-                          const uint32_t *vch, uint32_t nch, const std::vector<uint64_t> &q, uint32_t alpha,
-                          uint32_t *d_out) {
-    const uint32_t *h = induce_host_rows_later(c, sc, n, rows, nrows, vch, nch, q, alpha, d_out);
-    sync(c);
-    return *h;
+    uint32_t *sum = reinterpret_cast<uint32_t *>(sc.pin(4));
+    induce_dev(c, sc, n, d_rows, (uint32_t)nrows, vch, nch, d_q, alpha, d_out, sum);
+    return sum;
 }
 
 // Variables folded by the next launch: all that are left if they split, else
@@ -1388,7 +1387,7 @@ bool verify_impl(lg_ctx *c, Scratch &sc, const lg_config &cfg, const lg::Proof &
     basis.emplace_back(c, 4ull << cfg.initial_log_m);
     bvars.push_back(cfg.initial_log_m);
     sep.push_back(1);
-    const uint32_t *h1 = induce_host_rows_later(c, sc, cfg.initial_log_m, rows, s, pe0.data(), cfg.initial_k, q, alpha,
+    const uint32_t *h1 = induce_host_rows_later(c, sc, cfg.initial_log_m, rows, s, pe0.data(), cfg.initial_k, q.data(), alpha,
                                                 basis.back().u32(), dop.rows, dop.q);  // :53-60
     // SumcheckVerifierInstance::new (src/ligerito.rs:172-192)
     size_t rd = 0;
@@ -1471,7 +1470,7 @@ bool verify_impl(lg_ctx *c, Scratch &sc, const lg_config &cfg, const lg::Proof &
         const uint32_t *rr = dense(P.recursive[i], s, 1ull << cfg.ks[i]);
         basis.emplace_back(c, 4ull << cfg.log_m[i]);
         bvars.push_back(cfg.log_m[i]);
-        const uint32_t *h = induce_host_rows_later(c, sc, cfg.log_m[i], rr, s, rs.data(), cfg.ks[i], q, al,
+        const uint32_t *h = induce_host_rows_later(c, sc, cfg.log_m[i], rr, s, rs.data(), cfg.ks[i], q.data(), al,
                                                    basis.back().u32(), dop.rows, dop.q);
         g = read_tr();  // introduce_new (src/ligerito.rs:212-220)
         {
@@ -2092,10 +2091,10 @@ lg_status lg_induce_sumcheck_poly(lg_ctx *c, uint32_t n, const uint32_t *rows, u
         if (queries[k] > 0xFFFFFFFFull) return LG_ERR_INVALID_ARGUMENT;
     return guarded(c, [&] {
         CK(c, cudaSetDevice(c->device));
-        std::vector<uint64_t> q(queries, queries + nrows);
         Scratch sc(c);
-        *enforced_sum = induce_host_rows(c, sc, n, rows, nrows, vch, nch, q, alpha, d_out);
+        const uint32_t *h = induce_host_rows_later(c, sc, n, rows, nrows, vch, nch, queries, alpha, d_out);
         sc.finish();
+        *enforced_sum = *h;
     });
 }
 
