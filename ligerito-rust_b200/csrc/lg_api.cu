@@ -335,12 +335,14 @@ void rs_encode(lg_ctx *c, const Code &code, const uint32_t *d_poly, uint32_t log
 }
 
 // ligero_commit (src/ligero.rs:70-95) into caller buffers
-void commit_into(lg_ctx *c, const uint32_t *d_poly, uint32_t log_m, uint32_t n, uint32_t *E, uint32_t *tree) {
+// (root: where the tree's root is also written, e.g. pinned host memory)
+void commit_into(lg_ctx *c, const uint32_t *d_poly, uint32_t log_m, uint32_t n, uint32_t *E, uint32_t *tree,
+                 uint32_t *root = nullptr) {
     const Code code = get_code(c, log_m);
     const uint64_t m = 1ull << log_m, rows = 4 * m;
     rs_encode(c, code, d_poly, log_m, n, E, rows);
     CK(c, lgk::leaf_hashes(c->L, E, rows, n, tree));
-    CK(c, lgk::merkle_upper(c->L, tree, rows));
+    CK(c, lgk::merkle_upper(c->L, tree, rows, 1, 0, root));
 }
 
 Witness commit(lg_ctx *c, const uint32_t *d_poly, uint32_t log_m, uint32_t n) {
@@ -596,22 +598,16 @@ uint32_t fold_step(uint32_t cur, uint32_t left, uint32_t B) {
 }
 // partial_eval by any number of challenges (host rs, or device d_rs), a few
 // of them per launch
-void partial_eval_dev(lg_ctx *c, const uint32_t *d_in, uint32_t log_len, const uint32_t *rs, uint32_t k,
+void partial_eval_dev(lg_ctx *c, Scratch &sc, const uint32_t *d_in, uint32_t log_len, const uint32_t *rs, uint32_t k,
                       uint32_t *d_out, const uint32_t *d_rs = nullptr) {
-    DBuf tmp[2];
     const uint32_t *src = d_in;
-    uint32_t cur = log_len, done = 0, which = 0;
+    uint32_t cur = log_len, done = 0;
     while (done < k) {
         const uint32_t kk = fold_step(cur, k - done, 1);
-        uint32_t *dst;
-        if (done + kk == k) dst = d_out;
-        else {
-            tmp[which] = DBuf(c, 4ull << (cur - kk));
-            dst = tmp[which].u32();
-        }
+        // (what lies between launches is at most a sixteenth of the input)
+        uint32_t *dst = done + kk == k ? d_out : static_cast<uint32_t *>(sc.dev(4ull << (cur - kk)));
         CK(c, lgk::fold_eq(c->L, src, dst, cur, kk, d_rs ? nullptr : rs + done, d_rs ? d_rs + done : nullptr));
         src = dst;
-        which ^= 1;
         cur -= kk;
         done += kk;
     }
@@ -698,7 +694,7 @@ void prove_impl(lg_ctx *c, Scratch &sc, const lg_config &cfg, const uint32_t *d_
     }
     uint32_t fv = cfg.initial_log_m;  // log2 |f|
     DBuf f(c, 4ull << fv);
-    partial_eval_dev(c, d_poly, cfg.initial_log_m + cfg.initial_log_n, nullptr, cfg.initial_k, f.u32(), pe0);  // :52-53
+    partial_eval_dev(c, sc, d_poly, cfg.initial_log_m + cfg.initial_log_n, nullptr, cfg.initial_k, f.u32(), pe0);  // :52-53
     dump_dev(c, "fold_challenges", 0, pe0, 4ull * cfg.initial_k);
     dump_dev(c, "folded", 0, f.p, 4ull << fv);
 
@@ -1450,7 +1446,7 @@ bool verify_impl(lg_ctx *c, Scratch &sc, const lg_config &cfg, const lg::Proof &
                 }
                 if (npts == 0 || npts > nv || (1ull << (nv - npts)) != fe.size()) throw VerifyPanic{};
                 DBuf d(c, 4ull << (nv - npts));
-                partial_eval_dev(c, basis[bi].u32(), nv, ris.data() + first, (uint32_t)npts, d.u32());
+                partial_eval_dev(c, sc, basis[bi].u32(), nv, ris.data() + first, (uint32_t)npts, d.u32());
                 parts.push_back(sc.download_later(d.u32(), fe.size()));
             }
             sc.finish();  // also decides the queued checks
@@ -2054,10 +2050,10 @@ lg_status lg_ligero_commit(lg_ctx *c, const uint32_t *d_poly, uint32_t log_m, ui
         return LG_ERR_INVALID_ARGUMENT;
     return guarded(c, [&] {
         CK(c, cudaSetDevice(c->device));
-        commit_into(c, d_poly, log_m, n, d_enc, reinterpret_cast<uint32_t *>(d_tree));
-        const uint64_t rows = 4ull << log_m;
-        if (root) d2h(c, root, d_tree + 32 * (2 * rows - 2), 32);
+        uint8_t *h = pinned(c, 32);
+        commit_into(c, d_poly, log_m, n, d_enc, reinterpret_cast<uint32_t *>(d_tree), reinterpret_cast<uint32_t *>(h));
         sync(c);
+        if (root) std::memcpy(root, h, 32);
     });
 }
 
@@ -2066,7 +2062,8 @@ lg_status lg_partial_eval(lg_ctx *c, const uint32_t *d_evals, uint32_t log_len, 
     if (!c || !d_evals || !rs || !d_out || k == 0 || k > log_len || log_len > 34) return LG_ERR_INVALID_ARGUMENT;
     return guarded(c, [&] {
         CK(c, cudaSetDevice(c->device));
-        partial_eval_dev(c, d_evals, log_len, rs, k, d_out);
+        Scratch sc(c);
+        partial_eval_dev(c, sc, d_evals, log_len, rs, k, d_out);
         sync(c);
     });
 }

@@ -1069,7 +1069,7 @@ __device__ __forceinline__ void narrow_climb(uint32_t *__restrict__ tree, uint64
 
 template <bool MA>
 __global__ void __launch_bounds__(256) k_merkle_narrow(uint32_t *__restrict__ tree, uint64_t in_off, uint64_t n_in,
-                                                       uint32_t *ticket, uint64_t tree_stride) {
+                                                       uint32_t *ticket, uint64_t tree_stride, uint32_t *root) {
     pdl_begin();
     tree += blockIdx.y * tree_stride;  // lockstep batch: proof blockIdx.y, its own ticket
     ticket += blockIdx.y;
@@ -1080,7 +1080,14 @@ __global__ void __launch_bounds__(256) k_merkle_narrow(uint32_t *__restrict__ tr
     __shared__ uint32_t last;
     const uint32_t per = (uint32_t)(n_in < kNarrowNodes ? n_in : kNarrowNodes), nb = gridDim.x;
     narrow_climb<MA>(tree, in_off, n_in, (uint64_t)blockIdx.x * per, per, buf_a, buf_b);
-    if (nb == 1) return;
+    // the root once more where the caller asks for it
+    auto copy_root = [&](uint64_t off) {
+        if (root && threadIdx.x < 8) root[threadIdx.x] = __ldcg(tree + 8 * off + threadIdx.x);
+    };
+    if (nb == 1) {
+        copy_root(in_off + 2 * n_in - 2);
+        return;
+    }
     // the layer of the blocks' roots
     uint64_t off = in_off, n = n_in;
     for (uint32_t m = per; m > 1; m >>= 1) { off += n; n >>= 1; }
@@ -1091,10 +1098,12 @@ __global__ void __launch_bounds__(256) k_merkle_narrow(uint32_t *__restrict__ tr
     __threadfence();
     if (threadIdx.x == 0) *ticket = 0;  // ready for the next launch on the stream
     narrow_climb<MA>(tree, off, n, 0, nb, buf_a, buf_b);
+    copy_root(in_off + 2 * n_in - 2);
 }
 
-cudaError_t merkle_upper(Launcher &L, uint32_t *tree, uint64_t num_leaves, uint32_t B, uint64_t tree_stride) {
-    if (num_leaves == 0 || (num_leaves & (num_leaves - 1)) || !L.tickets || B == 0 || B > kMaxTickets)
+cudaError_t merkle_upper(Launcher &L, uint32_t *tree, uint64_t num_leaves, uint32_t B, uint64_t tree_stride,
+                         uint32_t *root) {
+    if ((root && (B != 1 || num_leaves < 2)) || num_leaves == 0 || (num_leaves & (num_leaves - 1)) || !L.tickets || B == 0 || B > kMaxTickets)
         return cudaErrorInvalidValue;
     uint64_t off = 0, n = num_leaves;
     // Three layers per launch with a thread per 8 nodes while a layer has
@@ -1113,7 +1122,7 @@ cudaError_t merkle_upper(Launcher &L, uint32_t *tree, uint64_t num_leaves, uint3
             const uint64_t per = std::min<uint64_t>(n, kNarrowNodes);
             L.note(32.0 * B * (2 * n - 1), 0, (double)B * (n - 1));
             LGK_LAUNCH(L, "merkle_narrow", launch_k(hash_bound(n * B) ? k_merkle_narrow<true> : k_merkle_narrow<false>, dim3((unsigned)(n / per), B), 256, 0, L.stream,
-                                                    tree, off, n, L.tickets, tree_stride));
+                                                    tree, off, n, L.tickets, tree_stride, root));
             e = cudaGetLastError();
             n = 1;
         }

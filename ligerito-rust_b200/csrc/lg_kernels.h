@@ -195,9 +195,10 @@ cudaError_t leaf_hashes(Launcher &L, const uint32_t *E, uint64_t rows, uint32_t 
 cudaError_t leaf_hash_block(Launcher &L, const uint32_t *E, uint64_t rows, uint32_t ncols, uint32_t b0,
                             uint32_t nb, uint32_t *out);
 // All upper layers from the leaf layer at tree[0]; tree as 8-word nodes.
-// Needs the Launcher's tickets.
+// Needs the Launcher's tickets.  root (B = 1, at least two leaves): 8 words,
+// e.g. of pinned host memory, that also receive the root.
 cudaError_t merkle_upper(Launcher &L, uint32_t *tree, uint64_t num_leaves, uint32_t B = 1,
-                         uint64_t tree_stride = 0);
+                         uint64_t tree_stride = 0, uint32_t *root = nullptr);
 
 // --- gathers for openings (src/ligero.rs:40-51, src/merkle_tree.rs:98) ---
 // out = the nq opened rows (nq x ncols words), then count Merkle nodes (8
