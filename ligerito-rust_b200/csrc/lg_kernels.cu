@@ -694,9 +694,9 @@ static cudaError_t launch_tail(Launcher &L, int K, PassArgs a, unsigned blocks) 
 
 // Stage split of `words` words in all (rs: of a Reed-Solomon encoding, whose
 // first pass runs all four quarters of a pencil).
-//   * The last pass (tiles in shared memory) takes 6 stages, fewer when the
-//     transform is small: its blocks are then few and each waits for its
-//     tables, which double with every stage (2^12 x 64 columns: 37 us as 6 + 6,
+//   * The last pass (tiles in shared memory) takes 6 stages, fewer when that
+//     makes less than two full tiles an SM: its blocks are then few and each
+//     waits for its tables, which double with every stage (2^12 x 64 columns: 37 us as 6 + 6,
 //     24 as 4 + 3 + 5; 2^10 x 64: 24 as 4 + 6, 20 as 3 + 3 + 4; from 2^22 words
 //     on the splits lie within 8% of each other and past that 6 wins), or when
 //     a tile holds few vectors to share its tables (one of 2^22: 500 us with
@@ -709,12 +709,13 @@ static cudaError_t launch_tail(Launcher &L, int K, PassArgs a, unsigned blocks) 
 //     most 4 where the transform is small and more threads hide more latency
 //     (2^14 x 64: 37 us as 4 + 4 + 6, 31.5 as 3 + 3 + 3 + 5).
 // The autotuner may replace it per shape.
+constexpr uint64_t kTileWords = 64ull * kTailChunk;
 FftPlan default_fft_plan(uint32_t log_len, uint64_t words, uint32_t nvec, bool rs) {
     FftPlan pl;
     uint32_t kt = std::min<uint32_t>(6, log_len);
     if (log_len >= (rs ? 9u : 7u) && log_len <= 24) {  // (at most kMaxFftPasses passes)
-        if (words <= (1ull << 17)) kt = 4;
-        else if ((words <= (1ull << 20) || nvec < 8) && !(rs && log_len <= 10)) kt = 5;
+        if (words <= 32 * kTileWords) kt = 4;
+        else if ((words <= 2 * 148 * kTileWords || nvec < 8) && !(rs && log_len <= 10)) kt = 5;
     }
     const uint32_t rem = log_len - kt, most = kt < 6 ? 4 : 5, first = rs ? kRsFirstStages : most;
     uint32_t nps = 0;
@@ -886,16 +887,25 @@ __global__ void __launch_bounds__(128) k_leaf_hash(const uint32_t *__restrict__ 
     uint32_t cv[8];
     if (b0 == 0) b3_iv(cv);
     else load_node(out + 8 * i, cv);
+    // a block's words are loaded while the one before it is compressed
     const uint32_t *p = E + 16ull * b0 * rows + i;
-    for (uint32_t b = b0; b < b0 + nb_run; ++b, p += 16 * rows) {
-        uint32_t m[16];
+    uint32_t nx[16];
+    auto load = [&](uint32_t b) {
         if (16 * (b + 1) <= ncols) {
 #pragma unroll
-            for (uint32_t w = 0; w < 16; ++w) m[w] = __ldg(strided(p, w, rows4));
+            for (uint32_t w = 0; w < 16; ++w) nx[w] = __ldg(strided(p, w, rows4));
         } else {
 #pragma unroll
-            for (uint32_t w = 0; w < 16; ++w) m[w] = b * 16 + w < ncols ? __ldg(strided(p, w, rows4)) : 0u;
+            for (uint32_t w = 0; w < 16; ++w) nx[w] = b * 16 + w < ncols ? __ldg(strided(p, w, rows4)) : 0u;
         }
+        p += 16 * rows;
+    };
+    load(b0);
+    for (uint32_t b = b0; b < b0 + nb_run; ++b) {
+        uint32_t m[16];
+#pragma unroll
+        for (uint32_t w = 0; w < 16; ++w) m[w] = nx[w];
+        if (b + 1 < b0 + nb_run) load(b + 1);
         const bool last = b + 1 == nb;
         const uint32_t blen = last ? 4 * ncols - 64 * (nb - 1) : 64;
         const uint32_t flags = (b == 0 ? B3_CHUNK_START : 0u) | (last ? (B3_CHUNK_END | B3_ROOT) : 0u);
