@@ -355,32 +355,35 @@ Witness commit(lg_ctx *c, const uint32_t *d_poly, uint32_t log_m, uint32_t n) {
     return w;
 }
 
-// Hash units of the host-input commitment: 32 columns (two BLAKE3 blocks of
-// every leaf) when there are at least 64, else 16 (one block).  The last
-// FFT pass runs once per unit, and its table work per tile does not shrink
-// with the columns, so a 16-column unit costs about as much GPU time per
-// column as its copy takes and the compute falls behind the copy; 32
-// keeps it ahead.
-uint32_t host_hash_unit(uint32_t n) { return n >= 64 ? 32 : std::min<uint32_t>(16, n); }
+// Hash units of the host-input commitment, in columns (16 are one BLAKE3 block
+// of every leaf).  A unit, once its columns are in, gets the last FFT pass and
+// its blocks of every leaf.  The last pass's table work per tile does not
+// shrink with the columns (2^18 rows: 117 us for 16 columns, 168 for 32), so
+// 32 columns a unit; but the first two units of at least 64 columns take 16,
+// because the GPU waits for the copy until then and can hash them meanwhile.
+std::vector<uint32_t> host_hash_units(uint32_t n) {
+    std::vector<uint32_t> u;
+    for (uint32_t j = 0; j < n; j += u.back()) u.push_back(std::min(n - j, n >= 64 && j >= 32 ? 32u : 16u));
+    return u;
+}
 
-// Copy groups of the host-input commitment (column counts, in order): the
-// first unit arrives as 1/8, 1/8, 1/4, 1/2 of it (a 16-column unit as 1/4,
-// 1/4, 1/2) so that compute starts after a few columns, the last as 1/2,
-// 1/4, 1/4 (a 16-column unit as two halves) so that little work remains
-// after the last bytes land, the units between whole.
+// Copy groups of the host-input commitment (column counts, in order; a unit is
+// whole groups): the first unit arrives as 1/4, 1/4, 1/2 of it so that compute
+// starts after a few columns, the last with its end in quarters of 16 columns
+// so that little work remains after the last bytes land, the units between
+// whole.  At 2^24 from pinned memory (19 us of copy a column) the last of 4
+// columns and a unit's last pass and hashes then end 0.28 ms after the copy.
 std::vector<uint32_t> host_copy_groups(uint32_t n) {
-    const uint32_t U = host_hash_unit(n), units = (n + U - 1) / U;
+    const std::vector<uint32_t> units = host_hash_units(n);
     std::vector<uint32_t> g;
-    for (uint32_t u = 0; u < units; ++u) {
-        const uint32_t cols = std::min(U, n - u * U);
-        if (u == 0 && cols == 32) {
-            g.insert(g.end(), {4, 4, 8, 16});
-        } else if (u == 0 && cols >= 8 && cols % 4 == 0) {
+    for (size_t u = 0; u < units.size(); ++u) {
+        const uint32_t cols = units[u];
+        if (u == 0 && cols >= 8 && cols % 4 == 0) {
             g.insert(g.end(), {cols / 4, cols / 4, cols / 2});
-        } else if (u + 1 == units && cols == 32) {
-            g.insert(g.end(), {16, 8, 8});
-        } else if (u + 1 == units && cols >= 8 && cols % 2 == 0) {
-            g.insert(g.end(), {cols / 2, cols / 2});
+        } else if (u + 1 == units.size() && cols == 32) {
+            g.insert(g.end(), {16, 8, 4, 4});
+        } else if (u + 1 == units.size() && cols >= 8 && cols % 4 == 0) {
+            g.insert(g.end(), {cols / 2, cols / 4, cols / 4});
         } else {
             g.push_back(cols);
         }
@@ -392,7 +395,7 @@ std::vector<uint32_t> host_copy_groups(uint32_t n) {
 // columns travel in groups (host_copy_groups) on the copy stream; the
 // compute stream waits for each group and, while the next is in flight,
 // runs its scale-and-spread and the FFT passes but the last (columns are
-// independent).  Each hash unit (host_hash_unit), once all its groups are
+// independent).  Each hash unit (host_hash_units), once all its groups are
 // in, gets the last FFT pass and its BLAKE3 blocks of every leaf: a leaf is
 // the row's words in column order and 16 words are one BLAKE3 block, so
 // columns 16b .. 16b+15 are block b of each leaf's chunk, chained through
@@ -410,8 +413,9 @@ Witness commit_from_host(lg_ctx *c, Scratch &sc, const uint32_t *h_poly, uint32_
     cudaPointerAttributes attr{};
     const bool pinned_src = cudaPointerGetAttributes(&attr, h_poly) == cudaSuccess && attr.type == cudaMemoryTypeHost;
     cudaGetLastError();
-    const std::vector<uint32_t> groups = host_copy_groups(n);
-    const uint32_t U = host_hash_unit(n);
+    const std::vector<uint32_t> groups = host_copy_groups(n), units = host_hash_units(n);
+    size_t unit = 0;
+    uint32_t ju = 0;  // the unit's first column
     // staging for pageable input: two pinned chunks, reused after their copy
     constexpr size_t kChunk = 4u << 20;
     uint8_t *slot[2] = {nullptr, nullptr};
@@ -447,13 +451,13 @@ Witness commit_from_host(lg_ctx *c, Scratch &sc, const uint32_t *h_poly, uint32_
         uint32_t *Eg = w.E.u32() + (uint64_t)j0 * rows;
         rs_encode(c, code, d_poly + (uint64_t)j0 * m, log_m, cols, Eg, rows, lgk::FFT_HEAD);
         j0 += cols;
-        if (j0 % U == 0 || j0 == n) {  // a hash unit is complete
-            const uint32_t u = (j0 - 1) / U, ju = u * U, ucols = j0 - ju;
+        if (j0 == ju + units[unit]) {  // a hash unit is complete
+            const uint32_t ucols = units[unit++];
             CK(c, lgk::fft_vectors(c->L, w.E.u32() + (uint64_t)ju * rows, code.tw, log_m, ucols, rows, 4, m, 4, false,
                                    lgk::FFT_LAST));
             // the unit's BLAKE3 blocks of every leaf, chained after the earlier units'
-            const uint32_t b0 = ju / 16, nb = (ucols + 15) / 16;
-            CK(c, lgk::leaf_hash_block(c->L, w.E.u32(), rows, n, b0, nb, w.tree.u32()));
+            CK(c, lgk::leaf_hash_block(c->L, w.E.u32(), rows, n, ju / 16, (ucols + 15) / 16, w.tree.u32()));
+            ju = j0;
         }
     }
     CK(c, lgk::merkle_upper(c->L, w.tree.u32(), rows));
