@@ -373,11 +373,16 @@ std::vector<uint32_t> host_hash_units(uint32_t n) {
 // so that little work remains after the last bytes land, the units between
 // whole.  At 2^24 from pinned memory (19 us of copy a column) the last of 4
 // columns and a unit's last pass and hashes then end 0.28 ms after the copy.
-std::vector<uint32_t> host_copy_groups(uint32_t n) {
+// A group costs the host about 15 us of copy, event and launch calls, so
+// groups of a unit join until they have kGroupBytes (2^20 from pageable
+// memory: 4 groups instead of 8).
+constexpr size_t kGroupBytes = 1u << 20;
+std::vector<uint32_t> host_copy_groups(uint32_t n, size_t col_bytes) {
     const std::vector<uint32_t> units = host_hash_units(n);
-    std::vector<uint32_t> g;
+    std::vector<uint32_t> out, g;
     for (size_t u = 0; u < units.size(); ++u) {
         const uint32_t cols = units[u];
+        g.clear();
         if (u == 0 && cols >= 8 && cols % 4 == 0) {
             g.insert(g.end(), {cols / 4, cols / 4, cols / 2});
         } else if (u + 1 == units.size() && cols == 32) {
@@ -387,8 +392,15 @@ std::vector<uint32_t> host_copy_groups(uint32_t n) {
         } else {
             g.push_back(cols);
         }
+        uint32_t join = 0;
+        for (size_t i = 0; i < g.size(); ++i) {
+            join += g[i];
+            if (i + 1 < g.size() && join * col_bytes < kGroupBytes) continue;
+            out.push_back(join);
+            join = 0;
+        }
     }
-    return g;
+    return out;
 }
 
 // The first commitment of a proof whose polynomial is on the host: the
@@ -401,19 +413,37 @@ std::vector<uint32_t> host_copy_groups(uint32_t n) {
 // columns 16b .. 16b+15 are block b of each leaf's chunk, chained through
 // the leaf slots of the tree.  After the last unit only the upper tree
 // remains.
+// Small polynomials travel whole instead: a group's calls cost the host more
+// than its share of the copy hides.  Measured proofs, in groups -> whole:
+// from pinned memory (50 GB/s) 2^16 270 -> 185 us, 2^18 286 -> 230, 2^20
+// 438 -> 335, 2^21 498 -> 486, and 2^22 in groups 700 (the copy alone is
+// 325 of it); from pageable memory (the staging copy runs at 13 GB/s) 2^16
+// 286 -> 194 us, 2^18 328 -> 292, 2^19 in groups 400.
+constexpr size_t kWholePinned = 8u << 20, kWholePageable = 1u << 20;
 Witness commit_from_host(lg_ctx *c, Scratch &sc, const uint32_t *h_poly, uint32_t *d_poly, uint32_t log_m,
                          uint32_t n) {
     const Code code = get_code(c, log_m);
     const uint64_t m = 1ull << log_m, rows = 4 * m;
+    cudaPointerAttributes attr{};
+    const bool pinned_src = cudaPointerGetAttributes(&attr, h_poly) == cudaSuccess && attr.type == cudaMemoryTypeHost;
+    cudaGetLastError();
+    const size_t total = 4 * m * n;
+    if (total <= (pinned_src ? kWholePinned : kWholePageable)) {
+        const void *src = h_poly;
+        if (!pinned_src) {
+            uint8_t *h = sc.pin(total);
+            std::memcpy(h, h_poly, total);
+            src = h;
+        }
+        CK(c, cudaMemcpyAsync(d_poly, src, total, cudaMemcpyHostToDevice, c->stream));
+        return commit(c, d_poly, log_m, n);
+    }
     Witness w;
     w.rows = rows;
     w.cols = n;
     w.E = DBuf(c, rows * n * 4);
     w.tree = DBuf(c, (2 * rows - 1) * 32);
-    cudaPointerAttributes attr{};
-    const bool pinned_src = cudaPointerGetAttributes(&attr, h_poly) == cudaSuccess && attr.type == cudaMemoryTypeHost;
-    cudaGetLastError();
-    const std::vector<uint32_t> groups = host_copy_groups(n), units = host_hash_units(n);
+    const std::vector<uint32_t> groups = host_copy_groups(n, 4 * m), units = host_hash_units(n);
     size_t unit = 0;
     uint32_t ju = 0;  // the unit's first column
     // staging for pageable input: two pinned chunks, reused after their copy
