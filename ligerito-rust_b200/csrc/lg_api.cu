@@ -653,11 +653,11 @@ void absorb3(lg::Transcript &fs, const std::array<uint32_t, 3> &s) { fs.absorb_u
 // prover (src/prover.rs:15-199).  The transcript runs on the device
 // (lg_fs.cu) up to yr: each challenge is squeezed into device memory
 // right after what it depends on is absorbed, and the kernels read it from
-// there, so the whole proof is queued without a host round trip.  yr is
-// then downloaded with the transcript state and the host finishes the
-// transcript (absorbing yr is long serial hashing) and the last opening.
-// Roots, sumcheck triples and openings are downloaded asynchronously and
-// materialised at the end; a failed prover assertion flagged on the device
+// there, so the whole proof is queued without a host round trip.  The last
+// sumcheck step writes yr, the transcript state, the roots and the triples
+// into pinned memory, and the host finishes the transcript (absorbing yr is
+// long serial hashing) and the last opening.  Openings are downloaded
+// asynchronously and materialised at the end; a failed prover assertion flagged on the device
 // (src/ligerito.rs:35,52, get_distinct_queries) raises ProverAssert there.
 void prove_impl(lg_ctx *c, Scratch &sc, const lg_config &cfg, const uint32_t *d_poly, uint64_t len, lg::Proof &P,
                 const uint32_t *h_poly = nullptr) {
@@ -666,7 +666,7 @@ void prove_impl(lg_ctx *c, Scratch &sc, const lg_config &cfg, const uint32_t *d_
     for (uint32_t i = 0; i < steps; ++i) nrounds += cfg.ks[i];
     const uint32_t ntri = 1 + nrounds + (steps - 1);  // sumcheck triples, in transcript order
     uint32_t *chal = static_cast<uint32_t *>(sc.dev(4ull * (cfg.initial_k + nrounds + 3 * steps + 4)));
-    // What the host reads at the end, in one run of words (one download): the
+    // What the host reads at the end, in one run of words: the
     // transcript state; s0, s1, s2, enforced sum per triple, then the fused
     // steps' block ticket; the roots (the transcript kernel absorbing one
     // copies it here; the tree itself may be freed before the download); yr.
@@ -747,7 +747,8 @@ void prove_impl(lg_ctx *c, Scratch &sc, const lg_config &cfg, const uint32_t *d_
     w0.tree.reset();
     DBuf f2(c, 4ull << (fv - 1)), B2(c, 4ull << (fv - 1));
     DBuf bi;  // the basis a step starts by gluing into B (none at the first)
-    bool yr_there = false;
+    // the end run's host copy, when the last step wrote it itself
+    uint32_t *end_h = nullptr;
     for (uint32_t i = 0; i < steps; ++i) {
         // The last commitment is final here: a side stream brings its matrix
         // and tree to the host during this step's rounds, so the final
@@ -800,9 +801,12 @@ void prove_impl(lg_ctx *c, Scratch &sc, const lg_config &cfg, const uint32_t *d_
                 next_chal(s.rounds - 1);
                 s.fo = i == steps - 1 ? yr_d : f2.u32();
                 s.Bo = B2.u32(); s.fs = fs;
+                if (i == steps - 1) {
+                    end_h = reinterpret_cast<uint32_t *>(sc.pin(4 * end_words));
+                    s.end = end_d; s.end_words = (uint32_t)end_words; s.mirror = end_h;
+                }
                 CK(c, lgk::sum_step(c->L, s));
-                if (s.fo != yr_d) std::swap(f, f2);
-                else yr_there = true;
+                if (i < steps - 1) std::swap(f, f2);
                 std::swap(B, B2);
                 fv -= s.rounds;
                 round_no += s.rounds;
@@ -827,8 +831,11 @@ void prove_impl(lg_ctx *c, Scratch &sc, const lg_config &cfg, const uint32_t *d_
             r = rn;
         }
         if (i == steps - 1) {  // :104-143
-            if (!yr_there) CK(c, cudaMemcpyAsync(yr_d, f.p, 4ull << fv, cudaMemcpyDeviceToDevice, c->stream));
-            const uint32_t *h = sc.download_later(end_d, end_words);
+            const uint32_t *h = end_h;
+            if (!h) {
+                CK(c, cudaMemcpyAsync(yr_d, f.p, 4ull << fv, cudaMemcpyDeviceToDevice, c->stream));
+                h = sc.download_later(end_d, end_words);
+            }
             if (h_E) CK(c, cudaStreamWaitEvent(c->stream, c->copy_ev[6], 0));
             sync(c);
             const auto *hs = reinterpret_cast<const lgk::FsState *>(h);

@@ -1616,6 +1616,8 @@ struct SumStepArgs {
     uint32_t *chal;              // the opening's challenges and the rounds' after them; !eval: the first round's is there
     uint32_t *fo, *Bo;           // 2^(log_len - rounds) words
     FsState *fs;
+    const uint32_t *end;  // mirror: end_words words from here go to pinned memory at the end
+    uint32_t end_words, *mirror;
 };
 // in shared memory, without its words
 struct SumStepShared {
@@ -1749,6 +1751,12 @@ __global__ void __launch_bounds__(kSumThreads) k_sum_step(SumStepArgs a, RoundSt
     if (c == 0)
         for (uint32_t i = tid; i < fsd::kFsStateWords; i += kSumThreads)
             reinterpret_cast<uint32_t *>(a.fs)[i] = reinterpret_cast<const uint32_t *>(&sh.S)[i];
+    // The last step of a proof hands the host its results itself: a copy after
+    // the kernel cost 7 us of a 2^16 proof's 186.
+    if (a.mirror) {
+        cluster_sync();  // the other blocks' words of `end` are written
+        for (uint32_t i = c * kSumThreads + tid; i < a.end_words; i += C * kSumThreads) a.mirror[i] = __ldcg(a.end + i);
+    }
 }
 static size_t sum_step_smem(uint32_t log_len, uint32_t C, bool bi) {
     return 4 * kTabWords + ((sizeof(SumStepShared) + 15) & ~size_t(15)) + ((bi ? 12ull : 8ull) << log_len) / C;
@@ -1768,10 +1776,12 @@ bool sum_step_fits(uint32_t log_len, uint32_t rounds, uint32_t NB, bool glue) {
 }
 cudaError_t sum_step(Launcher &L, const SumStep &s, uint32_t NB, const RoundStrides &st) {
     const uint32_t C = sum_step_cluster(s.log_len, s.rounds, NB, s.bi != nullptr);
-    if (C == 0 || NB == 0 || NB > 65535 || s.nsq > 2 || (s.eval && s.nsq == 0)) return cudaErrorInvalidValue;
+    if (C == 0 || NB == 0 || NB > 65535 || s.nsq > 2 || (s.eval && s.nsq == 0) || (s.mirror && NB != 1))
+        return cudaErrorInvalidValue;
     SumStepArgs a;
     a.f = s.f; a.B = s.B; a.bi = s.bi; a.log_len = s.log_len; a.rounds = s.rounds; a.eval = s.eval; a.nsq = s.nsq;
     a.tri = s.tri; a.chal = s.chal; a.fo = s.fo; a.Bo = s.Bo; a.fs = s.fs;
+    a.end = s.end; a.end_words = s.end_words; a.mirror = s.mirror;
     const size_t smem = sum_step_smem(s.log_len, C, s.bi != nullptr);
     if (smem > 48 * 1024) cudaFuncSetAttribute(k_sum_step, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
     const double n = (double)NB * (1ull << s.log_len);

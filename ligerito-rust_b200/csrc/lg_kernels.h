@@ -354,6 +354,10 @@ struct SumStep {
     uint32_t nsq = 0;
     uint32_t *tri = nullptr, *chal = nullptr, *fo = nullptr, *Bo = nullptr;
     FsState *fs = nullptr;
+    // the proof's last step: end_words words from `end` on (fs, tri and fo lie
+    // in them) are copied to pinned host memory when the step is done
+    const uint32_t *end = nullptr;
+    uint32_t end_words = 0, *mirror = nullptr;
 };
 bool sum_step_fits(uint32_t log_len, uint32_t rounds, uint32_t NB, bool glue);
 cudaError_t sum_step(Launcher &L, const SumStep &s, uint32_t NB = 1, const RoundStrides &st = RoundStrides{});
