@@ -2458,7 +2458,7 @@ __global__ void __launch_bounds__(256) k_ligero_check(const uint32_t *__restrict
     if (threadIdx.x == 0) {
         uint32_t d = 0, s = 0;
         for (uint32_t w = 0; w < (blockDim.x >> 5); ++w) { d ^= part[0][w]; s ^= part[1][w]; }
-        if (d != s) atomicOr(bad, 1u);
+        if (d != s) *bad = 1u;
     }
 }
 cudaError_t ligero_check(Launcher &L, const uint32_t *rows, const uint64_t *row_off, uint32_t nrows,
