@@ -920,9 +920,18 @@ struct BatchOpened {
     uint64_t stride;
     const uint64_t *q;
 };
+// The batch's last opening, whose rows no kernel reads again: the gather
+// writes it straight into pinned memory (only the nodes there are cross the
+// bus, not room for the most there can be), beside the download of the words
+// that every proof ends with.
+struct BatchEnd {
+    const uint32_t *run;   // those words: the node counts among them,
+    size_t words, counts;  // from run + counts on
+    const uint32_t *h = nullptr;  // their host copy, valid after finish()
+};
 BatchOpened open_rows_batch(lg_ctx *c, Scratch &sc, const BatchWitness &w, lgk::FsState *fs, const uint32_t *absorb,
                             uint64_t absorb_stride, uint32_t nsq, uint32_t *out, uint64_t out_stride,
-                            const std::vector<lg::Opening *> &ops, uint32_t *mirror) {
+                            const std::vector<lg::Opening *> &ops, uint32_t *mirror, BatchEnd *end = nullptr) {
     const uint32_t nq = LG_NUM_QUERIES, B = w.B;
     uint32_t depth = 0;
     while ((1ull << depth) < w.rows) ++depth;
@@ -930,8 +939,10 @@ BatchOpened open_rows_batch(lg_ctx *c, Scratch &sc, const BatchWitness &w, lgk::
     const uint64_t os = ((uint64_t)nq * w.cols + (uint64_t)cap * 8 + 1 + 3) & ~3ull;  // words per proof
     uint64_t *d_q = static_cast<uint64_t *>(sc.dev(8ull * nq * B));
     uint64_t *d_nodes = static_cast<uint64_t *>(sc.dev(8ull * cap * B));
-    uint32_t *d_out = static_cast<uint32_t *>(sc.dev(4ull * os * B));
-    uint32_t *d_cnt = d_out + (uint64_t)nq * w.cols + (uint64_t)cap * 8;
+    uint32_t *d_out = reinterpret_cast<uint32_t *>(end ? (void *)sc.pin(4ull * os * B) : sc.dev(4ull * os * B));
+    uint32_t *d_cnt = end ? const_cast<uint32_t *>(end->run) + end->counts
+                          : d_out + (uint64_t)nq * w.cols + (uint64_t)cap * 8;
+    const uint64_t cs = end ? 1 : os;  // words between the proofs' counts
     lgk::FsQueries a;
     a.src = absorb;
     a.nwords = absorb ? 8 : 0;
@@ -950,24 +961,26 @@ BatchOpened open_rows_batch(lg_ctx *c, Scratch &sc, const BatchWitness &w, lgk::
     fst.mirror = 8;
     fst.q = nq;
     fst.nodes = cap;
-    fst.nnodes = os;
+    fst.nnodes = cs;
     CK(c, lgk::fs_queries(c->L, fs, a, B, fst));
+    if (end) end->h = sc.download_side(end->run, end->words);
     lgk::GatherStrides gst;
     gst.E = w.e_stride();
     gst.q = nq;
     gst.tree = w.t_stride();
     gst.nodes = cap;
-    gst.count = os;
+    gst.count = cs;
     gst.out = os;
     CK(c, lgk::gather_opening(c->L, w.E.u32(), w.rows, w.cols, d_q, nq, w.tree.u32(), d_nodes, cap, d_cnt, d_out, B,
                               gst));
-    const uint32_t *h = sc.download_side(d_out, os * B);
+    const uint32_t *h = end ? d_out : sc.download_side(d_out, os * B);
     const uint32_t cols = w.cols;
-    sc.finalizers.push_back([h, nq, cap, cols, os, ops]() {
+    const uint32_t *hc = end ? end->h + end->counts : h + (uint64_t)nq * cols + (uint64_t)cap * 8;
+    sc.finalizers.push_back([h, hc, cs, nq, cap, cols, os, ops]() {
         for (size_t b = 0; b < ops.size(); ++b) {
             const uint32_t *hb = h + b * os;
             ops[b]->rows.assign_fixed(hb, nq, cols);
-            const uint32_t nr = std::min(hb[(uint64_t)nq * cols + (uint64_t)cap * 8], cap);
+            const uint32_t nr = std::min(hc[b * cs], cap);
             ops[b]->merkle.assign_fixed(reinterpret_cast<const uint8_t *>(hb + (uint64_t)nq * cols), nr, 32);
         }
     });
@@ -1046,14 +1059,21 @@ void prove_batch_impl(lg_ctx *c, Scratch &sc, const lg_config &cfg, const uint32
     // per-proof strides (words): challenges, then triples + the fused
     // steps' ticket
     const uint64_t CH = (cfg.initial_k + nrounds + 3 * steps + 4 + 3) & ~3u, TR = 4ull * ntri + 4;
-    auto *fs = static_cast<lgk::FsState *>(sc.dev(sizeof(lgk::FsState) * B));
+    // What the host reads at the end, in one run of words: the transcript
+    // states, the triples, each root's copies (8 words a proof), the last
+    // opening's node counts, yr.
+    constexpr size_t kFsW = sizeof(lgk::FsState) / 4;
+    const uint32_t fve = cfg.initial_log_m - nrounds;  // log2 |yr|
+    const size_t o_tri = (kFsW * B + 3) & ~size_t(3), o_roots = o_tri + TR * B, o_cnt = o_roots + 8ull * B * (steps + 1);
+    const size_t o_yr = (o_cnt + B + 3) & ~size_t(3), end_words = o_yr + ((size_t)B << fve);
+    uint32_t *end_d = static_cast<uint32_t *>(sc.dev(4 * end_words));
+    auto *fs = reinterpret_cast<lgk::FsState *>(end_d);
     uint32_t *chal = static_cast<uint32_t *>(sc.dev(4ull * CH * B));
-    uint32_t *tri = static_cast<uint32_t *>(sc.dev(4ull * TR * B));
+    uint32_t *tri = end_d + o_tri, *yr_d = end_d + o_yr;
     uint32_t nchal = 0, ntri_used = 0;
     auto next_chal = [&](uint32_t n) { uint32_t *p = chal + nchal; nchal += n; return p; };
     auto next_tri = [&]() { return tri + 4 * ntri_used++; };
-    // each root's copies (8 words a proof), downloaded together at the end
-    uint32_t *roots = static_cast<uint32_t *>(sc.dev(32ull * B * (steps + 1)));
+    uint32_t *roots = end_d + o_roots;
     auto each = [&](auto get) {
         std::vector<decltype(get(P[0]))> v;
         for (auto *p : P) v.push_back(get(p));
@@ -1122,6 +1142,7 @@ void prove_batch_impl(lg_ctx *c, Scratch &sc, const lg_config &cfg, const uint32
     w0.tree.reset();
 
     DBuf f2(c, (4ull << (fv - 1)) * B), B2(c, (4ull << (fv - 1)) * B);
+    bool yr_there = false;
     DBuf bi;
     for (uint32_t i = 0; i < steps; ++i) {
         const uint32_t nsq = i ? 2 : 1, rounds = cfg.ks[i];
@@ -1144,11 +1165,12 @@ void prove_batch_impl(lg_ctx *c, Scratch &sc, const lg_config &cfg, const uint32
                 for (uint32_t j = whole ? 0 : 1; j < s.rounds; ++j) next_tri();
                 s.chal = whole ? ec : r;
                 next_chal(s.rounds - 1);
-                s.fo = f2.u32(); s.Bo = B2.u32(); s.fs = fs;
+                s.fo = i == steps - 1 ? yr_d : f2.u32(); s.Bo = B2.u32(); s.fs = fs;
                 lgk::RoundStrides st = rstr(fv);
                 st.fo = st.go = 1ull << (fv - s.rounds);
                 CK(c, lgk::sum_step(c->L, s, B, st));
-                std::swap(f, f2);
+                if (i < steps - 1) std::swap(f, f2);
+                else yr_there = true;
                 std::swap(Bv, B2);
                 fv -= s.rounds;
                 k = rounds;
@@ -1170,21 +1192,21 @@ void prove_batch_impl(lg_ctx *c, Scratch &sc, const lg_config &cfg, const uint32
             // queries and their node list, and one gather opens every
             // proof -- no host round trip inside the batch.
             const uint64_t ny = 1ull << fv;
+            if (!yr_there)
+                CK(c, cudaMemcpyAsync(yr_d, f.p, 4 * ny * B, cudaMemcpyDeviceToDevice, c->stream));
             for (uint64_t off = 0; off < ny; off += 1024) {
                 lgk::FsStep a;
-                a.src = f.u32() + off;
+                a.src = yr_d + off;
                 a.nwords = (uint32_t)std::min<uint64_t>(1024, ny - off);
                 lgk::FsStrides st;
                 st.src = ny;
                 CK(c, lgk::fs_step(c->L, fs, a, B, st));
             }
+            BatchEnd end{end_d, end_words, o_cnt};
             open_rows_batch(c, sc, wprev, fs, nullptr, 0, 0, nullptr, 0,
-                            each([](lg::Proof *p) { return &p->final_; }), nullptr);
-            // (f is freed when this returns: its copy is queued now)
-            const uint32_t *hy = sc.download_later(f.u32(), ny * B);
-            const lgk::FsState *hs = sc.download_later(fs, B);
-            const uint32_t *ht = sc.download_later(tri, TR * B);
-            const uint32_t *hr = sc.download_later(roots, 8ull * B * (steps + 1));
+                            each([](lg::Proof *p) { return &p->final_; }), nullptr, &end);
+            const uint32_t *he = end.h, *hy = he + o_yr, *ht = he + o_tri, *hr = he + o_roots;
+            const auto *hs = reinterpret_cast<const lgk::FsState *>(he);
             std::vector<char> *flags = &bad;
             sc.finalizers.push_back([hy, hs, ht, hr, steps, ny, ntri, TR, P, flags]() {
                 for (size_t b = 0; b < P.size(); ++b) {
