@@ -226,7 +226,7 @@ __device__ __forceinline__ void pencil_stages(uint32_t (&v)[1 << KP], const uint
             v[y] ^= v[x];
         } else {
             v[y] ^= v[x];
-            v[x] ^= tab_mul_sa(sm, base, off, v[y]);
+            if (!ZERO0 || tp != 0) v[x] ^= tab_mul_sa(sm, base, off, v[y]);
             if (leaf) v[x] ^= leaf_rest(tp, v[y]);
         }
     }
@@ -268,7 +268,11 @@ __device__ __forceinline__ void issue_unit(const uint32_t *src, uint32_t cs, uin
 // a unit's rows into shared memory, the next unit's issued as soon as this
 // one's values are in registers (K = 6 at 2^12 x 1472 columns x 4: 143 us
 // without, 100 us with them).
-template <int K, bool INV>
+// ZERO0: the pass at the root of a whole transform, whose single group is the
+// leftmost of its layers: 1 + 1/2 + 1/4 .. stages' worth of its products are
+// with twiddle zero and left out (4 stages at 2^20 x 64 columns 157 -> 112 us,
+// of which 82 are its words' way from and to memory).
+template <int K, bool INV, bool ZERO0>
 __global__ void __launch_bounds__(256, K <= 4 ? 4 : (K == 5 ? 3 : 2)) k_fft_pass(PassArgs a) {
     pdl_begin();
     extern __shared__ __align__(16) uint8_t smraw[];
@@ -348,7 +352,7 @@ __global__ void __launch_bounds__(256, K <= 4 ? 4 : (K == 5 ? 3 : 2)) k_fft_pass
             prefetch();
         }
         if (!here) continue;
-        pencil_stages<K, 0, INV>(v, smraw, 0, 0);
+        pencil_stages<K, 0, INV, ZERO0>(v, smraw, 0, 0);
 #pragma unroll
         for (uint32_t t = 0; t < R; ++t) *strided(base, t, S4) = v[t];
     }
@@ -616,7 +620,7 @@ static unsigned wave_grid(const void *kernel, std::atomic<int> *occ_c, uint64_t 
     return (unsigned)std::min<uint64_t>(units, (uint64_t)sms * o);
 }
 
-template <bool INV>
+template <bool INV, bool ZERO0>
 static cudaError_t launch_pass(Launcher &L, int K, PassArgs a, unsigned threads) {
     char nmbuf[48];
     std::snprintf(nmbuf, sizeof nmbuf, "%s_L%u_K%d_n%u", INV ? "ifft_pass" : "fft_pass", a.L, K, a.nvec);
@@ -630,10 +634,10 @@ static cudaError_t launch_pass(Launcher &L, int K, PassArgs a, unsigned threads)
 #define LGK_CASE(k)                                                                                  \
     case k: {                                                                                        \
         static std::atomic<int> occ[2][257];                                                         \
-        const void *fn = reinterpret_cast<const void *>(k_fft_pass<k, INV>);                         \
+        const void *fn = reinterpret_cast<const void *>(k_fft_pass<k, INV, ZERO0>);                         \
         if (smem_max > 48 * 1024) cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_max); \
         const unsigned blocks = wave_grid(fn, &occ[a.bulk][threads], a.units, threads, smem);        \
-        LGK_LAUNCH(L, nmbuf, launch_k(k_fft_pass<k, INV>, blocks, threads, smem, L.stream, a));      \
+        LGK_LAUNCH(L, nmbuf, launch_k(k_fft_pass<k, INV, ZERO0>, blocks, threads, smem, L.stream, a));      \
         break;                                                                                       \
     }
         LGK_CASE(1) LGK_CASE(2) LGK_CASE(3) LGK_CASE(4) LGK_CASE(5) LGK_CASE(6)
@@ -705,9 +709,11 @@ static cudaError_t launch_tail(Launcher &L, int K, PassArgs a, unsigned blocks) 
 //     cost 40 us a stage at 2^20 x 64, 4 stages 41; 6 stages and a first pass
 //     of 5 over all quarters need so many registers and so much code that they
 //     lose (2^16 x 64 x 4: 225 us as 5 + 5 + 6, 207 as 3 + 3 + 4 + 6).  So as
-//     few passes of at most 5 (4) as will do, the shorter ones first; of at
-//     most 4 where the transform is small and more threads hide more latency
-//     (2^14 x 64: 37 us as 4 + 4 + 6, 31.5 as 3 + 3 + 3 + 5).
+//     few passes of at most 5 (4) as will do; of at most 4 where the transform
+//     is small and more threads hide more latency (2^14 x 64: 37 us as 4 + 4 +
+//     6, 31.5 as 3 + 3 + 3 + 5).  In an encoding the shorter ones come first; a
+//     plain transform's first pass leaves many products out, so there the
+//     longer ones do (inverse 2^20 x 64: 790 -> 759 us).
 // The autotuner may replace it per shape.
 constexpr uint64_t kTileWords = 64ull * kTailChunk;
 FftPlan default_fft_plan(uint32_t log_len, uint64_t words, uint32_t nvec, bool rs) {
@@ -721,7 +727,7 @@ FftPlan default_fft_plan(uint32_t log_len, uint64_t words, uint32_t nvec, bool r
     uint32_t nps = 0;
     while (rem > 0 && (nps == 0 || first + most * (nps - 1) < rem)) ++nps;
     pl.np = nps + 1;
-    for (uint32_t i = 0; i < nps && i < kMaxFftPasses; ++i) pl.ks[i] = rem / nps + (nps - i <= rem % nps ? 1 : 0);
+    for (uint32_t i = 0; i < nps && i < kMaxFftPasses; ++i) pl.ks[i] = rem / nps + (rs ? nps - i <= rem % nps : i < rem % nps);
     if (nps < kMaxFftPasses) pl.ks[nps] = kt;
     return pl;
 }
@@ -847,9 +853,13 @@ cudaError_t fft_vectors(Launcher &L, uint32_t *data, const uint32_t *tw, uint32_
         const bool src_aligned = !a.src || ((uintptr_t)a.src % 16 == 0 && a.src_col_stride % 4 == 0);
         // rows of at least 32 words: below that a bulk copy moves too little
         a.bulk = aligned && src_aligned && a.log_S >= 5;
+        // each stage's first node is the first of its layer, whose twiddle is zero
+        const bool zero0 = d0 == 0 && Q == 1 && (root_base & (root_base - 1)) == 0;
         cudaError_t e = a.src     ? launch_rs_first(L, (int)K, a, B)
-                        : inverse ? launch_pass<true>(L, (int)K, a, B)
-                                  : launch_pass<false>(L, (int)K, a, B);
+                        : zero0   ? (inverse ? launch_pass<true, true>(L, (int)K, a, B)
+                                             : launch_pass<false, true>(L, (int)K, a, B))
+                        : inverse ? launch_pass<true, false>(L, (int)K, a, B)
+                                  : launch_pass<false, false>(L, (int)K, a, B);
         if (e != cudaSuccess) return e;
     }
     return cudaSuccess;
