@@ -343,6 +343,7 @@ __global__ void __launch_bounds__(256, K <= 4 ? 4 : (K == 5 ? 3 : 2)) k_fft_pass
 #pragma unroll
                     for (uint32_t t = 0; t < R; ++t) v[t] = buf[t * B + tid];
                 }
+                fence_async();    // these reads before the next copies' writes: a barrier alone does not order the two proxies
                 __syncthreads();  // the values are in registers: the next unit's copies may land
                 if (u + 1 < u1) issue();
             } else if (here) {
@@ -437,6 +438,7 @@ __global__ void __launch_bounds__(256, K <= 4 ? 3 : 2) k_rs_first(PassArgs a) {
 #pragma unroll
                 for (uint32_t t = 0; t < R; ++t) v[t] = buf[t * B + tid];
             }
+            fence_async();    // these reads before the next copies' writes: a barrier alone does not order the two proxies
             __syncthreads();  // the values are in registers: the next unit's copies may land
             if (u + nb < U) issue(u + nb);
         } else if (mine) {
