@@ -125,7 +125,7 @@ def kernel_rooflines(stats, work, hbm_peak_gbs, peak_kind, pipes):
         int_ops = INT_OPS_PER_MULT * m + INT_OPS_PER_COMPRESSION * c
         t_hbm = b / (hbm_peak_gbs * 1e9)
         t_int = int_ops / int_peak if int_peak else 0.0
-        t_lds = (m * 8 / 32) / lds_peak if (lds_peak and name.startswith(("fft", "ifft", "fold", "rs_scale", "axpy",
+        t_lds = (m * 8 / 32) / lds_peak if (lds_peak and name.startswith(("fft", "ifft", "fold", "axpy",
                                                                            "induce_main", "eval013"))) else 0.0
         bound = max((t_hbm, "hbm"), (t_int, "int32"), (t_lds, "smem_lookups"))
         row = {"launches": n, "ms": round(ms, 4), "ms_per_launch": round(ms / n, 5),

@@ -77,20 +77,9 @@ __device__ __forceinline__ void mbar_wait(uint64_t *bar, uint32_t parity, uint32
 
 constexpr uint32_t kTail = 0x8299u;  // x^32 mod p
 
-__device__ __forceinline__ uint32_t red_small(uint32_t t) {
-    // t * (x^15 + x^9 + x^7 + x^4 + x^3 + 1) for deg t <= 16 (no overflow)
-    return t ^ (t << 3) ^ (t << 4) ^ (t << 7) ^ (t << 9) ^ (t << 15);
-}
-
 __device__ __forceinline__ uint32_t gf_mulx(uint32_t a) {
     return (a << 1) ^ ((uint32_t)((int32_t)a >> 31) & kTail);
 }
-// a * x^k for 1 <= k <= 16
-template <int K>
-__device__ __forceinline__ uint32_t gf_mulxk(uint32_t a) {
-    return (a << K) ^ red_small(a >> (32 - K));
-}
-
 // hi x^32 + lo mod p.  The tail x^15 + x^9 + x^7 + x^4 + x^3 + 1 is
 // (1 + x^3)(1 + x^4) + x^9 + x^15; one wide multiply gives both words of a
 // shifted hi.
@@ -217,24 +206,6 @@ __device__ __forceinline__ void tab_build_warp(uint32_t *T, uint32_t c, int lane
 #pragma unroll
     for (int j = 0; j < 4; ++j) T[32 * j + lane] = v[j];
 }
-// The same table with the products on the logic pipe only (shifts and
-// XORs): fewer instructions than tab_build_warp's multiply-add form, which
-// pays off where the kernel is bound by instruction issue and a table
-// serves few products (rs_scale builds one per matrix row: 47.3 M against
-// 52.9 M warp instructions per launch at 2^24).
-__device__ __forceinline__ void tab_build_warp_logic(uint32_t *T, uint32_t c, int lane) {
-    const uint32_t c1 = gf_mulx(c), c2 = gf_mulx(c1), c3 = gf_mulx(c2);
-    const int e = lane & 15;
-    uint32_t v = ((e & 1) ? c : 0u) ^ ((e & 2) ? c1 : 0u) ^ ((e & 4) ? c2 : 0u) ^ ((e & 8) ? c3 : 0u);
-    if (lane & 16) v = gf_mulxk<4>(v);
-    T[lane] = v;
-    v = gf_mulxk<8>(v);
-    T[32 + lane] = v;
-    v = gf_mulxk<8>(v);
-    T[64 + lane] = v;
-    v = gf_mulxk<8>(v);
-    T[96 + lane] = v;
-}
 // The tables of two constants interleaved: entry (w, e) = (c0 e x^(4w),
 // c1 e x^(4w)) in 8 bytes at byte 128 w + 8 e (1 KB a pair).  For values
 // multiplied by both constants (tab2_mul_sa) the nibble spreads and byte
@@ -258,9 +229,6 @@ __device__ __forceinline__ T *strided(T *p, uint32_t t, uint32_t stride_bytes) {
     return r;
 }
 
-__device__ __forceinline__ uint32_t shared_addr(const void *p) {
-    return (uint32_t)__cvta_generic_to_shared(p);
-}
 // Product with the table at byte offset base + off of the shared array
 // `sm`, off a constant after unrolling.  Byte j of a (b) holds 4 * nibble 2j
 // (2j+1) of w, the byte offset of that window's entry; a four-byte dot

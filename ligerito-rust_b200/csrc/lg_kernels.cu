@@ -975,10 +975,6 @@ __device__ __forceinline__ void hash_node(const uint32_t *l, const uint32_t *r, 
 // and hashes the 7 nodes of the three layers above them, keeping at most
 // three pending hashes; every lane does full work, so these launches run
 // at hashing throughput.
-__device__ __forceinline__ void hash_pair(const uint32_t (&l)[8], const uint32_t (&r)[8], uint32_t (&o)[8]) {
-    hash_node(l, r, o);
-}
-
 __global__ void __launch_bounds__(128) k_merkle_thread3(uint32_t *__restrict__ tree, uint64_t in_off, uint64_t n_in,
                                                         uint64_t tree_stride) {
     pdl_begin();
@@ -997,7 +993,7 @@ __global__ void __launch_bounds__(128) k_merkle_thread3(uint32_t *__restrict__ t
     load_node(src + 8, r);
 #pragma unroll 1
     for (uint32_t i = 0; i < 7; ++i) {
-        hash_pair(l, r, h);
+        hash_node(l, r, h);
         const uint64_t at = (i == 6)                ? off3 + t
                             : (i == 2 || i == 5)    ? off2 + 2 * t + (i == 5)
                                                     : off1 + 4 * t + (i < 2 ? i : i - 1);
@@ -1813,7 +1809,6 @@ cudaError_t sum_step(Launcher &L, const SumStep &s, uint32_t NB, const RoundStri
 InducePlan induce_plan(uint32_t n, uint32_t nq) {
     InducePlan p;
     p.b = std::min<uint32_t>(n, 9);
-    p.needs_zero = false;  // induce_prep zeroes the output
     (void)nq;
     return p;
 }
@@ -2294,7 +2289,7 @@ cudaError_t induce_fused(Launcher &L, const InducePlan &p, const uint32_t *d_row
     const size_t words = (1ull << p.b) + (1ull << (n - p.b));
     const int in_smem = words <= 10240;  // with the static arrays, under the 48 KB that needs no opt-in
     // one block a query: more than the device holds at 256 threads go out with
-    // 128, twice as many at a time (23 x 148 queries of 2^12: 40 -> 30 us)
+    // 128, twice as many at a time (23 x 148 queries of 2^12: 55 -> 48 us)
     const unsigned threads = (uint64_t)nq * B > 148 * 8 ? 128 : 256;
     LGK_LAUNCH(L, "induce_sp", launch_k(k_induce_sp, dim3(nq, B), threads, in_smem ? 4 * words : 0, L.stream, d_rows, glen,
                                         d_q, nq, alpha, n, p.b, args, d_rs, ilog2u(glen), d_alpha, d_apow, d_lo, d_hi,

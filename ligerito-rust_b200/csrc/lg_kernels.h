@@ -244,11 +244,10 @@ cudaError_t axpy(Launcher &L, uint32_t *B, const uint32_t *bi, uint32_t log_len,
 
 // --- induce_sumcheck_poly basis (src/sumcheck_polys.rs:74-160) ------------
 // basis[t] = sum_k apow[k] * prod_{bit i of t} S[k*n + i]; S = per-query
-// subspace values (sks_at_x).  induce_basis writes all of out (2^n words);
-// a plan with needs_zero set (none currently) wants out zeroed first.
+// subspace values (sks_at_x).  induce_basis writes all of out (2^n words).
 // The enforced sum (the sum of the setup's per-query contributions) lands
 // in d_sum (1 word).
-struct InducePlan { uint32_t b; bool needs_zero; };  // b: low bits of t in Lo
+struct InducePlan { uint32_t b; };  // b: low bits of t in Lo
 // per-proof strides: opened rows, queries, subspace values, alpha powers
 // (2 nq words), Lo / Hi vectors, basis out, enforced sum, challenges, alpha
 struct InduceStrides {

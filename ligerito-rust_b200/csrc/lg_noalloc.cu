@@ -109,10 +109,8 @@ extern "C" lg_status lg_induce_sumcheck_poly_noalloc(void *stream, uint32_t n, c
     lgk::Launcher L;
     L.stream = static_cast<cudaStream_t>(stream);
     err = lgk::induce_setup(L, d_rows, 1u << nch, gr, d_queries, nrows, alpha, n, sks, d_S, d_apow);
-    // The output is accumulated across query groups when the plan splits
-    // them, so it must start at zero; the scratch regions are fully written
-    // before they are read and need no clearing.
-    if (err == cudaSuccess && plan.needs_zero) err = cudaMemsetAsync(d_basis_out, 0, 4ull << n, L.stream);
+    // (the output and the scratch regions are fully written before they are
+    // read and need no clearing)
     if (err == cudaSuccess)
         err = lgk::induce_basis(L, plan, d_S, d_apow, n, nrows, d_lo, d_hi, d_basis_out, d_enforced_sum);
     return err == cudaSuccess ? LG_OK : LG_ERR_CUDA;
