@@ -334,6 +334,25 @@ void rs_encode(lg_ctx *c, const Code &code, const uint32_t *d_poly, uint32_t log
     }
 }
 
+// A caller's polynomial (n columns of 2^log_m) that lies partly inside the
+// buffer of its code words, moved out of it: the first pass of a column writes
+// where other columns' words may still be unread.
+struct EncodeInput {
+    DBuf moved;
+    const uint32_t *p;
+    EncodeInput(lg_ctx *c, const uint32_t *d_poly, uint32_t log_m, uint32_t n, const uint32_t *d_enc) : p(d_poly) {
+        const uint64_t words = (uint64_t)n << log_m;
+        if (!overlap(d_poly, words, d_enc, 4 * words)) return;
+        moved = DBuf(c, 4 * words);
+        CK(c, cudaMemcpyAsync(moved.p, d_poly, 4 * words, cudaMemcpyDeviceToDevice, c->stream));
+        p = moved.u32();
+    }
+    static bool overlap(const uint32_t *a, uint64_t na, const uint32_t *b, uint64_t nb) {
+        const uintptr_t x = (uintptr_t)a, y = (uintptr_t)b;
+        return x < y + 4 * nb && y < x + 4 * na;
+    }
+};
+
 // ligero_commit (src/ligero.rs:70-95) into caller buffers
 // (root: where the tree's root is also written, e.g. pinned host memory)
 void commit_into(lg_ctx *c, const uint32_t *d_poly, uint32_t log_m, uint32_t n, uint32_t *E, uint32_t *tree,
@@ -2123,7 +2142,8 @@ lg_status lg_rs_encode_cols(lg_ctx *c, const uint32_t *d_poly, uint32_t log_m, u
     return guarded(c, [&] {
         CK(c, cudaSetDevice(c->device));
         const Code code = get_code(c, log_m);
-        rs_encode(c, code, d_poly, log_m, n, d_enc, 4ull << log_m);
+        const EncodeInput in(c, d_poly, log_m, n, d_enc);
+        rs_encode(c, code, in.p, log_m, n, d_enc, 4ull << log_m);
         sync(c);
     });
 }
@@ -2135,7 +2155,8 @@ lg_status lg_ligero_commit(lg_ctx *c, const uint32_t *d_poly, uint32_t log_m, ui
     return guarded(c, [&] {
         CK(c, cudaSetDevice(c->device));
         uint8_t *h = pinned(c, 32);
-        commit_into(c, d_poly, log_m, n, d_enc, reinterpret_cast<uint32_t *>(d_tree), reinterpret_cast<uint32_t *>(h));
+        const EncodeInput in(c, d_poly, log_m, n, d_enc);
+        commit_into(c, in.p, log_m, n, d_enc, reinterpret_cast<uint32_t *>(d_tree), reinterpret_cast<uint32_t *>(h));
         sync(c);
         if (root) std::memcpy(root, h, 32);
     });
