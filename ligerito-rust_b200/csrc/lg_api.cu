@@ -334,6 +334,12 @@ void rs_encode(lg_ctx *c, const Code &code, const uint32_t *d_poly, uint32_t log
     }
 }
 
+// do na words at a and nb words at b share any
+bool overlap(const uint32_t *a, uint64_t na, const uint32_t *b, uint64_t nb) {
+    const uintptr_t x = (uintptr_t)a, y = (uintptr_t)b;
+    return x < y + 4 * nb && y < x + 4 * na;
+}
+
 // A caller's polynomial (n columns of 2^log_m) that lies partly inside the
 // buffer of its code words, moved out of it: the first pass of a column writes
 // where other columns' words may still be unread.
@@ -346,10 +352,6 @@ struct EncodeInput {
         moved = DBuf(c, 4 * words);
         CK(c, cudaMemcpyAsync(moved.p, d_poly, 4 * words, cudaMemcpyDeviceToDevice, c->stream));
         p = moved.u32();
-    }
-    static bool overlap(const uint32_t *a, uint64_t na, const uint32_t *b, uint64_t nb) {
-        const uintptr_t x = (uintptr_t)a, y = (uintptr_t)b;
-        return x < y + 4 * nb && y < x + 4 * na;
     }
 };
 
@@ -642,20 +644,23 @@ const uint32_t *induce_host_rows_later(lg_ctx *c, Scratch &sc, uint32_t n, const
     return sum;
 }
 
-// Variables folded by the next launch: all that are left if they split, else
-// at most 6.
-uint32_t fold_step(uint32_t cur, uint32_t left, uint32_t B) {
-    if (lgk::fold_splits(cur, left, B)) return left;
+// Variables folded by the next launch: all that are left (at most `most`) if
+// they split, else at most 6.
+uint32_t fold_step(uint32_t cur, uint32_t left, uint32_t B, uint32_t most = lgk::kMaxFold) {
+    if (left <= most && lgk::fold_splits(cur, left, B)) return left;
     return std::min<uint32_t>(6, left);
 }
 // partial_eval by any number of challenges (host rs, or device d_rs), a few
-// of them per launch
+// of them per launch.  One launch takes more than six only when d_out lies
+// apart from d_in: its blocks write while others may still read, where two
+// launches have a vector of their own between them.
 void partial_eval_dev(lg_ctx *c, Scratch &sc, const uint32_t *d_in, uint32_t log_len, const uint32_t *rs, uint32_t k,
                       uint32_t *d_out, const uint32_t *d_rs = nullptr) {
     const uint32_t *src = d_in;
     uint32_t cur = log_len, done = 0;
+    const uint32_t most = overlap(d_in, 1ull << log_len, d_out, 1ull << (log_len - k)) ? 6 : lgk::kMaxFold;
     while (done < k) {
-        const uint32_t kk = fold_step(cur, k - done, 1);
+        const uint32_t kk = fold_step(cur, k - done, 1, src == d_in ? most : lgk::kMaxFold);
         // (what lies between launches is at most a sixteenth of the input)
         uint32_t *dst = done + kk == k ? d_out : static_cast<uint32_t *>(sc.dev(4ull << (cur - kk)));
         CK(c, lgk::fold_eq(c->L, src, dst, cur, kk, d_rs ? nullptr : rs + done, d_rs ? d_rs + done : nullptr));
