@@ -373,7 +373,10 @@ __device__ void fs_step_warps(FsState &S, FsWork &W, const uint32_t *data, uint3
     const uint32_t all = st.nw + na + nsq;  // < 32: at most one full block
     const bool chain = all >= 16;
     if (threadIdx.x >= 32) {
-        if (nsq == 0 && !chain) return;
+        if (nsq == 0 && !chain) {  // nothing to hash: only let warp 0 know that the state is read
+            asm volatile("bar.arrive 1, 64;" ::: "memory");
+            return;
+        }
         uint32_t blk[16];
         const uint32_t i = (lane - 1) / 2, t = (lane - 1) & 1;
         if (lane == 0) {
@@ -395,7 +398,10 @@ __device__ void fs_step_warps(FsState &S, FsWork &W, const uint32_t *data, uint3
     // warp 0: the words that stay pending, read before anything is written
     const uint32_t rem = all & 15, next = lane < rem ? st.word((all & ~15u) + lane) : 0u;
     if (nsq == 0 && !chain) {
+        // warp 1 decides by S.nw too: with the new count it would schedule a
+        // block that nobody hashes, and leave its arrivals on the barriers
         __syncwarp();
+        asm volatile("bar.sync 1, 64;" ::: "memory");
         if (lane < 16) S.w[lane] = next;
         if (lane == 0) { S.nw = rem; S.total += 4ull * na; }
         __syncwarp();
