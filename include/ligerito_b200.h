@@ -101,6 +101,12 @@ uint64_t lg_ctx_launch_count(const lg_ctx *ctx); /* kernels this context launche
  * NULL: *len = the size with its NUL).  No reference counterpart. */
 lg_status lg_ctx_set_autotune(lg_ctx *ctx, int enabled);
 lg_status lg_tuned_choices(char *buf, uint64_t *len);
+/* Looks that a kernel takes at most for one of its own asynchronous copies to
+ * arrive before it gives up (2^18 at first, about a third of a second).  A call
+ * one of whose kernels gave up returns LG_ERR_CUDA and leaves the context
+ * usable; its outputs are not defined.  0: every such wait gives up (to test a
+ * program's handling of it).  No reference counterpart. */
+lg_status lg_ctx_set_copy_wait_limit(lg_ctx *ctx, uint32_t tries);
 /* Per-kernel CUDA-event timing (off by default); stats accumulate until reset. */
 lg_status lg_ctx_set_kernel_timing(lg_ctx *ctx, int enabled);
 lg_status lg_ctx_kernel_stats(lg_ctx *ctx, uint32_t index, char *name, size_t name_cap,

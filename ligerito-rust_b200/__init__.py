@@ -102,6 +102,7 @@ def _load() -> ctypes.CDLL:
         "lg_ctx_synchronize": (i32, [P]),
         "lg_ctx_launch_count": (u64, [P]),
         "lg_ctx_set_kernel_timing": (i32, [P, i32]),
+        "lg_ctx_set_copy_wait_limit": (i32, [P, u32]),
         "lg_ctx_kernel_stats": (i32, [P, u32, ctypes.c_char_p, ctypes.c_size_t, P, P]),
         "lg_ctx_reset_kernel_stats": (i32, [P]),
         "lg_ctx_kernel_work": (i32, [P, u32, P, P, P]),
@@ -414,6 +415,11 @@ class Context:
 
     def set_autotune(self, enabled: bool) -> None:
         _check(lib.lg_ctx_set_autotune(self.handle, 1 if enabled else 0), self)
+
+    def set_copy_wait_limit(self, tries: int = 1 << 18) -> None:
+        """Looks a kernel takes for one of its own copies before it gives up
+        and its call fails (lg_ctx_set_copy_wait_limit)."""
+        _check(lib.lg_ctx_set_copy_wait_limit(self.handle, tries), self)
 
     def reset_kernel_stats(self) -> None:
         _check(lib.lg_ctx_reset_kernel_stats(self.handle), self)

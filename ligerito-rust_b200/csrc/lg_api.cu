@@ -1604,6 +1604,7 @@ lg_status guarded(lg_ctx *c, F &&f) {
         cudaStreamSynchronize(c->stream);
         if (c->copy_stream) cudaStreamSynchronize(c->copy_stream);
         cudaGetLastError();
+        *c->L.fault = 0;  // it belongs to the call that failed
     };
     try {
         f();
@@ -1912,6 +1913,11 @@ lg_status lg_tuned_choices(char *buf, uint64_t *len) {
     if (*len < s.size() + 1) { *len = s.size() + 1; return LG_ERR_INVALID_ARGUMENT; }
     std::memcpy(buf, s.c_str(), s.size() + 1);
     *len = s.size() + 1;
+    return LG_OK;
+}
+lg_status lg_ctx_set_copy_wait_limit(lg_ctx *c, uint32_t tries) {
+    if (!c) return LG_ERR_INVALID_ARGUMENT;
+    c->L.copy_tries = tries;
     return LG_OK;
 }
 lg_status lg_ctx_set_kernel_timing(lg_ctx *c, int on) {

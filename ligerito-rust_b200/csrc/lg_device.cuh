@@ -16,6 +16,8 @@
 #pragma once
 #include <cstdint>
 
+#include "lg_kernels.h"
+
 namespace lgd {
 
 // Programmatic dependent launch: wait until the previous grid on the
@@ -58,21 +60,28 @@ __device__ __forceinline__ void bulk_store(void *dst, const void *src, uint32_t 
 __device__ __forceinline__ void bulk_store_wait() {
     asm volatile("cp.async.bulk.commit_group;\n\tcp.async.bulk.wait_group 0;" ::: "memory");
 }
-// Waits for the barrier's phase of that parity; a wait that does not end
-// within the limit (a copy that never completes) is reported in *fault, a
-// word of host memory that the host looks at after it synchronises.
-__device__ __forceinline__ void mbar_wait(uint64_t *bar, uint32_t parity, uint32_t *fault) {
+// Whether the barrier's phase of that parity completes within `tries` looks
+// (1.4 us each on a barrier that nothing completes: kCopyTries are 0.36 s).
+__device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity, uint32_t tries) {
     const uint32_t a = (uint32_t)__cvta_generic_to_shared(bar);
-    for (uint32_t tries = 0; tries < (1u << 18); ++tries) {
+    for (; tries > 0; --tries) {
         uint32_t done;
         asm volatile(
             "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
             : "=r"(done)
             : "r"(a), "r"(parity)
             : "memory");
-        if (done) return;
+        if (done) return true;
     }
-    *reinterpret_cast<volatile uint32_t *>(fault) = 1;
+    return false;
+}
+// A block one of whose threads saw its wait run out (a copy that does not
+// complete) ends with this: *fault, a word of host memory that the host looks
+// at after it synchronises, is set, and the copies still on their way have
+// once more that long to land before the block's shared memory goes to another.
+__device__ __forceinline__ void mbar_gave_up(uint64_t *bar, uint32_t parity, uint32_t *fault) {
+    if (threadIdx.x == 0) *reinterpret_cast<volatile uint32_t *>(fault) = 1;
+    mbar_wait(bar, parity, lgk::kCopyTries);
 }
 
 constexpr uint32_t kTail = 0x8299u;  // x^32 mod p

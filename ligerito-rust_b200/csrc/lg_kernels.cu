@@ -115,7 +115,7 @@ struct PassArgs {
     uint64_t col_stride, q_stride;
     uint32_t L, d0, log_S, nvec, bpg, root_base;  // bpg: strided passes, units per (q, P)
     uint32_t bulk;                                // strided passes: rows come in by bulk copies
-    uint32_t *fault;                              // set when a copy's wait gives up
+    uint32_t *fault, tries;                       // copies: set when a wait gives up, after so many looks
     uint32_t vchunk, nchunks;  // last pass: vectors per block, blocks per (q, P)
     uint64_t units;            // strided passes: (group, chunk) work units
     const uint32_t *src;       // strided passes: input, when not data (FftSrc)
@@ -337,14 +337,18 @@ __global__ void __launch_bounds__(256, K <= 4 ? 4 : (K == 5 ? 3 : 2)) k_fft_pass
             if (u + 1 < u1) prefetch();
         } else {
             if (a.bulk) {
-                mbar_wait(bar, parity, a.fault);
-                parity ^= 1;
+                const bool there = mbar_wait(bar, parity, a.tries);
                 if (here) {
 #pragma unroll
                     for (uint32_t t = 0; t < R; ++t) v[t] = buf[t * B + tid];
                 }
-                fence_async();    // these reads before the next copies' writes: a barrier alone does not order the two proxies
-                __syncthreads();  // the values are in registers: the next unit's copies may land
+                fence_async();  // these reads before the next copies' writes: a barrier alone does not order the two proxies
+                // the values are in registers: the next unit's copies may land
+                if (__syncthreads_or(!there)) {
+                    mbar_gave_up(bar, parity, a.fault);
+                    return;
+                }
+                parity ^= 1;
                 if (u + 1 < u1) issue();
             } else if (here) {
 #pragma unroll
@@ -380,6 +384,7 @@ __global__ void __launch_bounds__(256, K <= 4 ? 3 : 2) k_rs_first(PassArgs a) {
     const uint32_t B = blockDim.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nw = B >> 5;
     uint32_t *buf = reinterpret_cast<uint32_t *>(smraw + 4 * QT);  // a.bulk: [R][B]
     uint64_t *bar = reinterpret_cast<uint64_t *>(buf + R * B);
+    volatile uint32_t *gave_up = reinterpret_cast<uint32_t *>(bar + 1);  // a thread's wait ran out
     // units blockIdx.x, + gridDim.x, ...: every SM's blocks get the same number
     // of units to one (contiguous shares of 9 or 10 units a block left SMs
     // with 27 to 30)
@@ -394,6 +399,7 @@ __global__ void __launch_bounds__(256, K <= 4 ? 3 : 2) k_rs_first(PassArgs a) {
     if (a.bulk) {
         if (tid == 0) {
             mbar_init(bar, 1);
+            *gave_up = 0;
             fence_async();
         }
         __syncthreads();
@@ -424,22 +430,23 @@ __global__ void __launch_bounds__(256, K <= 4 ? 3 : 2) k_rs_first(PassArgs a) {
         T[3 * (QT / 16) + e] = make_uint4(c1.x ^ c2.x ^ d.x, c1.y ^ c2.y ^ d.y, c1.z ^ c2.z ^ d.z, c1.w ^ c2.w ^ d.w);
     }
     __syncthreads();
-    uint32_t parity = 0;
-    for (uint32_t u = u0; u < U; u += nb) {
+    uint32_t parity = 0, u = u0;
+    for (; u < U; u += nb) {
         const uint32_t g = u * B + tid;
         const bool mine = g < G;
         const uint32_t col = g >> a.log_S, o = g & smask;
         uint32_t v[R];
         const uint32_t *pp = a.pis + o;
         if (a.bulk) {
-            mbar_wait(bar, parity, a.fault);
-            parity ^= 1;
+            if (!mbar_wait(bar, parity, a.tries)) *gave_up = 1;
             if (mine) {
 #pragma unroll
                 for (uint32_t t = 0; t < R; ++t) v[t] = buf[t * B + tid];
             }
-            fence_async();    // these reads before the next copies' writes: a barrier alone does not order the two proxies
+            fence_async();  // these reads before the next copies' writes: a barrier alone does not order the two proxies
             __syncthreads();  // the values are in registers: the next unit's copies may land
+            parity ^= 1;
+            if (*gave_up) u = U;  // this unit's words are worth nothing, and it is the last
             if (u + nb < U) issue(u + nb);
         } else if (mine) {
             const uint32_t *lb = a.src + (uint64_t)col * scs + o;
@@ -494,6 +501,7 @@ __global__ void __launch_bounds__(256, K <= 4 ? 3 : 2) k_rs_first(PassArgs a) {
             }
         }
     }
+    if (a.bulk && *gave_up) mbar_gave_up(bar, parity ^ 1, a.fault);
 }
 
 // The node tables of a last pass's tile (see build_pass_tables): slots of
@@ -539,7 +547,7 @@ __global__ void __launch_bounds__(256, 4) k_fft_tail(PassArgs a) {
     for (uint32_t j = threadIdx.x; j < nvec; j += blockDim.x)
         bulk_load(tile + j * STRIDE, gbase + j * a.col_stride, 4 * R, bar);
     TailTables<K>::build(smraw, a, q, P);
-    mbar_wait(bar, 0, a.fault);
+    const bool there = mbar_wait(bar, 0, a.tries);
 
     // Two register phases: KA stages on pencils of 2^KA values at stride
     // 2^KB, then KB stages on contiguous pencils of 2^KB values.  Work items
@@ -575,15 +583,14 @@ __global__ void __launch_bounds__(256, 4) k_fft_tail(PassArgs a) {
             for (int i = 0; i < RB / 4; ++i) p[i] = make_uint4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
         }
     };
-    if (!INV) {
-        phase_a();
-        __syncthreads();
-        phase_b();
-    } else {
-        phase_b();
-        __syncthreads();
-        phase_a();
+    if (!INV) phase_a();
+    else phase_b();
+    if (__syncthreads_or(!there)) {
+        mbar_gave_up(bar, 0, a.fault);
+        return;
     }
+    if (!INV) phase_b();
+    else phase_a();
     fence_async();  // this thread's tile words, before the copies out
     __syncthreads();
     for (uint32_t j = threadIdx.x; j < nvec; j += blockDim.x)
@@ -826,7 +833,7 @@ cudaError_t fft_vectors(Launcher &L, uint32_t *data, const uint32_t *tw, uint32_
         a.src_q_stride = 0;
         a.pis = a.src ? src->pis : nullptr;
         a.L = log_len; a.d0 = d0; a.log_S = log_len - d0 - K;
-        a.nvec = nvec; a.root_base = root_base; a.fault = L.fault;
+        a.nvec = nvec; a.root_base = root_base; a.fault = L.fault; a.tries = L.copy_tries;
         const bool tail = a.log_S == 0 && K >= 4 && aligned;
         {
             // every vector read (the source once when all Q subtrees share

@@ -20,6 +20,9 @@ constexpr size_t kDtabWords = kMaxFftPasses * 63 * 128;
 // commitments), so a steady run of proofs builds none
 constexpr uint32_t kDtabSlots = 4;
 
+// looks a kernel takes at most for one of its own copies to arrive
+constexpr uint32_t kCopyTries = 1u << 18;
+
 // A stage split of an FFT: np passes of ks[i] stages, the last one in tiles.
 struct FftPlan {
     uint32_t np = 0;
@@ -49,9 +52,9 @@ struct Launcher {
     // tickets of kernels whose last block to finish does the final step
     uint32_t *tickets = nullptr;
     // a word of pinned host memory, owned by the context: a kernel whose wait
-    // for one of its copies gave up sets it, and the context reports it at
-    // its next synchronisation
-    uint32_t *fault = nullptr;
+    // for one of its copies gave up (after copy_tries looks) sets it, and the
+    // context reports it at its next synchronisation
+    uint32_t *fault = nullptr, copy_tries = kCopyTries;
     struct DtabKey {
         const uint32_t *tw = nullptr;
         uint32_t log_len = 0, root_base = 0, plan = 0;
