@@ -121,7 +121,7 @@ lg_status lg_ctx_kernel_work(lg_ctx *ctx, uint32_t index, double *hbm_bytes, dou
                              double *blake3_compressions);
 uint64_t lg_ctx_device_bytes_in_use(const lg_ctx *ctx);
 /* Device bytes a context keeps between calls (its arena, reserved on its
- * first call, and its FFT tables), and the bytes of the code / twiddle
+ * first proof, its FFT tables and fold workspace), and the bytes of the code / twiddle
  * tables that all contexts on a device share (ReedSolomonEncoding::new's
  * twiddles and pis per size, src/reed_solomon.rs:49-64), held while a
  * context on that device exists. */
