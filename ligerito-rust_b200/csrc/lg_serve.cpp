@@ -50,12 +50,13 @@ struct Request {
     lg_proof *proof = nullptr;
 };
 
-// Device bytes one proof holds at its peak: the input when it is on the
-// host, the first encoded matrix (16 bytes per coefficient), its tree (4
-// per coefficient at 64 columns, 8 allowed for narrower matrices), the folded
-// vectors and the per-context arenas.
+// Device bytes one proof holds at its peak, while the second commitment stands
+// beside the first: the input when it is on the host, both encoded matrices (16
+// bytes per coefficient of theirs) and trees (256 a row of the polynomial's
+// matrix), the folded vector and its basis, and the per-context arenas.
 uint64_t footprint(const lg_config &c, uint64_t len, int on_device) {
-    uint64_t b = 16 * len + 8 * len + (len >> c.initial_k) * 4 * 4 + (48ull << 20);
+    const uint64_t f = 1ull << c.initial_log_m;
+    uint64_t b = 16 * len + 256 * f + 16 * f + (256ull << c.log_m[0]) + 8 * f + (48ull << 20);
     if (!on_device) b += 4 * len;
     return b;
 }
