@@ -108,7 +108,7 @@ INT_OPS_PER_MULT, INT_OPS_PER_COMPRESSION = 16, 800
 SERIAL_KERNELS = ("fs_", "opening_check", "ligero_check")
 
 
-def kernel_rooflines(stats, work, hbm_peak_gbs, peak_kind, pipes):
+def kernel_rooflines(stats, work, general, hbm_peak_gbs, peak_kind, pipes):
     """Per-kernel roofline of one proof.  For each kernel: its compulsory HBM
     bytes over the measured copy bandwidth, its INT32 operations over the
     measured LOP3 rate (the integer logic pipe, which binds the table
@@ -125,8 +125,7 @@ def kernel_rooflines(stats, work, hbm_peak_gbs, peak_kind, pipes):
         int_ops = INT_OPS_PER_MULT * m + INT_OPS_PER_COMPRESSION * c
         t_hbm = b / (hbm_peak_gbs * 1e9)
         t_int = int_ops / int_peak if int_peak else 0.0
-        t_lds = (m * 8 / 32) / lds_peak if (lds_peak and name.startswith(("fft", "ifft", "fold", "axpy",
-                                                                           "induce_main", "eval013"))) else 0.0
+        t_lds = ((m - general.get(name, 0.0)) * 8 / 32) / lds_peak if lds_peak else 0.0
         bound = max((t_hbm, "hbm"), (t_int, "int32"), (t_lds, "smem_lookups"))
         row = {"launches": n, "ms": round(ms, 4), "ms_per_launch": round(ms / n, 5),
                "hbm_bytes": int(b), "gf_mults": int(m), "blake3_compressions": int(c),
@@ -299,10 +298,10 @@ def run_ours(args):
     ctx.reset_kernel_stats()
     lg.prover(cfg, poly, ctx)
     stats = ctx.kernel_stats()
-    work = ctx.kernel_work()
+    work, general = ctx.kernel_work(), ctx.kernel_general_mults()
     ctx.set_kernel_timing(False)
     peak, peak_kind = _peaks()
-    roofline = kernel_rooflines(stats, work, peak, peak_kind, pipes)
+    roofline = kernel_rooflines(stats, work, general, peak, peak_kind, pipes)
 
     cpu = None
     if rank == 0 and world == 1 and not args.no_cpu_baseline:
@@ -387,7 +386,7 @@ def run_prove_large(args):
     ctx.set_kernel_timing(True)
     ctx.reset_kernel_stats()
     lg.prover(cfg, poly, ctx)
-    stats, work = ctx.kernel_stats(), ctx.kernel_work()
+    stats, work, general = ctx.kernel_stats(), ctx.kernel_work(), ctx.kernel_general_mults()
     ctx.set_kernel_timing(False)
     peak, peak_kind = _peaks()
     print(json.dumps({"workload": "prove28", "metric": "prove ms at 2^28 (generated config, seed 2)",
@@ -397,7 +396,7 @@ def run_prove_large(args):
                       "e2e": {"value": round(a.elapsed_time(b), 3), "unit": "ms",
                               "h2d_bytes_per_step": 4 * cfg.poly_len, "d2h_bytes_per_step": len(pb2)},
                       "clocks": clocks, "data": "synthetic (SplitMix64 seed 2)",
-                      "roofline": kernel_rooflines(stats, work, peak, peak_kind, pipes)}), flush=True)
+                      "roofline": kernel_rooflines(stats, work, general, peak, peak_kind, pipes)}), flush=True)
 
 
 def run_micro(args):
@@ -438,13 +437,13 @@ def run_micro(args):
     ctx.set_kernel_timing(True)
     ctx.reset_kernel_stats()
     run()
-    stats, work = ctx.kernel_stats(), ctx.kernel_work()
+    stats, work, general = ctx.kernel_stats(), ctx.kernel_work(), ctx.kernel_general_mults()
     ctx.set_kernel_timing(False)
     peak, peak_kind = _peaks()
     print(json.dumps({"workload": w, "metric": metric, "value": round(statistics.median(times), 4) if times else None,
                       "unit": "ms", "steps": args.steps, "warmup": args.warmup, "higher_is_better": False,
                       "data": "synthetic (SplitMix64 seed 1)",
-                      "roofline": kernel_rooflines(stats, work, peak, peak_kind, lg.measure_pipe_peaks(0))}),
+                      "roofline": kernel_rooflines(stats, work, general, peak, peak_kind, lg.measure_pipe_peaks(0))}),
           flush=True)
 
 

@@ -119,6 +119,9 @@ lg_status lg_ctx_reset_kernel_stats(lg_ctx *ctx);
  * device's peak rates.  No reference counterpart (measurement only). */
 lg_status lg_ctx_kernel_work(lg_ctx *ctx, uint32_t index, double *hbm_bytes, double *gf_mults,
                              double *blake3_compressions);
+/* Those of entry `index`'s multiplications that do not go by a table of one
+ * factor's multiples (general products: integer multiplies, no lookups). */
+lg_status lg_ctx_kernel_general_mults(lg_ctx *ctx, uint32_t index, double *gf_mults);
 uint64_t lg_ctx_device_bytes_in_use(const lg_ctx *ctx);
 /* Device bytes a context keeps between calls (its arena, reserved on its
  * first proof, its FFT tables and fold workspace), and the bytes of the code / twiddle

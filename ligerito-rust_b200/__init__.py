@@ -106,6 +106,7 @@ def _load() -> ctypes.CDLL:
         "lg_ctx_kernel_stats": (i32, [P, u32, ctypes.c_char_p, ctypes.c_size_t, P, P]),
         "lg_ctx_reset_kernel_stats": (i32, [P]),
         "lg_ctx_kernel_work": (i32, [P, u32, P, P, P]),
+        "lg_ctx_kernel_general_mults": (i32, [P, u32, P]),
         "lg_ctx_set_autotune": (i32, [P, i32]),
         "lg_tuned_choices": (i32, [P, P]),
         "lg_measure_pipe_peaks": (i32, [i32, P, u32]),
@@ -411,6 +412,14 @@ class Context:
                                                         ctypes.byref(c)) == 0:
             out[names[i]] = (float(b.value), float(m.value), float(c.value))
             i += 1
+        return out
+
+    def kernel_general_mults(self) -> dict:
+        """name -> those of kernel_work's multiplications that go by no table."""
+        out, m = {}, ctypes.c_double()
+        for i, name in enumerate(self.kernel_stats()):
+            if lib.lg_ctx_kernel_general_mults(self.handle, i, ctypes.byref(m)) == 0:
+                out[name] = float(m.value)
         return out
 
     def set_autotune(self, enabled: bool) -> None:

@@ -1965,7 +1965,7 @@ lg_status lg_ctx_kernel_stats(lg_ctx *c, uint32_t index, char *name, size_t cap,
     if (ms) *ms = it->second.second;
     return LG_OK;
 }
-lg_status lg_ctx_kernel_work(lg_ctx *c, uint32_t index, double *bytes, double *mults, double *comps) {
+static lg_status kernel_work(lg_ctx *c, uint32_t index, lgk::Launcher::Work *out) {
     if (!c) return LG_ERR_INVALID_ARGUMENT;
     lg_status st = guarded(c, [&] { sync(c); c->L.resolve(); });
     if (st != LG_OK) return st;
@@ -1973,12 +1973,23 @@ lg_status lg_ctx_kernel_work(lg_ctx *c, uint32_t index, double *bytes, double *m
     auto it = c->L.stats.begin();
     std::advance(it, index);
     const auto w = c->L.work.find(it->first);
-    const lgk::Launcher::Work none{};
-    const lgk::Launcher::Work &x = w == c->L.work.end() ? none : w->second;
+    if (w != c->L.work.end()) *out = w->second;
+    return LG_OK;
+}
+lg_status lg_ctx_kernel_work(lg_ctx *c, uint32_t index, double *bytes, double *mults, double *comps) {
+    lgk::Launcher::Work x{};
+    const lg_status st = kernel_work(c, index, &x);
+    if (st != LG_OK) return st;
     if (bytes) *bytes = x.bytes;
     if (mults) *mults = x.mults;
     if (comps) *comps = x.comps;
     return LG_OK;
+}
+lg_status lg_ctx_kernel_general_mults(lg_ctx *c, uint32_t index, double *mults) {
+    lgk::Launcher::Work x{};
+    const lg_status st = kernel_work(c, index, &x);
+    if (st == LG_OK && mults) *mults = x.general;
+    return st;
 }
 lg_status lg_ctx_reset_kernel_stats(lg_ctx *c) {
     if (!c) return LG_ERR_INVALID_ARGUMENT;

@@ -45,6 +45,7 @@ void Launcher::end(const char *name, cudaEvent_t a) {
     t.bytes += w.bytes;
     t.mults += w.mults;
     t.comps += w.comps;
+    t.general += w.general;
 }
 void Launcher::resolve() {
     for (auto &p : pending) {
@@ -98,7 +99,7 @@ cudaError_t rs_scale_spread(Launcher &L, const uint32_t *poly, const uint32_t *p
                             uint32_t log_m, uint32_t n) {
     uint64_t total = (uint64_t)n << log_m;
     unsigned blocks = (unsigned)std::min<uint64_t>((total + 255) / 256, 148ull * 16);
-    L.note(20.0 * total, (double)total);
+    L.note(20.0 * total, (double)total, 0, (double)total);
     LGK_LAUNCH(L, "rs_scale_spread", launch_k(k_rs_scale_spread, blocks, 256, 0, L.stream, poly, pis, E, log_m, total));
     return cudaGetLastError();
 }
@@ -835,12 +836,20 @@ cudaError_t fft_vectors(Launcher &L, uint32_t *data, const uint32_t *tw, uint32_
         a.L = log_len; a.d0 = d0; a.log_S = log_len - d0 - K;
         a.nvec = nvec; a.root_base = root_base; a.fault = L.fault; a.tries = L.copy_tries;
         const bool tail = a.log_S == 0 && K >= 4 && aligned;
+        // the root of a whole transform: each stage's first node is the first of
+        // its layer, whose twiddle is zero
+        const bool zero0 = !tail && !a.src && d0 == 0 && Q == 1 && (root_base & (root_base - 1)) == 0;
         {
-            // every vector read (the source once when all Q subtrees share
-            // it) and written once; one product per butterfly and stage
-            const double words = (double)Q * nvec * (1ull << log_len);
-            if (a.src) L.note(4.0 * (words / Q + words), words / Q + words / 2 * K);
-            else L.note(8.0 * words, words / 2 * K);
+            // every vector read (the source once for all quarters) and written
+            // once; a product a butterfly and stage, but those with twiddle zero
+            // that the pass leaves out (see k_fft_pass and k_rs_first)
+            const double words = (double)Q * nvec * (1ull << log_len), R = 1u << K;
+            if (a.src) {
+                const double in = words / Q, table = R + 2 * (K - 1) * R - (R / 2 - 1);  // a pencil's
+                L.note(4.0 * (in + words), in / R * (R + table), 0, in);
+            } else {
+                L.note(8.0 * words, words / 2 * K - (zero0 ? words * (1 - 1 / R) : 0));
+            }
         }
         if (tail) {
             a.vchunk = std::min<uint32_t>(nvec, kTailChunk);
@@ -862,8 +871,6 @@ cudaError_t fft_vectors(Launcher &L, uint32_t *data, const uint32_t *tw, uint32_
         const bool src_aligned = !a.src || ((uintptr_t)a.src % 16 == 0 && a.src_col_stride % 4 == 0);
         // rows of at least 32 words: below that a bulk copy moves too little
         a.bulk = aligned && src_aligned && a.log_S >= 5;
-        // each stage's first node is the first of its layer, whose twiddle is zero
-        const bool zero0 = d0 == 0 && Q == 1 && (root_base & (root_base - 1)) == 0;
         cudaError_t e = a.src     ? launch_rs_first(L, (int)K, a, B)
                         : zero0   ? (inverse ? launch_pass<true, true>(L, (int)K, a, B)
                                              : launch_pass<false, true>(L, (int)K, a, B))
@@ -1424,7 +1431,7 @@ cudaError_t fold_eq(Launcher &L, const uint32_t *in, uint32_t *out, uint32_t log
     }
     if (choice == kFoldSplit && few) {
         const dim3 grid((unsigned)((M + 255) / 256) * 8, B);
-        L.note(B * (4.0 * (M << k) + 4.0 * M), (double)B * M * (1u << k));
+        L.note(B * (4.0 * (M << k) + 4.0 * M), (double)B * M * ((1u << k) + (k >= 8 ? 16 : 8)));
         switch (k) {
 #define LGK_CASE(kk, kh)                                                                                   \
     case kk:                                                                                               \
@@ -1512,7 +1519,7 @@ cudaError_t eval013(Launcher &L, const uint32_t *f, const uint32_t *g, uint32_t 
     const uint64_t half = 1ull << (log_len - 1);
     const dim3 blocks((unsigned)std::max<uint64_t>(1, std::min<uint64_t>((half + 255) / 256, 148ull * 4)), B);
     const FsTail t = tail ? *tail : FsTail{};
-    L.note(16.0 * B * half, 3.0 * B * half);
+    L.note(16.0 * B * half, 3.0 * B * half, 0, 3.0 * B * half);
     LGK_LAUNCH(L, "eval013", launch_k(k_eval013, blocks, 256, 0, L.stream, f, g, half, acc3, t, st));
     return cudaGetLastError();
 }
@@ -1572,7 +1579,7 @@ cudaError_t fold_round(Launcher &L, const uint32_t *f, const uint32_t *B, uint32
     if (log_len < 2 || NB == 0 || NB > 65535) return cudaErrorInvalidValue;
     const uint64_t quarter = 1ull << (log_len - 2);
     const dim3 blocks((unsigned)std::max<uint64_t>(1, std::min<uint64_t>((quarter + 255) / 256, 148ull * 4)), NB);
-    L.note(48.0 * NB * quarter, 7.0 * NB * quarter);
+    L.note(48.0 * NB * quarter, 7.0 * NB * quarter, 0, 3.0 * NB * quarter);
     LGK_LAUNCH(L, "fold_round", launch_k(k_fold_round, blocks, 256, 0, L.stream, f, B, quarter, r, d_r, fo, Bo, acc3,
                                          tail ? *tail : FsTail{}, st));
     return cudaGetLastError();
@@ -1800,7 +1807,7 @@ cudaError_t sum_step(Launcher &L, const SumStep &s, uint32_t NB, const RoundStri
     const size_t smem = sum_step_smem(s.log_len, C, s.bi != nullptr);
     if (smem > 48 * 1024) cudaFuncSetAttribute(k_sum_step, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
     const double n = (double)NB * (1ull << s.log_len);
-    L.note(12.0 * n, 7.0 * n / 2);
+    L.note(12.0 * n, 7.0 * n / 2, 0, 3.0 * n / 2);
     LGK_LAUNCH(L, "fold_round", launch_kc(k_sum_step, dim3(C, NB), kSumThreads, C, smem, L.stream, a, st, C));
     return cudaGetLastError();
 }
@@ -1888,7 +1895,8 @@ cudaError_t induce_setup(Launcher &L, const uint32_t *d_rows, uint32_t glen, con
     if (!d_rs)
         for (uint32_t j = 0; j < glen; ++j) args.gr[j] = gr[j];
     for (uint32_t i = 0; i + 1 < n && i < 32; ++i) args.sks[i] = sks[i];
-    L.note(4.0 * B * nq * (glen + n + 2), (double)B * nq * (glen + 2 * n + 20));
+    const double products = (double)B * nq * (glen + 2 * n + 20);
+    L.note(4.0 * B * nq * (glen + n + 2), products, 0, products);
     LGK_LAUNCH(L, "induce_setup", launch_k(k_induce_setup, dim3((nq + 3) / 4, B), 128, 0, L.stream, d_rows, glen, d_q,
                                            nq, alpha, n, args, d_S, d_apow, d_rs, ilog2u(glen), d_alpha, st));
     return cudaGetLastError();
@@ -2129,7 +2137,7 @@ cudaError_t induce_basis(Launcher &L, const InducePlan &p, const uint32_t *d_S, 
                          uint32_t B, const InduceStrides &st) {
     if (B == 0 || B > 65535) return cudaErrorInvalidValue;
     const double vec = (double)nq * ((1ull << p.b) + (1ull << (n - p.b)));  // Lo and Hi words
-    L.note(4.0 * B * vec, B * vec);
+    L.note(4.0 * B * vec, B * vec, 0, B * vec);
     const size_t words = (1ull << p.b) + (1ull << (n - p.b));
     const int in_smem = words <= 12288;  // 48 KB: no opt-in needed
     LGK_LAUNCH(L, "induce_prep", launch_k(k_induce_prep, dim3(nq, B), 256, in_smem ? 4 * words : 0, L.stream, d_S,
@@ -2292,7 +2300,8 @@ cudaError_t induce_fused(Launcher &L, const InducePlan &p, const uint32_t *d_row
         for (uint32_t j = 0; j < glen; ++j) args.gr[j] = gr[j];
     for (uint32_t i = 0; i + 1 < n && i < 32; ++i) args.sks[i] = sks[i];
     const double vec = (double)nq * ((1ull << p.b) + (1ull << (n - p.b)));
-    L.note(4.0 * B * (vec + nq * (glen + 2)), B * (vec + nq * (glen + 2.0 * n + 20)));
+    const double products = B * (vec + nq * (glen + 2.0 * n + 20));
+    L.note(4.0 * B * (vec + nq * (glen + 2)), products, 0, products);
     const size_t words = (1ull << p.b) + (1ull << (n - p.b));
     const int in_smem = words <= 10240;  // with the static arrays, under the 48 KB that needs no opt-in
     // one block a query: more than the device holds at 256 threads go out with

@@ -70,12 +70,15 @@ struct Launcher {
     std::vector<cudaEvent_t> free_events;
     std::map<std::string, std::pair<uint64_t, double>> stats;  // name -> (launches, ms)
     // Algorithmic work of the timed launches, by kernel name: compulsory HBM
-    // bytes, GF(2^32) multiplications, BLAKE3 compressions.  A launcher
-    // states the next launch's work with note(); end() books it.
-    struct Work { double bytes = 0, mults = 0, comps = 0; };
+    // bytes, GF(2^32) multiplications (general: those of them that do not go
+    // by a table), BLAKE3 compressions.  A launcher states the next launch's
+    // work with note(); end() books it.
+    struct Work { double bytes = 0, mults = 0, comps = 0, general = 0; };
     std::map<std::string, Work> work;
     Work next_work;
-    void note(double bytes, double mults, double comps = 0) { next_work = {bytes, mults, comps}; }
+    void note(double bytes, double mults, double comps = 0, double general = 0) {
+        next_work = {bytes, mults, comps, general};
+    }
 
     cudaEvent_t get_event();
     void begin(const char *name, cudaEvent_t *a);
