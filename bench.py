@@ -106,6 +106,7 @@ class ClockSampler:
 # XORs), 8 shared-memory wavefronts per 32 table multiplications.
 INT_OPS_PER_MULT, INT_OPS_PER_COMPRESSION = 16, 800
 SERIAL_KERNELS = ("fs_", "opening_check", "ligero_check")
+CLUSTER_STEP = "fold_round"  # rounds of a sumcheck step, the transcript between them
 
 
 def kernel_rooflines(stats, work, general, hbm_peak_gbs, peak_kind, pipes):
@@ -134,7 +135,7 @@ def kernel_rooflines(stats, work, general, hbm_peak_gbs, peak_kind, pipes):
                "frac_int32": round(t_int / t, 4) if t > 0 and int_peak else None}
         if t_lds:
             row["frac_smem_lookups"] = round(t_lds / t, 4)
-        if name.startswith(SERIAL_KERNELS) or bound[0] == 0.0:
+        if name.startswith(SERIAL_KERNELS) or name == CLUSTER_STEP or bound[0] == 0.0:
             row["bound"], row["frac"] = "latency (serial chain)", None
         else:
             row["bound"], row["frac"] = bound[1], round(bound[0] / t, 4) if t > 0 else None

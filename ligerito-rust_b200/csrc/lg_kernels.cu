@@ -1580,7 +1580,7 @@ cudaError_t fold_round(Launcher &L, const uint32_t *f, const uint32_t *B, uint32
     const uint64_t quarter = 1ull << (log_len - 2);
     const dim3 blocks((unsigned)std::max<uint64_t>(1, std::min<uint64_t>((quarter + 255) / 256, 148ull * 4)), NB);
     L.note(48.0 * NB * quarter, 7.0 * NB * quarter, 0, 3.0 * NB * quarter);
-    LGK_LAUNCH(L, "fold_round", launch_k(k_fold_round, blocks, 256, 0, L.stream, f, B, quarter, r, d_r, fo, Bo, acc3,
+    LGK_LAUNCH(L, "fold_round_grid", launch_k(k_fold_round, blocks, 256, 0, L.stream, f, B, quarter, r, d_r, fo, Bo, acc3,
                                          tail ? *tail : FsTail{}, st));
     return cudaGetLastError();
 }
@@ -1806,8 +1806,14 @@ cudaError_t sum_step(Launcher &L, const SumStep &s, uint32_t NB, const RoundStri
     a.end = s.end; a.end_words = s.end_words; a.mirror = s.mirror;
     const size_t smem = sum_step_smem(s.log_len, C, s.bi != nullptr);
     if (smem > 48 * 1024) cudaFuncSetAttribute(k_sum_step, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-    const double n = (double)NB * (1ull << s.log_len);
-    L.note(12.0 * n, 7.0 * n / 2, 0, 3.0 * n / 2);
+    // the opening triple takes 3 general products a pair of words, the glue one
+    // table product a word, a round 4 and 3 for four words; the rounds' words
+    // halve
+    const double n = (double)NB * (1ull << s.log_len), out = n / (1u << s.rounds), folded = 2 * (n - out) / 4;
+    const double opening = s.eval ? 1.5 * n : 0, glue = s.bi ? n : 0;
+    L.note(8.0 * n + 4.0 * glue + 8.0 * out, opening + glue + 7.0 * folded, 0, opening + 3.0 * folded);
+    // (the name of the rounds in a cluster; a round over the whole device, bound
+    // otherwise, is a fold_round_grid)
     LGK_LAUNCH(L, "fold_round", launch_kc(k_sum_step, dim3(C, NB), kSumThreads, C, smem, L.stream, a, st, C));
     return cudaGetLastError();
 }

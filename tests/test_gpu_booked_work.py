@@ -45,3 +45,21 @@ def test_encode_first_pass_products(lg, ctx, log_m, n):
     assert K == 3 or table == 105  # of 4 stages
     assert work[name][1] == (n << log_m) / R * (R + table)
     assert general[name] == n << log_m  # the scaling
+
+
+def test_cluster_steps_are_booked_apart(lg, ctx):
+    # folded vectors of 2^14 and 2^12, a launch each
+    cfg = lg.ProverConfig(2, (1 << 14, 1 << 6), [(1 << 12, 4), (1 << 10, 4)], 6, [2, 2])
+    poly = lg.splitmix_coeffs_device(2, cfg.poly_len, ctx)
+    stats, work, general = _booked(ctx, lambda: lg.prover(cfg, poly, ctx))
+    assert stats["fold_round"][0] == 2 and "fold_round_grid" not in stats
+    # an opening triple is 3 products a pair of words, the second step's glue
+    # one a word, a round 4 by the table and 3 others for four words
+    steps = [(1 << 14, 0), (1 << 12, 1)]
+    assert work["fold_round"][1] == sum(1.5 * n + g * n + 1.75 * (n + n / 2) for n, g in steps)
+    assert general["fold_round"] == sum(1.5 * n + 0.75 * (n + n / 2) for n, _ in steps)
+    # 2^17: one round over the device, then a launch for the rest
+    cfg = lg.ProverConfig(1, (1 << 17, 2), [(1 << 14, 8)], 1, [3])
+    poly = lg.splitmix_coeffs_device(2, cfg.poly_len, ctx)
+    stats, _, _ = _booked(ctx, lambda: lg.prover(cfg, poly, ctx))
+    assert stats["fold_round"][0] == 1 and stats["fold_round_grid"][0] == 1
