@@ -101,6 +101,12 @@ uint64_t lg_ctx_launch_count(const lg_ctx *ctx); /* kernels this context launche
  * NULL: *len = the size with its NUL).  No reference counterpart. */
 lg_status lg_ctx_set_autotune(lg_ctx *ctx, int enabled);
 lg_status lg_tuned_choices(char *buf, uint64_t *len);
+/* The stage split of this context's transforms: those of as many stages as the
+ * sum run in `passes` <= 6 passes of stages[i] in 1..6 each (an encoding's first
+ * one of at most 5: it fails with LG_ERR_CUDA otherwise), before any tuned or
+ * default split; transforms of other lengths are not affected.  passes = 0:
+ * none.  Every split gives the same results.  No reference counterpart. */
+lg_status lg_ctx_set_fft_split(lg_ctx *ctx, const uint32_t *stages, uint32_t passes);
 /* Looks that a kernel takes at most for one of its own asynchronous copies to
  * arrive before it gives up (2^18 at first, about a third of a second).  A call
  * one of whose kernels gave up returns LG_ERR_CUDA and leaves the context

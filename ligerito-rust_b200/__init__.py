@@ -103,6 +103,7 @@ def _load() -> ctypes.CDLL:
         "lg_ctx_launch_count": (u64, [P]),
         "lg_ctx_set_kernel_timing": (i32, [P, i32]),
         "lg_ctx_set_copy_wait_limit": (i32, [P, u32]),
+        "lg_ctx_set_fft_split": (i32, [P, P, u32]),
         "lg_ctx_kernel_stats": (i32, [P, u32, ctypes.c_char_p, ctypes.c_size_t, P, P]),
         "lg_ctx_reset_kernel_stats": (i32, [P]),
         "lg_ctx_kernel_work": (i32, [P, u32, P, P, P]),
@@ -424,6 +425,12 @@ class Context:
 
     def set_autotune(self, enabled: bool) -> None:
         _check(lib.lg_ctx_set_autotune(self.handle, 1 if enabled else 0), self)
+
+    def set_fft_split(self, stages: Sequence[int] = ()) -> None:
+        """Stages of each pass of the transforms of sum(stages) stages
+        (lg_ctx_set_fft_split); empty: the default split again."""
+        s = _u32(list(stages))
+        _check(lib.lg_ctx_set_fft_split(self.handle, s.ctypes.data, len(s)), self)
 
     def set_copy_wait_limit(self, tries: int = 1 << 18) -> None:
         """Looks a kernel takes for one of its own copies before it gives up

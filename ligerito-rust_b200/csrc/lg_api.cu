@@ -1943,6 +1943,17 @@ lg_status lg_tuned_choices(char *buf, uint64_t *len) {
     *len = s.size() + 1;
     return LG_OK;
 }
+lg_status lg_ctx_set_fft_split(lg_ctx *c, const uint32_t *stages, uint32_t passes) {
+    if (!c || passes > lgk::kMaxFftPasses || (passes && !stages)) return LG_ERR_INVALID_ARGUMENT;
+    lgk::FftPlan pl;
+    pl.np = passes;
+    for (uint32_t i = 0; i < passes; ++i) {
+        if (stages[i] < 1 || stages[i] > 6) return LG_ERR_INVALID_ARGUMENT;
+        pl.ks[i] = stages[i];
+    }
+    c->L.split = pl;
+    return LG_OK;
+}
 lg_status lg_ctx_set_copy_wait_limit(lg_ctx *c, uint32_t tries) {
     if (!c) return LG_ERR_INVALID_ARGUMENT;
     c->L.copy_tries = tries;

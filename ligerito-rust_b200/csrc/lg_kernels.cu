@@ -786,7 +786,9 @@ cudaError_t fft_vectors(Launcher &L, uint32_t *data, const uint32_t *tw, uint32_
     // (nor does the size of one group change the default)
     const uint64_t words = passes == FFT_ALL ? (uint64_t)Q * nvec << log_len : ~0ull;
     FftPlan plan = default_fft_plan(log_len, words, passes == FFT_ALL ? nvec : ~0u, src != nullptr || passes != FFT_ALL);
-    if (passes == FFT_ALL && !L.forced_plan) {
+    if (L.split.np && plan_valid(L.split, log_len)) {
+        plan = L.split;
+    } else if (passes == FFT_ALL && !L.forced_plan) {
         const TuneKey tk{L.device, log_len, nvec, Q, src != nullptr, inverse, 0};
         if (!tuned_fft_plan(tk, &plan) && L.autotune) {
             cudaError_t e = tune_fft(L, tk, data, tw, col_stride, q_stride, root_base, src, &plan);

@@ -42,6 +42,7 @@ struct Launcher {
     // fastest for the process; forced_plan overrides the split (tuning runs).
     bool autotune = false;
     const FftPlan *forced_plan = nullptr;
+    FftPlan split;  // np > 0: the split of every transform of as many stages
     int forced_fold = 0;
     // device scratch of kDtabSlots x kDtabWords, owned by the context: sets
     // of the FFT passes' shared twiddle tables (fft_vectors), rebuilt in
