@@ -249,6 +249,7 @@ struct Scratch {
     void finish() {
         sync(c);
         if (side) CK(c, cudaStreamSynchronize(c->copy_stream));
+        side = false;
         for (auto &f : finalizers) f();
         finalizers.clear();
     }
@@ -269,8 +270,10 @@ struct Scratch {
         return p;
     }
     ~Scratch() {
-        if (pin_overflow.empty()) return;
-        // copies into the extra blocks may still be in flight after an error
+        if (pin_overflow.empty() && !(side && !dev_overflow.empty())) return;
+        // after an error, copies into the extra pinned blocks may still be in
+        // flight, and the copy stream may still read device buffers that go
+        // back in the other stream's order
         cudaStreamSynchronize(c->stream);
         if (c->copy_stream) cudaStreamSynchronize(c->copy_stream);
         for (uint8_t *p : pin_overflow) cudaFreeHost(p);
