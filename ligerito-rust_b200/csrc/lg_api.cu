@@ -623,7 +623,7 @@ void induce_dev(lg_ctx *c, Scratch &sc, uint32_t n, const uint32_t *d_rows, uint
                 const uint32_t *d_vch = nullptr, const uint32_t *d_alpha = nullptr) {
     std::vector<uint32_t> gr = d_vch ? std::vector<uint32_t>() : lg::lagrange_basis(vch, nch);
     std::vector<uint32_t> sks = lg::eval_sk_at_vks(1ull << n);
-    lgk::InducePlan plan = lgk::induce_plan(n, nq);
+    lgk::InducePlan plan = lgk::induce_plan(n);
     uint32_t *d_S = static_cast<uint32_t *>(sc.dev(4ull * nq * std::max<uint32_t>(n, 1)));
     uint32_t *d_apow = static_cast<uint32_t *>(sc.dev(8ull * nq));
     uint32_t *d_lo = static_cast<uint32_t *>(sc.dev(4ull * nq << plan.b));
@@ -1046,7 +1046,7 @@ void induce_batch(lg_ctx *c, Scratch &sc, uint32_t n, const uint32_t *d_rows, ui
                   uint32_t nch, const uint64_t *d_q, uint32_t *d_out, uint32_t *d_sum, uint64_t sum_stride,
                   const uint32_t *d_vch, const uint32_t *d_alpha, uint64_t chal_stride, uint32_t B) {
     std::vector<uint32_t> sks = lg::eval_sk_at_vks(1ull << n);
-    const lgk::InducePlan plan = lgk::induce_plan(n, nq);
+    const lgk::InducePlan plan = lgk::induce_plan(n);
     lgk::InduceStrides st;
     st.rows = rows_stride;
     st.q = nq;

@@ -120,7 +120,7 @@ struct PassArgs {
     uint32_t vchunk, nchunks;  // last pass: vectors per block, blocks per (q, P)
     uint64_t units;            // strided passes: (group, chunk) work units
     const uint32_t *src;       // strided passes: input, when not data (FftSrc)
-    uint64_t src_col_stride, src_q_stride;
+    uint64_t src_col_stride;
     const uint32_t *pis;       // k_rs_first: the row scaling
 };
 
@@ -833,7 +833,6 @@ cudaError_t fft_vectors(Launcher &L, uint32_t *data, const uint32_t *tw, uint32_
         a.dtab = reinterpret_cast<const uint4 *>(dtab + (size_t)p * 63 * kTabWords);
         a.src = (src && p == 0) ? src->p : nullptr;
         a.src_col_stride = src ? src->col_stride : 0;
-        a.src_q_stride = 0;
         a.pis = a.src ? src->pis : nullptr;
         a.L = log_len; a.d0 = d0; a.log_S = log_len - d0 - K;
         a.nvec = nvec; a.root_base = root_base; a.fault = L.fault; a.tries = L.copy_tries;
@@ -1828,10 +1827,9 @@ cudaError_t sum_step(Launcher &L, const SumStep &s, uint32_t NB, const RoundStri
 // reference's doubling order exactly).  The main kernel gives each warp one
 // query at a time: the warp builds the table of Hi_k[block] and multiplies
 // the whole Lo_k vector by it.
-InducePlan induce_plan(uint32_t n, uint32_t nq) {
+InducePlan induce_plan(uint32_t n) {
     InducePlan p;
     p.b = std::min<uint32_t>(n, 9);
-    (void)nq;
     return p;
 }
 
@@ -1977,13 +1975,13 @@ __global__ void k_induce_prep(const uint32_t *__restrict__ S, const uint32_t *__
 // lane's share of Lo_k; at the segment's end the warps' sums meet in
 // shared memory and go to out (zeroed by induce_prep) by store when the
 // segment covers all queries, else by XOR.
-template <int ACC>  // ACC = max(1, 2^b / 32) words per lane
-__global__ void __launch_bounds__(256, ACC <= 16 ? 3 : 2) k_induce_main(const uint32_t *__restrict__ lo, const uint32_t *__restrict__ hi,
+template <int ACC>  // ACC = max(1, 2^b / 32) words per lane (b <= 9)
+__global__ void __launch_bounds__(256, 3) k_induce_main(const uint32_t *__restrict__ lo, const uint32_t *__restrict__ hi,
                                                      uint32_t n, uint32_t b, uint32_t nq, uint32_t B,
                                                      uint32_t *__restrict__ out, InduceStrides st) {
     pdl_begin();
     __shared__ __align__(128) uint32_t tabs[8][kTabWords];
-    __shared__ uint32_t red[32 * 32];
+    __shared__ uint32_t red[512];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
     const uint32_t nlo = 1u << b, nhi = 1u << (n - b);
     const uint64_t P = (uint64_t)B * nhi * nq;
@@ -2179,7 +2177,7 @@ static cudaError_t launch_induce_main(Launcher &L, const InducePlan &p, uint32_t
     switch (std::max<uint32_t>(1, (1u << p.b) / 32)) {
 #define LGK_CASE(a) \
     case a: LGK_LAUNCH(L, "induce_main", launch_k(k_induce_main<a>, induce_grid<a>(work), 256, 0, L.stream, d_lo, d_hi, n, p.b, nq, B, out, st)); break;
-        LGK_CASE(1) LGK_CASE(2) LGK_CASE(4) LGK_CASE(8) LGK_CASE(16) LGK_CASE(32)
+        LGK_CASE(1) LGK_CASE(2) LGK_CASE(4) LGK_CASE(8) LGK_CASE(16)
 #undef LGK_CASE
         default: return cudaErrorInvalidValue;
     }

@@ -37,7 +37,7 @@ inline uint32_t plan_code(const FftPlan &p) {  // a compact key (3 bits a pass)
 struct Launcher {
     cudaStream_t stream = nullptr;
     int device = 0;
-    // Autotuning (see tune_fft / tuned_fold_blocks): when set, the first call
+    // Autotuning (see tune_fft and tune_fold): when set, the first call
     // of a shape times the candidates on scratch buffers and keeps the
     // fastest for the process; forced_plan overrides the split (tuning runs).
     bool autotune = false;
@@ -260,7 +260,7 @@ struct InducePlan { uint32_t b; };  // b: low bits of t in Lo
 struct InduceStrides {
     uint64_t rows = 0, q = 0, S = 0, apow = 0, lo = 0, hi = 0, out = 0, sum = 0, rs = 0, alpha = 0;
 };
-InducePlan induce_plan(uint32_t n, uint32_t nq);
+InducePlan induce_plan(uint32_t n);
 cudaError_t induce_basis(Launcher &L, const InducePlan &p, const uint32_t *d_S, const uint32_t *d_apow,
                          uint32_t n, uint32_t nq, uint32_t *d_scratch_lo, uint32_t *d_scratch_hi,
                          uint32_t *out, uint32_t *d_sum, uint32_t B = 1, const InduceStrides &st = InduceStrides{});

@@ -72,7 +72,7 @@ extern "C" lg_status lg_induce_sumcheck_poly_noalloc(void *stream, uint32_t n, c
     if (!d_rows || !v_challenges || !d_queries || !d_basis_out || !d_enforced_sum || nch == 0 || nch > 8 ||
         nrows == 0 || n > 28)
         return LG_ERR_INVALID_ARGUMENT;
-    const lgk::InducePlan plan = lgk::induce_plan(n, nrows);
+    const lgk::InducePlan plan = lgk::induce_plan(n);
     const uint64_t w_S = round256((uint64_t)nrows * (n ? n : 1));
     const uint64_t w_apow = round256(2ull * nrows);
     const uint64_t w_lo = round256((uint64_t)nrows << plan.b);
