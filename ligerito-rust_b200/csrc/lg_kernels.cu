@@ -527,7 +527,9 @@ struct TailTables {
     }
 };
 
-template <int K, bool INV>
+// BULK: tiles in and out by bulk copies (launch_tail); an instantiation of its
+// own, because both forms in one cost the bulk one 0.6% (2^20 x 64).
+template <int K, bool INV, bool BULK>
 __global__ void __launch_bounds__(256, 4) k_fft_tail(PassArgs a) {
     pdl_begin();
     constexpr int KA = K / 2, KB = K - KA, RB = 1 << KB, R = 1 << K, STRIDE = R + 4;
@@ -539,16 +541,34 @@ __global__ void __launch_bounds__(256, 4) k_fft_tail(PassArgs a) {
     uint32_t *tile = reinterpret_cast<uint32_t *>(smraw + TailTables<K>::kSlots * 512);
     uint64_t *bar = reinterpret_cast<uint64_t *>(tile + a.vchunk * STRIDE);
     uint32_t *gbase = a.data + (uint64_t)chunk * a.vchunk * a.col_stride + q * a.q_stride + ((uint64_t)P << K);
-    if (threadIdx.x == 0) {
-        mbar_init(bar, 1);
-        fence_async();
-        mbar_expect(bar, 4 * R * nvec);
+    [[maybe_unused]] bool there = true;
+    if constexpr (BULK) {
+        if (threadIdx.x == 0) {
+            mbar_init(bar, 1);
+            fence_async();
+            mbar_expect(bar, 4 * R * nvec);
+        }
+        __syncthreads();
+        for (uint32_t j = threadIdx.x; j < nvec; j += blockDim.x)
+            bulk_load(tile + j * STRIDE, gbase + j * a.col_stride, 4 * R, bar);
+        TailTables<K>::build(smraw, a, q, P);
+        there = mbar_wait(bar, 0, a.tries);
+    } else {
+        constexpr uint32_t D = R / 16;  // 16-byte pieces a thread: 64 vectors, 256 threads
+        uint4 d[D];
+#pragma unroll
+        for (uint32_t k = 0; k < D; ++k) {
+            const uint32_t i = threadIdx.x + k * blockDim.x, j = i / (R / 4);
+            if (j < nvec) d[k] = *reinterpret_cast<const uint4 *>(gbase + j * a.col_stride + 4 * (i % (R / 4)));
+        }
+        TailTables<K>::build(smraw, a, q, P);
+#pragma unroll
+        for (uint32_t k = 0; k < D; ++k) {
+            const uint32_t i = threadIdx.x + k * blockDim.x, j = i / (R / 4);
+            if (j < nvec) *reinterpret_cast<uint4 *>(tile + j * STRIDE + 4 * (i % (R / 4))) = d[k];
+        }
+        __syncthreads();
     }
-    __syncthreads();
-    for (uint32_t j = threadIdx.x; j < nvec; j += blockDim.x)
-        bulk_load(tile + j * STRIDE, gbase + j * a.col_stride, 4 * R, bar);
-    TailTables<K>::build(smraw, a, q, P);
-    const bool there = mbar_wait(bar, 0, a.tries);
 
     // Two register phases: KA stages on pencils of 2^KA values at stride
     // 2^KB, then KB stages on contiguous pencils of 2^KB values.  Work items
@@ -586,17 +606,28 @@ __global__ void __launch_bounds__(256, 4) k_fft_tail(PassArgs a) {
     };
     if (!INV) phase_a();
     else phase_b();
-    if (__syncthreads_or(!there)) {
-        mbar_gave_up(bar, 0, a.fault);
-        return;
+    if constexpr (BULK) {
+        if (__syncthreads_or(!there)) {
+            mbar_gave_up(bar, 0, a.fault);
+            return;
+        }
+    } else {
+        __syncthreads();
     }
     if (!INV) phase_b();
     else phase_a();
-    fence_async();  // this thread's tile words, before the copies out
-    __syncthreads();
-    for (uint32_t j = threadIdx.x; j < nvec; j += blockDim.x)
-        bulk_store(gbase + j * a.col_stride, tile + j * STRIDE, 4 * R);
-    bulk_store_wait();  // the tile is read, and the words are written when the grid ends
+    if constexpr (!BULK) {
+        __syncthreads();
+        for (uint32_t i = threadIdx.x; i < nvec * (R / 4); i += blockDim.x)
+            *reinterpret_cast<uint4 *>(gbase + (uint64_t)(i / (R / 4)) * a.col_stride + 4 * (i % (R / 4))) =
+                *reinterpret_cast<const uint4 *>(tile + (i / (R / 4)) * STRIDE + 4 * (i % (R / 4)));
+    } else {
+        fence_async();  // this thread's tile words, before the copies out
+        __syncthreads();
+        for (uint32_t j = threadIdx.x; j < nvec; j += blockDim.x)
+            bulk_store(gbase + j * a.col_stride, tile + j * STRIDE, 4 * R);
+        bulk_store_wait();
+    }
 }
 
 constexpr uint32_t kMinPassThreads = 64;
@@ -687,19 +718,23 @@ static cudaError_t launch_tail(Launcher &L, int K, PassArgs a, unsigned blocks) 
     const int smem_max = (int)tail_smem(K, kTailChunk);
     uint32_t vp2 = 1;
     while (vp2 < a.vchunk) vp2 <<= 1;
-    // A thread per pencil of a phase (vectors x 2^(K - K/2), the larger one)
-    // up to 256 threads; with enough tiles for several blocks a SM, 128: two
-    // pencils a thread and more tiles in flight hide a tile's table fill and
-    // barriers better (2^18 points: 64 columns 279 -> 265 us, 32 columns 195 ->
-    // 168 us; 64 tiles of 64 columns 10.7 us with 256, 12.8 with 128).
-    const unsigned threads = std::max<unsigned>(32, std::min<unsigned>(blocks >= 148 * 4 ? 128 : 256, vp2 << (K - K / 2)));
-    switch (K) {
-#define LGK_CASE(k)                                                                                 \
-    case k:                                                                                         \
-        cudaFuncSetAttribute(k_fft_tail<k, INV>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_max);   \
-        LGK_LAUNCH(L, nmbuf, launch_k(k_fft_tail<k, INV>, blocks, threads, smem, L.stream, a));           \
+    // Enough tiles for several blocks a SM: the tile in and out by bulk copies,
+    // which leave the load/store unit to the lookups, a thread per pencil of a
+    // phase (vectors x 2^(K - K/2), the larger one) and at most 128: two pencils
+    // a thread and more tiles in flight hide a tile's table fill and barriers
+    // better (2^18 points: 64 columns 279 -> 265 us, 32 columns 195 -> 168 us).
+    // Fewer tiles wait for their own latency: plain 16-byte loads and stores
+    // without the copies' hand-over, and 256 threads to fill the tables (2^6 x
+    // 64: 11.5 -> 10.3 us, 2^6 x 3: 15.2 -> 9.8; 590 tiles of 64 18.5 -> 17.8).
+    const bool bulk = blocks >= 148 * 4;
+    const unsigned threads = bulk ? std::max<unsigned>(32, std::min<unsigned>(128, vp2 << (K - K / 2))) : 256;
+    switch (2 * K + bulk) {
+#define LGK_CASE(k, b)                                                                                         \
+    case 2 * k + b:                                                                                            \
+        cudaFuncSetAttribute(k_fft_tail<k, INV, b>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_max);    \
+        LGK_LAUNCH(L, nmbuf, launch_k(k_fft_tail<k, INV, b>, blocks, threads, smem, L.stream, a));             \
         break;
-        LGK_CASE(4) LGK_CASE(5) LGK_CASE(6)
+        LGK_CASE(4, false) LGK_CASE(5, false) LGK_CASE(6, false) LGK_CASE(4, true) LGK_CASE(5, true) LGK_CASE(6, true)
 #undef LGK_CASE
         default: return cudaErrorInvalidValue;
     }

@@ -14,14 +14,16 @@ def own(lg):
     c.close()
 
 
-# 6: the last pass alone; 11 x 601 and 21: strided passes of 5 stages with bulk
-# copies; 17 x 3: four stages in registers, then the last pass
-@pytest.mark.parametrize("log_n,batch", [(6, 5), (11, 601), (17, 3), (21, 1)])
+# the last pass alone and after four stages in registers, in at least four tiles
+# an SM (fewer go without copies); strided passes of 5 and 6 stages with bulk
+# copies, whose last pass waits for none
+@pytest.mark.parametrize("stages,batch", [((6,), 64 * 600), ((4, 6), 64 * 40), ((5, 6), 601), ((6, 5), 601)])
 @pytest.mark.parametrize("inverse", [False, True])
-def test_transform_reports_and_recovers(lg, own, log_n, batch, inverse):
+def test_transform_reports_and_recovers(lg, own, stages, batch, inverse):
     import torch
 
-    call = lg.ifft if inverse else lg.fft
+    log_n, call = sum(stages), lg.ifft if inverse else lg.fft
+    own.set_fft_split(stages)
     src = lg.splitmix_coeffs_device(log_n, batch << log_n, own)
     want = src.clone()
     call(want, log_n, own)
