@@ -742,35 +742,52 @@ static cudaError_t launch_tail(Launcher &L, int K, PassArgs a, unsigned blocks) 
 }
 
 // Stage split of `words` words in all (rs: of a Reed-Solomon encoding, whose
-// first pass runs all four quarters of a pencil).
-//   * The last pass (tiles in shared memory) takes 6 stages, fewer when that
-//     makes less than two full tiles an SM: its blocks are then few and each
-//     waits for its tables, which double with every stage (2^12 x 64 columns: 37 us as 6 + 6,
-//     24 as 4 + 3 + 5; 2^10 x 64: 24 as 4 + 6, 20 as 3 + 3 + 4; from 2^22 words
-//     on the splits lie within 8% of each other and past that 6 wins), or when
-//     a tile holds few vectors to share its tables (one of 2^22: 500 us with
-//     6, 340 with 5).
-//   * The strided passes before it hold a 2^K-value pencil a thread.  5 stages
-//     cost 40 us a stage at 2^20 x 64, 4 stages 41; 6 stages and a first pass
-//     of 5 over all quarters need so many registers and so much code that they
-//     lose (2^16 x 64 x 4: 225 us as 5 + 5 + 6, 207 as 3 + 3 + 4 + 6).  So as
-//     few passes of at most 5 (4) as will do; of at most 4 where the transform
-//     is small and more threads hide more latency (2^14 x 64: 37 us as 4 + 4 +
-//     6, 31.5 as 3 + 3 + 3 + 5).  In an encoding the shorter ones come first; a
-//     plain transform's first pass leaves many products out, so there the
-//     longer ones do (inverse 2^20 x 64: 790 -> 759 us).
+// first pass runs all four quarters of a pencil; aligned: the last pass can run
+// in tiles in shared memory).  The lines lie where the best splits of 2^5 ..
+// 2^18 points x 1 .. 3000 vectors change; over them this rule is on average
+// within 2% of each shape's best split.
+//   * A tile of the last pass waits for its tables, which double with every
+//     stage.  A few tiles' waits are the launch's latency anyway (below 2^14
+//     words: 6 stages; but never a strided pass of fewer than 3).  With up to two
+//     tiles an SM, 5 stages (2^14 x 8: 24.9 us as 3 + 3 + 3 + 5, 25.5 as 3 + 2 + 3
+//     + 6; inverse 2^13 x 130: 30.3 us as 4 + 4 + 5, 30.8 as 4 + 3 + 6); past
+//     that 6 again (2^10 x 3000: 35.9 us as 4 + 6, 37.3 as 5 + 5), unless a tile
+//     holds few vectors (one of 2^22: 500 us with 6, 340 with 5).
+//   * The strided passes before it hold a 2^K-value pencil a thread: at most 4
+//     stages where more threads hide more latency, 5 in large transforms, whose
+//     passes cost their products.  An encoding's first pass has four times the
+//     work a thread, so passes of 3 serve it longer (2^15 x 40: 85 us as 3 + 3 +
+//     3 + 6, 89 as 4 + 5 + 6).  In an encoding the shorter passes come first; a
+//     plain transform's first pass leaves many products out, so there the longer
+//     ones do (inverse 2^20 x 64: 790 -> 759 us).
+//   * Without tiles a thread of the last pass reads 2^K words in a row: 4 stages
+//     are the most whose warps' lines stay in L1 (2^12 x 500: 49 us as 4 + 4 + 4,
+//     77 as 3 + 4 + 5; 2^18 x 8: 86 and 128).
 // The autotuner may replace it per shape.
-constexpr uint64_t kTileWords = 64ull * kTailChunk;
-FftPlan default_fft_plan(uint32_t log_len, uint64_t words, uint32_t nvec, bool rs) {
-    FftPlan pl;
-    uint32_t kt = std::min<uint32_t>(6, log_len);
-    if (log_len >= (rs ? 9u : 7u) && log_len <= 24) {  // (at most kMaxFftPasses passes)
-        if (words <= 32 * kTileWords) kt = 4;
-        else if ((words <= 2 * 148 * kTileWords || nvec < 8) && !(rs && log_len <= 10)) kt = 5;
+constexpr uint64_t kTwoTilesAnSm = 2 * 148 * 64ull * kTailChunk;  // of 6 stages
+FftPlan default_fft_plan(uint32_t log_len, uint64_t words, uint32_t nvec, bool rs, bool aligned) {
+    uint32_t kt, most;
+    if (!aligned) {
+        kt = 4;
+        most = words < (1u << 18) ? 3 : 4;
+    } else if (log_len <= 6) {
+        kt = most = log_len;
+    } else if (rs) {
+        kt = words < (1u << 16) ? 6 : words <= kTwoTilesAnSm || nvec < 8 ? 5 : 6;
+        most = words <= kTwoTilesAnSm ? 3 : words < (1u << 24) ? 4 : 5;
+    } else if (words < (1u << 14)) {
+        kt = std::max(4u, std::min(6u, log_len - 3));
+        most = 4;
+    } else {
+        kt = words <= kTwoTilesAnSm || nvec < 8 ? 5 : 6;
+        most = words < (1u << 23) ? 4 : 5;
     }
-    const uint32_t rem = log_len - kt, most = kt < 6 ? 4 : 5, first = rs ? kRsFirstStages : most;
+    kt = std::min(kt, log_len);
+    while (kt + most * (kMaxFftPasses - 1) < log_len) ++most;
+    const uint32_t rem = log_len - kt, first = rs ? std::min(most, kRsFirstStages) : most;
     uint32_t nps = 0;
     while (rem > 0 && (nps == 0 || first + most * (nps - 1) < rem)) ++nps;
+    FftPlan pl;
     pl.np = nps + 1;
     for (uint32_t i = 0; i < nps && i < kMaxFftPasses; ++i) pl.ks[i] = rem / nps + (rs ? nps - i <= rem % nps : i < rem % nps);
     if (nps < kMaxFftPasses) pl.ks[nps] = kt;
@@ -819,8 +836,9 @@ cudaError_t fft_vectors(Launcher &L, uint32_t *data, const uint32_t *tw, uint32_
     // head / last calls on column groups must agree on the split, so only
     // whole transforms take tuned plans
     // (nor does the size of one group change the default)
+    const bool aligned = ((uintptr_t)data % 16 == 0) && (col_stride % 4 == 0) && (q_stride % 4 == 0);
     const uint64_t words = passes == FFT_ALL ? (uint64_t)Q * nvec << log_len : ~0ull;
-    FftPlan plan = default_fft_plan(log_len, words, passes == FFT_ALL ? nvec : ~0u, src != nullptr || passes != FFT_ALL);
+    FftPlan plan = default_fft_plan(log_len, words, passes == FFT_ALL ? nvec : ~0u, src != nullptr || passes != FFT_ALL, aligned);
     if (L.split.np && plan_valid(L.split, log_len)) {
         plan = L.split;
     } else if (passes == FFT_ALL && !L.forced_plan) {
@@ -858,7 +876,6 @@ cudaError_t fft_vectors(Launcher &L, uint32_t *data, const uint32_t *tw, uint32_
     const uint32_t *dtab = L.dtab + slot * kDtabWords;
     uint32_t nvec_p2 = 1;
     while (nvec_p2 < nvec) nvec_p2 <<= 1;
-    const bool aligned = ((uintptr_t)data % 16 == 0) && (col_stride % 4 == 0) && (q_stride % 4 == 0);
     for (uint32_t pi = 0; pi < np; ++pi) {
         const uint32_t p = inverse ? np - 1 - pi : pi;
         if ((passes == FFT_HEAD && p == np - 1) || (passes == FFT_LAST && p != np - 1)) continue;
@@ -2590,7 +2607,7 @@ std::map<TuneKey, int> g_fold_bps;
 // Candidate splits: the last pass 4-6 stages, the strided passes before it
 // 3-6 each (at most kMaxFftPasses passes), the default first.
 std::vector<FftPlan> fft_candidates(uint32_t log_len, uint64_t words, uint32_t nvec, bool rs) {
-    std::vector<FftPlan> out{default_fft_plan(log_len, words, nvec, rs)};
+    std::vector<FftPlan> out{default_fft_plan(log_len, words, nvec, rs, true)};
     if (log_len <= 6) return out;
     auto add = [&](const FftPlan &p) {
         for (auto &q : out)
@@ -2641,7 +2658,7 @@ cudaError_t tune_fft(Launcher &L, const TuneKey &k, uint32_t *data, const uint32
         (src && cudaMallocAsync(&ss, 4 * src_extent, L.stream) != cudaSuccess)) {
         cudaGetLastError();
         if (sd) cudaFreeAsync(sd, L.stream);
-        *out = default_fft_plan(k.log_len, words, k.nvec, src != nullptr);
+        *out = default_fft_plan(k.log_len, words, k.nvec, src != nullptr, true);
         return cudaSuccess;
     }
     FftSrc s2;
@@ -2656,7 +2673,7 @@ cudaError_t tune_fft(Launcher &L, const TuneKey &k, uint32_t *data, const uint32
     cudaEventCreate(&b);
     const bool timing = L.timing;
     L.timing = false;
-    FftPlan best = default_fft_plan(k.log_len, words, k.nvec, src != nullptr);
+    FftPlan best = default_fft_plan(k.log_len, words, k.nvec, src != nullptr, true);
     float best_ms = 1e30f;
     cudaError_t err = cudaSuccess;
     for (const FftPlan &c : fft_candidates(k.log_len, words, k.nvec, src != nullptr)) {

@@ -145,7 +145,7 @@ struct TuneKey {
     bool operator<(const TuneKey &o) const;
 };
 constexpr uint32_t kRsFirstStages = 4;  // stages of a Reed-Solomon first pass by default
-FftPlan default_fft_plan(uint32_t log_len, uint64_t words, uint32_t nvec, bool rs);
+FftPlan default_fft_plan(uint32_t log_len, uint64_t words, uint32_t nvec, bool rs, bool aligned);
 bool tuned_fft_plan(const TuneKey &k, FftPlan *out);
 cudaError_t tune_fft(Launcher &L, const TuneKey &k, uint32_t *data, const uint32_t *tw, uint64_t col_stride,
                      uint64_t q_stride, uint32_t root_base, const struct FftSrc *src, FftPlan *out);

@@ -42,7 +42,7 @@ def test_encode_first_pass_products(lg, ctx, log_m, n):
     K = int(name.split("_K")[1].split("_")[0])
     R = 1 << K
     table = R + 4 * (K - 1) * R // 2 - (R // 2 - 1)
-    assert K == 3 or table == 105  # of 4 stages
+    assert K != 4 or table == 105
     assert work[name][1] == (n << log_m) / R * (R + table)
     assert general[name] == n << log_m  # the scaling
 

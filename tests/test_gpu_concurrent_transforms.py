@@ -76,12 +76,12 @@ def test_encodings(lg, ctx, stages, n):
 
 
 def test_proofs_with_a_strided_pass_of_five(lg, ctx):
-    # 2^21: the first commitment's default split is 4 + 5 + 6
     cfg = lg.config_for_size(21)
     poly = lg.splitmix_coeffs_device(21, cfg.poly_len, ctx)
     want = lg.prover(cfg, poly, ctx).to_bytes()
 
     def work(c):
+        c.set_fft_split((4, 5, 6))  # the first commitment's columns
         for _ in range(2):
             assert lg.prover(cfg, poly, c).to_bytes() == want
 
