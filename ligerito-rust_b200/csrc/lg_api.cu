@@ -447,10 +447,10 @@ std::vector<uint32_t> host_copy_groups(uint32_t n, size_t col_bytes) {
 // Small polynomials travel whole instead: a group's calls cost the host more
 // than its share of the copy hides.  Measured proofs, in groups -> whole:
 // from pinned memory (50 GB/s) 2^16 270 -> 185 us, 2^18 286 -> 230, 2^20
-// 438 -> 335, 2^21 498 -> 486, and 2^22 in groups 700 (the copy alone is
-// 325 of it); from pageable memory (the staging copy runs at 13 GB/s) 2^16
+// 438 -> 335, but 2^21 of 64 columns 462 -> 478, of 16 and 128 701 -> 835 and
+// 436 -> 459; from pageable memory (the staging copy runs at 13 GB/s) 2^16
 // 286 -> 194 us, 2^18 328 -> 292, 2^19 in groups 400.
-constexpr size_t kWholePinned = 8u << 20, kWholePageable = 1u << 20;
+constexpr size_t kWholePinned = 4u << 20, kWholePageable = 1u << 20;
 Witness commit_from_host(lg_ctx *c, Scratch &sc, const uint32_t *h_poly, uint32_t *d_poly, uint32_t log_m,
                          uint32_t n) {
     const Code code = get_code(c, log_m);
