@@ -1446,10 +1446,12 @@ __global__ void __launch_bounds__(256) k_fold_split(const uint32_t *__restrict__
 
 // Few outputs: the split form, where one thread an output would leave most of
 // the device idle (2^10 outputs of 64 terms on 4 blocks: 5.8 us, split 3.6).
+// Sixteen terms leave a cluster's blocks two each, less than their exchange
+// costs (2^14 words by 4, a call: 17.8 us, split 19.1).
 // More than 6 variables at once only for very few outputs: 2^22 words by 9
 // take 22 us so, 13 us as 6 and then 3.
 bool fold_splits(uint32_t log_len, uint32_t k, uint32_t B) {
-    if (k < 4 || k > kMaxFold || log_len < k) return false;
+    if (k < 5 || k > kMaxFold || log_len < k) return false;
     const uint64_t chunks = (((1ull << (log_len - k)) + 255) / 256) * B;
     return chunks <= (k <= 6 ? 64 : 8);
 }
@@ -1490,7 +1492,7 @@ cudaError_t fold_eq(Launcher &L, const uint32_t *in, uint32_t *out, uint32_t log
     case kk:                                                                                               \
         LGK_LAUNCH(L, "fold_eq", launch_kc(k_fold_split<kh, kk - kh>, grid, 256, 8, 0, L.stream, in, out, M, c, d_rs, st)); \
         break;
-            LGK_CASE(4, 3) LGK_CASE(5, 3) LGK_CASE(6, 3) LGK_CASE(7, 3) LGK_CASE(8, 4) LGK_CASE(9, 4)
+            LGK_CASE(5, 3) LGK_CASE(6, 3) LGK_CASE(7, 3) LGK_CASE(8, 4) LGK_CASE(9, 4)
 #undef LGK_CASE
         }
         return cudaGetLastError();
