@@ -726,8 +726,9 @@ static cudaError_t launch_tail(Launcher &L, int K, PassArgs a, unsigned blocks) 
     // Fewer tiles wait for their own latency: plain 16-byte loads and stores
     // without the copies' hand-over, and 256 threads to fill the tables (2^6 x
     // 64: 11.5 -> 10.3 us, 2^6 x 3: 15.2 -> 9.8; 590 tiles of 64 18.5 -> 17.8).
-    const bool bulk = blocks >= 148 * 4;
-    const unsigned threads = bulk ? std::max<unsigned>(32, std::min<unsigned>(128, vp2 << (K - K / 2))) : 256;
+    // Tiles of fewer than 8 vectors are all table fill: no copies either.
+    const bool many = blocks >= 148 * 4, bulk = many && a.vchunk >= 8;
+    const unsigned threads = many ? std::max<unsigned>(32, std::min<unsigned>(128, vp2 << (K - K / 2))) : 256;
     switch (2 * K + bulk) {
 #define LGK_CASE(k, b)                                                                                         \
     case 2 * k + b:                                                                                            \
@@ -774,13 +775,13 @@ FftPlan default_fft_plan(uint32_t log_len, uint64_t words, uint32_t nvec, bool r
         kt = most = log_len;
     } else if (rs) {
         kt = words < (1u << 16) ? 6 : words <= kTwoTilesAnSm || nvec < 8 ? 5 : 6;
-        most = words <= kTwoTilesAnSm ? 3 : words < (1u << 24) ? 4 : 5;
+        most = words <= kTwoTilesAnSm ? 3 : words < (1u << 24) || nvec < 8 ? 4 : 5;
     } else if (words < (1u << 14)) {
         kt = std::max(4u, std::min(6u, log_len - 3));
         most = 4;
     } else {
         kt = words <= kTwoTilesAnSm || nvec < 8 ? 5 : 6;
-        most = words < (1u << 23) ? 4 : 5;
+        most = words < (1u << 23) || nvec < 8 ? 4 : 5;
     }
     kt = std::min(kt, log_len);
     while (kt + most * (kMaxFftPasses - 1) < log_len) ++most;

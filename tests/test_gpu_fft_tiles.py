@@ -14,10 +14,14 @@ def split(ctx):
     ctx.set_fft_split()
 
 
-# 591 and 592 tiles: the last without bulk copies and the first with them
-@pytest.mark.parametrize("stages,batch", [
-    ((k,), b) for k in (4, 5, 6) for b in (1, 2, 7, 63, 64, 65, 130, 591 * 64, 591 * 64 + 1, 592 * 64)
-] + [((5, 6), 64 * 18), ((5, 6), 64 * 18 + 1), ((5, 6), 64 * 19), ((4, 4), 64 * 37 + 3), ((3, 5), 5), ((4, 6), 1)])
+ALONE = [((k,), b) for k in (4, 5, 6) for b in (1, 2, 7, 63, 64, 65, 130, 591 * 64, 591 * 64 + 1, 592 * 64)]
+AFTER = [((5, 6), 64 * 18), ((5, 6), 64 * 18 + 1), ((5, 6), 64 * 19), ((4, 4), 64 * 37 + 3), ((3, 5), 5), ((4, 6), 1)]
+FEW = [((5, 5, 6), b) for b in (1, 7, 8, 9)]
+
+
+# 591 and 592 tiles: the last without bulk copies and the first with them; many
+# tiles of few vectors, with copies from 8 vectors on
+@pytest.mark.parametrize("stages,batch", ALONE + AFTER + FEW)
 def test_tiles(lg, ref, ctx, split, stages, batch):
     log_n = sum(stages)
     v = rng.integers(0, 2**32, size=batch << log_n, dtype=np.uint64).astype(np.uint32)
