@@ -129,11 +129,11 @@ lg_status lg_ctx_kernel_work(lg_ctx *ctx, uint32_t index, double *hbm_bytes, dou
  * factor's multiples (general products: integer multiplies, no lookups). */
 lg_status lg_ctx_kernel_general_mults(lg_ctx *ctx, uint32_t index, double *gf_mults);
 uint64_t lg_ctx_device_bytes_in_use(const lg_ctx *ctx);
-/* Device bytes a context keeps between calls (its arena, reserved on its
- * first proof, its FFT tables and fold workspace), and the bytes of the code / twiddle
- * tables that all contexts on a device share (ReedSolomonEncoding::new's
- * twiddles and pis per size, src/reed_solomon.rs:49-64), held while a
- * context on that device exists. */
+/* Device bytes a context keeps between calls (its arena, reserved by its
+ * first proof or verification, its FFT tables and fold workspace), and the
+ * bytes of the code / twiddle tables that all contexts on a device share
+ * (ReedSolomonEncoding::new's twiddles and pis per size,
+ * src/reed_solomon.rs:49-64), held while a context on that device exists. */
 uint64_t lg_ctx_device_bytes_cached(const lg_ctx *ctx);
 uint64_t lg_device_table_bytes(int device);
 
@@ -288,7 +288,8 @@ lg_status lg_ifft(lg_ctx *ctx, uint32_t *d_data, uint32_t log_n, uint64_t batch)
 /* ReedSolomonEncoding::new(2^log_m, 2^(log_m+2)).encode_non_systematic on
  * every column of poly2flatmat: src/reed_solomon.rs:104-113 with
  * src/ligero.rs:11-38.  d_poly: n columns of 2^log_m (column j at
- * j*2^log_m); d_encoded: n columns of 2^(log_m+2), column-major. */
+ * j*2^log_m); d_encoded: n columns of 2^(log_m+2), column-major.  d_poly may
+ * lie inside d_encoded: it is then moved to a buffer of its own first. */
 lg_status lg_rs_encode_cols(lg_ctx *ctx, const uint32_t *d_poly, uint32_t log_m, uint32_t n,
                             uint32_t *d_encoded);
 

@@ -11,8 +11,9 @@
 // message is kept as big-endian words.
 //
 // Squeeze i of a batch finalises the state after i+1 more counters, so one
-// thread compresses the full blocks that the absorbed words and the counters
-// complete (the only serial part), then every thread finalises its own clone.
+// warp compresses the full blocks that the absorbed words and the counters
+// complete (the only serial part; their schedules come from other warps), then
+// every thread finalises its own clone.
 #include <cstdint>
 
 #include "lg_device.cuh"
