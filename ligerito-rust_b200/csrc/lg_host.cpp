@@ -8,6 +8,9 @@
 #if defined(__x86_64__)
 #include <immintrin.h>
 #endif
+#if defined(__linux__)
+#include <sys/mman.h>
+#endif
 
 namespace lg {
 
@@ -676,7 +679,23 @@ std::vector<uint32_t> lagrange_basis(const uint32_t *rs, size_t k) {
     return cur;
 }
 
+// Pages of [p, p + bytes) that are about to be written anyway, asked for in one
+// system call: new memory otherwise costs a fault every 4 KiB (1.3 us; 512 KiB
+// of a 2^17 polynomial 200 us, 30 so), which also waits for whatever holds the
+// process's memory map, such as another thread's pinned allocation.
+void prefault(void *p, size_t bytes) {
+#ifdef MADV_POPULATE_WRITE
+    constexpr uintptr_t kPage = 4096;
+    const uintptr_t a = ((uintptr_t)p + kPage - 1) & ~(kPage - 1), e = ((uintptr_t)p + bytes) & ~(kPage - 1);
+    if (e > a + 16 * kPage) madvise(reinterpret_cast<void *>(a), e - a, MADV_POPULATE_WRITE);
+#else
+    (void)p;
+    (void)bytes;
+#endif
+}
+
 void splitmix_fill(uint64_t seed, uint32_t *out, uint64_t n, uint64_t first) {
+    prefault(out, 4 * n);
     for (uint64_t i = 0; i < n; ++i) {
         uint64_t z = seed + (first + i + 1) * 0x9E3779B97F4A7C15ull;
         z = (z ^ (z >> 30)) * 0xBF58476D1CE4E5B9ull;

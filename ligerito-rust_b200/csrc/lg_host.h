@@ -143,6 +143,7 @@ std::vector<uint32_t> lagrange_basis(const uint32_t *rs, size_t k);
 // next_s (src/binary_fft.rs:100-107)
 inline uint32_t next_s(uint32_t s, uint32_t c) { return gf_mul(s, s) ^ gf_mul(c, s); }
 
+void prefault(void *p, size_t bytes);
 void splitmix_fill(uint64_t seed, uint32_t *out, uint64_t n, uint64_t first_index = 0);
 
 }  // namespace lg

@@ -209,6 +209,9 @@ lg_status lg_server_submit(lg_server *s, const lg_config *cfg, const uint32_t *p
     r->len = len;
     r->on_device = poly_on_device;
     if (copy_input && !poly_on_device) {
+        // (without it a submission's copy took longer than the proof of the one before)
+        r->owned.reserve(len);
+        lg::prefault(r->owned.data(), 4 * len);
         r->owned.assign(poly, poly + len);
         r->poly = r->owned.data();
     } else {
